@@ -25,6 +25,7 @@ COMMON = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-ffp-con
                  "-I" + os.path.join(ROOT, "include"), "-I" + CSRC]
 UNITS = {
     "jgb_fp64.cu": ["-fmad=false"],
+    "jgb_path64.cu": ["-fmad=false"],
     "jgb_mixed.cu": ["-prec-div=false", "-ftz=true"],
     "jgb_api.cu": [],
     "jgb_noalloc.cu": [],

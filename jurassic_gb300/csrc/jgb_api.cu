@@ -20,6 +20,7 @@
 #include "jgb_common.cuh"
 #include "jgb_internal.h"
 #include "jgb_ctx.h"
+#include "jgb_path64.cuh"
 
 extern "C" const double jgb_continua_blob[];
 extern "C" const long jgb_continua_count;
@@ -72,6 +73,7 @@ void ctm_coefficients(double nu, double* out) {
       out[5] = sfac * c296;
       out[6] = c260 / c296;
       out[7] = cfrn * fscal;
+      out[14] = c260 > 0 && c296 > 0 ? std::log(out[6]) : std::nan("");
     }
   }
   auto cia = [&](int ob, int obeta, int onu, int n, double* o) {
@@ -129,6 +131,7 @@ TblDev tbl_view(const jgb_ctx* x) {
   T.ue = x->t_ue.as<float2>();
   T.sr = x->s_sr.as<double>();
   T.srf = x->s_srf.as<float>();
+  T.srd = x->s_srd.as<double2>();
   T.st = x->s_st.as<double>();
   return T;
 }
@@ -334,6 +337,179 @@ __global__ void k_mask_keys(int nray, int nd, const unsigned char* mask, const i
   int m = 0;
   for (int id = 0; id < nd; id++) m += mask[(long long)id * nray + r] ? 0 : 1;
   key[r] = (m << 13) | min(count[r], 8191);
+}
+
+// Records derived from the uploaded tables, made at the first forward model
+// after an upload: row records and interleaved rows of both paths, and the
+// emitters whose p and T grids are identical for all channels, so that their
+// brackets are found once per LOS point (mixed: float grids; FP64: the grids
+// of the channels that have a table).
+int prepare_tables(jgb_ctx* x, cudaStream_t s) {
+  if (!x->meta_stale) return JGB_OK;
+  const CtlDev& c = x->c;
+  const size_t tp = x->tp, tt = x->tt;
+  auto same_grid = [&](size_t a, size_t b, auto& p, auto& t) {
+    return x->h_np[b] == x->h_np[a] &&
+           std::equal(x->h_nt.begin() + a * tp, x->h_nt.begin() + (a + 1) * tp,
+                      x->h_nt.begin() + b * tp) &&
+           std::equal(p.begin() + a * tp, p.begin() + (a + 1) * tp, p.begin() + b * tp) &&
+           std::equal(t.begin() + a * tp * tt, t.begin() + (a + 1) * tp * tt, t.begin() + b * tp * tt);
+  };
+  x->grid_mask = x->grid_mask64 = 0;
+  if (tp * tt < 32768)  // rows of a p-T cell packed in 16 bits
+    for (int g = 0; g < c.ng; g++) {
+      bool same = x->h_np[g] >= 30;
+      for (int id = 1; id < c.nd && same; id++)
+        same = same_grid(g, (size_t)id * c.ng + g, x->h_pf, x->h_tf);
+      if (same) x->grid_mask |= 1u << g;
+      int ref = 0;
+      while (ref < c.nd && x->h_np[(size_t)ref * c.ng + g] < 30) ref++;
+      if (ref == c.nd) ref = 0;  // no channel has a table: nothing reads the grid
+      same = true;
+      for (int id = ref + 1; id < c.nd && same; id++)
+        same = x->h_np[(size_t)id * c.ng + g] < 30 ||
+               same_grid((size_t)ref * c.ng + g, (size_t)id * c.ng + g, x->h_p, x->h_t);
+      if (same) x->grid_mask64 |= 1u << g;
+      x->grid_ref[g] = ref;
+    }
+  const long long nrow = (long long)c.nd * c.ng * x->tp * x->tt;
+  launch_rowmeta(nrow, x->tu, x->t_nu.as<int>(), x->t_u.as<float>(), x->t_eps.as<float>(),
+                 x->t_tf.as<float>(), c.formod == 0, x->t_meta.as<float4>(), x->t_ue.as<float2>(), s);
+  const int one = 1;
+  CK(cudaMemcpyAsync(x->t_mono.p, &one, sizeof(int), cudaMemcpyHostToDevice, s));
+  launch_rows_mono(nrow, x->tu, x->t_nu.as<int>(), x->t_u.as<float>(), x->t_eps.as<float>(),
+                   x->t_mono.as<int>(), s);
+  CK(cudaGetLastError());
+  x->meta_stale = false;
+  return JGB_OK;
+}
+
+// The tiles of 32 rays of a batch: rays by descending key, three groups that
+// never share a tile (k_tiles), then the tiles' point offsets; P.perm, P.toff
+// (device) and the offsets on the host.
+int plan_tiles(jgb_ctx* x, int nray, const int* keys, const int* count, int ntile, int nfirst,
+               int tfirst, int nsecond, int tsecond, MixedPlan& P, std::vector<long long>& toff_h,
+               cudaStream_t s) {
+  CK(x->tiles_keys2.reserve(sizeof(int) * (size_t)nray));
+  CK(x->tiles_vals.reserve(sizeof(int) * 2 * (size_t)nray));
+  CK(x->tiles_perm.reserve(sizeof(int) * 32 * (size_t)ntile));
+  CK(x->tiles_len.reserve(sizeof(int) * (size_t)ntile));
+  CK(x->tiles_off.reserve(sizeof(long long) * (size_t)(2 * ntile + 2)));
+  int* vals_in = x->tiles_vals.as<int>();
+  int* vals_out = vals_in + nray;
+  k_iota<<<(nray + 255) / 256, 256, 0, s>>>(nray, vals_in);
+  size_t sb = 0, sb2 = 0;
+  long long* toff = x->tiles_off.as<long long>();
+  long long* tpts = toff + ntile + 1;
+  const bool sorted = nray > 32 || tfirst < ntile;  // one tile's rays keep any order
+  if (sorted) {
+    cub::DeviceRadixSort::SortPairsDescending(nullptr, sb, keys, x->tiles_keys2.as<int>(), vals_in,
+                                              vals_out, nray, 0, 32, s);
+    CK(x->scan_tmp.reserve(sb + 16));
+    cub::DeviceRadixSort::SortPairsDescending(x->scan_tmp.p, sb, keys, x->tiles_keys2.as<int>(),
+                                              vals_in, vals_out, nray, 0, 32, s);
+  }
+  P.ntile = ntile;
+  P.perm = x->tiles_perm.as<int>();
+  P.tlen = x->tiles_len.as<int>();
+  P.toff = toff;
+  P.tile0 = 0;
+  P.tile1 = ntile;
+  k_tiles<<<(ntile + 127) / 128, 128, 0, s>>>(nray, ntile, nfirst, tfirst, nsecond, tsecond, count,
+                                               sorted ? vals_out : vals_in, P.perm, P.tlen, tpts);
+  CK(cudaMemsetAsync(toff, 0, sizeof(long long), s));
+  cub::DeviceScan::InclusiveSum(nullptr, sb2, tpts, toff + 1, ntile, s);
+  CK(x->scan_tmp.reserve(std::max(sb, sb2) + 16));
+  cub::DeviceScan::InclusiveSum(x->scan_tmp.p, sb2, tpts, toff + 1, ntile, s);
+  toff_h.resize(ntile + 1);
+  CK(cudaMemcpyAsync(toff_h.data(), toff, sizeof(long long) * (ntile + 1), cudaMemcpyDeviceToHost, s));
+  CK(cudaStreamSynchronize(s));
+  return JGB_OK;
+}
+
+// FP64 path of a traced batch: chunks of tiles whose workspaces stay within
+// kPath64Bytes (per-point fields within a quarter of it), and of channels
+// where one tile alone would exceed it.
+constexpr size_t kPath64Bytes = size_t(4) << 30;
+
+int run_path64(jgb_ctx* x, const BatchDev& b, const LosDev& L, cudaStream_t s, int* launches) {
+  const CtlDev& c = x->c;
+  const int nray = b.nray, ntile = (nray + 31) / 32;
+  int rc = prepare_tables(x, s);
+  if (rc) return rc;
+  if (x->srd_stale) {
+    launch_src_channel_major(c.nd, x->s_st.as<double>(), x->s_sr.as<double>(), x->s_srd.as<double2>(), s);
+    x->srd_stale = false;
+  }
+  const int* keys = L.count;
+  if (b.skip_masked && nray > 32) {
+    CK(x->tiles_keys.reserve(sizeof(int) * (size_t)nray));
+    k_mask_keys<<<(nray + 255) / 256, 256, 0, s>>>(nray, c.nd, b.mask, L.count, x->tiles_keys.as<int>());
+    keys = x->tiles_keys.as<int>();
+  }
+  MixedPlan Pm{};
+  std::vector<long long> toff;
+  rc = plan_tiles(x, nray, keys, L.count, ntile, nray, ntile, nray, ntile, Pm, toff, s);
+  if (rc) return rc;
+  size_t bfd, bfu;
+  path64_point_bytes(c, &bfd, &bfu);
+  const size_t bch = 32 * sizeof(double) * (size_t)(c.ng + 2);  // per (point, channel)
+  struct Chunk {
+    int t0, t1, ndc, longest;
+  };
+  std::vector<Chunk> chunks;
+  size_t need_f = 0, need_w = 0;
+  for (int t = 0; t < ntile;) {
+    Chunk k{t, t, c.nd, 0};
+    auto pts = [&](int t1) { return (size_t)(toff[t1] - toff[k.t0]); };
+    do {
+      k.longest = std::max(k.longest, (int)(toff[k.t1 + 1] - toff[k.t1]));
+      k.t1++;
+    } while (k.t1 < ntile && k.t1 - k.t0 < 65535 && pts(k.t1 + 1) * (bfd + bfu) <= kPath64Bytes / 4 &&
+             pts(k.t1 + 1) * c.nd * bch <= kPath64Bytes);
+    const size_t np = std::max<size_t>(pts(k.t1), 1);
+    if (np * c.nd * bch > kPath64Bytes) k.ndc = (int)std::max<size_t>(kPath64Bytes / (np * bch), 1);
+    need_f = std::max(need_f, np * (bfd + bfu));
+    need_w = std::max(need_w, np * k.ndc * bch +
+                                  sizeof(int) * 32 * (size_t)(k.t1 - k.t0) * k.ndc * std::max(c.ng, 1));
+    chunks.push_back(k);
+    t = k.t1;
+  }
+  CK(x->tiles_data.reserve(need_f));
+  CK(x->seg.reserve(need_w));
+  CK(cudaEventRecord(x->ev[4], s));
+  Path64 P{};
+  P.perm = Pm.perm;
+  P.toff = Pm.toff;
+  P.shared = x->grid_mask64;
+  std::copy(x->grid_ref, x->grid_ref + kMaxG, P.gref);
+  P.mono = x->t_mono.as<int>();
+  const TblDev T = tbl_view(x);
+  const ChanDev ch = chan_view(x);
+  for (const Chunk& k : chunks) {
+    const size_t np = std::max<size_t>((size_t)(toff[k.t1] - toff[k.t0]), 1);
+    P.tile0 = k.t0;
+    P.tile1 = k.t1;
+    P.pt0 = toff[k.t0];
+    P.fd = x->tiles_data.as<double>();
+    P.fu = reinterpret_cast<unsigned*>(x->tiles_data.as<char>() + np * bfd);
+    if (k.longest > 0) launch_prep64(c, T, L, P, k.longest, s);
+    for (int id = 0; id < c.nd; id += k.ndc) {
+      P.id0 = id;
+      P.id1 = std::min(c.nd, id + k.ndc);
+      const size_t ndc = P.id1 - P.id0;
+      P.om = x->seg.as<double>();
+      P.se = P.om + np * ndc * c.ng * 32;
+      P.stop = reinterpret_cast<int*>(P.se + np * ndc * 2 * 32);
+      // four lanes per ray while the warps of one per ray leave schedulers idle
+      const long long warps = (long long)(k.t1 - k.t0) * ndc * c.ng;
+      launch_path64(c, T, ch, b, L, P, std::max(k.longest, 1), warps <= 2LL * x->sms ? 4 : 1, s);
+      CK(cudaGetLastError());
+      *launches += 3;
+    }
+    *launches += 1;
+  }
+  return JGB_OK;
 }
 
 float elapsed(cudaEvent_t a, cudaEvent_t b) {
@@ -566,43 +742,16 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
   TblDev T = tbl_view(x);
   int launches = 4 + (c.hydz >= 0) + trace_launches;
   if (precision == JGB_FP64) {
-    double* refl = nullptr;
-    if (need_refl) {
-      CK(x->refl.reserve(sizeof(double) * 2 * (size_t)cap * c.nd));
-      refl = x->refl.as<double>();
-    }
-    CK(cudaEventRecord(x->ev[4], s));
-    launch_path_fp64(c, T, ch, bo, L, refl, s);
-    launches += 1;
+    const int rc = run_path64(x, bo, L, s, &launches);
+    if (rc) return rc;
   } else {
     if (x->srf_stale) {
       launch_src_to_float(c.nd, x->s_sr.as<double>(), x->s_srf.as<float>(), s);
       x->srf_stale = false;
     }
-    if (x->meta_stale) {
-      // emitters whose (float) p and T grids are identical for all channels:
-      // their brackets are found once per LOS point in the tile packing
-      x->grid_mask = 0;
-      if ((long long)x->tp * x->tt < 32768)  // rows of a p-T cell packed in 16 bits
-        for (int g = 0; g < c.ng; g++) {
-          bool same = x->h_np[g] >= 30;
-          for (int id = 1; id < c.nd && same; id++) {
-            const size_t a = (size_t)g, b = (size_t)id * c.ng + g;
-            same = x->h_np[b] == x->h_np[a] &&
-                   std::equal(x->h_nt.begin() + a * x->tp, x->h_nt.begin() + (a + 1) * x->tp,
-                              x->h_nt.begin() + b * x->tp) &&
-                   std::equal(x->h_pf.begin() + a * x->tp, x->h_pf.begin() + (a + 1) * x->tp,
-                              x->h_pf.begin() + b * x->tp) &&
-                   std::equal(x->h_tf.begin() + a * x->tp * x->tt,
-                              x->h_tf.begin() + (a + 1) * x->tp * x->tt,
-                              x->h_tf.begin() + b * x->tp * x->tt);
-          }
-          if (same) x->grid_mask |= 1u << g;
-        }
-      launch_rowmeta((long long)c.nd * c.ng * x->tp * x->tt, x->tu, x->t_nu.as<int>(),
-                     x->t_u.as<float>(), x->t_eps.as<float>(), x->t_tf.as<float>(),
-                     c.formod == 0, x->t_meta.as<float4>(), x->t_ue.as<float2>(), s);
-      x->meta_stale = false;
+    {
+      const int rc = prepare_tables(x, s);
+      if (rc) return rc;
     }
     // resumed perturbations: start points and the base rays' snapshot lists
     const ResumeSpec* rs = x->resume;
@@ -791,14 +940,6 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
       nplain_end = nray;
     }
     CK(x->tiles_keys.reserve(sizeof(int) * (size_t)nray));
-    CK(x->tiles_keys2.reserve(sizeof(int) * (size_t)nray));
-    CK(x->tiles_vals.reserve(sizeof(int) * 2 * (size_t)nray));
-    CK(x->tiles_perm.reserve(sizeof(int) * 32 * (size_t)ntile));
-    CK(x->tiles_len.reserve(sizeof(int) * (size_t)ntile));
-    CK(x->tiles_off.reserve(sizeof(long long) * (size_t)(2 * ntile + 2)));
-    int* vals_in = x->tiles_vals.as<int>();
-    int* vals_out = vals_in + nray;
-    k_iota<<<(nray + 255) / 256, 256, 0, s>>>(nray, vals_in);
     const int* keys = L.count;
     if (rs) {
       k_resume_keys<<<(nray + 255) / 256, 256, 0, s>>>(nray, nbase_rays, c.nd, b.mask, b.skip_masked,
@@ -811,33 +952,14 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
                                                       x->tiles_keys.as<int>());
       keys = x->tiles_keys.as<int>();
     }
-    size_t sbytes = 0;
-    cub::DeviceRadixSort::SortPairsDescending(nullptr, sbytes, keys, x->tiles_keys2.as<int>(),
-                                              vals_in, vals_out, nray, 0, 32, s);
-    CK(x->scan_tmp.reserve(std::max(sbytes, tmp_bytes) + 16));
-    cub::DeviceRadixSort::SortPairsDescending(x->scan_tmp.p, sbytes, keys,
-                                              x->tiles_keys2.as<int>(), vals_in, vals_out, nray,
-                                              0, 32, s);
-    long long* tpts = x->tiles_off.as<long long>() + ntile + 1;
-    long long* toff = x->tiles_off.as<long long>();
     MixedPlan Pm{};
-    Pm.ntile = ntile;
-    Pm.perm = x->tiles_perm.as<int>();
-    Pm.tlen = x->tiles_len.as<int>();
-    Pm.toff = toff;
-    Pm.tile0 = 0;
-    Pm.tile1 = ntile;
-    k_tiles<<<(ntile + 127) / 128, 128, 0, s>>>(nray, ntile, rs ? nbase_rays : nray, tfirst,
-                                                 nplain_end, tsecond, L.count, vals_out, Pm.perm,
-                                                 Pm.tlen, tpts);
-    CK(cudaMemsetAsync(toff, 0, sizeof(long long), s));
-    size_t sb2 = 0;
-    cub::DeviceScan::InclusiveSum(nullptr, sb2, tpts, toff + 1, ntile, s);
-    CK(x->scan_tmp.reserve(std::max(std::max(sbytes, tmp_bytes), sb2) + 16));
-    cub::DeviceScan::InclusiveSum(x->scan_tmp.p, sb2, tpts, toff + 1, ntile, s);
-    long long tile_points = 0;
-    CK(cudaMemcpyAsync(&tile_points, toff + ntile, sizeof(long long), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
+    std::vector<long long> toff_h;
+    {
+      const int rc = plan_tiles(x, nray, keys, L.count, ntile, rs ? nbase_rays : nray, tfirst,
+                                nplain_end, tsecond, Pm, toff_h, s);
+      if (rc) return rc;
+    }
+    const long long tile_points = toff_h[ntile];
     Pm.brmask = x->grid_mask;
     Pm.nfield = mixed_nfield(c, Pm.brmask);
     CK(x->tiles_data.reserve(sizeof(float) * 32 * (size_t)std::max(tile_points, 1LL) * Pm.nfield));
@@ -1449,7 +1571,9 @@ int jgb_create(const jgb_ctl* ctl, int device, jgb_ctx** out) {
             x->d_ctm.reserve(sizeof(double) * ctm.size()) == cudaSuccess &&
             x->s_st.reserve(sizeof(double) * kNS) == cudaSuccess &&
             x->s_sr.reserve(sizeof(double) * kNS * c.nd) == cudaSuccess &&
-            x->s_srf.reserve(sizeof(float) * kNS * c.nd) == cudaSuccess;
+            x->s_srf.reserve(sizeof(float) * kNS * c.nd) == cudaSuccess &&
+            x->s_srd.reserve(sizeof(double2) * kNS * c.nd) == cudaSuccess &&
+            x->t_mono.reserve(sizeof(int)) == cudaSuccess;
   ok = ok && cudaMemcpy(x->d_nu.p, x->nu.data(), sizeof(double) * c.nd, cudaMemcpyHostToDevice) == cudaSuccess;
   ok = ok && cudaMemcpy(x->d_window.p, x->window.data(), sizeof(int) * c.nd, cudaMemcpyHostToDevice) == cudaSuccess;
   if (c.ncl) ok = ok && cudaMemcpy(x->d_clnu.p, x->clnu.data(), sizeof(double) * c.ncl, cudaMemcpyHostToDevice) == cudaSuccess;
@@ -1477,7 +1601,7 @@ void jgb_destroy(jgb_ctx* x) {
   }
   DevBuf* bufs[] = {&x->d_nu, &x->d_window, &x->d_clnu, &x->d_sfnu, &x->d_ctm, &x->t_np,
                     &x->t_p, &x->t_nt, &x->t_t, &x->t_nu, &x->t_u, &x->t_eps, &x->t_pf,
-                    &x->t_tf, &x->t_meta, &x->t_ue, &x->s_st, &x->s_sr, &x->s_srf, &x->b_levoff, &x->b_rayoff,
+                    &x->t_tf, &x->t_meta, &x->t_ue, &x->t_mono, &x->s_st, &x->s_sr, &x->s_srf, &x->s_srd, &x->b_levoff, &x->b_rayoff,
                     &x->b_rayobs, &x->b_lev, &x->b_scal, &x->b_geo, &x->b_rad, &x->b_tau,
                     &x->b_tp, &x->b_mask, &x->b_p, &x->los_off, &x->los_cnt, &x->los_cnt64,
                     &x->los_sft, &x->los_ends, &x->los_planes, &x->scan_tmp, &x->err_word,
@@ -1517,6 +1641,8 @@ int jgb_tables_init(jgb_ctx* x, int tp, int tt, int tu) {
   x->h_nt.assign(ndg * tp, 0);
   x->h_pf.assign(ndg * tp, 0.f);
   x->h_tf.assign(ndg * tp * tt, 0.f);
+  x->h_p.assign(ndg * tp, 0.0);
+  x->h_t.assign(ndg * tp * tt, 0.0);
   CK(x->t_np.reserve(sizeof(int) * std::max<size_t>(ndg, 1)));
   CK(x->t_p.reserve(sizeof(double) * std::max<size_t>(ndg * tp, 1)));
   CK(x->t_nt.reserve(sizeof(int) * std::max<size_t>(ndg * tp, 1)));
@@ -1573,6 +1699,8 @@ int jgb_set_table(jgb_ctx* x, int id, int ig, int np, const double* p, const int
   std::copy(ntv.begin(), ntv.end(), x->h_nt.begin() + dg * x->tp);
   std::copy(pf.begin(), pf.end(), x->h_pf.begin() + dg * x->tp);
   std::copy(tf.begin(), tf.end(), x->h_tf.begin() + dg * x->tp * x->tt);
+  std::copy(pv.begin(), pv.end(), x->h_p.begin() + dg * x->tp);
+  std::copy(tv.begin(), tv.end(), x->h_t.begin() + dg * x->tp * x->tt);
   CK(cudaMemcpy(x->t_p.as<double>() + dg * x->tp, pv.data(), sizeof(double) * x->tp, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(x->t_pf.as<float>() + dg * x->tp, pf.data(), sizeof(float) * x->tp, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(x->t_nt.as<int>() + dg * x->tp, ntv.data(), sizeof(int) * x->tp, cudaMemcpyHostToDevice));
@@ -1652,7 +1780,7 @@ int jgb_set_filter(jgb_ctx* x, int id, int n, const double* fnu, const double* f
   CK(cudaStreamSynchronize(x->stream));
   tmp.release();
   x->src_set[id] = 1;
-  x->srf_stale = true;
+  x->srf_stale = x->srd_stale = true;
   return JGB_OK;
 }
 
@@ -1662,7 +1790,7 @@ int jgb_set_srcfunc(jgb_ctx* x, const double* sr) {
   cudaSetDevice(x->device);
   CK(cudaMemcpy(x->s_sr.p, sr, sizeof(double) * kNS * x->c.nd, cudaMemcpyHostToDevice));
   std::fill(x->src_set.begin(), x->src_set.end(), 1);
-  x->srf_stale = true;
+  x->srf_stale = x->srd_stale = true;
   return JGB_OK;
 }
 

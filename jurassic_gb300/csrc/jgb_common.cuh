@@ -111,6 +111,22 @@ __host__ __device__ inline double planck(double t, double nu) {
   return kC1 * (nu * nu * nu) / expm1(kC2 * nu / t);
 }
 
+// Solar zenith angle (sza, jurassic.c:5183-5219)
+__device__ inline double solar_zenith(double sec, double lon, double lat) {
+  const double d = sec / 86400 - 0.5;
+  const double g = (357.529 + 0.98560028 * d) * (kPI / 180.0);
+  const double q = 280.459 + 0.98564736 * d;
+  const double l = (q + 1.915 * sin(g) + 0.020 * sin(2 * g)) * (kPI / 180.0);
+  const double e = (23.439 - 0.00000036 * d) * (kPI / 180.0);
+  const double dec = asin(sin(e) * sin(l));
+  const double ra = atan2(cos(e) * sin(l), cos(l));
+  const double gmst = 18.697374558 + 24.06570982441908 * d;
+  const double lst = gmst + lon / 15;
+  const double h = lst / 12 * kPI - ra;
+  const double latr = lat * (kPI / 180.0);
+  return acos(sin(latr) * sin(dec) + cos(latr) * cos(dec) * cos(h)) * (180.0 / kPI);
+}
+
 // ---------------------------------------------------------------------------
 // Device-resident views (plain pointers into context-owned buffers)
 
@@ -141,6 +157,7 @@ struct TblDev {
   const float4* rowmeta;  // row records of the mixed path (EGA: 2 float4 per row, CGA: 1)
   const float2* ue;    // rows interleaved {u[i], eps[i]} (mixed path)
   const double* sr;    // source function [kNS][nd]
+  const double2* srd;  // source function, channel-major: value and slope [nd][kNS]
   const float* srf;    // source function, channel-major float [nd][kNS]
   const double* st;    // source-function temperatures [kNS]
 };

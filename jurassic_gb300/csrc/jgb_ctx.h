@@ -75,15 +75,20 @@ struct jgb_ctx {
   std::vector<int> h_nt;
   std::vector<float> h_pf, h_tf;
   unsigned grid_mask = 0;
+  // the same for the FP64 path: FP64 grids, the emitters whose grids are the
+  // same for every channel with a table, and one such channel of each
+  std::vector<double> h_p, h_t;
+  unsigned grid_mask64 = 0;
+  int grid_ref[jgb::kMaxG] = {};
   // field of view: nfov samples (dz, w) on the device, pencil-beam scratch
   int nfov = 0;
   jgb::DevBuf d_fov, fov_raw;
-  jgb::DevBuf t_np, t_p, t_nt, t_t, t_nu, t_u, t_eps, t_pf, t_tf, t_meta, t_ue;
+  jgb::DevBuf t_np, t_p, t_nt, t_t, t_nu, t_u, t_eps, t_pf, t_tf, t_meta, t_ue, t_mono;
   bool meta_stale = true;
   // source function
-  jgb::DevBuf s_st, s_sr, s_srf;
+  jgb::DevBuf s_st, s_sr, s_srf, s_srd;
   std::vector<char> src_set;
-  bool srf_stale = true;
+  bool srf_stale = true, srd_stale = true;
   // per-call scratch
   jgb::DevBuf b_levoff, b_rayoff, b_rayobs, b_lev, b_scal, b_geo, b_rad, b_tau, b_tp, b_mask, b_p;
   jgb::DevBuf los_off, los_cnt, los_cnt64, los_sft, los_ends, los_planes, scan_tmp, err_word;

@@ -446,22 +446,6 @@ __device__ inline double continuum_beta(const CtlDev& c, const double* cc, doubl
   return beta;
 }
 
-// Solar zenith angle (sza, jurassic.c:5183-5219)
-__device__ inline double solar_zenith(double sec, double lon, double lat) {
-  const double d = sec / 86400 - 0.5;
-  const double g = (357.529 + 0.98560028 * d) * (kPI / 180.0);
-  const double q = 280.459 + 0.98564736 * d;
-  const double l = (q + 1.915 * sin(g) + 0.020 * sin(2 * g)) * (kPI / 180.0);
-  const double e = (23.439 - 0.00000036 * d) * (kPI / 180.0);
-  const double dec = asin(sin(e) * sin(l));
-  const double ra = atan2(cos(e) * sin(l), cos(l));
-  const double gmst = 18.697374558 + 24.06570982441908 * d;
-  const double lst = gmst + lon / 15;
-  const double h = lst / 12 * kPI - ra;
-  const double latr = lat * (kPI / 180.0);
-  return acos(sin(latr) * sin(dec) + cos(latr) * cos(dec) * cos(h)) * (180.0 / kPI);
-}
-
 // Per-(observation, channel) constants derived from the atmosphere record.
 __device__ inline void obs_channel_consts(const CtlDev& c, const ChanDev& ch, const double* s,
                                           int id, double* cloud, bool* has_cloud,

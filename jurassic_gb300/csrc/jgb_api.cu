@@ -535,10 +535,10 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
   if (c.hydz >= 0) launch_hydrostatic(c, b, const_cast<double*>(b.p), s);
   CK(cudaEventRecord(x->ev[2], s));
 
-  // ray tracing.  Mixed precision traces in one pass: a small batch into
-  // fixed slabs of NLOS points per ray, a large one into capacities from a
-  // geometric bound of every ray's LOS points; if a ray outgrows its bound,
-  // or in FP64, the rays are counted first (count, scan, fill).
+  // ray tracing, in one pass: a small mixed-precision batch into fixed slabs
+  // of NLOS points per ray, others into capacities from a geometric bound of
+  // every ray's LOS points; if a ray outgrows its bound, or the capacities do
+  // not fit the device, the rays are counted first (count, scan, fill).
   const long long slab = c.nlos_max;
   // resumed perturbations (EGA; the Curtis-Godson sums run from the first
   // point) can be traced from their base rays' walks (TraceResume).  The
@@ -554,9 +554,14 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
   }
   int trace_launches = 0;  // kernels of the resumed tracing beyond one fill
   enum { kSlab, kBound, kCount } mode =
-      precision != JGB_MIXED ? kCount
-      : (long long)nray * slab <= kSinglePassPoints ? kSlab
+      precision == JGB_MIXED && (long long)nray * slab <= kSinglePassPoints ? kSlab
       : x->los_bound_scale > 0 ? kBound : kCount;
+  const double* slopes = nullptr;  // FP64: slopes of the level intervals
+  if (precision == JGB_FP64) {
+    CK(x->lev_slopes.reserve(level_slope_bytes(c, b.nlev)));
+    launch_level_slopes(c, b, x->lev_slopes.as<double>(), s);
+    slopes = x->lev_slopes.as<double>();
+  }
   CK(x->los_cnt.reserve(sizeof(int) * (size_t)std::max(nray, 1)));
   CK(x->los_cnt64.reserve(sizeof(long long) * (size_t)(nray + 1)));
   CK(x->los_off.reserve(sizeof(long long) * (size_t)(nray + 1)));
@@ -587,7 +592,7 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
       else if (precision == JGB_MIXED)
         launch_trace_count_mixed(c, b, L, d_err, s);
       else
-        launch_trace_count(c, ch, b, L, d_err, s);
+        launch_trace_count(c, b, L, slopes, d_err, s);
       CK(cudaGetLastError());
       passes += mode == kCount;
       k_widen<<<(nray + 255) / 256, 256, 0, s>>>(nray, L.count, cnt64);
@@ -602,11 +607,16 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
       if (h_err & kErrLosOverflow) return fail(x, JGB_ERR_LOS, "Too many LOS points!");
     }
     cap = std::max(total, 1LL);
-    const int nplanes = 8 + c.ng + c.nw + (c.formod == 0 ? 3 * c.ng : 0);
-    const int nfplanes = 5 + c.ng + c.nw + (c.formod == 0 ? 3 * c.ng : 0);
-    CK(x->los_planes.reserve(precision == JGB_MIXED
-                                 ? (sizeof(double) + sizeof(float) * nfplanes) * (size_t)cap
-                                 : sizeof(double) * (size_t)cap * nplanes));
+    const int nplanes = 5 + c.ng + c.nw + (c.formod == 0 ? 3 * c.ng : 0);
+    const size_t plane_bytes = precision == JGB_MIXED
+                                   ? (sizeof(double) + sizeof(float) * nplanes) * (size_t)cap
+                                   : sizeof(double) * (size_t)cap * nplanes;
+    if (mode == kBound && x->los_planes.reserve(plane_bytes) == cudaErrorMemoryAllocation) {
+      (void)cudaGetLastError();  // the exact counts may still fit
+      mode = kCount;
+      continue;
+    }
+    CK(x->los_planes.reserve(plane_bytes));
     double* P = x->los_planes.as<double>();
     if (precision == JGB_MIXED) {  // z in FP64, the point data in FP32 planes
       float* F = reinterpret_cast<float*>(P + cap);
@@ -622,16 +632,15 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
       L.f.cgu = L.f.cgt + (long long)c.ng * cap;
     }
     L.cap = cap;
-    L.z = P + 0 * cap;
-    if (precision != JGB_MIXED) {
-      L.lon = P + 1 * cap;
-      L.lat = P + 2 * cap;
-      L.p = P + 3 * cap;
-      L.t = P + 4 * cap;
-      L.ds = P + 5 * cap;
-      L.aux = P + 6 * cap;
-      L.qh2o = P + 7 * cap;
-      L.u = P + 8 * cap;
+    if (precision == JGB_MIXED) {
+      L.z = P;
+    } else {
+      L.p = P + 0 * cap;
+      L.t = P + 1 * cap;
+      L.ds = P + 2 * cap;
+      L.aux = P + 3 * cap;
+      L.qh2o = P + 4 * cap;
+      L.u = P + 5 * cap;
       L.kw = L.u + (long long)c.ng * cap;
       L.cgp = L.kw + (long long)c.nw * cap;
       L.cgt = L.cgp + (long long)c.ng * cap;
@@ -683,7 +692,7 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
         launch_trace_fill_resumed(c, b, L, vout, 0, npr, R, 2, d_err, s);
         trace_launches += 6;  // plan, iota, the sort's three passes, the fill
       }
-    } else if (precision == JGB_MIXED) {
+    } else {
       // rays ordered by capacity (longest first) when the capacities are
       // bounds of the real lengths: a warp's rays then walk similar lengths
       const int* order = nullptr;
@@ -704,9 +713,11 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
                                                   bits, s);
         order = vout;
       }
-      launch_trace_fill_mixed(c, b, L, order, d_err, s);
-    } else
-      launch_trace_fill(c, ch, b, L, d_err, s);
+      if (precision == JGB_MIXED)
+        launch_trace_fill_mixed(c, b, L, order, d_err, s);
+      else
+        launch_trace_fill(c, b, L, order, slopes, d_err, s);
+    }
     CK(cudaGetLastError());
     passes++;
     if (mode == kCount) break;
@@ -1604,7 +1615,7 @@ void jgb_destroy(jgb_ctx* x) {
                     &x->t_tf, &x->t_meta, &x->t_ue, &x->t_mono, &x->s_st, &x->s_sr, &x->s_srf, &x->s_srd, &x->b_levoff, &x->b_rayoff,
                     &x->b_rayobs, &x->b_lev, &x->b_scal, &x->b_geo, &x->b_rad, &x->b_tau,
                     &x->b_tp, &x->b_mask, &x->b_p, &x->los_off, &x->los_cnt, &x->los_cnt64,
-                    &x->los_sft, &x->los_ends, &x->los_planes, &x->scan_tmp, &x->err_word,
+                    &x->los_sft, &x->los_ends, &x->los_planes, &x->lev_slopes, &x->scan_tmp, &x->err_word,
                     &x->tiles_perm, &x->tiles_keys, &x->tiles_keys2, &x->tiles_vals,
                     &x->tiles_off, &x->tiles_len, &x->tiles_data, &x->refl, &x->seg,
                     &x->rs_start, &x->rs_lists, &x->rs_snap, &x->rs_base, &x->rs_seg, &x->rs_trace,

@@ -201,7 +201,8 @@ struct LosDev {
   int ng, nw;
   bool cga;
   // planes [point]
-  double *z, *lon, *lat, *p, *t, *ds, *aux, *qh2o;
+  double* z;            // mixed precision only
+  double *p, *t, *ds, *aux, *qh2o;
   double* u;            // [ng][cap]
   double* kw;           // [nw][cap]
   double *cgp, *cgt, *cgu;  // [ng][cap] (CGA only)

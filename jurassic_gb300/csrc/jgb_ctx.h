@@ -91,7 +91,7 @@ struct jgb_ctx {
   bool srf_stale = true, srd_stale = true;
   // per-call scratch
   jgb::DevBuf b_levoff, b_rayoff, b_rayobs, b_lev, b_scal, b_geo, b_rad, b_tau, b_tp, b_mask, b_p;
-  jgb::DevBuf los_off, los_cnt, los_cnt64, los_sft, los_ends, los_planes, scan_tmp, err_word;
+  jgb::DevBuf los_off, los_cnt, los_cnt64, los_sft, los_ends, los_planes, lev_slopes, scan_tmp, err_word;
   jgb::DevBuf tiles_perm, tiles_keys, tiles_keys2, tiles_vals, tiles_off, tiles_len, tiles_data;
   jgb::DevBuf refl;
   // finite-difference Jacobian: expanded batch and bookkeeping

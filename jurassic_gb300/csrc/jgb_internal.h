@@ -10,8 +10,12 @@ struct jgb_engine;
 
 namespace jgb {
 
-// jgb_fp64.cu
-void launch_trace_count(const CtlDev& c, const ChanDev& ch, const BatchDev& b, const LosDev& L,
+// jgb_fp64.cu: ray tracing.  slopes: the level intervals' slopes
+// (launch_level_slopes into level_slope_bytes) or nullptr, which forms them
+// as the rays go
+size_t level_slope_bytes(const CtlDev& c, long long nlev);
+void launch_level_slopes(const CtlDev& c, const BatchDev& b, double* slopes, cudaStream_t s);
+void launch_trace_count(const CtlDev& c, const BatchDev& b, const LosDev& L, const double* slopes,
                         unsigned* err, cudaStream_t s);
 // jgb_fp64.cu: field-of-view convolution + BT + mask of pencil-beam results
 void launch_fov(const CtlDev& c, const BatchDev& b, const double* prad, const double* ptau,
@@ -51,8 +55,8 @@ void launch_trace_fill_resumed(const CtlDev& c, const BatchDev& b, const LosDev&
                                unsigned* err, cudaStream_t s);
 void launch_los_bound_mixed(const CtlDev& c, const BatchDev& b, double scale, int* cap,
                             cudaStream_t s);
-void launch_trace_fill(const CtlDev& c, const ChanDev& ch, const BatchDev& b, const LosDev& L,
-                       unsigned* err, cudaStream_t s);
+void launch_trace_fill(const CtlDev& c, const BatchDev& b, const LosDev& L, const int* order,
+                       const double* slopes, unsigned* err, cudaStream_t s);
 void launch_path_fp64(const CtlDev& c, const TblDev& T, const ChanDev& ch, const BatchDev& b,
                       const LosDev& L, double* refl_scratch, cudaStream_t s);
 void launch_srcfunc(int nd, int id0, int nch, const int* fn_off, const double* fnu,

@@ -204,7 +204,7 @@ extern "C" int jgb_formod_batch_dev_noalloc(jgb_ctx* x, const jgb_batch* db) {
   const long long nm = (long long)c.nd * nray;
   k_noalloc_mask<<<(unsigned)((nm + 255) / 256), 256, 0, s>>>(nm, b.rad, base + o_mask);
   if (c.hydz >= 0) launch_hydrostatic(c, b, const_cast<double*>(b.p), s);
-  launch_trace_count(c, v.ch, b, L, d_err, s);
+  launch_trace_count(c, b, L, nullptr, d_err, s);
   k_noalloc_scan<<<1, 1024, 0, s>>>(nray, L.count, L.off);
   long long total = 0;
   unsigned h_err = 0;
@@ -232,20 +232,17 @@ extern "C" int jgb_formod_batch_dev_noalloc(jgb_ctx* x, const jgb_batch* db) {
   }
   double* P = reinterpret_cast<double*>(base + o_planes);
   L.cap = cap;
-  L.z = P + 0 * cap;
-  L.lon = P + 1 * cap;
-  L.lat = P + 2 * cap;
-  L.p = P + 3 * cap;
-  L.t = P + 4 * cap;
-  L.ds = P + 5 * cap;
-  L.aux = P + 6 * cap;
-  L.qh2o = P + 7 * cap;
-  L.u = P + 8 * cap;
+  L.p = P + 0 * cap;
+  L.t = P + 1 * cap;
+  L.ds = P + 2 * cap;
+  L.aux = P + 3 * cap;
+  L.qh2o = P + 4 * cap;
+  L.u = P + 5 * cap;
   L.kw = L.u + (long long)c.ng * cap;
   L.cgp = L.kw + (long long)c.nw * cap;
   L.cgt = L.cgp + (long long)c.ng * cap;
   L.cgu = L.cgt + (long long)c.ng * cap;
-  launch_trace_fill(c, v.ch, b, L, d_err, s);
+  launch_trace_fill(c, b, L, nullptr, nullptr, d_err, s);
   double* refl = need_refl ? reinterpret_cast<double*>(base + o_refl) : nullptr;
   launch_path_fp64(c, v.T, v.ch, b, L, refl, s);
   cudaEventRecord(x->ev[1], s);

@@ -10,6 +10,8 @@ struct jgb_engine;
 
 namespace jgb {
 
+struct DevBuf;
+
 // jgb_fp64.cu: ray tracing.  slopes: the level intervals' slopes
 // (launch_level_slopes into level_slope_bytes) or nullptr, which forms them
 // as the rays go
@@ -161,10 +163,11 @@ int ctx_view(jgb_ctx* x, CtxView* out);  // fills *out; returns JGB_ERR_STATE if
 // jgb_normal.cu: batched normal-equation products on device buffers.
 // Problems are concatenated (K blocks m_i x n_i, A blocks n_i x n_i, ...);
 // sel (host, nullptr = all) picks the problems computed, the others' blocks
-// are left untouched.  At most 65535 selected problems per call.
+// are left untouched.  At most 65535 selected problems per call.  split: the
+// operand blocks' buffer of the context whose stream s is.
 int normal_equations_dev(int nret, const int* m, const int* n, const double* K, const double* w,
                          const double* dy, double* A, double* b, int precision, const int* sel,
-                         void* desc_dev, cudaStream_t s);
+                         void* desc_dev, DevBuf& split, cudaStream_t s);
 size_t normal_desc_bytes(int nret);
 int ctx_fail(jgb_ctx* x, int code, const char* msg);
 

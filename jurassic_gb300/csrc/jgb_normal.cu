@@ -15,12 +15,11 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
-#include <map>
-#include <mutex>
-#include <utility>
+#include <vector>
 
 #include "../../include/jurassic_gb300.h"
 #include "jgb_common.cuh"
+#include "jgb_ctx.h"
 #include "jgb_internal.h"
 
 namespace jgb {
@@ -55,8 +54,6 @@ __device__ __forceinline__ unsigned tf32_of(float x) {
   asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
   return r;
 }
-
-__device__ unsigned g_tc_err;  // a tensor-core wait gave up (results invalid)
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
@@ -137,13 +134,30 @@ __global__ void k_wait_selftest(int arrive, unsigned long long* out) {
 // words (the FP64 pipe of GB300 is narrow): for a normal float the high word
 // is the sign, the exponent rebiased by 1023 - 127 and the top 20 mantissa
 // bits, the low word the last 3 mantissa bits; zero, subnormal, infinite
-// and NaN inputs take the conversion instruction.
+// and NaN inputs take the conversion instruction, in a call: inline it
+// becomes a predicated conversion that every value pays for (16 cycles of the
+// SM per warp).
+__device__ __noinline__ double f2d_rare(float f) { return (double)f; }
+
 __device__ __forceinline__ double f2d_bits(float f) {
   const unsigned u = __float_as_uint(f);
-  const unsigned e = u & 0x7f800000u;
-  if (e == 0u || e == 0x7f800000u) return (double)f;
+  if ((u & 0x7fffffffu) - 0x00800000u >= 0x7f000000u)
+    return u == 0u ? 0.0 : f2d_rare(f);
   const unsigned hi = (u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + (896u << 20));
   return __hiloint2double((int)hi, (int)(u << 29));
+}
+
+// (float)x, rounded to nearest even on the integer pipe; results outside the
+// normal range, infinities and NaN by the conversion (as above, in a call).
+__device__ __noinline__ float d2f_rare(double x) { return (float)x; }
+
+__device__ __forceinline__ float d2f_bits(double x) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const unsigned mag = hi & 0x7fffffffu, rest = lo & 0x1fffffffu;
+  if (mag - (897u << 20) >= (253u << 20)) return (mag | lo) == 0u ? __uint_as_float(hi) : d2f_rare(x);
+  const unsigned f = ((mag - (896u << 20)) << 3) | (lo >> 29);
+  return __uint_as_float((hi & 0x80000000u) |
+                         (f + (rest > 0x10000000u || (rest == 0x10000000u && (f & 1u)) ? 1u : 0u)));
 }
 
 // X = sqrt(W)[K | dy] of every problem, formed once in FP64 and split into
@@ -172,7 +186,7 @@ __global__ void __launch_bounds__(128) k_split_x(const NeDesc* desc, const doubl
       float x = 0.f;
       if (row < d.m && col < na) {
         const double v = col < d.n ? Kall[d.koff + (long long)row * d.n + col] : dyall[d.moff + row];
-        x = (float)(v * wall[d.moff + row]);
+        x = d2f_bits(v * wall[d.moff + row]);
       }
       const float hi = __uint_as_float(tf32_of(x));
       const int o = tc_off(tid, k) >> 2;
@@ -253,7 +267,8 @@ __device__ __forceinline__ void epi_sync() {
 // memory is freed.
 __global__ void __launch_bounds__(kNeThreads, 2) k_normal_tc(const NeDesc* desc, int nsel,
                                                              long long ntiles, const float* xbuf,
-                                                             double* Aall, double* ball) {
+                                                             double* Aall, double* ball,
+                                                             unsigned* err) {
   extern __shared__ __align__(1024) unsigned char tc_smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   uint64_t* full = reinterpret_cast<uint64_t*>(tc_smem + kBarOff);  // [kStages]
@@ -443,7 +458,7 @@ __global__ void __launch_bounds__(kNeThreads, 2) k_normal_tc(const NeDesc* desc,
       }
     }
   }
-  if (!ok) atomicOr(&g_tc_err, 1u);
+  if (!ok) atomicOr(err, 1u);
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   if (warp == 1)
@@ -481,36 +496,13 @@ __global__ void k_normal_fp64(const NeDesc* desc, const double* Kall, const doub
 
 }  // namespace
 
-// Grow-only scratch for the split X planes, one per device; calls that use
-// it are ordered on their stream (the engine and the entry points run on
-// their context's stream; concurrent streams on one device would share it).
-static float* split_buffer(size_t bytes, cudaStream_t s) {
-  static std::mutex mu;
-  static std::map<int, std::pair<void*, size_t>> bufs;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
-  std::lock_guard<std::mutex> lock(mu);
-  auto& b = bufs[dev];
-  if (b.second < bytes) {
-    if (b.first) {
-      cudaStreamSynchronize(s);
-      cudaFree(b.first);
-    }
-    b.first = nullptr;
-    b.second = 0;
-    const size_t want = bytes + bytes / 4;
-    if (cudaMalloc(&b.first, want) != cudaSuccess) return nullptr;
-    b.second = want;
-  }
-  return static_cast<float*>(b.first);
-}
-
 int normal_equations_dev(int nret, const int* m, const int* n, const double* K, const double* w,
                          const double* dy, double* A, double* b, int precision, const int* sel,
-                         void* desc_dev, cudaStream_t s) {
+                         void* desc_dev, DevBuf& split, cudaStream_t s) {
   // descriptors of the selected problems (host -> device scratch provided by
   // the caller); offsets follow the concatenation of all nret problems
-  NeDesc* hd = new NeDesc[nret];
+  // (one more entry holds the tensor-core kernel's error word)
+  std::vector<NeDesc> hd(nret + 1);
   long long ko = 0, mo = 0, ao = 0, bo = 0, xo = 0, ntiles = 0;
   int maxn = 0, maxblk = 0, nsel = 0;
   for (int i = 0; i < nret; i++) {
@@ -528,37 +520,31 @@ int normal_equations_dev(int nret, const int* m, const int* n, const double* K, 
     ao += (long long)n[i] * n[i];
     bo += n[i];
   }
-  if (nsel == 0) {
-    delete[] hd;
-    return JGB_OK;
-  }
-  if (nsel > 65535) {
-    delete[] hd;
-    return JGB_ERR_ARG;
-  }
-  cudaError_t e = cudaMemcpyAsync(desc_dev, hd, sizeof(NeDesc) * nsel, cudaMemcpyHostToDevice, s);
-  cudaStreamSynchronize(s);
-  delete[] hd;
-  if (e != cudaSuccess) return JGB_ERR_CUDA;
+  if (nsel == 0) return JGB_OK;
+  if (nsel > 65535) return JGB_ERR_ARG;
+  hd[nsel] = NeDesc{};
+  // pageable memory: staged by the time the call returns
+  if (cudaMemcpyAsync(desc_dev, hd.data(), sizeof(NeDesc) * (nsel + 1), cudaMemcpyHostToDevice, s) !=
+      cudaSuccess)
+    return JGB_ERR_CUDA;
   if (precision == JGB_MIXED) {
-    // operand blocks in a grow-only buffer of the current device (held to exit)
-    float* xbuf = split_buffer(sizeof(float) * (size_t)xo, s);
-    if (!xbuf) return JGB_ERR_CUDA;
+    // operand blocks in the context's buffer (its calls run one after another)
+    if (split.reserve(sizeof(float) * (size_t)xo) != cudaSuccess) return JGB_ERR_CUDA;
+    float* xbuf = split.as<float>();
     const NeDesc* dd = static_cast<const NeDesc*>(desc_dev);
     k_split_x<<<dim3((unsigned)(maxblk < 4096 ? maxblk : 4096), nsel), 128, 0, s>>>(dd, K, w, dy,
                                                                                       xbuf);
     cudaFuncSetAttribute(k_normal_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
-    const unsigned zero = 0;
-    cudaMemcpyToSymbolAsync(g_tc_err, &zero, sizeof(zero), 0, cudaMemcpyHostToDevice, s);
+    unsigned* err = reinterpret_cast<unsigned*>(static_cast<NeDesc*>(desc_dev) + nsel);
     // persistent: two CTAs per SM (or one per tile when there are fewer)
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
       return JGB_ERR_CUDA;
     const unsigned grid = (unsigned)(ntiles < 2LL * sms ? ntiles : 2LL * sms);
-    k_normal_tc<<<grid, kNeThreads, kTcSmem, s>>>(dd, nsel, ntiles, xbuf, A, b);
+    k_normal_tc<<<grid, kNeThreads, kTcSmem, s>>>(dd, nsel, ntiles, xbuf, A, b, err);
     unsigned herr = 0;
-    cudaMemcpyFromSymbolAsync(&herr, g_tc_err, sizeof(herr), 0, cudaMemcpyDeviceToHost, s);
+    cudaMemcpyAsync(&herr, err, sizeof(herr), cudaMemcpyDeviceToHost, s);
     if (cudaStreamSynchronize(s) != cudaSuccess || herr) return JGB_ERR_CUDA;
   } else {
     const long long nel = (long long)maxn * (maxn + 1) / 2 + maxn;
@@ -568,7 +554,7 @@ int normal_equations_dev(int nret, const int* m, const int* n, const double* K, 
   return cudaGetLastError() == cudaSuccess ? JGB_OK : JGB_ERR_CUDA;
 }
 
-size_t normal_desc_bytes(int nret) { return sizeof(NeDesc) * (size_t)nret; }
+size_t normal_desc_bytes(int nret) { return sizeof(NeDesc) * ((size_t)nret + 1); }
 
 int wait_selftest(int device, int arrive, int* timed_out, double* seconds) {
   if (!timed_out || !seconds) return JGB_ERR_ARG;
@@ -627,7 +613,7 @@ extern "C" int jgb_normal_equations(jgb_ctx* x, int nret, const int* m, const in
   cudaMemcpyAsync(dK, K, sizeof(double) * sk, cudaMemcpyHostToDevice, s);
   cudaMemcpyAsync(dw, w, sizeof(double) * sm, cudaMemcpyHostToDevice, s);
   cudaMemcpyAsync(ddy, dy, sizeof(double) * sm, cudaMemcpyHostToDevice, s);
-  rc = normal_equations_dev(nret, m, n, dK, dw, ddy, dA, db, precision, nullptr, ddesc, s);
+  rc = normal_equations_dev(nret, m, n, dK, dw, ddy, dA, db, precision, nullptr, ddesc, x->ne_split, s);
   if (rc == JGB_OK) {
     cudaMemcpyAsync(A, dA, sizeof(double) * sa, cudaMemcpyDeviceToHost, s);
     cudaMemcpyAsync(b, db, sizeof(double) * sb, cudaMemcpyDeviceToHost, s);
@@ -653,27 +639,23 @@ extern "C" int jgb_normal_equations_dev(jgb_ctx* x, int nret, const int* m, cons
   cudaSetDevice(v.device);
   for (int i = 0; i < nret; i++)
     if (m[i] <= 0 || n[i] <= 0) return ctx_fail(x, JGB_ERR_ARG, "empty retrieval");
-  void* ddesc = nullptr;
-  if (cudaMalloc(&ddesc, normal_desc_bytes(nret)) != cudaSuccess)
+  // descriptors in the context's buffer, under its lock
+  if (x->ne_desc.reserve(normal_desc_bytes(nret)) != cudaSuccess)
     return ctx_fail(x, JGB_ERR_CUDA, "cudaMalloc failed");
-  cudaEvent_t e0, e1;
-  cudaEventCreate(&e0);
-  cudaEventCreate(&e1);
+  void* ddesc = x->ne_desc.p;
+  cudaEvent_t e0 = x->ev[0], e1 = x->ev[1];
   cudaStream_t s = v.stream;
   // descriptors are uploaded (and the stream synchronised) inside; the
   // events bracket the kernel launch that follows
-  rc = normal_equations_dev(nret, m, n, K, w, dy, A, b, precision, nullptr, ddesc, s);
+  rc = normal_equations_dev(nret, m, n, K, w, dy, A, b, precision, nullptr, ddesc, x->ne_split, s);
   // time a second identical launch only when asked: the first one above
   // included the descriptor upload
   if (rc == JGB_OK && kernel_ms) {
     cudaEventRecord(e0, s);
-    rc = normal_equations_dev(nret, m, n, K, w, dy, A, b, precision, nullptr, ddesc, s);
+    rc = normal_equations_dev(nret, m, n, K, w, dy, A, b, precision, nullptr, ddesc, x->ne_split, s);
     cudaEventRecord(e1, s);
   }
   if (cudaStreamSynchronize(s) != cudaSuccess) rc = JGB_ERR_CUDA;
   if (rc == JGB_OK && kernel_ms) cudaEventElapsedTime(kernel_ms, e0, e1);
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  cudaFree(ddesc);
   return rc ? ctx_fail(x, rc, "normal-equation kernel failed") : JGB_OK;
 }

@@ -1370,7 +1370,7 @@ int lm_iteration(jgb_engine* E, WorkSet& w) {
   // K^T W K into covn and K^T W dy into bvec; covn replaces cov where the
   // kernel was (re)computed for this iteration
   rc = normal_equations_dev(nret, w.mvec.data(), w.nvec.data(), w.Kd, w.w, w.dy, w.covn, w.bvec,
-                            E->precision, A.data(), w.nedesc, s);
+                            E->precision, A.data(), w.nedesc, x->ne_split, s);
   if (rc) return ctx_error(x, rc, "normal-equation kernel failed");
   rc = put_flags(E, w, N);
   if (rc) return rc;
@@ -1444,7 +1444,7 @@ int finish_requests(jgb_engine* E, WorkSet& w) {
   if (err_ana && any_ok) {
     // the final covariance is FP64 in both precision modes
     rc = normal_equations_dev(nret, w.mvec.data(), w.nvec.data(), w.Kd, w.w, w.dy, w.covn, w.bvec,
-                              JGB_FP64, ok.data(), w.nedesc, s);
+                              JGB_FP64, ok.data(), w.nedesc, x->ne_split, s);
     if (rc) return ctx_error(x, rc, "normal-equation kernel failed");
     rc = put_flags(E, w, ok);
     if (rc) return rc;

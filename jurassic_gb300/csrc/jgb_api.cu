@@ -131,6 +131,7 @@ TblDev tbl_view(const jgb_ctx* x) {
   T.ue = x->t_ue.as<float2>();
   T.sr = x->s_sr.as<double>();
   T.srf = x->s_srf.as<float>();
+  T.chanf = x->d_chanf.as<float>();
   T.srd = x->s_srd.as<double2>();
   T.st = x->s_st.as<double>();
   return T;
@@ -374,11 +375,8 @@ int prepare_tables(jgb_ctx* x, cudaStream_t s) {
     }
   const long long nrow = (long long)c.nd * c.ng * x->tp * x->tt;
   launch_rowmeta(nrow, x->tu, x->t_nu.as<int>(), x->t_u.as<float>(), x->t_eps.as<float>(),
-                 x->t_tf.as<float>(), c.formod == 0, x->t_meta.as<float4>(), x->t_ue.as<float2>(), s);
-  const int one = 1;
-  CK(cudaMemcpyAsync(x->t_mono.p, &one, sizeof(int), cudaMemcpyHostToDevice, s));
-  launch_rows_mono(nrow, x->tu, x->t_nu.as<int>(), x->t_u.as<float>(), x->t_eps.as<float>(),
-                   x->t_mono.as<int>(), s);
+                 c.formod == 0, x->t_meta.as<float4>(), x->t_ue.as<float2>(), s);
+  launch_chan_consts(c, chan_view(x), x->d_chanf.as<float>(), s);
   CK(cudaGetLastError());
   x->meta_stale = false;
   return JGB_OK;
@@ -427,11 +425,71 @@ int plan_tiles(jgb_ctx* x, int nray, const int* keys, const int* count, int ntil
   return JGB_OK;
 }
 
-// FP64 path of a traced batch: chunks of tiles whose workspaces stay within
-// kPath64Bytes (per-point fields within a quarter of it), and of channels
-// where one tile alone would exceed it.
-constexpr size_t kPath64Bytes = size_t(4) << 30;
+// Workspace of the path between its kernels (segments of every point, channel
+// and emitter): a batch runs in chunks of tiles within it, of channels where
+// one tile alone would exceed it.  4 GiB is 1.4 % of the device and gives the
+// emitters' kernel tens of warps per scheduler.
+constexpr size_t kPathBytes = size_t(4) << 30;
 
+struct PathChunk {
+  int t0, t1;   // tiles
+  int ndc;      // channels at a time
+  int longest;  // points of the longest tile
+};
+
+// point_bytes, chan_bytes: workspace of a tile point, and of one per channel;
+// tile_bytes: of a (tile, channel).  The largest needs in *need_points (limited
+// to a quarter of kPathBytes) and *need_chan.
+void path_chunks(const std::vector<long long>& toff, int nd, size_t point_bytes, size_t chan_bytes,
+                 size_t tile_bytes, std::vector<PathChunk>& out, size_t* need_points,
+                 size_t* need_chan) {
+  const int ntile = (int)toff.size() - 1;
+  for (int t = 0; t < ntile;) {
+    PathChunk k{t, t, nd, 0};
+    auto pts = [&](int t1) { return (size_t)(toff[t1] - toff[k.t0]); };
+    do {
+      k.longest = std::max(k.longest, (int)(toff[k.t1 + 1] - toff[k.t1]));
+      k.t1++;
+    } while (k.t1 < ntile && k.t1 - k.t0 < 65535 && pts(k.t1 + 1) * point_bytes <= kPathBytes / 4 &&
+             pts(k.t1 + 1) * nd * chan_bytes <= kPathBytes);
+    const size_t np = std::max<size_t>(pts(k.t1), 1);
+    if (np * nd * chan_bytes > kPathBytes) k.ndc = (int)std::max<size_t>(kPathBytes / (np * chan_bytes), 1);
+    if (need_points) *need_points = std::max(*need_points, np * point_bytes);
+    *need_chan = std::max(*need_chan, np * k.ndc * chan_bytes + (size_t)(k.t1 - k.t0) * k.ndc * tile_bytes);
+    out.push_back(k);
+    t = k.t1;
+  }
+}
+
+// The autotuner of the mixed path: times every variant of the emitters'
+// kernel on a chunk (the results are the same) and keeps the fastest;
+// JGB_PATH_VARIANT takes one without timing.
+int tune_gas(jgb_ctx* x, const TblDev& T, const BatchDev& b, const LosDev& L, const MixedPlan& P,
+             cudaStream_t s) {
+  const int nv = path_gas_variants();
+  if (const char* force = getenv("JGB_PATH_VARIANT")) {
+    x->path_variant = ((atoi(force) % nv) + nv) % nv;
+    return JGB_OK;
+  }
+  x->tune_ms.clear();
+  float best = 1e30f;
+  for (int v = 0; v < nv; v++) {
+    CK(cudaEventRecord(x->ev[4], s));
+    launch_gas_m(x->c, T, b, L, P, 1, v, s);
+    CK(cudaEventRecord(x->ev[5], s));
+    CK(cudaEventSynchronize(x->ev[5]));
+    float ms = 0;
+    cudaEventElapsedTime(&ms, x->ev[4], x->ev[5]);
+    x->tune_ms.push_back(ms);
+    if (ms < best) {
+      best = ms;
+      x->path_variant = v;
+    }
+  }
+  return JGB_OK;
+}
+
+// FP64 path of a traced batch.
 int run_path64(jgb_ctx* x, const BatchDev& b, const LosDev& L, cudaStream_t s, int* launches) {
   const CtlDev& c = x->c;
   const int nray = b.nray, ntile = (nray + 31) / 32;
@@ -454,27 +512,10 @@ int run_path64(jgb_ctx* x, const BatchDev& b, const LosDev& L, cudaStream_t s, i
   size_t bfd, bfu;
   path64_point_bytes(c, &bfd, &bfu);
   const size_t bch = 32 * sizeof(double) * (size_t)(c.ng + 2);  // per (point, channel)
-  struct Chunk {
-    int t0, t1, ndc, longest;
-  };
-  std::vector<Chunk> chunks;
+  std::vector<PathChunk> chunks;
   size_t need_f = 0, need_w = 0;
-  for (int t = 0; t < ntile;) {
-    Chunk k{t, t, c.nd, 0};
-    auto pts = [&](int t1) { return (size_t)(toff[t1] - toff[k.t0]); };
-    do {
-      k.longest = std::max(k.longest, (int)(toff[k.t1 + 1] - toff[k.t1]));
-      k.t1++;
-    } while (k.t1 < ntile && k.t1 - k.t0 < 65535 && pts(k.t1 + 1) * (bfd + bfu) <= kPath64Bytes / 4 &&
-             pts(k.t1 + 1) * c.nd * bch <= kPath64Bytes);
-    const size_t np = std::max<size_t>(pts(k.t1), 1);
-    if (np * c.nd * bch > kPath64Bytes) k.ndc = (int)std::max<size_t>(kPath64Bytes / (np * bch), 1);
-    need_f = std::max(need_f, np * (bfd + bfu));
-    need_w = std::max(need_w, np * k.ndc * bch +
-                                  sizeof(int) * 32 * (size_t)(k.t1 - k.t0) * k.ndc * std::max(c.ng, 1));
-    chunks.push_back(k);
-    t = k.t1;
-  }
+  path_chunks(toff, c.nd, bfd + bfu, bch, 32 * sizeof(int) * (size_t)std::max(c.ng, 1), chunks,
+              &need_f, &need_w);
   CK(x->tiles_data.reserve(need_f));
   CK(x->seg.reserve(need_w));
   CK(cudaEventRecord(x->ev[4], s));
@@ -483,10 +524,9 @@ int run_path64(jgb_ctx* x, const BatchDev& b, const LosDev& L, cudaStream_t s, i
   P.toff = Pm.toff;
   P.shared = x->grid_mask64;
   std::copy(x->grid_ref, x->grid_ref + kMaxG, P.gref);
-  P.mono = x->t_mono.as<int>();
   const TblDev T = tbl_view(x);
   const ChanDev ch = chan_view(x);
-  for (const Chunk& k : chunks) {
+  for (const PathChunk& k : chunks) {
     const size_t np = std::max<size_t>((size_t)(toff[k.t1] - toff[k.t0]), 1);
     P.tile0 = k.t0;
     P.tile1 = k.t1;
@@ -748,8 +788,6 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
     bo.rad = x->fov_raw.as<double>();
     bo.tau = bo.rad + (size_t)c.nd * nray;
   }
-  // reflection needs per-point source and emissivity per channel
-  const bool need_refl = c.sftype >= 2 && c.nsf > 0;
   TblDev T = tbl_view(x);
   int launches = 4 + (c.hydz >= 0) + trace_launches;
   if (precision == JGB_FP64) {
@@ -977,18 +1015,6 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
     Pm.data = x->tiles_data.as<float>();
     launch_pack_tiles_n(c, tbl_view(x), L, Pm, tile_points, s);
     CK(cudaGetLastError());
-    float* refl = nullptr;
-    if (need_refl) {
-      CK(x->refl.reserve(sizeof(float) * 2 * (size_t)cap * c.nd));
-      refl = x->refl.as<float>();
-    }
-    // a batch with too few tiles to fill the device is latency-bound: split
-    // the path over the emitters (ng warps per tile and channel)
-    const long long split_warps = (long long)ntile * c.nd * c.ng;
-    const bool split = !rs && c.ng > 1 &&
-                       (x->path_split == 1 || (x->path_split < 0 && split_warps <= 32LL * x->sms));
-    Pm.seg_eps = nullptr;
-    Pm.seg_sat = nullptr;
     if (rs) {
       // bases (saving the states), then the perturbations (starting from them)
       Pm.start = rstart;
@@ -1016,46 +1042,53 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
       launch_path_resume(c, T, ch, bo, L, Pm, s);
       launches += 10;
       x->stats.resume_skip = resume_skip;
-    } else if (split) {
-      const size_t nseg = (size_t)std::max(tile_points, 1LL) * c.nd * c.ng * 32;
-      CK(x->seg.reserve(nseg * (sizeof(float) + 1)));
-      Pm.seg_eps = x->seg.as<float>();
-      Pm.seg_sat = reinterpret_cast<unsigned char*>(Pm.seg_eps + nseg);
-      CK(cudaEventRecord(x->ev[4], s));
-      launch_path_split(c, T, ch, bo, L, Pm, refl, s);
-      launches += 7;
-    } else if (x->path_variant < 0 && !rs) {
-      // autotune: time every register cap with both block shapes on this
-      // batch (results are identical)
-      const char* force = getenv("JGB_PATH_VARIANT");
-      if (force) {
-        x->path_variant = atoi(force) % path_mixed_variants();
-      } else {
-        float best = 1e30f;
-        x->tune_ms.clear();
-        auto trial = [&](int v) -> int {
-          CK(cudaEventRecord(x->ev[4], s));
-          launch_path_mixed(c, T, ch, bo, L, Pm, refl, v, s);
-          CK(cudaEventRecord(x->ev[5], s));
-          CK(cudaEventSynchronize(x->ev[5]));
-          const float ms = elapsed(x->ev[4], x->ev[5]);
-          x->tune_ms.push_back(ms);
-          if (ms < best) {
-            best = ms;
-            x->path_variant = v;
+    } else {
+      if (c.ncl > 0) {
+        CK(x->cloudf.reserve(sizeof(float) * (size_t)c.nd * nray));
+        launch_cloud_m(c, ch, bo, x->cloudf.as<float>(), s);
+        Pm.cloud = x->cloudf.as<float>();
+        launches += 1;
+      }
+      Pm.nseg = std::max(c.ng, 2);
+      // chunks of tiles whose segments stay within kPathBytes (and of channels
+      // where one tile alone would not)
+      const size_t bch = 32 * sizeof(float) * (size_t)Pm.nseg;
+      std::vector<PathChunk> chunks;
+      size_t need = 0;
+      path_chunks(toff_h, c.nd, 0, bch, 32 * sizeof(int) * (size_t)std::max(c.ng, 1), chunks, nullptr, &need);
+      CK(x->seg.reserve(need));
+      // a batch that leaves the schedulers idle gives each ray four lanes
+      const long long warps = (long long)ntile * c.nd * c.ng;
+      const int lanes = x->path_split == 1 || (x->path_split < 0 && warps <= 8LL * x->sms) ? 4 : 1;
+      bool timed = false;
+      for (const PathChunk& k : chunks) {
+        Pm.tile0 = k.t0;
+        Pm.tile1 = k.t1;
+        Pm.pt0 = toff_h[k.t0];
+        const size_t np = std::max<size_t>((size_t)(toff_h[k.t1] - toff_h[k.t0]), 1);
+        for (int id = 0; id < c.nd; id += k.ndc) {
+          Pm.id0 = id;
+          Pm.id1 = std::min(c.nd, id + k.ndc);
+          Pm.seg = x->seg.as<float>();
+          Pm.stop = reinterpret_cast<int*>(x->seg.as<char>() + np * (Pm.id1 - Pm.id0) * bch);
+          int variant = x->path_variant;
+          if (lanes == 1 && variant < 0 && warps > 32LL * x->sms) {
+            const int rc = tune_gas(x, T, bo, L, Pm, s);
+            if (rc) return rc;
+            variant = x->path_variant;
           }
-          return JGB_OK;
-        };
-        for (int v = 0; v < path_mixed_variants(); v++) {
-          const int rc = trial(v);
-          if (rc) return rc;
+          // few tiles: no consecutive ones to share rows between
+          if (variant < 0) variant = 6;
+          if (k.t1 - k.t0 < 8) variant %= 4;
+          if (!timed) CK(cudaEventRecord(x->ev[4], s));
+          timed = true;
+          launch_gas_m(c, T, bo, L, Pm, lanes, variant, s);
+          launch_seg_scan_m(c, T, ch, bo, L, Pm, std::max(k.longest, 1), s);
+          CK(cudaGetLastError());
+          launches += 3;
         }
       }
-    }
-    if (!split && !rs) {
-      CK(cudaEventRecord(x->ev[4], s));
-      launch_path_mixed(c, T, ch, bo, L, Pm, refl, x->path_variant, s);
-      launches += 6;
+      launches += 5;
     }
   }
   CK(cudaGetLastError());
@@ -1584,7 +1617,7 @@ int jgb_create(const jgb_ctl* ctl, int device, jgb_ctx** out) {
             x->s_sr.reserve(sizeof(double) * kNS * c.nd) == cudaSuccess &&
             x->s_srf.reserve(sizeof(float) * kNS * c.nd) == cudaSuccess &&
             x->s_srd.reserve(sizeof(double2) * kNS * c.nd) == cudaSuccess &&
-            x->t_mono.reserve(sizeof(int)) == cudaSuccess;
+            x->d_chanf.reserve(chan_const_bytes(c)) == cudaSuccess;
   ok = ok && cudaMemcpy(x->d_nu.p, x->nu.data(), sizeof(double) * c.nd, cudaMemcpyHostToDevice) == cudaSuccess;
   ok = ok && cudaMemcpy(x->d_window.p, x->window.data(), sizeof(int) * c.nd, cudaMemcpyHostToDevice) == cudaSuccess;
   if (c.ncl) ok = ok && cudaMemcpy(x->d_clnu.p, x->clnu.data(), sizeof(double) * c.ncl, cudaMemcpyHostToDevice) == cudaSuccess;
@@ -1610,14 +1643,14 @@ void jgb_destroy(jgb_ctx* x) {
     for (jgb_engine* E : x->engines) engine_detach(E);
     x->engines.clear();
   }
-  DevBuf* bufs[] = {&x->d_nu, &x->d_window, &x->d_clnu, &x->d_sfnu, &x->d_ctm, &x->t_np,
+  DevBuf* bufs[] = {&x->d_nu, &x->d_window, &x->d_clnu, &x->d_sfnu, &x->d_ctm, &x->d_chanf, &x->cloudf, &x->t_np,
                     &x->t_p, &x->t_nt, &x->t_t, &x->t_nu, &x->t_u, &x->t_eps, &x->t_pf,
-                    &x->t_tf, &x->t_meta, &x->t_ue, &x->t_mono, &x->s_st, &x->s_sr, &x->s_srf, &x->s_srd, &x->b_levoff, &x->b_rayoff,
+                    &x->t_tf, &x->t_meta, &x->t_ue, &x->s_st, &x->s_sr, &x->s_srf, &x->s_srd, &x->b_levoff, &x->b_rayoff,
                     &x->b_rayobs, &x->b_lev, &x->b_scal, &x->b_geo, &x->b_rad, &x->b_tau,
                     &x->b_tp, &x->b_mask, &x->b_p, &x->los_off, &x->los_cnt, &x->los_cnt64,
                     &x->los_sft, &x->los_ends, &x->los_planes, &x->lev_slopes, &x->scan_tmp, &x->err_word,
                     &x->tiles_perm, &x->tiles_keys, &x->tiles_keys2, &x->tiles_vals,
-                    &x->tiles_off, &x->tiles_len, &x->tiles_data, &x->refl, &x->ne_desc, &x->ne_split, &x->seg,
+                    &x->tiles_off, &x->tiles_len, &x->tiles_data, &x->ne_desc, &x->ne_split, &x->seg,
                     &x->rs_start, &x->rs_lists, &x->rs_snap, &x->rs_base, &x->rs_seg, &x->rs_trace,
                     &x->d_fov, &x->fov_raw,
                     &x->kx_levoff, &x->kx_rayoff, &x->kx_rayobs, &x->kx_src, &x->kx_lev,

@@ -142,6 +142,10 @@ struct CtlDev {
   int fov;   // field-of-view convolution on: path kernels write pencil values only
 };
 
+// Mark in a row record's count: the row falls somewhere, or its columns reach
+// 2^125 (see jgb_mixed.cu).
+constexpr int kOddRow = 0x40000000;
+
 // Emissivity tables, dense with capacities tp x tt x tu per (channel, emitter).
 struct TblDev {
   int tp, tt, tu;
@@ -154,10 +158,11 @@ struct TblDev {
   const float* eps;    // [nd*ng*tp*tt*tu]
   const float* pf;     // float copies of p and t for the mixed path
   const float* tf;
-  const float4* rowmeta;  // row records of the mixed path (EGA: 2 float4 per row, CGA: 1)
+  const float4* rowmeta;  // row records (EGA: 2 float4 per row, CGA: 1; layouts in jgb_mixed.cu)
   const float2* ue;    // rows interleaved {u[i], eps[i]} (mixed path)
   const double* sr;    // source function [kNS][nd]
   const double2* srd;  // source function, channel-major: value and slope [nd][kNS]
+  const float* chanf;  // channel constants of the mixed path
   const float* srf;    // source function, channel-major float [nd][kNS]
   const double* st;    // source-function temperatures [kNS]
 };

@@ -65,7 +65,7 @@ struct jgb_ctx {
   double retp_zmin = 0, retp_zmax = 0, rett_zmin = 0, rett_zmax = 0;
   int ret_flags[7] = {0, 0, 0, 0, 0, 0, 0};
   // device constants
-  jgb::DevBuf d_nu, d_window, d_clnu, d_sfnu, d_ctm;
+  jgb::DevBuf d_nu, d_window, d_clnu, d_sfnu, d_ctm, d_chanf;
   // tables
   int tp = 0, tt = 0, tu = 0;
   bool tables_init = false;
@@ -83,7 +83,7 @@ struct jgb_ctx {
   // field of view: nfov samples (dz, w) on the device, pencil-beam scratch
   int nfov = 0;
   jgb::DevBuf d_fov, fov_raw;
-  jgb::DevBuf t_np, t_p, t_nt, t_t, t_nu, t_u, t_eps, t_pf, t_tf, t_meta, t_ue, t_mono;
+  jgb::DevBuf t_np, t_p, t_nt, t_t, t_nu, t_u, t_eps, t_pf, t_tf, t_meta, t_ue;
   bool meta_stale = true;
   // source function
   jgb::DevBuf s_st, s_sr, s_srf, s_srd;
@@ -93,7 +93,7 @@ struct jgb_ctx {
   jgb::DevBuf b_levoff, b_rayoff, b_rayobs, b_lev, b_scal, b_geo, b_rad, b_tau, b_tp, b_mask, b_p;
   jgb::DevBuf los_off, los_cnt, los_cnt64, los_sft, los_ends, los_planes, lev_slopes, scan_tmp, err_word;
   jgb::DevBuf tiles_perm, tiles_keys, tiles_keys2, tiles_vals, tiles_off, tiles_len, tiles_data;
-  jgb::DevBuf refl;
+  jgb::DevBuf cloudf;   // mixed path: cloud extinction per (channel, ray)
   jgb::DevBuf ne_desc, ne_split;  // normal equations: descriptors, operand blocks
   // finite-difference Jacobian: expanded batch and bookkeeping
   jgb::DevBuf kx_levoff, kx_rayoff, kx_rayobs, kx_src, kx_lev, kx_scal, kx_geo, kx_rad, kx_tau, kx_tp,
@@ -102,9 +102,9 @@ struct jgb_ctx {
   // copies of the second chunk of a host batch overlap the first's compute
   cudaStream_t copy_stream = nullptr;
   cudaEvent_t pev[3] = {};
-  int path_variant = -1;  // mixed path kernel variant chosen by the autotuner
+  int path_variant = -1;  // variant of the mixed path's emitter kernel chosen by the autotuner
   double los_bound_scale = 1.0;  // factor on the per-ray LOS bound (0: count first)
-  int path_split = -1;    // path split over emitters: -1 when latency-bound, 0 never, 1 always
+  int path_split = -1;    // four lanes per ray in the mixed path: -1 small batches, 0 never, 1 always
   int fd_resume = 1;      // resume perturbed paths from their base's state: 0 never,
                           // 1 when the estimated schedule is shorter, 2 always,
                           // 3 always and with the emitters shared with the base
@@ -115,7 +115,7 @@ struct jgb_ctx {
   // retrieval engines made from this context (detached by jgb_destroy)
   std::vector<jgb_engine*> engines;
   int sms = 152;          // multiprocessors of the device
-  jgb::DevBuf seg;        // segment emissivities and flags of the split path
+  jgb::DevBuf seg;        // workspace of the path between its kernels
   std::vector<float> tune_ms;
   jgb_stats stats{};
   std::string err;

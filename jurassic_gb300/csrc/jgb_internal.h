@@ -82,17 +82,17 @@ struct MixedPlan {
   float* data;          // tile planes
   int nfield;
   unsigned brmask;      // emitters with p-T brackets precomputed per LOS point
-  // split path (latency-bound batches): segment emissivity and saturation
-  // flag of every (tile point, channel, emitter, lane), else nullptr
-  float* seg_eps;
-  unsigned char* seg_sat;
-  // tiles [tile0, tile1) of this launch
+  // a chunk of the path (k_gas_m, k_seg_m, k_scan_m): tiles [tile0, tile1)
+  // with pt0 = toff[tile0], channels [id0, id1); seg[((point * channels +
+  // channel) * nseg + emitter) * 32 + lane] the segment emissivities, stop the
+  // point where each (tile, channel, emitter, lane) saturates
   int tile0, tile1;
-  // block shape of the path kernel: 0 = the 4 warps of a block take 4
-  // channels of one tile (they share the tile's LOS data), 1 = one channel
-  // of 4 consecutive tiles (they share the table rows: similar rays at
-  // similar p-T)
-  int tile_major;
+  long long pt0;
+  int id0, id1;
+  int nseg;
+  float* seg;
+  int* stop;
+  const float* cloud;   // [nd][nray] cloud extinction (NaN: none), nullptr: no clouds
   // resumed forward models (finite-difference perturbations): start[r] is
   // the LOS point ray r starts at (its state read from snap, slot r); ray r
   // saves the path state for the rays snap_ray[k] before its point
@@ -122,26 +122,27 @@ struct MixedPlan {
 int mixed_nfield(const CtlDev& c, unsigned brmask);
 void launch_pack_tiles_n(const CtlDev& c, const TblDev& T, const LosDev& L, const MixedPlan& P,
                          long long total_tile_points, cudaStream_t s);
-// register-cap variants of the path kernel (each with both block shapes:
-// variant v = cap + path_mixed_caps() * shape)
-int path_mixed_caps();
-int path_mixed_variants();
-// the path split over emitters: one warp per (tile, channel, emitter) for the
-// emitter path states, then the combination and radiance per (tile, channel)
-void launch_path_split(const CtlDev& c, const TblDev& T, const ChanDev& ch, const BatchDev& b,
-                       const LosDev& L, const MixedPlan& P, float* refl_scratch, cudaStream_t s);
+// the path of a chunk: the emitters' paths (lanes_per_ray 1 or 4; variant:
+// the autotuner's choice for 1), then segments and sums
+int path_gas_variants();
+void launch_gas_m(const CtlDev& c, const TblDev& T, const BatchDev& b, const LosDev& L,
+                  const MixedPlan& P, int lanes_per_ray, int variant, cudaStream_t s);
+void launch_seg_scan_m(const CtlDev& c, const TblDev& T, const ChanDev& ch, const BatchDev& b,
+                       const LosDev& L, const MixedPlan& P, int longest, cudaStream_t s);
+void launch_cloud_m(const CtlDev& c, const ChanDev& ch, const BatchDev& b, float* out,
+                    cudaStream_t s);
+// FP32 channel constants of the path
+size_t chan_const_bytes(const CtlDev& c);
+void launch_chan_consts(const CtlDev& c, const ChanDev& ch, float* out, cudaStream_t s);
 // the path of tiles [P.tile0, P.tile1) with resume points and state snapshots
 void launch_path_resume(const CtlDev& c, const TblDev& T, const ChanDev& ch, const BatchDev& b,
                         const LosDev& L, const MixedPlan& P, cudaStream_t s);
 // words of one saved path state (per ray and channel)
 int path_state_words(const CtlDev& c);
-void launch_path_mixed(const CtlDev& c, const TblDev& T, const ChanDev& ch, const BatchDev& b,
-                       const LosDev& L, const MixedPlan& P, float* refl_scratch, int variant,
-                       cudaStream_t s);
 void launch_src_to_float(int nd, const double* sr, float* srf, cudaStream_t s);
 void launch_tables_to_float(long long n, const double* src, float* dst, cudaStream_t s);
-void launch_rowmeta(long long nrow, int tu, const int* nu, const float* u, const float* e,
-                    const float* tf, int cga, float4* meta, float2* ue, cudaStream_t s);
+void launch_rowmeta(long long nrow, int tu, const int* nu, const float* u, const float* e, int cga,
+                    float4* meta, float2* ue, cudaStream_t s);
 
 // jgb_retrieval.cu: frees an engine's device and pinned memory and unties
 // it from its context (which is being destroyed); the handle then accepts

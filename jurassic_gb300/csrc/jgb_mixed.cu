@@ -71,50 +71,22 @@ constexpr unsigned kNoBracket = 0x80000000u;
 // only on a miss.  Any valid bracket gives the same interpolated value, so
 // the result does not depend on the hint.
 
-struct RowF {
-  unsigned off;          // row start in the u and eps arrays
-  int n;
-  float u0, un, e0, en;  // first/last entries of the row
-  float t;               // temperature of the row
-};
-
 // Row r = (dg * tp + ip) * tt + it from its record; 32-bit row arithmetic
 // (the table upload checks that rows x TU < 2^32).  EGA records are 32
-// bytes, {u[0], u[n-1], eps[0], eps[n-1]} and {n (int bits), t, 0, 0}: both
-// ends of a row are tested before any search (the path emissivity starts
-// below the rows and saturates above them).  CGA records are 16 bytes,
-// {n, t, u[0], eps[0]}: a column above a row brackets at n-2, and the
+// bytes, {u[0], eps[0], eps[n-1], n} and {u[n-1], a, 0, 0}, where a = log(1 -
+// eps[n-1]) / u[n-1]: the first half places the path emissivity against the
+// row before any search (it starts below the rows and saturates above them),
+// the second is read where a column leaves the row.  CGA records are 16
+// bytes, {n, 0, u[0], eps[0]}: a column above a row brackets at n-2, and the
 // search brings the row's last entries.
-// With the temperature weights precomputed (PRE) a row's temperature is not
-// needed: EGA then reads only the count n of the second half of the record.
-template <bool CGA, bool PRE = false>
-__device__ __forceinline__ RowF rowf_at(const TblDev& T, unsigned r) {
-  RowF w;
-  w.off = r * (unsigned)T.tu;
-  if (CGA) {
-    const float4 m = __ldg(T.rowmeta + r);
-    w.n = __float_as_int(m.x);
-    w.t = m.y;
-    w.u0 = m.z;
-    w.e0 = m.w;
-    w.un = w.en = 0.f;
-  } else {
-    const float4 m = __ldg(T.rowmeta + 2 * r);
-    if (PRE) {
-      w.n = __ldg(reinterpret_cast<const int*>(T.rowmeta + 2 * r + 1));
-      w.t = 0.f;
-    } else {
-      const float4 m2 = __ldg(T.rowmeta + 2 * r + 1);
-      w.n = __float_as_int(m2.x);
-      w.t = m2.y;
-    }
-    w.u0 = m.x;
-    w.un = m.y;
-    w.e0 = m.z;
-    w.en = m.w;
-  }
-  return w;
-}
+// kOddRow in n marks a row that falls somewhere or whose columns reach 2^125:
+// such rows take corner_odd (full-range divisions, no assumption on the
+// order), the others divide by __fdividef, which gives the bits of the
+// full-range division for divisors below 2^126 in a quarter of its
+// instructions.
+// Where results of several kernels must agree to the bit, sums of products
+// name their fused form; left to the compiler it depends on the block that a
+// value is used in.
 
 // A bracket index i with the grid values at i and i + 1.
 struct Bracket {
@@ -165,6 +137,11 @@ __device__ __forceinline__ Bracket2 hunt2(const float2* g, int n, float x, int h
   return Bracket2{i, __ldg(g + i), __ldg(g + i + 1)};
 }
 
+// Emissivity between the entries a and b {u, eps} at column u (LIN).
+__device__ __forceinline__ float between(float2 a, float2 b, float u) {
+  return __fmaf_rn(__fdividef(__fsub_rn(b.y, a.y), __fsub_rn(b.x, a.x)), __fsub_rn(u, a.x), a.y);
+}
+
 // Emissivity of one table row (corner of the p-T cell) for the extended
 // path: EGA u = intpol_tbl_u(e_path) + du, CGA u = ucg; then
 // intpol_tbl_eps(u) (jurassic.c:3799-3891, 3895-3967).  In EGA the bracket
@@ -174,54 +151,91 @@ __device__ __forceinline__ Bracket2 hunt2(const float2* g, int n, float x, int h
 // The bracket is the same either way, so the value is too.  h is the
 // search hint carried along the path: of the emissivity-row search in EGA,
 // of the column-row search in CGA (EGA's column search starts from the
-// emissivity bracket, or from the row start below the table).
+// emissivity bracket, or from the row start below the table).  m: the first
+// half of the row's record.
 template <bool CGA>
-__device__ __forceinline__ float corner_eps(const TblDev& T, const RowF& r, float e_path, float du,
-                                            float ucg, unsigned short& h) {
-  const float2* row = T.ue + r.off;
+__device__ __forceinline__ float corner_eps(const TblDev& T, unsigned r, const float4 m,
+                                            float e_path, float du, float ucg,
+                                            unsigned short& h) {
+  const float2* row = T.ue + r * (unsigned)T.tu;
   if (CGA) {  // intpol_tbl_eps(ucg), the row's last entries from the search
+    const int n = __float_as_int(m.x);
     const float uc = ucg;
-    if (uc < r.u0) return r.e0 / r.u0 * uc;
-    const Bracket2 k = hunt2<0>(row, r.n, uc, h);
+    if (uc < m.z) return __fdividef(m.w, m.z) * uc;
+    const Bracket2 k = hunt2<0>(row, n, uc, h);
     h = (unsigned short)k.i;
     if (uc > k.b.x) {
-      const float a = log1pf(-k.b.y) / k.b.x;
+      const float a = __fdividef(log1pf(-k.b.y), k.b.x);
       return -expm1f(a * uc);
     }
-    return k.a.y + (k.b.y - k.a.y) / (k.b.x - k.a.x) * (uc - k.a.x);
+    return between(k.a, k.b, uc);
   }
+  const float2* rec = reinterpret_cast<const float2*>(T.rowmeta + 2 * r + 1);  // {u[n-1], a}
+  const int n = __float_as_int(m.w);
   float uq;
-  int ib = -1;
-  float u_lo = 0.f, u_hi = 0.f, e_lo = 0.f, e_hi = 0.f;
-  if (CGA) {
-    uq = ucg;
+  int ib = 0;
+  if (e_path < m.y) {
+    uq = __fadd_rn(__fmul_rn(__fdividef(m.x, m.y), e_path), du);
+    if (uq < m.x) return __fdividef(m.y, m.x) * uq;
+  } else if (e_path > m.z) {
+    uq = __fadd_rn(__fdividef(log1pf(-e_path), __ldg(rec).y), du);
   } else {
-    if (e_path < r.e0) {
-      uq = r.u0 / r.e0 * e_path;
-    } else if (e_path > r.en) {
-      const float a = log1pf(-r.en) / r.un;
-      uq = log1pf(-e_path) / a;
-    } else {
-      const Bracket2 k = hunt2<1>(row, r.n, e_path, h);
-      h = (unsigned short)k.i;
-      ib = k.i;
-      e_lo = k.a.y;
-      e_hi = k.b.y;
-      u_lo = k.a.x;
-      u_hi = k.b.x;
-      uq = u_lo + (u_hi - u_lo) / (e_hi - e_lo) * (e_path - e_lo);
-    }
-    uq = uq + du;
+    const Bracket2 k = hunt2<1>(row, n, e_path, h);
+    h = (unsigned short)k.i;
+    ib = k.i;
+    uq = __fadd_rn(__fmaf_rn(__fdividef(__fsub_rn(k.b.x, k.a.x), __fsub_rn(k.b.y, k.a.y)),
+                             __fsub_rn(e_path, k.a.y), k.a.x), du);
+    if (uq >= k.a.x && uq < k.b.x)
+      return between(k.a, k.b, uq);
   }
-  if (uq < r.u0) return r.e0 / r.u0 * uq;
-  if (uq > r.un) {
-    const float a = log1pf(-r.en) / r.un;
+  if (uq < m.x) return __fdividef(m.y, m.x) * uq;
+  const float2 top = __ldg(rec);
+  if (uq > top.x) return -expm1f(top.y * uq);
+  const Bracket2 k = hunt2<0>(row, n, uq, ib);
+  return between(k.a, k.b, uq);
+}
+
+// The same for a row marked kOddRow.
+template <bool CGA>
+__device__ __noinline__ float corner_odd(const float2* row, int n, float e_path, float du,
+                                         float ucg, unsigned short* h) {
+  n &= ~kOddRow;
+  const float2 first = __ldg(row), last = __ldg(row + n - 1);
+  if (CGA) {
+    if (ucg < first.x) return first.y / first.x * ucg;
+    const Bracket2 k = hunt2<0>(row, n, ucg, *h);
+    *h = (unsigned short)k.i;
+    if (ucg > k.b.x) {
+      const float a = log1pf(-k.b.y) / k.b.x;
+      return -expm1f(a * ucg);
+    }
+    return k.a.y + (k.b.y - k.a.y) / (k.b.x - k.a.x) * (ucg - k.a.x);
+  }
+  float uq, u_lo = 0.f, u_hi = 0.f, e_lo = 0.f, e_hi = 0.f;
+  int ib = -1;
+  if (e_path < first.y) {
+    uq = __fmul_rn(first.x / first.y, e_path);
+  } else if (e_path > last.y) {
+    const float a = log1pf(-last.y) / last.x;
+    uq = log1pf(-e_path) / a;
+  } else {
+    const Bracket2 k = hunt2<1>(row, n, e_path, *h);
+    *h = (unsigned short)k.i;
+    ib = k.i;
+    e_lo = k.a.y;
+    e_hi = k.b.y;
+    u_lo = k.a.x;
+    u_hi = k.b.x;
+    uq = u_lo + (u_hi - u_lo) / (e_hi - e_lo) * (e_path - e_lo);
+  }
+  uq = __fadd_rn(uq, du);
+  if (uq < first.x) return first.y / first.x * uq;
+  if (uq > last.x) {
+    const float a = log1pf(-last.y) / last.x;
     return -expm1f(a * uq);
   }
-  if (!CGA && ib >= 0 && uq >= u_lo && uq < u_hi)
-    return e_lo + (e_hi - e_lo) / (u_hi - u_lo) * (uq - u_lo);
-  const Bracket2 k = hunt2<0>(row, r.n, uq, CGA ? (int)h : (ib >= 0 ? ib : 0));
-  if (CGA) h = (unsigned short)k.i;
+  if (ib >= 0 && uq >= u_lo && uq < u_hi) return e_lo + (e_hi - e_lo) / (u_hi - u_lo) * (uq - u_lo);
+  const Bracket2 k = hunt2<0>(row, n, uq, max(ib, 0));
   return k.a.y + (k.b.y - k.a.y) / (k.b.x - k.a.x) * (uq - k.a.x);
 }
 
@@ -340,8 +354,7 @@ __device__ __forceinline__ Bracket pbracket_f(const float* g, int n, float x, in
 constexpr int kStateWords = 5;  // t, e, ipr, 2 words of 16-bit corner hints
 constexpr float kTauStop = 1e-12f;  // path transmittance below which the walk stops
 constexpr int kChanConsts = 16;  // constants of a warp's channel
-constexpr int kThreadFloats = 2;  // per-thread values kept in shared memory
-constexpr int kPathThreads = 128;  // threads of a path block: 4 warps = 4 channels
+constexpr int kPathThreads = 128;  // threads of a path block
 
 // Per (channel, emitter) state carried along the path: transmittance t and
 // emissivity e of the extended path (each accurate where it is small), the
@@ -351,6 +364,86 @@ struct GasState {
   int ipr;
   unsigned short h[4];
 };
+
+// Interpolations of the cell's corners in temperature and pressure.
+__device__ __forceinline__ float mix_f(float y0, float y1, float w) {
+  return __fmaf_rn(__fsub_rn(y1, y0), w, y0);
+}
+
+// The path's emissivity becomes e: the segment's emissivity; *sat is set where
+// the reference's segment transmittance becomes zero.
+__device__ __forceinline__ float extend_f(float e, GasState& s, bool& sat) {
+  e = fminf(fmaxf(e, 0.f), 1.f);
+  const float te = __fsub_rn(1.f, e);  // exact for e >= 0.5
+  const float rt = __fdividef(1.f, s.t);
+  const float eps = (s.e < 0.5f) ? __fmul_rn(__fsub_rn(e, s.e), rt) : __fmaf_rn(-te, rt, 1.f);
+  if (e >= 1.f) sat = true;
+  s.t = te;
+  s.e = e;
+  return eps;
+}
+
+// The p-T cell of one LOS point in table dg: rows ra, ra + 1 at the lower
+// pressure, rc, rc + 1 at the upper one, and the weights in pressure (w) and
+// temperature (a, b).
+struct CellF {
+  unsigned ra, rc;
+  float w, a, b;
+  bool ok;
+};
+
+// From the precomputed words (grids shared by all channels) ...
+__device__ __forceinline__ CellF cell_packed(const TblDev& T, long long dg, unsigned brw, float w,
+                                             float a, float b) {
+  const unsigned rb = (unsigned)dg * (unsigned)(T.tp * T.tt);
+  return CellF{rb + (brw & 0xffffu), rb + (brw >> 16), w, a, b, (brw & kNoBracket) == 0u};
+}
+
+// ... or found here, the pressure bracket from the last one (ipr).  The
+// temperature interpolation is then e00 + (e01 - e00) / (t1 - t0) (t - t0).
+struct CellFind {
+  CellF k;
+  float ta, tb, tc, td;
+};
+template <bool CGA>
+__device__ __forceinline__ CellFind cell_find(const TblDev& T, long long dg, int np, float pq,
+                                              float tq, int& ipr) {
+  CellFind f{};
+  const Bracket pb = pbracket_f(T.pf + dg * T.tp, np, pq, ipr);
+  ipr = pb.i;
+  const int* ntg = T.nt + dg * T.tp;
+  const int nt0 = __ldg(ntg + ipr), nt1 = __ldg(ntg + ipr + 1);
+  if (nt0 < 2 || nt1 < 2) return f;
+  const int it0 = bracket_regf(T.tf + (dg * T.tp + ipr) * T.tt, nt0, tq);
+  const int it1 = bracket_regf(T.tf + (dg * T.tp + ipr + 1) * T.tt, nt1, tq);
+  const unsigned rp = (unsigned)dg * (unsigned)T.tp + (unsigned)ipr;
+  f.k.ra = rp * (unsigned)T.tt + (unsigned)it0;
+  f.k.rc = (rp + 1u) * (unsigned)T.tt + (unsigned)it1;
+  f.k.ok = true;
+  f.ta = __ldg(T.tf + f.k.ra);
+  f.tb = __ldg(T.tf + f.k.ra + 1);
+  f.tc = __ldg(T.tf + f.k.rc);
+  f.td = __ldg(T.tf + f.k.rc + 1);
+  if (CGA && pq / pb.a > 0.f && pb.b / pb.a > 0.f)
+    f.k.w = __logf(pq / pb.a) / __logf(pb.b / pb.a);
+  else
+    f.k.w = (pq - pb.a) / (pb.b - pb.a);
+  return f;
+}
+
+// Temperature interpolation with the division in place.
+__device__ __forceinline__ float mix_t(float y0, float y1, float t0, float t1, float t) {
+  return __fmaf_rn(__fsub_rn(y1, y0) / __fsub_rn(t1, t0), __fsub_rn(t, t0), y0);
+}
+
+template <bool CGA>
+__device__ __forceinline__ float4 row_record(const TblDev& T, unsigned r) {
+  return __ldg(T.rowmeta + (CGA ? r : 2 * r));
+}
+template <bool CGA>
+__device__ __forceinline__ int row_count(const float4 m) {
+  return __float_as_int(CGA ? m.x : m.w);
+}
 
 // One (channel, emitter) at one LOS point (intpol_tbl_ega / intpol_tbl_cga,
 // jurassic.c:3710-3891).  Returns the segment emissivity; *sat is set where
@@ -363,10 +456,8 @@ __device__ __forceinline__ float gas_eps_f(const TblDev& T, long long dg, float 
                                            float tq, float du, float ucg, unsigned brw,
                                            float wpre, float wta, float wtb, GasState& s,
                                            bool& sat) {
-  constexpr bool cga = CGA;
   const bool pre = brw != (kNoBracket | 1u);
   if (pre && brw == kNoBracket) return 0.f;   // np < 30
-  const float* pg = T.pf + dg * T.tp;
   int np = 0;
   if (!pre) {
     np = __ldg(T.np + dg);
@@ -378,64 +469,202 @@ __device__ __forceinline__ float gas_eps_f(const TblDev& T, long long dg, float 
     sat = true;
     return 1.f;
   }
-  unsigned ra, rc;
-  float pa = 0.f, pb = 0.f;
-  if (pre) {
-    if (brw & kNoBracket) return 0.f;         // nt < 2 at this pressure
-    const unsigned rb = (unsigned)dg * (unsigned)(T.tp * T.tt);
-    ra = rb + (brw & 0xffffu);
-    rc = rb + (brw >> 16);
+  CellFind f{};
+  if (pre) f.k = cell_packed(T, dg, brw, wpre, wta, wtb);
+  else f = cell_find<CGA>(T, dg, np, pq, tq, s.ipr);
+  if (!f.k.ok) return 0.f;                    // nt < 2 at this pressure
+  const unsigned ra = f.k.ra, rc = f.k.rc;
+  const float4 m00 = row_record<CGA>(T, ra), m01 = row_record<CGA>(T, ra + 1u);
+  const float4 m10 = row_record<CGA>(T, rc), m11 = row_record<CGA>(T, rc + 1u);
+  const int n00 = row_count<CGA>(m00), n01 = row_count<CGA>(m01);
+  const int n10 = row_count<CGA>(m10), n11 = row_count<CGA>(m11);
+  if (min(min(n00, n01), min(n10, n11)) < 2) return 0.f;
+  float e00, e01, e10, e11;
+  if ((n00 | n01 | n10 | n11) & kOddRow) {
+    const unsigned tu = (unsigned)T.tu;
+    e00 = corner_odd<CGA>(T.ue + ra * tu, n00, s.e, du, ucg, &s.h[0]);
+    e01 = corner_odd<CGA>(T.ue + (ra + 1u) * tu, n01, s.e, du, ucg, &s.h[1]);
+    e10 = corner_odd<CGA>(T.ue + rc * tu, n10, s.e, du, ucg, &s.h[2]);
+    e11 = corner_odd<CGA>(T.ue + (rc + 1u) * tu, n11, s.e, du, ucg, &s.h[3]);
   } else {
-    const int* ntg = T.nt + dg * T.tp;
-    const Bracket pb_ = pbracket_f(pg, np, pq, s.ipr);
-    const int ipr = pb_.i;
-    s.ipr = ipr;
-    pa = pb_.a;
-    pb = pb_.b;
-    const int nt0 = __ldg(ntg + ipr), nt1 = __ldg(ntg + ipr + 1);
-    if (nt0 < 2 || nt1 < 2) return 0.f;
-    const int it0 = bracket_regf(T.tf + (dg * T.tp + ipr) * T.tt, nt0, tq);
-    const int it1 = bracket_regf(T.tf + (dg * T.tp + ipr + 1) * T.tt, nt1, tq);
-    const unsigned rp = (unsigned)dg * (unsigned)T.tp + (unsigned)ipr;
-    ra = rp * (unsigned)T.tt + (unsigned)it0;
-    rc = (rp + 1u) * (unsigned)T.tt + (unsigned)it1;
+    e00 = corner_eps<CGA>(T, ra, m00, s.e, du, ucg, s.h[0]);
+    e01 = corner_eps<CGA>(T, ra + 1u, m01, s.e, du, ucg, s.h[1]);
+    e10 = corner_eps<CGA>(T, rc, m10, s.e, du, ucg, s.h[2]);
+    e11 = corner_eps<CGA>(T, rc + 1u, m11, s.e, du, ucg, s.h[3]);
   }
-  float ea, eb, w;
-  if (pre) {
-    const RowF r00 = rowf_at<CGA, true>(T, ra), r01 = rowf_at<CGA, true>(T, ra + 1u);
-    const RowF r10 = rowf_at<CGA, true>(T, rc), r11 = rowf_at<CGA, true>(T, rc + 1u);
-    if (r00.n < 2 || r01.n < 2 || r10.n < 2 || r11.n < 2) return 0.f;
-    const float e00 = corner_eps<CGA>(T, r00, s.e, du, ucg, s.h[0]);
-    const float e01 = corner_eps<CGA>(T, r01, s.e, du, ucg, s.h[1]);
-    const float e10 = corner_eps<CGA>(T, r10, s.e, du, ucg, s.h[2]);
-    const float e11 = corner_eps<CGA>(T, r11, s.e, du, ucg, s.h[3]);
-    ea = e00 + (e01 - e00) * wta;
-    eb = e10 + (e11 - e10) * wtb;
-    w = wpre;
-  } else {
-    const RowF r00 = rowf_at<CGA>(T, ra), r01 = rowf_at<CGA>(T, ra + 1u);
-    const RowF r10 = rowf_at<CGA>(T, rc), r11 = rowf_at<CGA>(T, rc + 1u);
-    if (r00.n < 2 || r01.n < 2 || r10.n < 2 || r11.n < 2) return 0.f;
-    const float e00 = corner_eps<CGA>(T, r00, s.e, du, ucg, s.h[0]);
-    const float e01 = corner_eps<CGA>(T, r01, s.e, du, ucg, s.h[1]);
-    const float e10 = corner_eps<CGA>(T, r10, s.e, du, ucg, s.h[2]);
-    const float e11 = corner_eps<CGA>(T, r11, s.e, du, ucg, s.h[3]);
-    const float ta = r00.t, tb = r01.t, tc = r10.t, td = r11.t;
-    ea = e00 + (e01 - e00) / (tb - ta) * (tq - ta);
-    eb = e10 + (e11 - e10) / (td - tc) * (tq - tc);
-    if (cga && pq / pa > 0.f && pb / pa > 0.f)
-      w = __logf(pq / pa) / __logf(pb / pa);
-    else
-      w = (pq - pa) / (pb - pa);
+  const float ea = pre ? mix_f(e00, e01, wta) : mix_t(e00, e01, f.ta, f.tb, tq);
+  const float eb = pre ? mix_f(e10, e11, wtb) : mix_t(e10, e11, f.tc, f.td, tq);
+  return extend_f(mix_f(ea, eb, f.k.w), s, sat);
+}
+
+// Per-channel constants of the path in FP32 (chanf[id * kChanConsts]): nu,
+// CO2 296/260/230 K, H2O 296 K, log of its 260/296 K ratio, foreign, N2 B and
+// beta, O2 B and beta, then the continua of the channel as bits (1 CO2, 2 H2O,
+// 4 N2, 8 O2) and the window.
+constexpr int kChanSwitches = 11, kChanWindow = 12;
+
+__global__ void k_chan_consts(CtlDev c, ChanDev ch, float* out) {
+  const int id = blockIdx.x * blockDim.x + threadIdx.x;
+  if (id >= c.nd) return;
+  const double* cc = ch.ctm + (long long)id * kCtmStride;
+  float* k = out + id * kChanConsts;
+  k[0] = (float)ch.nu[id];
+  k[1] = (float)cc[1];
+  k[2] = (float)cc[2];
+  k[3] = (float)cc[3];
+  k[4] = (float)cc[5];
+  k[5] = (float)log(cc[6] > 0 ? cc[6] : 1.0);
+  k[6] = (float)cc[7];
+  k[7] = (float)cc[9];
+  k[8] = (float)cc[10];
+  k[9] = (float)cc[12];
+  k[10] = (float)cc[13];
+  const int on = (c.ig_co2 >= 0 && cc[0] != 0 ? 1 : 0) | (c.ig_h2o >= 0 && cc[4] != 0 ? 2 : 0) |
+                 (cc[8] != 0 ? 4 : 0) | (cc[11] != 0 ? 8 : 0);
+  k[kChanSwitches] = __int_as_float(on);
+  k[kChanWindow] = __int_as_float(c.nw > 0 ? ch.window[id] : 0);
+}
+
+// The channel's continua that the control set has on.
+__device__ __forceinline__ int continua_on(const CtlDev& c, float bits) {
+  return __float_as_int(bits) & ((c.ctm_co2 ? 1 : 0) | (c.ctm_h2o ? 2 : 0) | (c.ctm_n2 ? 4 : 0) |
+                                 (c.ctm_o2 ? 8 : 0));
+}
+
+// Extinction of a segment by the continua (ctmco2, ctmh2o, ctmn2, ctmo2)
+// added to beta; kc: the channel's constants, f: the point's fields.
+template <typename K>
+__device__ __forceinline__ float continua_f(const CtlDev& c, const Fields& F, K kc, int on,
+                                            const float* f, float p, float t, float ds,
+                                            float beta) {
+  const float pr = p / (float)kP0;
+  if (on & 1) {
+    const float co2_296 = kc[1], co2_260 = kc[2], co2_230 = kc[3];
+    const float d230 = t - 230.f, d260 = t - 260.f, d296 = t - 296.f;
+    const float ctw = d260 * 5.050505e-4f * d296 * co2_230 - d230 * 9.259259e-4f * d296 * co2_260 +
+                      d230 * 4.208754e-4f * d260 * co2_296;
+    const float uco2 = f[(F.g0 + c.ig_co2 * F.es + kFU) * 32];
+    beta += __fdividef(uco2, ds) * (float)(1.0 / (kNA * 1000.0)) * pr * ctw;
   }
-  float e = ea + (eb - ea) * w;
-  e = fminf(fmaxf(e, 0.f), 1.f);
-  const float te = 1.f - e;  // exact for e >= 0.5
-  const float eps = (s.e < 0.5f) ? (e - s.e) / s.t : 1.f - te / s.t;
-  if (e >= 1.f) sat = true;
-  s.t = te;
-  s.e = e;
-  return eps;
+  if (on & 2) {
+    const float q = f[F.qh2o * 32];
+    const float uh = f[(F.g0 + c.ig_h2o * F.es + kFU) * 32];
+    const float nu = kc[0], h2o_s296 = kc[4], h2o_lr = kc[5], h2o_frn = kc[6];
+    const float self = h2o_s296 * __expf(h2o_lr * (296.f - t) * (1.f / 36.f));
+    const float a1 = nu * (__fdividef(uh, ds) * 1e-20f) * tanhf(__fdividef(.7193876f, t) * nu);
+    beta += a1 * __fdividef(296.f, t) * pr * (q * self + (1.f - q) * h2o_frn);
+  }
+  if (on & 12) {
+    const float n2_b = kc[7], n2_beta = kc[8], o2_b = kc[9], o2_beta = kc[10];
+    const float x = __fdividef(pr * 273.f, t);
+    const float x2 = 0.1f * x * x;
+    if (on & 4)
+      beta += x2 * __expf(n2_beta * (1.f / 296.f - 1.f / t)) * 0.79f * n2_b *
+              (0.79f + 0.21f * (1.294f - 0.4545f * t / 296.f));
+    if (on & 8) beta += x2 * __expf(o2_beta * (1.f / 296.f - 1.f / t)) * 0.21f * o2_b;
+  }
+  return beta;
+}
+
+// Source function (formod_srcfunc) of a channel's table at temperature t.
+__device__ __forceinline__ float source_f(const float* srf, float t) {
+  const float st0 = (float)kTMIN, sdt = (float)((kTMAX - kTMIN) / (kNS - 1.0));
+  const float xs = (t - st0) / sdt;
+  int is = (int)xs;
+  is = is < 0 ? 0 : (is > kNS - 2 ? kNS - 2 : is);
+  const float s0 = __ldg(srf + is), s1 = __ldg(srf + is + 1);
+  return s0 + (s1 - s0) * (xs - (float)is);
+}
+
+// Emissivity of a segment from the emitters' E, the extinction beta and the
+// length.
+__device__ __forceinline__ float segment_f(float E, float beta, float ds) {
+  return E + (1.f - E) * (-expm1f(-beta * ds));
+}
+
+// E of a segment joined with another emitter's emissivity.
+__device__ __forceinline__ float join_f(float E, float eg) {
+  return __fmaf_rn(__fsub_rn(1.f, E), eg, E);
+}
+
+// One segment (v = src * eps, m = 1 - eps) added to the Kahan-compensated
+// radiance sum and the path transmittance.
+__device__ __forceinline__ void add_f(float v, float m, float& rad, float& comp, float& tau) {
+  const float y = __fmaf_rn(v, tau, -comp);
+  const float sum = __fadd_rn(rad, y);
+  comp = __fsub_rn(__fsub_rn(sum, rad), y);
+  rad = sum;
+  tau = __fmul_rn(tau, m);
+}
+
+// Cloud extinction and surface emissivity of a (ray, channel).
+__device__ __forceinline__ float cloud_of(const CtlDev& c, const ChanDev& ch, const BatchDev& b,
+                                          int r, int id, bool* has) {
+  const double* s = b.scal + (long long)b.ray_obs[r] * b.nscal;
+  *has = c.ncl > 0 && s[1] > 0;
+  if (!*has) return 0.f;
+  const double nu = ch.nu[id];
+  const int icl = bracket_irr(ch.clnu, c.ncl, nu);
+  return (float)lin(ch.clnu[icl], s[2 + icl], ch.clnu[icl + 1], s[2 + icl + 1], nu);
+}
+
+__device__ __forceinline__ float sfeps_of(const CtlDev& c, const ChanDev& ch, const BatchDev& b,
+                                          int r, int id) {
+  if (c.nsf <= 0) return 1.f;
+  const double* se = b.scal + (long long)b.ray_obs[r] * b.nscal + 5 + c.ncl;
+  const double nu = ch.nu[id];
+  const int isf = bracket_irr(ch.sfnu, c.nsf, nu);
+  return (float)lin(ch.sfnu[isf], se[isf], ch.sfnu[isf + 1], se[isf + 1], nu);
+}
+
+// Surface emission, reflection and solar term (jurassic.c:3264-3328), BT
+// conversion and mask.  seg: the n segments {src * eps, 1 - eps} step apart
+// where the surface reflects, else nullptr.
+__device__ __forceinline__ void write_radiance(const CtlDev& c, const TblDev& T, const ChanDev& ch,
+                                               const BatchDev& b, const LosDev& L, int id, int r,
+                                               float rad, float tau, const float* seg,
+                                               long long step, int n) {
+  const double nu = ch.nu[id];
+  double radd = (double)rad;
+  const double sft = L.sft[r];
+  if (c.sftype >= 1 && sft > 0) {
+    const float sfeps = sfeps_of(c, ch, b, r, id);
+    const float ssf = source_f(T.srf + (long long)id * kNS, (float)sft);
+    radd += (double)(sfeps * ssf * tau);
+    if (seg) {
+      float tr = 1.f;
+      double acc = 0;
+      for (int ip = n - 1; ip >= 0; ip--) {
+        acc += (double)(seg[ip * step] * tr);
+        tr *= seg[ip * step + 32];
+      }
+      radd += acc * (double)tau * (double)(1.f - sfeps);
+      if (c.sftype >= 3) {
+        const double* e6 = L.ends + 6LL * r;
+        const double sza2 = c.sfsza < 0 ? solar_zenith(b.geo[r], e6[4], e6[5]) : c.sfsza;
+        if (sza2 < 89.999) {
+          double x0[3], x1[3];
+          to_cart(e6[3], e6[4], e6[5], x0);
+          to_cart(e6[0], e6[1], e6[2], x1);
+          for (int i = 0; i < 3; i++) x1[i] -= x0[i];
+          const double cosa = (x0[0] * x1[0] + x0[1] * x1[1] + x0[2] * x1[2]) /
+                              sqrt(x0[0] * x0[0] + x0[1] * x0[1] + x0[2] * x0[2]) /
+                              sqrt(x1[0] * x1[0] + x1[1] * x1[1] + x1[2] * x1[2]);
+          const double rcos = cosa / cos(sza2 * (kPI / 180.0));
+          radd += 6.764e-5 / (2. * kPI) * planck(kTSUN, nu) * tr * (1 - sfeps) * tau * rcos;
+        }
+      }
+    }
+  }
+  const long long oi = (long long)id * b.nray + r;
+  if (c.fov) {  // pencil beam only: FOV convolution, BT and mask follow in k_fov
+    b.rad[oi] = radd;
+    b.tau[oi] = (double)tau;
+    return;
+  }
+  if (c.write_bbt) radd = kC2 * nu / log1p(kC1 * (nu * nu * nu) / radd);
+  b.rad[oi] = b.mask[oi] ? __longlong_as_double(0x7ff8000000000000LL) : radd;
+  b.tau[oi] = (double)tau;
 }
 
 // The emitter loop runs over a runtime count with the per-emitter state in
@@ -444,96 +673,45 @@ __device__ __forceinline__ float gas_eps_f(const TblDev& T, long long dg, float 
 // enough warps resident to hide load latency, and thread-local arrays spill
 // through L1 into L2.
 // MINB is the minimum number of resident blocks per SM requested from the
-// register allocator (1 = no cap); the variants are chosen by the autotuner.
-// SPLIT: the emitters' segment emissivities come from k_path_gas (P.seg_eps,
-// P.seg_sat) instead of being computed here; everything else is this same
-// code, so both forms give the same results.
-// RESUME: rays start at P.start[r] from a saved state and save states for
-// other rays (finite-difference perturbations that leave a path prefix
-// unchanged); the arithmetic of every point is the same.
-template <int MINB, bool CGA, bool SPLIT = false, bool RESUME = false, bool SHARE = false,
-          int NT = kPathThreads>
-__global__ void __launch_bounds__(NT, MINB) k_path_mixed(CtlDev c, TblDev T, ChanDev ch,
-                                                          BatchDev b, LosDev L, MixedPlan P,
-                                                          float* refl) {
+// register allocator.  This form (all emitters of a point in one warp, sums
+// along the way) serves the resumed batches of finite-difference
+// perturbations: rays start at P.start[r] from a saved state and save states
+// for other rays that share a path prefix.  Other batches take k_gas_m,
+// k_seg_m and k_scan_m, whose arithmetic per point is the same.
+template <int MINB, bool CGA, bool SHARE>
+__global__ void __launch_bounds__(kPathThreads, MINB) k_path_mixed(CtlDev c, TblDev T, ChanDev ch,
+                                                                   BatchDev b, LosDev L,
+                                                                   MixedPlan P) {
+  constexpr int nth = kPathThreads;
   const int ng = c.ng;
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
-  constexpr int W = NT / 32;  // warps of a block
-  int tile, id;
-  if (P.tile_major) {  // one channel of W consecutive tiles
-    tile = P.tile0 + (int)(blockIdx.x / c.nd) * W + warp;
-    id = (int)(blockIdx.x % c.nd);
-  } else {             // W channels of one tile
-    const int nchb = (c.nd + W - 1) / W;
-    tile = P.tile0 + blockIdx.x / nchb;
-    id = (blockIdx.x % nchb) * W + warp;
-  }
-  if (tile >= P.tile1 || id >= c.nd) return;
+  constexpr int W = nth / 32;  // warps of a block
+  // one channel of W consecutive tiles: the perturbations of one observation
+  // share table rows
+  const int tile = P.tile0 + (int)(blockIdx.x / c.nd) * W + warp;
+  const int id = (int)(blockIdx.x % c.nd);
+  if (tile >= P.tile1) return;
   int r = P.perm[tile * 32 + lane];
   if (r >= 0 && b.obs_skip && b.obs_skip[b.ray_obs[r]]) r = -1;  // lane idle, outputs untouched
   const bool skip = r >= 0 && b.skip_masked && b.mask[(long long)id * b.nray + r];
   const int n = r >= 0 && !skip ? L.count[r] : 0;
   const Fields F = fields_of(c, P.brmask);
   const float* base = P.data + P.toff[tile] * (long long)F.n * 32 + lane;
-  constexpr bool cga = CGA;
-  const double nud = ch.nu[id];
-  const float nu = (float)nud;
-
-  // per-(observation, channel) constants
-  float cloud = 0.f, sfeps = 1.f;
-  bool has_cloud = false;
-  if (r >= 0) {
-    const double* s = b.scal + (long long)b.ray_obs[r] * b.nscal;
-    has_cloud = c.ncl > 0 && s[1] > 0;
-    if (has_cloud) {
-      const int icl = bracket_irr(ch.clnu, c.ncl, nud);
-      cloud = (float)lin(ch.clnu[icl], s[2 + icl], ch.clnu[icl + 1], s[2 + icl + 1], nud);
-    }
-    if (c.nsf > 0) {
-      const double* se = s + 5 + c.ncl;
-      const int isf = bracket_irr(ch.sfnu, c.nsf, nud);
-      sfeps = (float)lin(ch.sfnu[isf], se[isf], ch.sfnu[isf + 1], se[isf + 1], nud);
-    }
-  }
-  const int w = c.nw > 0 ? ch.window[id] : 0;
-  const double* cc = ch.ctm + (long long)id * kCtmStride;
-  const bool co2_on = c.ctm_co2 && c.ig_co2 >= 0 && cc[0] != 0;
-  const bool h2o_on = c.ctm_h2o && c.ig_h2o >= 0 && cc[4] != 0;
-  const bool n2_on = c.ctm_n2 && cc[8] != 0;
-  const bool o2_on = c.ctm_o2 && cc[11] != 0;
-  const float st0 = (float)kTMIN, sdt = (float)((kTMAX - kTMIN) / (kNS - 1.0));
 
   // per-emitter path state in shared memory, word-major per thread:
-  // sh[(g * kStateWords + w) * NT + threadIdx.x]
+  // sh[(g * kStateWords + w) * nth + threadIdx.x]
   extern __shared__ unsigned sh_state[];
-  constexpr int nth = NT;
   const int tid = threadIdx.x;
-  // behind the state: the channel's constants (kChanConsts words per warp:
-  // continuum coefficients, [11] channel index, [12] window index) and
-  // kThreadFloats per thread (cloud extinction, surface emissivity), read
-  // where used so that they hold no registers across the emitter loop
+  // behind the state: the channel's constants per warp and each thread's
+  // cloud extinction, read where used so that they hold no registers across
+  // the emitter loop
   float* const sh_tail = reinterpret_cast<float*>(sh_state + kStateWords * nth * (ng > 0 ? ng : 1));
   volatile float* kc = sh_tail + warp * kChanConsts;
-  volatile int* kci = reinterpret_cast<volatile int*>(sh_tail + warp * kChanConsts);
-  volatile float* kthr = sh_tail + (nth / 32) * kChanConsts + tid;  // [0], [nth]
-  if (lane == 0) {
-    kc[0] = nu;
-    kc[1] = (float)cc[1];
-    kc[2] = (float)cc[2];
-    kc[3] = (float)cc[3];
-    kc[4] = (float)cc[5];
-    kc[5] = (float)log(cc[6] > 0 ? cc[6] : 1.0);
-    kc[6] = (float)cc[7];
-    kc[7] = (float)cc[9];
-    kc[8] = (float)cc[10];
-    kc[9] = (float)cc[12];
-    kc[10] = (float)cc[13];
-    kci[11] = id;
-    kci[12] = w;
-  }
-  kthr[0] = cloud;
-  kthr[nth] = sfeps;
+  volatile float* kthr = sh_tail + W * kChanConsts + tid;
+  if (lane < kChanConsts) kc[lane] = T.chanf[id * kChanConsts + lane];
+  bool has_cloud = false;
+  kthr[0] = r >= 0 ? cloud_of(c, ch, b, r, id, &has_cloud) : 0.f;
   __syncwarp();
   // the pressure-bracket word is only used where the bracket is searched
   // here (pre = false); with a precomputed bracket it keeps its initial -1
@@ -560,7 +738,7 @@ __global__ void __launch_bounds__(NT, MINB) k_path_mixed(CtlDev c, TblDev T, Cha
     for (int k = 0; k < 2; k++)
       q[(3 + k) * nth] = (unsigned)st.h[2 * k] | ((unsigned)st.h[2 * k + 1] << 16);
   };
-  for (int g = 0; g < ng && !SPLIT; g++) {
+  for (int g = 0; g < ng; g++) {
     GasState st;
     st.t = 1.f;
     st.e = 0.f;
@@ -569,13 +747,8 @@ __global__ void __launch_bounds__(NT, MINB) k_path_mixed(CtlDev c, TblDev T, Cha
     for (int k = 0; k < 4; k++) st.h[k] = 0;
     sstore(g, st);
   }
-  // split form: segment emissivities of (point, this channel, emitter g) at
-  // seg0 + ip * segstride + g * 32
-  const long long segstride = (long long)c.nd * ng * 32;
-  const long long seg0 = SPLIT ? ((P.toff[tile] * c.nd + id) * ng) * 32 + lane : 0;
   const long long dg0 = (long long)id * ng;
   float rad = 0.f, comp = 0.f, tau = 1.f;
-  const bool do_refl = refl != nullptr && r >= 0 && c.sftype >= 2 && sfeps < 1.f && L.sft[r] > 0;
 
   // resume: the state words of every emitter and rad, comp, tau
   const int sw = kStateWords * ng;
@@ -587,7 +760,7 @@ __global__ void __launch_bounds__(NT, MINB) k_path_mixed(CtlDev c, TblDev T, Cha
     q[sw + 2] = tau;
   };
   int start = 0, sn = 0, se = 0;
-  if (RESUME && n > 0) {
+  if (n > 0) {
     start = P.start[r];
     if (start > 0) {
       const float* q = P.snap + ((long long)r * c.nd + id) * (sw + 3);
@@ -616,22 +789,14 @@ __global__ void __launch_bounds__(NT, MINB) k_path_mixed(CtlDev c, TblDev T, Cha
 
   // resumed lanes join the warp's walk at their own start point: every
   // iteration reads one point of the tile for all lanes (coalesced)
-  int ip0 = start;
-  if (RESUME) {
-    const unsigned wmin = __reduce_min_sync(0xffffffffu, n > 0 ? (unsigned)start : 0xffffffffu);
-    ip0 = wmin == 0xffffffffu ? 0 : (int)wmin;
-  }
-  for (int ip = ip0; ip < n; ip++) {
-    if (RESUME && ip < start) continue;
-    // opaque from here on: the rest of the path adds at most max(src) tau,
-    // below 1e-10 of the radiance (not with surface reflection, whose sum
-    // needs every point)
-    if (tau < kTauStop && !do_refl) {
+  const unsigned wmin = __reduce_min_sync(0xffffffffu, n > 0 ? (unsigned)start : 0xffffffffu);
+  for (int ip = wmin == 0xffffffffu ? 0 : (int)wmin; ip < n; ip++) {
+    if (ip < start) continue;
+    if (tau < kTauStop) {  // opaque from here on (see k_scan_m)
       walked = ip;
       break;
     }
-    if (RESUME)
-      for (; sn < se && P.snap_ip[sn] == ip; sn++) snap_write(P.snap_ray[sn]);
+    for (; sn < se && P.snap_ip[sn] == ip; sn++) snap_write(P.snap_ray[sn]);
     // the base stopped here: the shared emitters continue from its final states
     if (SHARE && rb >= 0 && ip == nvalid) {
       const unsigned* q = P.seg_final + ((long long)rb * c.nd + id) * sw;
@@ -651,29 +816,24 @@ __global__ void __launch_bounds__(NT, MINB) k_path_mixed(CtlDev c, TblDev T, Cha
 #pragma unroll 1
     for (int g = 0; g < ng; g++) {
       float eg;
-      if (SPLIT) {
-        const long long o = seg0 + ip * segstride + g * 32;
-        eg = P.seg_eps[o];
-        if (P.seg_sat[o]) sat = true;
-      } else if (SHARE && shared && g != pg) {
+      if (SHARE && shared && g != pg) {
         eg = P.seg_base[sbase * ng + g];
         if ((satm_in >> g) & 1u) sat = true;
       } else {
         constexpr int es = kEmitterFields(CGA), kb = kFBr(CGA);
         const float* fg = f + (F.g0 + g * es) * 32;
-        const float du = cga ? 0.f : fg[kFU * 32];
-        const float pq = cga ? fg[kFCgp * 32] : p;
-        const float tq = cga ? fg[kFCgt * 32] : t;
-        const float ucg = cga ? fg[kFCgu * 32] : 0.f;
+        const float du = CGA ? 0.f : fg[kFU * 32];
+        const float pq = CGA ? fg[kFCgp * 32] : p;
+        const float tq = CGA ? fg[kFCgt * 32] : t;
+        const float ucg = CGA ? fg[kFCgu * 32] : 0.f;
         const bool brg = (P.brmask >> g) & 1u;
         const unsigned brw = brg ? __float_as_uint(fg[kb * 32]) : (kNoBracket | 1u);
         const float wpre = brg ? fg[(kb + 1) * 32] : 0.f;
         const float wta = brg ? fg[(kb + 2) * 32] : 0.f;
         const float wtb = brg ? fg[(kb + 3) * 32] : 0.f;
         GasState st = sload(g, brg);
-        const long long dg = dg0 + g;  // (channel, emitter)
         bool sg = false;
-        eg = gas_eps_f<CGA>(T, dg, pq, tq, du, ucg, brw, wpre, wta, wtb, st, sg);
+        eg = gas_eps_f<CGA>(T, dg0 + g, pq, tq, du, ucg, brw, wpre, wta, wtb, st, sg);
         sstore(g, st, brg);
         if (sg) sat = true;
         if (SHARE && seg_write) {
@@ -681,224 +841,313 @@ __global__ void __launch_bounds__(NT, MINB) k_path_mixed(CtlDev c, TblDev T, Cha
           if (sg) satm_out |= 1u << g;
         }
       }
-      E = E + (1.f - E) * eg;
+      E = join_f(E, eg);
     }
     if (SHARE && seg_write) P.seg_satm[sbase] = satm_out;
-    // extinction and continua
-    float beta = c.nw > 0 ? f[(F.kw0 + w) * 32] : 0.f;
-    if (has_cloud) beta += f[F.aux * 32] * kthr[0];
-    const float pr = p / (float)kP0;
-    if (co2_on) {
-      const float co2_296 = kc[1], co2_260 = kc[2], co2_230 = kc[3];
-      const float d230 = t - 230.f, d260 = t - 260.f, d296 = t - 296.f;
-      const float ctw = d260 * 5.050505e-4f * d296 * co2_230 - d230 * 9.259259e-4f * d296 * co2_260 +
-                        d230 * 4.208754e-4f * d260 * co2_296;
-      const float uco2 = f[(F.g0 + c.ig_co2 * F.es + kFU) * 32];
-      beta += (uco2 / ds) * (float)(1.0 / (kNA * 1000.0)) * pr * ctw;
-    }
-    if (h2o_on) {
-      const float q = f[F.qh2o * 32];
-      const float uh = f[(F.g0 + c.ig_h2o * F.es + kFU) * 32];
-      const float nu = kc[0], h2o_s296 = kc[4], h2o_lr = kc[5], h2o_frn = kc[6];
-      const float self = h2o_s296 * __expf(h2o_lr * (296.f - t) * (1.f / 36.f));
-      const float a1 = nu * ((uh / ds) * 1e-20f) * tanhf(.7193876f / t * nu);
-      beta += a1 * (296.f / t) * pr * (q * self + (1.f - q) * h2o_frn);
-    }
-    if (n2_on || o2_on) {
-      const float n2_b = kc[7], n2_beta = kc[8], o2_b = kc[9], o2_beta = kc[10];
-      const float x = pr * 273.f / t;
-      const float x2 = 0.1f * x * x;
-      if (n2_on)
-        beta += x2 * __expf(n2_beta * (1.f / 296.f - 1.f / t)) * 0.79f * n2_b *
-                (0.79f + 0.21f * (1.294f - 0.4545f * t / 296.f));
-      if (o2_on) beta += x2 * __expf(o2_beta * (1.f / 296.f - 1.f / t)) * 0.21f * o2_b;
-    }
-    // source function (formod_srcfunc); the channel index is re-read from
-    // shared memory so that the table pointer holds no registers in the loop
-    const float* srf = T.srf + (long long)kci[11] * kNS;
-    const float xs = (t - st0) / sdt;
-    int is = (int)xs;
-    is = is < 0 ? 0 : (is > kNS - 2 ? kNS - 2 : is);
-    const float s0 = __ldg(srf + is), s1 = __ldg(srf + is + 1);
-    const float src = s0 + (s1 - s0) * (xs - (float)is);
-    float eps = 0.f;
     if (!sat) {
-      eps = E + (1.f - E) * (-expm1f(-beta * ds));
-      // Kahan-compensated radiance sum
-      const float y = src * eps * tau - comp;
-      const float tsum = rad + y;
-      comp = (tsum - rad) - y;
-      rad = tsum;
-      tau *= (1.f - eps);
-    }
-    if (do_refl) {
-      float* sc = refl + 2 * (L.off[r] * c.nd);
-      sc[2 * ((long long)ip * c.nd + id)] = src;
-      sc[2 * ((long long)ip * c.nd + id) + 1] = eps;
+      float beta = c.nw > 0 ? f[(F.kw0 + __float_as_int(kc[kChanWindow])) * 32] : 0.f;
+      if (has_cloud) beta = __fmaf_rn(f[F.aux * 32], kthr[0], beta);
+      beta = continua_f(c, F, kc, continua_on(c, kc[kChanSwitches]), f, p, t, ds, beta);
+      const float src = source_f(T.srf + (long long)id * kNS, t);
+      const float eps = segment_f(E, beta, ds);
+      add_f(__fmul_rn(src, eps), __fsub_rn(1.f, eps), rad, comp, tau);
     }
   }
   // states for resume points beyond the end of this walk (a path that became
   // opaque earlier hands its final state on, so the resumed rays stop too)
-  if (RESUME)
-    for (; sn < se; sn++) snap_write(P.snap_ray[sn]);
+  for (; sn < se; sn++) snap_write(P.snap_ray[sn]);
   if (SHARE && seg_write) {  // what a perturbed ray needs past this walk
     P.seg_nvalid[(long long)r * c.nd + id] = walked;
     unsigned* q = P.seg_final + ((long long)r * c.nd + id) * sw;
     for (int k = 0; k < sw; k++) q[k] = sh_state[k * nth + tid];
   }
   if (r < 0) return;
-
-  const double nud2 = ch.nu[id];
-  const float sfeps2 = kthr[nth];
-  const float* srf = T.srf + (long long)id * kNS;
-  double radd = (double)rad;
-  const double sft = L.sft[r];
-  if (c.sftype >= 1 && sft > 0) {
-    const float xs = ((float)sft - st0) / sdt;
-    int is = (int)xs;
-    is = is < 0 ? 0 : (is > kNS - 2 ? kNS - 2 : is);
-    const float s0 = srf[is], s1 = srf[is + 1];
-    const float ssf = s0 + (s1 - s0) * (xs - (float)is);
-    radd += (double)(sfeps2 * ssf * tau);
-    if (do_refl) {
-      const float* sc = refl + 2 * (L.off[r] * c.nd);
-      float tr = 1.f;
-      double acc = 0;
-      for (int ip = n - 1; ip >= 0; ip--) {
-        const float src = sc[2 * ((long long)ip * c.nd + id)];
-        const float e = sc[2 * ((long long)ip * c.nd + id) + 1];
-        acc += (double)(src * e * tr);
-        tr *= (1.f - e);
-      }
-      radd += acc * (double)tau * (double)(1.f - sfeps2);
-      if (c.sftype >= 3) {
-        const double* e6 = L.ends + 6LL * r;
-        // solar zenith angle (sza, jurassic.c:5183-5219) and incidence
-        const double d = b.geo[r] / 86400 - 0.5;
-        const double g = (357.529 + 0.98560028 * d) * (kPI / 180.0);
-        const double qq = 280.459 + 0.98564736 * d;
-        const double l = (qq + 1.915 * sin(g) + 0.020 * sin(2 * g)) * (kPI / 180.0);
-        const double ee = (23.439 - 0.00000036 * d) * (kPI / 180.0);
-        const double dec = asin(sin(ee) * sin(l));
-        const double ra = atan2(cos(ee) * sin(l), cos(l));
-        const double lst = 18.697374558 + 24.06570982441908 * d + e6[4] / 15;
-        const double h = lst / 12 * kPI - ra;
-        const double latr = e6[5] * (kPI / 180.0);
-        const double sza2 = c.sfsza < 0 ? acos(sin(latr) * sin(dec) + cos(latr) * cos(dec) * cos(h)) *
-                                              (180.0 / kPI)
-                                        : c.sfsza;
-        if (sza2 < 89.999) {
-          double x0[3], x1[3];
-          to_cart(e6[3], e6[4], e6[5], x0);
-          to_cart(e6[0], e6[1], e6[2], x1);
-          for (int i = 0; i < 3; i++) x1[i] -= x0[i];
-          const double cosa = (x0[0] * x1[0] + x0[1] * x1[1] + x0[2] * x1[2]) /
-                              sqrt(x0[0] * x0[0] + x0[1] * x0[1] + x0[2] * x0[2]) /
-                              sqrt(x1[0] * x1[0] + x1[1] * x1[1] + x1[2] * x1[2]);
-          const double rcos = cosa / cos(sza2 * (kPI / 180.0));
-          radd += 6.764e-5 / (2. * kPI) * planck(kTSUN, nud2) * tr * (1 - sfeps2) * tau * rcos;
-        }
-      }
-    }
-  }
-  const long long oi = (long long)id * b.nray + r;
-  if (c.fov) {  // pencil beam only: FOV convolution, BT and mask follow in k_fov
-    b.rad[oi] = radd;
-    b.tau[oi] = (double)tau;
-    return;
-  }
-  if (c.write_bbt) radd = kC2 * nud2 / log1p(kC1 * (nud2 * nud2 * nud2) / radd);
-  b.rad[oi] = b.mask[oi] ? __longlong_as_double(0x7ff8000000000000LL) : radd;
-  b.tau[oi] = (double)tau;
+  write_radiance(c, T, ch, b, L, id, r, rad, tau, nullptr, 0, 0);
 }
 
-// Emitter path states of the split form: one warp per (tile, channel,
-// emitter) walks the tile's points with the state of that emitter only and
-// writes every segment emissivity and saturation flag.  The emitters' states
-// are independent along the path (intpol_tbl_ega / intpol_tbl_cga keep one
-// tau_path per emitter); only their combination per point couples them, and
-// that is left to k_path_mixed<..., SPLIT>.  A latency-bound batch (few
-// tiles) so runs ng warps where the fused form runs one.
-template <bool CGA>
-__global__ void __launch_bounds__(128) k_path_gas(CtlDev c, TblDev T, BatchDev b, LosDev L,
-                                                  MixedPlan P) {
-  const int lane = threadIdx.x & 31;
-  const int ng = c.ng;
-  const long long per_tile = (long long)c.nd * ng;
-  const long long wg = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
-  const int tile = (int)(wg / per_tile);
-  if (tile >= P.ntile) return;
-  const int rem = (int)(wg - (long long)tile * per_tile);
-  const int id = rem / ng, g = rem - id * ng;
-  int r = P.perm[tile * 32 + lane];
-  if (r >= 0 && b.obs_skip && b.obs_skip[b.ray_obs[r]]) r = -1;
-  const bool skip = r >= 0 && b.skip_masked && b.mask[(long long)id * b.nray + r];
-  const int n = r >= 0 && !skip ? L.count[r] : 0;
-  const Fields F = fields_of(c, P.brmask);
-  const float* base = P.data + P.toff[tile] * (long long)F.n * 32 + lane;
-  constexpr bool cga = CGA;
+// ---------------------------------------------------------------------------
+// the path of a batch, in three kernels
+//
+// k_gas_m: the emitters' paths are independent (one tau_path per emitter in
+// intpol_tbl_ega / intpol_tbl_cga), so a warp walks a tile's points for one
+// (channel, emitter) with the state in registers and writes the segment
+// emissivities.  LPR = 4 gives each ray four lanes, one per corner of the p-T
+// cell, for batches that leave the device idle.  shape 1: the warps of a
+// block take consecutive tiles of one (channel, emitter), whose rows they
+// share in L1; shape 0: consecutive channels of one tile.
+template <bool CGA, int LPR, int MINB>
+__global__ void __launch_bounds__(kPathThreads, MINB) k_gas_m(CtlDev c, TblDev T, BatchDev b,
+                                                              LosDev L, MixedPlan P, int shape) {
+  constexpr int W = kPathThreads / 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int ng = c.ng, ndc = P.id1 - P.id0;
+  int tl, idl, g, part8 = 0;
+  if (LPR == 4 || shape == 0) {
+    long long w = (long long)blockIdx.x * W + warp;
+    idl = (int)(w % ndc);
+    w /= ndc;
+    g = (int)(w % ng);
+    w /= ng;
+    if (LPR == 4) {
+      part8 = (int)(w & 3);
+      w >>= 2;
+    }
+    tl = (int)w;
+  } else {
+    const unsigned per = (unsigned)(ndc * ng);
+    tl = (int)(blockIdx.x / per) * W + warp;
+    const unsigned rem = blockIdx.x % per;
+    idl = (int)(rem / ng);
+    g = (int)(rem % ng);
+  }
+  if (tl >= P.tile1 - P.tile0) return;
+  const int tile = P.tile0 + tl, id = P.id0 + idl;
   const long long dg = (long long)id * ng + g;
-  const long long segstride = (long long)c.nd * ng * 32;
-  const long long seg0 = ((P.toff[tile] * c.nd + id) * ng + g) * 32 + lane;
+  const int np = __ldg(T.np + dg);
+  if (np < 30) return;  // no table: k_seg_m leaves this emitter out
+  const int rl = LPR == 4 ? part8 * 8 + (lane >> 2) : lane, corner = lane & 3;
+  int r = P.perm[tile * 32 + rl];
+  if (r >= 0 && b.obs_skip && b.obs_skip[b.ray_obs[r]]) r = -1;
+  if (r >= 0 && b.skip_masked && b.mask[(long long)id * b.nray + r]) r = -1;
+  const int n = r >= 0 ? L.count[r] : 0;
+  const Fields F = fields_of(c, P.brmask);
+  constexpr int es = kEmitterFields(CGA), kb = kFBr(CGA);
+  const float* f = P.data + P.toff[tile] * (long long)F.n * 32 + rl;
+  const float* fg = f + (F.g0 + g * es) * 32;
+  const int fstep = F.n * 32;
+  const long long lp0 = P.toff[tile] - P.pt0;
+  float* out = P.seg + ((lp0 * ndc + idl) * P.nseg + g) * 32 + rl;
+  const long long ostep = (long long)ndc * P.nseg * 32;
+  const bool brg = (P.brmask >> g) & 1u;
   GasState st;
   st.t = 1.f;
   st.e = 0.f;
   st.ipr = -1;
 #pragma unroll
   for (int k = 0; k < 4; k++) st.h[k] = 0;
-  const unsigned brbit = (P.brmask >> g) & 1u;
-  for (int ip = 0; ip < n; ip++) {
-    const float* f = base + (long long)ip * F.n * 32;
-    constexpr int es = kEmitterFields(CGA), kb = kFBr(CGA);
-    const float* fg = f + (F.g0 + g * es) * 32;
-    const float du = cga ? 0.f : fg[kFU * 32];
-    const float pq = cga ? fg[kFCgp * 32] : f[F.p * 32];
-    const float tq = cga ? fg[kFCgt * 32] : f[F.t * 32];
-    const float ucg = cga ? fg[kFCgu * 32] : 0.f;
-    const unsigned brw = brbit ? __float_as_uint(fg[kb * 32]) : (kNoBracket | 1u);
-    const float wpre = brbit ? fg[(kb + 1) * 32] : 0.f;
-    const float wta = brbit ? fg[(kb + 2) * 32] : 0.f;
-    const float wtb = brbit ? fg[(kb + 3) * 32] : 0.f;
-    bool sat = false;
-    const float eg = gas_eps_f<CGA>(T, dg, pq, tq, du, ucg, brw, wpre, wta, wtb, st, sat);
-    const long long o = seg0 + ip * segstride;
-    P.seg_eps[o] = eg;
-    P.seg_sat[o] = sat ? 1 : 0;
+  int stop = n;  // the first point that is saturated: all later ones are too
+  if (LPR == 1) {
+    for (int ip = 0; ip < n; ip++) {
+      const float du = CGA ? 0.f : fg[kFU * 32];
+      const float pq = CGA ? fg[kFCgp * 32] : brg ? 0.f : f[F.p * 32];
+      const float tq = CGA ? fg[kFCgt * 32] : brg ? 0.f : f[F.t * 32];
+      const float ucg = CGA ? fg[kFCgu * 32] : 0.f;
+      const unsigned brw = brg ? __float_as_uint(fg[kb * 32]) : (kNoBracket | 1u);
+      const float wpre = brg ? fg[(kb + 1) * 32] : 0.f;
+      const float wta = brg ? fg[(kb + 2) * 32] : 0.f;
+      const float wtb = brg ? fg[(kb + 3) * 32] : 0.f;
+      bool sat = false;
+      const float eg = gas_eps_f<CGA>(T, dg, pq, tq, du, ucg, brw, wpre, wta, wtb, st, sat);
+      if (sat) {
+        stop = ip;
+        break;
+      }
+      *out = eg;
+      out += ostep;
+      f += fstep;
+      fg += fstep;
+    }
+    if (r >= 0) P.stop[((long long)(tl * ndc + idl) * ng + g) * 32 + rl] = stop;
+    return;
   }
+  const int nmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)n);
+  // the next point's fields are loaded ahead of this point's chain
+  float nu = 0.f, npq = 0.f, ntq = 0.f, nw = 0.f, na = 0.f, nb = 0.f;
+  unsigned nbr = kNoBracket | 1u;
+  auto fetch = [&](int ip) {
+    if (ip >= n) return;
+    const float* q = fg + (long long)ip * fstep;
+    nu = CGA ? q[kFCgu * 32] : q[kFU * 32];
+    if (brg) {
+      nbr = __float_as_uint(q[kb * 32]);
+      nw = q[(kb + 1) * 32];
+      na = q[(kb + 2) * 32];
+      nb = q[(kb + 3) * 32];
+    } else {
+      npq = CGA ? q[kFCgp * 32] : f[(long long)ip * fstep + F.p * 32];
+      ntq = CGA ? q[kFCgt * 32] : f[(long long)ip * fstep + F.t * 32];
+    }
+  };
+  fetch(0);
+  for (int ip = 0; ip < nmax; ip++) {
+    bool on = ip < n && stop == n;
+    if (on && st.t < 1e-9f) {
+      stop = ip;
+      on = false;
+    }
+    if (!__any_sync(0xffffffffu, on)) break;
+    const float u = nu, pq = npq, tq = ntq;
+    CellFind cf{};
+    if (brg) cf.k = cell_packed(T, dg, nbr, nw, na, nb);
+    else if (on) cf = cell_find<CGA>(T, dg, np, pq, tq, st.ipr);
+    fetch(ip + 1);
+    float mine = 0.f;
+    int cnt = 0;
+    if (on && cf.k.ok) {
+      const unsigned row = ((corner & 2) ? cf.k.rc : cf.k.ra) + (corner & 1);
+      const float4 m = row_record<CGA>(T, row);
+      cnt = row_count<CGA>(m);
+      if (cnt >= 2)
+        mine = (cnt & kOddRow)
+                   ? corner_odd<CGA>(T.ue + row * (unsigned)T.tu, cnt, st.e, u, u, &st.h[0])
+                   : corner_eps<CGA>(T, row, m, st.e, u, u, st.h[0]);
+    }
+    const bool ok = ((__ballot_sync(0xffffffffu, cnt >= 2) >> (lane & ~3)) & 15u) == 15u;
+    const float ox = __shfl_xor_sync(0xffffffffu, mine, 1);
+    const float lo = (corner & 1) ? ox : mine, hi = (corner & 1) ? mine : ox;
+    const float et = brg ? mix_f(lo, hi, (corner & 2) ? cf.k.b : cf.k.a)
+                         : (corner & 2) ? mix_t(lo, hi, cf.tc, cf.td, tq)
+                                        : mix_t(lo, hi, cf.ta, cf.tb, tq);
+    const float oy = __shfl_xor_sync(0xffffffffu, et, 2);
+    const float ea = (corner & 2) ? oy : et, eb = (corner & 2) ? et : oy;
+    if (on) {
+      bool sat = false;
+      const float eg = ok ? extend_f(mix_f(ea, eb, cf.k.w), st, sat) : 0.f;
+      if (sat) stop = ip;
+      else if (corner == 0) out[ip * ostep] = eg;
+    }
+  }
+  if (r >= 0 && corner == 0) P.stop[((long long)(tl * ndc + idl) * ng + g) * 32 + rl] = stop;
 }
 
-// Row records of the mixed path (layouts at rowf_at); rows with fewer than
-// two entries are never interpolated and get zeros.
+// k_seg_m: one warp per (point, channel) joins the emitters' segments with the
+// continua, clouds and extinction and leaves src * eps and 1 - eps in the
+// first two of the point's entries.  Every point at once: nothing here
+// depends on the path.
+__global__ void __launch_bounds__(kPathThreads) k_seg_m(CtlDev c, TblDev T, BatchDev b, LosDev L,
+                                                        MixedPlan P) {
+  const int lane = threadIdx.x & 31;
+  const int ng = c.ng, ndc = P.id1 - P.id0, nchb = (ndc + 3) / 4;
+  const int idl = (int)(blockIdx.x % nchb) * 4 + (threadIdx.x >> 5);
+  const int ip = (int)(blockIdx.x / nchb);
+  const int tl = (int)blockIdx.y, tile = P.tile0 + tl;
+  if (idl >= ndc) return;
+  const int id = P.id0 + idl;
+  const int r = P.perm[tile * 32 + lane];
+  if (r < 0 || ip >= L.count[r]) return;
+  if (b.obs_skip && b.obs_skip[b.ray_obs[r]]) return;
+  if (b.skip_masked && b.mask[(long long)id * b.nray + r]) return;
+  const Fields F = fields_of(c, P.brmask);
+  const long long pt = P.toff[tile] + ip;
+  const float* f = P.data + pt * F.n * 32 + lane;
+  float* seg = P.seg + ((pt - P.pt0) * ndc + idl) * (long long)P.nseg * 32 + lane;
+  const int* st = P.stop + (long long)(tl * ndc + idl) * ng * 32 + lane;
+  float E = 0.f;
+  for (int g = 0; g < ng; g++) {
+    if (__ldg(T.np + (long long)id * ng + g) < 30) continue;
+    if (ip >= st[g * 32]) return;  // saturated: k_scan_m stops before
+    E = join_f(E, seg[g * 32]);
+  }
+  const float* kc = T.chanf + id * kChanConsts;
+  const float p = f[F.p * 32], t = f[F.t * 32], ds = f[F.ds * 32];
+  float beta = c.nw > 0 ? f[(F.kw0 + __float_as_int(kc[kChanWindow])) * 32] : 0.f;
+  if (P.cloud) {
+    const float cl = P.cloud[(long long)id * b.nray + r];
+    if (cl == cl) beta = __fmaf_rn(f[F.aux * 32], cl, beta);
+  }
+  beta = continua_f(c, F, kc, continua_on(c, kc[kChanSwitches]), f, p, t, ds, beta);
+  const float src = source_f(T.srf + (long long)id * kNS, t);
+  const float eps = segment_f(E, beta, ds);
+  seg[0] = __fmul_rn(src, eps);
+  seg[32] = __fsub_rn(1.f, eps);
+}
+
+// Cloud extinction of every (channel, ray), NaN without a cloud.
+__global__ void k_cloud_m(CtlDev c, ChanDev ch, BatchDev b, float* out) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= (long long)c.nd * b.nray) return;
+  bool has = false;
+  const float v = cloud_of(c, ch, b, (int)(i % b.nray), (int)(i / b.nray), &has);
+  out[i] = has ? v : __int_as_float(0x7fc00000);
+}
+
+// k_scan_m: one thread per (ray, channel) sums the segments along the path.
+// It stops at the first saturated emitter (nothing adds after it) and, without
+// surface reflection, once the path transmittance is below kTauStop: the rest
+// adds at most max(src) tau, below 1e-10 of the radiance.
+__global__ void __launch_bounds__(kPathThreads) k_scan_m(CtlDev c, TblDev T, ChanDev ch, BatchDev b,
+                                                         LosDev L, MixedPlan P) {
+  const int lane = threadIdx.x & 31;
+  const int ng = c.ng, ndc = P.id1 - P.id0;
+  const long long w = (long long)blockIdx.x * (kPathThreads / 32) + (threadIdx.x >> 5);
+  const int idl = (int)(w % ndc), tl = (int)(w / ndc);
+  if (tl >= P.tile1 - P.tile0) return;
+  const int tile = P.tile0 + tl, id = P.id0 + idl;
+  const int r = P.perm[tile * 32 + lane];
+  if (r < 0 || (b.obs_skip && b.obs_skip[b.ray_obs[r]])) return;
+  int n = b.skip_masked && b.mask[(long long)id * b.nray + r] ? 0 : L.count[r];
+  const int* st = P.stop + (long long)(tl * ndc + idl) * ng * 32 + lane;
+  for (int g = 0; g < ng; g++)
+    if (n > 0 && __ldg(T.np + (long long)id * ng + g) >= 30) n = min(n, st[g * 32]);
+  const float* seg =
+      P.seg + ((P.toff[tile] - P.pt0) * ndc + idl) * (long long)P.nseg * 32 + lane;
+  const long long step = (long long)ndc * P.nseg * 32;
+  const bool refl = c.sftype >= 2 && c.nsf > 0 && L.sft[r] > 0 && sfeps_of(c, ch, b, r, id) < 1.f;
+  float rad = 0.f, comp = 0.f, tau = 1.f;
+  constexpr int U = 8;  // loads in flight ahead of the sums
+  for (int ip = 0; ip < n; ip += U) {
+    if (tau < kTauStop && !refl) break;
+    float v[U], m[U];
+#pragma unroll
+    for (int k = 0; k < U; k++) {
+      const bool in = ip + k < n;
+      v[k] = in ? seg[(ip + k) * step] : 0.f;
+      m[k] = in ? seg[(ip + k) * step + 32] : 1.f;
+    }
+#pragma unroll
+    for (int k = 0; k < U; k++)
+      if (ip + k < n && (refl || !(tau < kTauStop))) add_f(v[k], m[k], rad, comp, tau);
+  }
+  write_radiance(c, T, ch, b, L, id, r, rad, tau, refl ? seg : nullptr, step, n);
+}
+
+// Row records (layouts above); rows with fewer than two entries are never
+// interpolated and get zeros.
 __global__ void k_rowmeta(long long nrow, int tu, const int* nu, const float* u, const float* e,
-                          const float* tf, int cga, float4* meta) {
+                          int cga, float4* meta) {
   const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= nrow) return;
   const int n = nu[r];
   const float* ur = u + r * tu;
   const float* er = e + r * tu;
+  const float nf = __int_as_float(n);
   if (cga) {
-    meta[r] = make_float4(__int_as_float(n), tf[r], n >= 2 ? ur[0] : 0.f, n >= 2 ? er[0] : 0.f);
+    meta[r] = n >= 2 ? make_float4(nf, 0.f, ur[0], er[0]) : make_float4(nf, 0.f, 0.f, 0.f);
     return;
   }
-  float4 m = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (n >= 2) m = make_float4(ur[0], ur[n - 1], er[0], er[n - 1]);
+  float4 m = make_float4(0.f, 0.f, 0.f, nf), m2 = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (n >= 2) {
+    m = make_float4(ur[0], er[0], er[n - 1], nf);
+    m2 = make_float4(ur[n - 1], log1pf(-er[n - 1]) / ur[n - 1], 0.f, 0.f);
+  }
   meta[2 * r] = m;
-  meta[2 * r + 1] = make_float4(__int_as_float(n), tf[r], 0.f, 0.f);
+  meta[2 * r + 1] = m2;
 }
 
-// The rows interleaved {u[i], eps[i]}: a probe of one brings the other.
-__global__ void k_interleave(long long n, const float* u, const float* e, float2* ue) {
+// The rows interleaved {u[i], eps[i]}: a probe of one brings the other; marks
+// odd rows (kOddRow, from the entry that shows it).
+__global__ void k_interleave(long long n, int tu, const int* nu, const float* u, const float* e,
+                             int cga, float2* ue, float4* meta) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) ue[i] = make_float2(u[i], e[i]);
+  if (i >= n) return;
+  const float a = u[i], b = e[i];
+  ue[i] = make_float2(a, b);
+  const long long r = i / tu;
+  const int k = (int)(i - r * tu), cnt = nu[r];
+  if (cnt < 2 || k >= cnt) return;
+  const bool fine = fabsf(a) < 4.2535296e37f && fabsf(b) < 4.2535296e37f &&  // 2^125
+                    (k + 1 >= cnt || (a <= u[i + 1] && b <= e[i + 1]));
+  if (!fine)
+    atomicOr(reinterpret_cast<int*>(cga ? &meta[r].x : &meta[2 * r].w), kOddRow);
 }
 
-void launch_rowmeta(long long nrow, int tu, const int* nu, const float* u, const float* e,
-                    const float* tf, int cga, float4* meta, float2* ue, cudaStream_t s) {
+void launch_rowmeta(long long nrow, int tu, const int* nu, const float* u, const float* e, int cga,
+                    float4* meta, float2* ue, cudaStream_t s) {
   const int bs = 256;
   if (nrow > 0) {
-    k_rowmeta<<<(unsigned)((nrow + bs - 1) / bs), bs, 0, s>>>(nrow, tu, nu, u, e, tf, cga, meta);
+    k_rowmeta<<<(unsigned)((nrow + bs - 1) / bs), bs, 0, s>>>(nrow, tu, nu, u, e, cga, meta);
     const long long n = nrow * tu;
-    k_interleave<<<(unsigned)((n + bs - 1) / bs), bs, 0, s>>>(n, u, e, ue);
+    k_interleave<<<(unsigned)((n + bs - 1) / bs), bs, 0, s>>>(n, tu, nu, u, e, cga, ue, meta);
   }
 }
 
@@ -921,113 +1170,81 @@ void launch_pack_tiles_n(const CtlDev& c, const TblDev& T, const LosDev& L, cons
   k_pack_tiles<<<(unsigned)((nth + bs - 1) / bs), bs, 0, s>>>(c, T, L, P, total_tile_points);
 }
 
-// register caps of the autotuner's variants (minimum resident blocks per SM),
-// each with both 128-thread block shapes, and the tile-major shape with
-// 256-thread blocks (one channel of 8 consecutive tiles) at two caps
-int path_mixed_caps() { return 7; }
-int path_mixed_variants() { return 2 * path_mixed_caps() + 2; }
-
-size_t path_smem(const CtlDev& c, int nt) {
-  return sizeof(unsigned) * kStateWords * nt * (size_t)(c.ng > 0 ? c.ng : 1) +
-         sizeof(float) * ((nt / 32) * kChanConsts + kThreadFloats * nt);
+size_t path_smem(const CtlDev& c) {
+  return sizeof(unsigned) * kStateWords * kPathThreads * (size_t)(c.ng > 0 ? c.ng : 1) +
+         sizeof(float) * ((kPathThreads / 32) * kChanConsts + kPathThreads);
 }
 
-template <typename K>
-void launch_k(K kern, unsigned nblk, int nt, size_t smem, cudaStream_t s, const CtlDev& c,
-              const TblDev& T, const ChanDev& ch, const BatchDev& b, const LosDev& L,
-              const MixedPlan& P, float* refl) {
-  if (smem > 48 * 1024)  // many emitters: opt in to the larger shared memory
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  kern<<<nblk, nt, smem, s>>>(c, T, ch, b, L, P, refl);
-}
+// Variants of k_gas_m with one lane per ray, chosen by the autotuner: block
+// shape (v / 4) and minimum resident blocks per SM (v % 4: 8, 10, 12, 16, i.e.
+// at most 64, 48, 40 and 32 registers).
+int path_gas_variants() { return 8; }
 
 template <bool CGA>
-void launch_variant(const CtlDev& c, const TblDev& T, const ChanDev& ch, const BatchDev& b,
-                    const LosDev& L, const MixedPlan& P, float* refl, int variant,
-                    cudaStream_t s) {
-  MixedPlan Pv = P;
-  if (variant >= 2 * path_mixed_caps()) {  // 256 threads, one channel of 8 tiles
-    Pv.tile_major = 1;
-    const unsigned nblk = (unsigned)((long long)((P.ntile + 7) / 8) * c.nd);
-    const size_t smem = path_smem(c, 256);
-    if (variant == 2 * path_mixed_caps())
-      launch_k(k_path_mixed<4, CGA, false, false, false, 256>, nblk, 256, smem, s, c, T, ch, b, L, Pv, refl);
-    else
-      launch_k(k_path_mixed<5, CGA, false, false, false, 256>, nblk, 256, smem, s, c, T, ch, b, L, Pv, refl);
+void launch_gas_v(const CtlDev& c, const TblDev& T, const BatchDev& b, const LosDev& L,
+                  const MixedPlan& P, int lanes_per_ray, int variant, cudaStream_t s) {
+  const long long nt = P.tile1 - P.tile0, ndc = P.id1 - P.id0;
+  constexpr int W = kPathThreads / 32;
+  if (lanes_per_ray == 4) {
+    const unsigned nblk = (unsigned)((nt * ndc * c.ng * 4 + W - 1) / W);
+    k_gas_m<CGA, 4, 8><<<nblk, kPathThreads, 0, s>>>(c, T, b, L, P, 0);
     return;
   }
-  Pv.tile_major = variant >= path_mixed_caps() ? 1 : 0;
-  const int nchb = (c.nd + 3) / 4;
-  const unsigned nblk = Pv.tile_major ? (unsigned)((long long)((P.ntile + 3) / 4) * c.nd)
-                                      : (unsigned)((long long)P.ntile * nchb);
-  // state, then kChanConsts per warp and kThreadFloats per thread
-  const size_t smem = path_smem(c, kPathThreads);
-  switch (variant % path_mixed_caps()) {
-    case 1: launch_k(k_path_mixed<5, CGA>, nblk, kPathThreads, smem, s, c, T, ch, b, L, Pv, refl); break;
-    case 2: launch_k(k_path_mixed<6, CGA>, nblk, kPathThreads, smem, s, c, T, ch, b, L, Pv, refl); break;
-    case 3: launch_k(k_path_mixed<4, CGA>, nblk, kPathThreads, smem, s, c, T, ch, b, L, Pv, refl); break;
-    case 4: launch_k(k_path_mixed<8, CGA>, nblk, kPathThreads, smem, s, c, T, ch, b, L, Pv, refl); break;
-    case 5: launch_k(k_path_mixed<10, CGA>, nblk, kPathThreads, smem, s, c, T, ch, b, L, Pv, refl); break;
-    case 6: launch_k(k_path_mixed<12, CGA>, nblk, kPathThreads, smem, s, c, T, ch, b, L, Pv, refl); break;
-    default: launch_k(k_path_mixed<1, CGA>, nblk, kPathThreads, smem, s, c, T, ch, b, L, Pv, refl); break;
+  const int shape = variant / 4;
+  const unsigned nblk = (unsigned)(shape ? (nt + W - 1) / W * ndc * c.ng : (nt * ndc * c.ng + W - 1) / W);
+  switch (variant % 4) {
+    case 0: k_gas_m<CGA, 1, 8><<<nblk, kPathThreads, 0, s>>>(c, T, b, L, P, shape); break;
+    case 1: k_gas_m<CGA, 1, 10><<<nblk, kPathThreads, 0, s>>>(c, T, b, L, P, shape); break;
+    case 2: k_gas_m<CGA, 1, 12><<<nblk, kPathThreads, 0, s>>>(c, T, b, L, P, shape); break;
+    default: k_gas_m<CGA, 1, 16><<<nblk, kPathThreads, 0, s>>>(c, T, b, L, P, shape); break;
   }
 }
 
-void launch_path_mixed(const CtlDev& c, const TblDev& T, const ChanDev& ch, const BatchDev& b,
-                       const LosDev& L, const MixedPlan& P, float* refl_scratch, int variant,
-                       cudaStream_t s) {
-  if (c.formod == 0)
-    launch_variant<true>(c, T, ch, b, L, P, refl_scratch, variant, s);
-  else
-    launch_variant<false>(c, T, ch, b, L, P, refl_scratch, variant, s);
+void launch_gas_m(const CtlDev& c, const TblDev& T, const BatchDev& b, const LosDev& L,
+                  const MixedPlan& P, int lanes_per_ray, int variant, cudaStream_t s) {
+  if (c.ng <= 0) return;
+  if (c.formod == 0) launch_gas_v<true>(c, T, b, L, P, lanes_per_ray, variant, s);
+  else launch_gas_v<false>(c, T, b, L, P, lanes_per_ray, variant, s);
 }
 
-template <bool CGA>
-void launch_split(const CtlDev& c, const TblDev& T, const ChanDev& ch, const BatchDev& b,
-                  const LosDev& L, const MixedPlan& P, float* refl, size_t smem, cudaStream_t s) {
-  const long long warps = (long long)P.ntile * c.nd * c.ng;
-  k_path_gas<CGA><<<(unsigned)((warps + 3) / 4), 128, 0, s>>>(c, T, b, L, P);
-  if (smem > 48 * 1024)
-    cudaFuncSetAttribute(k_path_mixed<1, CGA, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem);
-  const unsigned nblk = (unsigned)((long long)P.ntile * ((c.nd + 3) / 4));
-  k_path_mixed<1, CGA, true><<<nblk, kPathThreads, smem, s>>>(c, T, ch, b, L, P, refl);
+void launch_seg_scan_m(const CtlDev& c, const TblDev& T, const ChanDev& ch, const BatchDev& b,
+                       const LosDev& L, const MixedPlan& P, int longest, cudaStream_t s) {
+  const long long nt = P.tile1 - P.tile0, ndc = P.id1 - P.id0, nchb = (ndc + 3) / 4;
+  k_seg_m<<<dim3((unsigned)(nchb * longest), (unsigned)nt), kPathThreads, 0, s>>>(c, T, b, L, P);
+  k_scan_m<<<(unsigned)((nt * ndc + 3) / 4), kPathThreads, 0, s>>>(c, T, ch, b, L, P);
 }
 
-void launch_path_split(const CtlDev& c, const TblDev& T, const ChanDev& ch, const BatchDev& b,
-                       const LosDev& L, const MixedPlan& P, float* refl_scratch, cudaStream_t s) {
-  const size_t smem = sizeof(unsigned) * kStateWords * kPathThreads * (size_t)(c.ng > 0 ? c.ng : 1) +
-                      sizeof(float) * (4 * kChanConsts + kThreadFloats * kPathThreads);
-  if (c.formod == 0)
-    launch_split<true>(c, T, ch, b, L, P, refl_scratch, smem, s);
-  else
-    launch_split<false>(c, T, ch, b, L, P, refl_scratch, smem, s);
+void launch_cloud_m(const CtlDev& c, const ChanDev& ch, const BatchDev& b, float* out,
+                    cudaStream_t s) {
+  const long long n = (long long)c.nd * b.nray;
+  k_cloud_m<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(c, ch, b, out);
 }
+
+void launch_chan_consts(const CtlDev& c, const ChanDev& ch, float* out, cudaStream_t s) {
+  k_chan_consts<<<(c.nd + 127) / 128, 128, 0, s>>>(c, ch, out);
+}
+
+size_t chan_const_bytes(const CtlDev& c) { return sizeof(float) * kChanConsts * (size_t)c.nd; }
 
 int path_state_words(const CtlDev& c) { return kStateWords * c.ng + 3; }
 
 void launch_path_resume(const CtlDev& c, const TblDev& T, const ChanDev& ch, const BatchDev& b,
-                        const LosDev& L, const MixedPlan& P0, cudaStream_t s) {
-  // block = one channel of 4 consecutive tiles (the perturbations of one
-  // observation share table rows)
-  MixedPlan P = P0;
-  P.tile_major = 1;
+                        const LosDev& L, const MixedPlan& P, cudaStream_t s) {
   const unsigned nblk = (unsigned)((long long)((P.tile1 - P.tile0 + 3) / 4) * c.nd);
   if (nblk == 0) return;
-  const size_t smem = sizeof(unsigned) * kStateWords * kPathThreads * (size_t)(c.ng > 0 ? c.ng : 1) +
-                      sizeof(float) * (4 * kChanConsts + kThreadFloats * kPathThreads);
+  const size_t smem = path_smem(c);
   auto go = [&](auto kern) {
-    if (smem > 48 * 1024)
+    if (smem > 48 * 1024)  // many emitters: opt in to the larger shared memory
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    kern<<<nblk, kPathThreads, smem, s>>>(c, T, ch, b, L, P, nullptr);
+    kern<<<nblk, kPathThreads, smem, s>>>(c, T, ch, b, L, P);
   };
   const bool share = P.seg_base != nullptr;
   if (c.formod == 0) {
-    if (share) go(k_path_mixed<8, true, false, true, true>);
-    else go(k_path_mixed<8, true, false, true, false>);
+    if (share) go(k_path_mixed<8, true, true>);
+    else go(k_path_mixed<8, true, false>);
   } else {
-    if (share) go(k_path_mixed<8, false, false, true, true>);
-    else go(k_path_mixed<8, false, false, true, false>);
+    if (share) go(k_path_mixed<8, false, true>);
+    else go(k_path_mixed<8, false, false>);
   }
 }
 

@@ -326,14 +326,14 @@ __device__ __noinline__ double u_above(float un, float en, double e) {
 
 // Emissivity of one corner of the cell: EGA intpol_tbl_eps(intpol_tbl_u(e) +
 // du), CGA intpol_tbl_eps(du).  ef = round_down_f(e), the row's count and
-// end entries come with the row record (EGA 32 bytes {u0, un, e0, en}, {n, t,
-// -, -}; CGA 16 bytes {n, t, u0, e0}).  Slopes between entries are formed in
+// end entries come with the row record (EGA {u0, e0, en, n}, {un, ...}; CGA {n,
+// ..., u0, e0}).  Slopes between entries are formed in
 // single precision, as the reference's LIN macro does on floats.  Where the
 // column u_eq + du stays in the bracket that inverts e, the emissivity
 // follows from the entries already loaded.
 template <bool CGA>
-__device__ __forceinline__ double corner64(const TblDev& T, unsigned r, bool mono, double e,
-                                           float ef, double du, int& h, bool& ok) {
+__device__ __forceinline__ double corner64(const TblDev& T, unsigned r, double e, float ef,
+                                           double du, int& h, bool& ok) {
   const float2* row = T.ue + (size_t)r * (unsigned)T.tu;
   float u0, e0, un = 0.f, en = 0.f;
   int n;
@@ -344,12 +344,14 @@ __device__ __forceinline__ double corner64(const TblDev& T, unsigned r, bool mon
     e0 = m.w;
   } else {
     const float4 m = __ldg(T.rowmeta + 2 * (size_t)r);
-    n = __ldg(reinterpret_cast<const int*>(T.rowmeta + 2 * (size_t)r + 1));
+    n = __float_as_int(m.w);
+    un = __ldg(reinterpret_cast<const float*>(T.rowmeta + 2 * (size_t)r + 1));
     u0 = m.x;
-    un = m.y;
-    e0 = m.z;
-    en = m.w;
+    e0 = m.y;
+    en = m.z;
   }
+  const bool mono = !(n & kOddRow);
+  n &= ~kOddRow;
   ok = n >= 2;
   if (!ok) return 0.0;
   // Both interpolations are y0 + (y1 - y0) / (x1 - x0) (x - x0): the lanes pick
@@ -441,7 +443,6 @@ __global__ void __launch_bounds__(128) k_gas64(CtlDev c, TblDev T, BatchDev b, L
   double* out = P.om + ((lp0 * ndc + idl) * ng + g) * 32 + rl;
   const long long ostep = (long long)ndc * ng * 32;
   const bool cell = (P.shared >> g) & 1u;
-  const bool mono = P.mono[0] != 0;
   const unsigned rb = (unsigned)dg * (unsigned)(T.tp * T.tt);
   int h[4] = {0, 0, 0, 0};
   double tau = 1.0;
@@ -494,7 +495,7 @@ __global__ void __launch_bounds__(128) k_gas64(CtlDev c, TblDev T, BatchDev b, L
     if (LPR == 4) {
       double mine = 0.0;
       if (have)
-        mine = corner64<CGA>(T, ((corner & 2) ? rc : ra) + (corner & 1), mono, e, ef, du, h[0], ok);
+        mine = corner64<CGA>(T, ((corner & 2) ? rc : ra) + (corner & 1), e, ef, du, h[0], ok);
       ok = ((__ballot_sync(0xffffffffu, ok) >> (lane & ~3)) & 15u) == 15u;
       const double ox = __shfl_xor_sync(0xffffffffu, mine, 1);
       const double lo = (corner & 1) ? ox : mine, hi = (corner & 1) ? mine : ox;
@@ -504,10 +505,10 @@ __global__ void __launch_bounds__(128) k_gas64(CtlDev c, TblDev T, BatchDev b, L
       eb = (corner & 2) ? et : oy;
     } else if (have) {
       bool k0, k1, k2, k3;
-      const double e00 = corner64<CGA>(T, ra, mono, e, ef, du, h[0], k0);
-      const double e01 = corner64<CGA>(T, ra + 1, mono, e, ef, du, h[1], k1);
-      const double e10 = corner64<CGA>(T, rc, mono, e, ef, du, h[2], k2);
-      const double e11 = corner64<CGA>(T, rc + 1, mono, e, ef, du, h[3], k3);
+      const double e00 = corner64<CGA>(T, ra, e, ef, du, h[0], k0);
+      const double e01 = corner64<CGA>(T, ra + 1, e, ef, du, h[1], k1);
+      const double e10 = corner64<CGA>(T, rc, e, ef, du, h[2], k2);
+      const double e11 = corner64<CGA>(T, rc + 1, e, ef, du, h[3], k3);
       ok = k0 && k1 && k2 && k3;
       ea = lin64(e00, e01, la);
       eb = lin64(e10, e11, lb);
@@ -699,28 +700,12 @@ __global__ void k_src_channel_major(int nd, const double* st, const double* sr, 
   srd[gid] = make_double2(s0, it + 1 < kNS ? (s1 - s0) / (st[it + 1] - st[it]) : 0.0);
 }
 
-// mono[0] = 0 where a row's u or eps ever falls (or is NaN)
-__global__ void k_rows_mono(long long n, int tu, const int* nu, const float* u, const float* e,
-                            int* mono) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int k = (int)(i % tu);
-  if (k + 1 >= nu[i / tu]) return;
-  if (!(u[i] <= u[i + 1] && e[i] <= e[i + 1])) *mono = 0;
-}
-
 }  // namespace
 
 void path64_point_bytes(const CtlDev& c, size_t* fd, size_t* fu) {
   const Fields64 F = fields64(c);
   *fd = sizeof(double) * 32 * (size_t)F.nfd;
   *fu = sizeof(unsigned) * 32 * (size_t)F.nfu;
-}
-
-void launch_rows_mono(long long nrow, int tu, const int* nu, const float* u, const float* e,
-                      int* mono, cudaStream_t s) {
-  const long long n = nrow * tu;
-  if (n > 0) k_rows_mono<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, tu, nu, u, e, mono);
 }
 
 void launch_src_channel_major(int nd, const double* st, const double* sr, double2* srd,

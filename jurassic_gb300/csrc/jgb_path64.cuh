@@ -16,7 +16,6 @@ struct Path64 {
   int id0, id1;           // channels of this chunk
   unsigned shared;        // emitters whose p-T grids are the same for every channel
   int gref[kMaxG];        // a channel with a table of each such emitter
-  const int* mono;        // [1] 1: no table row ever falls
   double* fd;             // per-point fields (k_prep64)
   unsigned* fu;
   double* om;             // segment transmittance of every (point, channel, emitter, lane)
@@ -26,8 +25,6 @@ struct Path64 {
 
 // bytes of the per-point fields (32 lanes)
 void path64_point_bytes(const CtlDev& c, size_t* fd, size_t* fu);
-void launch_rows_mono(long long nrow, int tu, const int* nu, const float* u, const float* e,
-                      int* mono, cudaStream_t s);
 void launch_src_channel_major(int nd, const double* st, const double* sr, double2* srd,
                               cudaStream_t s);
 // longest: points of the chunk's longest tile

@@ -374,8 +374,13 @@ int prepare_tables(jgb_ctx* x, cudaStream_t s) {
       x->grid_ref[g] = ref;
     }
   const long long nrow = (long long)c.nd * c.ng * x->tp * x->tt;
+  CK(cudaMemsetAsync(x->t_odd.p, 0, sizeof(int), s));
   launch_rowmeta(nrow, x->tu, x->t_nu.as<int>(), x->t_u.as<float>(), x->t_eps.as<float>(),
-                 c.formod == 0, x->t_meta.as<float4>(), x->t_ue.as<float2>(), s);
+                 c.formod == 0, x->t_meta.as<float4>(), x->t_ue.as<float2>(), x->t_odd.as<int>(), s);
+  int odd = 0;
+  CK(cudaMemcpyAsync(&odd, x->t_odd.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+  CK(cudaStreamSynchronize(s));
+  x->odd_rows = odd != 0;
   launch_chan_consts(c, chan_view(x), x->d_chanf.as<float>(), s);
   CK(cudaGetLastError());
   x->meta_stale = false;
@@ -1010,6 +1015,7 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
     }
     const long long tile_points = toff_h[ntile];
     Pm.brmask = x->grid_mask;
+    Pm.fast = !x->odd_rows && x->grid_mask == (1u << c.ng) - 1u;
     Pm.nfield = mixed_nfield(c, Pm.brmask);
     CK(x->tiles_data.reserve(sizeof(float) * 32 * (size_t)std::max(tile_points, 1LL) * Pm.nfield));
     Pm.data = x->tiles_data.as<float>();
@@ -1617,7 +1623,8 @@ int jgb_create(const jgb_ctl* ctl, int device, jgb_ctx** out) {
             x->s_sr.reserve(sizeof(double) * kNS * c.nd) == cudaSuccess &&
             x->s_srf.reserve(sizeof(float) * kNS * c.nd) == cudaSuccess &&
             x->s_srd.reserve(sizeof(double2) * kNS * c.nd) == cudaSuccess &&
-            x->d_chanf.reserve(chan_const_bytes(c)) == cudaSuccess;
+            x->d_chanf.reserve(chan_const_bytes(c)) == cudaSuccess &&
+            x->t_odd.reserve(sizeof(int)) == cudaSuccess;
   ok = ok && cudaMemcpy(x->d_nu.p, x->nu.data(), sizeof(double) * c.nd, cudaMemcpyHostToDevice) == cudaSuccess;
   ok = ok && cudaMemcpy(x->d_window.p, x->window.data(), sizeof(int) * c.nd, cudaMemcpyHostToDevice) == cudaSuccess;
   if (c.ncl) ok = ok && cudaMemcpy(x->d_clnu.p, x->clnu.data(), sizeof(double) * c.ncl, cudaMemcpyHostToDevice) == cudaSuccess;
@@ -1645,7 +1652,7 @@ void jgb_destroy(jgb_ctx* x) {
   }
   DevBuf* bufs[] = {&x->d_nu, &x->d_window, &x->d_clnu, &x->d_sfnu, &x->d_ctm, &x->d_chanf, &x->cloudf, &x->t_np,
                     &x->t_p, &x->t_nt, &x->t_t, &x->t_nu, &x->t_u, &x->t_eps, &x->t_pf,
-                    &x->t_tf, &x->t_meta, &x->t_ue, &x->s_st, &x->s_sr, &x->s_srf, &x->s_srd, &x->b_levoff, &x->b_rayoff,
+                    &x->t_tf, &x->t_meta, &x->t_ue, &x->t_odd, &x->s_st, &x->s_sr, &x->s_srf, &x->s_srd, &x->b_levoff, &x->b_rayoff,
                     &x->b_rayobs, &x->b_lev, &x->b_scal, &x->b_geo, &x->b_rad, &x->b_tau,
                     &x->b_tp, &x->b_mask, &x->b_p, &x->los_off, &x->los_cnt, &x->los_cnt64,
                     &x->los_sft, &x->los_ends, &x->los_planes, &x->lev_slopes, &x->scan_tmp, &x->err_word,

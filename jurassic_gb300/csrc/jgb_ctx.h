@@ -75,6 +75,7 @@ struct jgb_ctx {
   std::vector<int> h_nt;
   std::vector<float> h_pf, h_tf;
   unsigned grid_mask = 0;
+  bool odd_rows = false;  // tables with a row marked kOddRow
   // the same for the FP64 path: FP64 grids, the emitters whose grids are the
   // same for every channel with a table, and one such channel of each
   std::vector<double> h_p, h_t;
@@ -83,7 +84,7 @@ struct jgb_ctx {
   // field of view: nfov samples (dz, w) on the device, pencil-beam scratch
   int nfov = 0;
   jgb::DevBuf d_fov, fov_raw;
-  jgb::DevBuf t_np, t_p, t_nt, t_t, t_nu, t_u, t_eps, t_pf, t_tf, t_meta, t_ue;
+  jgb::DevBuf t_np, t_p, t_nt, t_t, t_nu, t_u, t_eps, t_pf, t_tf, t_meta, t_ue, t_odd;
   bool meta_stale = true;
   // source function
   jgb::DevBuf s_st, s_sr, s_srf, s_srd;

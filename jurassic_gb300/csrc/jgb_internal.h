@@ -82,6 +82,7 @@ struct MixedPlan {
   float* data;          // tile planes
   int nfield;
   unsigned brmask;      // emitters with p-T brackets precomputed per LOS point
+  bool fast;            // all of them, and no odd row in the tables
   // a chunk of the path (k_gas_m, k_seg_m, k_scan_m): tiles [tile0, tile1)
   // with pt0 = toff[tile0], channels [id0, id1); seg[((point * channels +
   // channel) * nseg + emitter) * 32 + lane] the segment emissivities, stop the
@@ -142,7 +143,7 @@ int path_state_words(const CtlDev& c);
 void launch_src_to_float(int nd, const double* sr, float* srf, cudaStream_t s);
 void launch_tables_to_float(long long n, const double* src, float* dst, cudaStream_t s);
 void launch_rowmeta(long long nrow, int tu, const int* nu, const float* u, const float* e, int cga,
-                    float4* meta, float2* ue, cudaStream_t s);
+                    float4* meta, float2* ue, int* any_odd, cudaStream_t s);
 
 // jgb_retrieval.cu: frees an engine's device and pinned memory and unties
 // it from its context (which is being destroyed); the handle then accepts

@@ -1,11 +1,14 @@
 // Mixed-precision forward model: FP32 path loop with compensated sums.
 //
 // Work decomposition: rays are sorted by LOS length and grouped into tiles
-// of 32 (one ray per lane); a warp walks one tile for one channel, so all
-// lanes of a warp read the same emissivity table (same channel, emitter)
-// at neighbouring rows and the same LOS plane entries (one 128-byte line
-// per field and point).  A block holds 4 warps = 4 channels of one tile,
-// which share the tile's LOS data through L1.
+// of 32 (one ray per lane), so all lanes of a warp read the same emissivity
+// table (same channel, emitter) at neighbouring rows and the same LOS plane
+// entries (one 128-byte line per field and point).  A batch runs through
+// three kernels: k_gas_m walks the points for one (tile, channel, emitter)
+// per warp, k_seg_m joins the emitters' segments of every (point, channel)
+// with the continua, k_scan_m sums them along the rays.  Resumed
+// finite-difference perturbations take one kernel for all three
+// (k_path_mixed), which saves and restores path states.
 //
 // Numerics (same algorithm as intpol_tbl_ega/cga, jurassic.c:3710-3891, and
 // formod_pencil, 3196-3338):
@@ -15,6 +18,8 @@
 //  * segment emissivities are combined as E <- E + (1 - E) eps_g (no
 //    cancellation for small eps), the continuum as -expm1(-beta ds);
 //  * the radiance sum is Kahan-compensated.
+#include <type_traits>
+
 #include "jgb_common.cuh"
 #include "jgb_internal.h"
 
@@ -24,7 +29,8 @@ namespace jgb {
 // factor, the extinction per window, then one block of kEmitterFields(CGA)
 // fields per emitter, emitter g's at g0 + g * es + k (k constant, so that a
 // warp addresses them from one base):
-//   EGA: u, br, pw, wa, wb;  CGA: u, cgp, cgt, cgu, br, pw, wa, wb.
+//   EGA: u, {br, pw, wa, wb};  CGA: u, cgp, cgt, cgu, {br, pw, wa, wb},
+// the braces 16 bytes per lane (one load).
 // For emitters whose p-T grids are shared by all channels, the
 // channel-independent part of the table interpolation is done once per LOS
 // point: br holds the rows of the point's p-T cell within a (channel,
@@ -122,7 +128,7 @@ __device__ __forceinline__ int bisect2(const float2* g, int lo, int hi, float x)
 // entry, or the one-entry pad after the last row) and then ignored.
 template <int C>
 __device__ __forceinline__ Bracket2 hunt2(const float2* g, int n, float x, int h) {
-  h = min(max(h, 0), n - 2);
+  h = min(h, n - 2);
   const float2 A = __ldg(g + h), B = __ldg(g + h + 1), D = __ldg(g + h + 2);
   const float a = comp<C>(A), b = comp<C>(B), c = comp<C>(D);
   // bracket h or h + 1: every x >= a when the probes reach the row's end
@@ -156,14 +162,14 @@ __device__ __forceinline__ float between(float2 a, float2 b, float u) {
 template <bool CGA>
 __device__ __forceinline__ float corner_eps(const TblDev& T, unsigned r, const float4 m,
                                             float e_path, float du, float ucg,
-                                            unsigned short& h) {
+                                            int& h) {
   const float2* row = T.ue + r * (unsigned)T.tu;
   if (CGA) {  // intpol_tbl_eps(ucg), the row's last entries from the search
     const int n = __float_as_int(m.x);
     const float uc = ucg;
     if (uc < m.z) return __fdividef(m.w, m.z) * uc;
     const Bracket2 k = hunt2<0>(row, n, uc, h);
-    h = (unsigned short)k.i;
+    h = k.i;
     if (uc > k.b.x) {
       const float a = __fdividef(log1pf(-k.b.y), k.b.x);
       return -expm1f(a * uc);
@@ -181,7 +187,7 @@ __device__ __forceinline__ float corner_eps(const TblDev& T, unsigned r, const f
     uq = __fadd_rn(__fdividef(log1pf(-e_path), __ldg(rec).y), du);
   } else {
     const Bracket2 k = hunt2<1>(row, n, e_path, h);
-    h = (unsigned short)k.i;
+    h = k.i;
     ib = k.i;
     uq = __fadd_rn(__fmaf_rn(__fdividef(__fsub_rn(k.b.x, k.a.x), __fsub_rn(k.b.y, k.a.y)),
                              __fsub_rn(e_path, k.a.y), k.a.x), du);
@@ -195,21 +201,25 @@ __device__ __forceinline__ float corner_eps(const TblDev& T, unsigned r, const f
   return between(k.a, k.b, uq);
 }
 
-// The same for a row marked kOddRow.
+// The same for a row marked kOddRow; the hint comes and goes by value (a
+// pointer to it would keep the hints of every row in local memory).
+struct OddCorner {
+  float e;
+  int h;
+};
 template <bool CGA>
-__device__ __noinline__ float corner_odd(const float2* row, int n, float e_path, float du,
-                                         float ucg, unsigned short* h) {
+__device__ __noinline__ OddCorner corner_odd(const float2* row, int n, float e_path, float du,
+                                             float ucg, int h) {
   n &= ~kOddRow;
   const float2 first = __ldg(row), last = __ldg(row + n - 1);
   if (CGA) {
-    if (ucg < first.x) return first.y / first.x * ucg;
-    const Bracket2 k = hunt2<0>(row, n, ucg, *h);
-    *h = (unsigned short)k.i;
+    if (ucg < first.x) return OddCorner{first.y / first.x * ucg, h};
+    const Bracket2 k = hunt2<0>(row, n, ucg, h);
     if (ucg > k.b.x) {
       const float a = log1pf(-k.b.y) / k.b.x;
-      return -expm1f(a * ucg);
+      return OddCorner{-expm1f(a * ucg), k.i};
     }
-    return k.a.y + (k.b.y - k.a.y) / (k.b.x - k.a.x) * (ucg - k.a.x);
+    return OddCorner{k.a.y + (k.b.y - k.a.y) / (k.b.x - k.a.x) * (ucg - k.a.x), k.i};
   }
   float uq, u_lo = 0.f, u_hi = 0.f, e_lo = 0.f, e_hi = 0.f;
   int ib = -1;
@@ -219,9 +229,8 @@ __device__ __noinline__ float corner_odd(const float2* row, int n, float e_path,
     const float a = log1pf(-last.y) / last.x;
     uq = log1pf(-e_path) / a;
   } else {
-    const Bracket2 k = hunt2<1>(row, n, e_path, *h);
-    *h = (unsigned short)k.i;
-    ib = k.i;
+    const Bracket2 k = hunt2<1>(row, n, e_path, h);
+    h = ib = k.i;
     e_lo = k.a.y;
     e_hi = k.b.y;
     u_lo = k.a.x;
@@ -229,14 +238,31 @@ __device__ __noinline__ float corner_odd(const float2* row, int n, float e_path,
     uq = u_lo + (u_hi - u_lo) / (e_hi - e_lo) * (e_path - e_lo);
   }
   uq = __fadd_rn(uq, du);
-  if (uq < first.x) return first.y / first.x * uq;
+  if (uq < first.x) return OddCorner{first.y / first.x * uq, h};
   if (uq > last.x) {
     const float a = log1pf(-last.y) / last.x;
-    return -expm1f(a * uq);
+    return OddCorner{-expm1f(a * uq), h};
   }
-  if (ib >= 0 && uq >= u_lo && uq < u_hi) return e_lo + (e_hi - e_lo) / (u_hi - u_lo) * (uq - u_lo);
+  if (ib >= 0 && uq >= u_lo && uq < u_hi)
+    return OddCorner{e_lo + (e_hi - e_lo) / (u_hi - u_lo) * (uq - u_lo), h};
   const Bracket2 k = hunt2<0>(row, n, uq, max(ib, 0));
-  return k.a.y + (k.b.y - k.a.y) / (k.b.x - k.a.x) * (uq - k.a.x);
+  return OddCorner{k.a.y + (k.b.y - k.a.y) / (k.b.x - k.a.x) * (uq - k.a.x), h};
+}
+
+// One corner of the cell from its record, whichever kind of row it is.  FAST
+// kernels run where no row is odd and every emitter's grids are shared by all
+// channels: the calls and the search for the cell cost registers even where
+// they are not taken.
+template <bool CGA, bool FAST>
+__device__ __forceinline__ float corner_any(const TblDev& T, unsigned r, const float4 m, int n,
+                                            float e_path, float du, float ucg,
+                                            int& h) {
+  if (!FAST && (n & kOddRow)) {
+    const OddCorner o = corner_odd<CGA>(T.ue + r * (unsigned)T.tu, n, e_path, du, ucg, h);
+    h = o.h;
+    return o.e;
+  }
+  return corner_eps<CGA>(T, r, m, e_path, du, ucg, h);
 }
 
 __device__ __forceinline__ int bracket_regf(const float* g, int n, float x) {
@@ -274,10 +300,7 @@ __global__ void k_pack_tiles(CtlDev c, TblDev T, LosDev L, MixedPlan P, long lon
   const int r = P.perm[tile * 32 + lane];
   const Fields F = fields_of(c, P.brmask);
   float* out = P.data + tp * (long long)F.n * 32 + lane;
-  if (r < 0 || ip >= L.count[r]) {
-    for (int f = 0; f < F.n; f++) out[f * 32] = 0.f;
-    return;
-  }
+  if (r < 0 || ip >= L.count[r]) return;  // never read
   const long long q = L.off[r] + ip;
   const LosDev::F32& Lf = L.f;
   out[F.p * 32] = Lf.p[q];
@@ -295,7 +318,6 @@ __global__ void k_pack_tiles(CtlDev c, TblDev T, LosDev L, MixedPlan P, long lon
       og[kFCgt * 32] = Lf.cgt[g * L.cap + q];
       og[kFCgu * 32] = Lf.cgu[g * L.cap + q];
     }
-    for (int k = 0; k < 4; k++) og[(kFBr(cgaf) + k) * 32] = 0.f;
   }
   // p-T brackets and interpolation weights on the grids of channel 0
   // (identical for every channel)
@@ -328,11 +350,8 @@ __global__ void k_pack_tiles(CtlDev c, TblDev T, LosDev L, MixedPlan P, long lon
           pw = (pq - pa) / (pb - pa);
       }
     }
-    float* og = out + (F.g0 + g * F.es + kFBr(cgaf)) * 32;
-    og[0] = __uint_as_float(wd);
-    og[32] = pw;
-    og[64] = wa;
-    og[96] = wb;
+    float* og = P.data + (tp * F.n + F.g0 + g * F.es + kFBr(cgaf)) * 32;
+    reinterpret_cast<float4*>(og)[lane] = make_float4(__uint_as_float(wd), pw, wa, wb);
   }
 }
 
@@ -358,11 +377,11 @@ constexpr int kPathThreads = 128;  // threads of a path block
 
 // Per (channel, emitter) state carried along the path: transmittance t and
 // emissivity e of the extended path (each accurate where it is small), the
-// pressure bracket and the search hints of the four table corners (16 bit).
+// pressure bracket and the search hints of the four table corners (below 2^16).
 struct GasState {
   float t, e;
   int ipr;
-  unsigned short h[4];
+  int h[4];
 };
 
 // Interpolations of the cell's corners in temperature and pressure.
@@ -393,10 +412,15 @@ struct CellF {
 };
 
 // From the precomputed words (grids shared by all channels) ...
-__device__ __forceinline__ CellF cell_packed(const TblDev& T, long long dg, unsigned brw, float w,
-                                             float a, float b) {
-  const unsigned rb = (unsigned)dg * (unsigned)(T.tp * T.tt);
-  return CellF{rb + (brw & 0xffffu), rb + (brw >> 16), w, a, b, (brw & kNoBracket) == 0u};
+__device__ __forceinline__ float4 cell_words(const float* block, int lane) {
+  return reinterpret_cast<const float4*>(block - lane)[lane];
+}
+__device__ __forceinline__ float4 no_cell() {
+  return make_float4(__uint_as_float(kNoBracket | 1u), 0.f, 0.f, 0.f);
+}
+__device__ __forceinline__ CellF cell_packed(const TblDev& T, long long dg, const float4 cw) {
+  const unsigned rb = (unsigned)dg * (unsigned)(T.tp * T.tt), brw = __float_as_uint(cw.x);
+  return CellF{rb + (brw & 0xffffu), rb + (brw >> 16), cw.y, cw.z, cw.w, (brw & kNoBracket) == 0u};
 }
 
 // ... or found here, the pressure bracket from the last one (ipr).  The
@@ -448,15 +472,15 @@ __device__ __forceinline__ int row_count(const float4 m) {
 // One (channel, emitter) at one LOS point (intpol_tbl_ega / intpol_tbl_cga,
 // jurassic.c:3710-3891).  Returns the segment emissivity; *sat is set where
 // the reference's segment transmittance becomes zero.
-// brw: packed bracket precomputed for the LOS point (grids shared by all
-// channels), or kNoBracket | 1 to search here; wpre, wta, wtb: the pressure
-// and temperature interpolation weights precomputed with it.
-template <bool CGA>
+// cw: the cell's rows and interpolation weights precomputed for the LOS point
+// (grids shared by all channels), or no_cell() to search here.
+template <bool CGA, bool FAST>
 __device__ __forceinline__ float gas_eps_f(const TblDev& T, long long dg, float pq,
-                                           float tq, float du, float ucg, unsigned brw,
-                                           float wpre, float wta, float wtb, GasState& s,
-                                           bool& sat) {
-  const bool pre = brw != (kNoBracket | 1u);
+                                           float tq, float du, float ucg, const float4 cw,
+                                           GasState& s, bool& sat) {
+  const unsigned brw = __float_as_uint(cw.x);
+  const float wta = cw.z, wtb = cw.w;
+  const bool pre = FAST || brw != (kNoBracket | 1u);
   if (pre && brw == kNoBracket) return 0.f;   // np < 30
   int np = 0;
   if (!pre) {
@@ -470,30 +494,29 @@ __device__ __forceinline__ float gas_eps_f(const TblDev& T, long long dg, float 
     return 1.f;
   }
   CellFind f{};
-  if (pre) f.k = cell_packed(T, dg, brw, wpre, wta, wtb);
+  if (pre) f.k = cell_packed(T, dg, cw);
   else f = cell_find<CGA>(T, dg, np, pq, tq, s.ipr);
   if (!f.k.ok) return 0.f;                    // nt < 2 at this pressure
   const unsigned ra = f.k.ra, rc = f.k.rc;
-  const float4 m00 = row_record<CGA>(T, ra), m01 = row_record<CGA>(T, ra + 1u);
-  const float4 m10 = row_record<CGA>(T, rc), m11 = row_record<CGA>(T, rc + 1u);
-  const int n00 = row_count<CGA>(m00), n01 = row_count<CGA>(m01);
-  const int n10 = row_count<CGA>(m10), n11 = row_count<CGA>(m11);
-  if (min(min(n00, n01), min(n10, n11)) < 2) return 0.f;
-  float e00, e01, e10, e11;
-  if ((n00 | n01 | n10 | n11) & kOddRow) {
-    const unsigned tu = (unsigned)T.tu;
-    e00 = corner_odd<CGA>(T.ue + ra * tu, n00, s.e, du, ucg, &s.h[0]);
-    e01 = corner_odd<CGA>(T.ue + (ra + 1u) * tu, n01, s.e, du, ucg, &s.h[1]);
-    e10 = corner_odd<CGA>(T.ue + rc * tu, n10, s.e, du, ucg, &s.h[2]);
-    e11 = corner_odd<CGA>(T.ue + (rc + 1u) * tu, n11, s.e, du, ucg, &s.h[3]);
-  } else {
-    e00 = corner_eps<CGA>(T, ra, m00, s.e, du, ucg, s.h[0]);
-    e01 = corner_eps<CGA>(T, ra + 1u, m01, s.e, du, ucg, s.h[1]);
-    e10 = corner_eps<CGA>(T, rc, m10, s.e, du, ucg, s.h[2]);
-    e11 = corner_eps<CGA>(T, rc + 1u, m11, s.e, du, ucg, s.h[3]);
+  // one pressure's pair of rows after the other (four records at a time cost
+  // more registers than their overlap gains)
+  float ea, eb;
+  {
+    const float4 m0 = row_record<CGA>(T, ra), m1 = row_record<CGA>(T, ra + 1u);
+    const int n0 = row_count<CGA>(m0), n1 = row_count<CGA>(m1);
+    if (min(n0, n1) < 2) return 0.f;
+    const float e0 = corner_any<CGA, FAST>(T, ra, m0, n0, s.e, du, ucg, s.h[0]);
+    const float e1 = corner_any<CGA, FAST>(T, ra + 1u, m1, n1, s.e, du, ucg, s.h[1]);
+    ea = pre ? mix_f(e0, e1, wta) : mix_t(e0, e1, f.ta, f.tb, tq);
   }
-  const float ea = pre ? mix_f(e00, e01, wta) : mix_t(e00, e01, f.ta, f.tb, tq);
-  const float eb = pre ? mix_f(e10, e11, wtb) : mix_t(e10, e11, f.tc, f.td, tq);
+  {
+    const float4 m0 = row_record<CGA>(T, rc), m1 = row_record<CGA>(T, rc + 1u);
+    const int n0 = row_count<CGA>(m0), n1 = row_count<CGA>(m1);
+    if (min(n0, n1) < 2) return 0.f;
+    const float e0 = corner_any<CGA, FAST>(T, rc, m0, n0, s.e, du, ucg, s.h[2]);
+    const float e1 = corner_any<CGA, FAST>(T, rc + 1u, m1, n1, s.e, du, ucg, s.h[3]);
+    eb = pre ? mix_f(e0, e1, wtb) : mix_t(e0, e1, f.tc, f.td, tq);
+  }
   return extend_f(mix_f(ea, eb, f.k.w), s, sat);
 }
 
@@ -678,7 +701,7 @@ __device__ __forceinline__ void write_radiance(const CtlDev& c, const TblDev& T,
 // perturbations: rays start at P.start[r] from a saved state and save states
 // for other rays that share a path prefix.  Other batches take k_gas_m,
 // k_seg_m and k_scan_m, whose arithmetic per point is the same.
-template <int MINB, bool CGA, bool SHARE>
+template <int MINB, bool CGA, bool SHARE, bool FAST>
 __global__ void __launch_bounds__(kPathThreads, MINB) k_path_mixed(CtlDev c, TblDev T, ChanDev ch,
                                                                    BatchDev b, LosDev L,
                                                                    MixedPlan P) {
@@ -724,8 +747,8 @@ __global__ void __launch_bounds__(kPathThreads, MINB) k_path_mixed(CtlDev c, Tbl
 #pragma unroll
     for (int k = 0; k < 2; k++) {
       const unsigned hw = q[(3 + k) * nth];
-      st.h[2 * k] = (unsigned short)(hw & 0xffffu);
-      st.h[2 * k + 1] = (unsigned short)(hw >> 16);
+      st.h[2 * k] = (int)(hw & 0xffffu);
+      st.h[2 * k + 1] = (int)(hw >> 16);
     }
     return st;
   };
@@ -826,14 +849,11 @@ __global__ void __launch_bounds__(kPathThreads, MINB) k_path_mixed(CtlDev c, Tbl
         const float pq = CGA ? fg[kFCgp * 32] : p;
         const float tq = CGA ? fg[kFCgt * 32] : t;
         const float ucg = CGA ? fg[kFCgu * 32] : 0.f;
-        const bool brg = (P.brmask >> g) & 1u;
-        const unsigned brw = brg ? __float_as_uint(fg[kb * 32]) : (kNoBracket | 1u);
-        const float wpre = brg ? fg[(kb + 1) * 32] : 0.f;
-        const float wta = brg ? fg[(kb + 2) * 32] : 0.f;
-        const float wtb = brg ? fg[(kb + 3) * 32] : 0.f;
+        const bool brg = FAST || ((P.brmask >> g) & 1u);
+        const float4 cw = brg ? cell_words(fg + kb * 32, lane) : no_cell();
         GasState st = sload(g, brg);
         bool sg = false;
-        eg = gas_eps_f<CGA>(T, dg0 + g, pq, tq, du, ucg, brw, wpre, wta, wtb, st, sg);
+        eg = gas_eps_f<CGA, FAST>(T, dg0 + g, pq, tq, du, ucg, cw, st, sg);
         sstore(g, st, brg);
         if (sg) sat = true;
         if (SHARE && seg_write) {
@@ -875,7 +895,13 @@ __global__ void __launch_bounds__(kPathThreads, MINB) k_path_mixed(CtlDev c, Tbl
 // cell, for batches that leave the device idle.  shape 1: the warps of a
 // block take consecutive tiles of one (channel, emitter), whose rows they
 // share in L1; shape 0: consecutive channels of one tile.
-template <bool CGA, int LPR, int MINB>
+// Bound by instruction issue and the L1 data pipe together (73 % and 62 %
+// busy on 62 nadir tiles x 100 channels x 5 emitters, 345 instructions per
+// point and emitter, DRAM 5 %): 12.3 ms for those 3.1e7 warp steps, against
+// 17 ms in a kernel that held all emitters of a channel in a warp (527
+// instructions, state in shared memory).  What the register count costs
+// shows in the variants: spilling forms take 13.8 ms, 64 registers 12.9 ms.
+template <bool CGA, int LPR, int MINB, bool FAST>
 __global__ void __launch_bounds__(kPathThreads, MINB) k_gas_m(CtlDev c, TblDev T, BatchDev b,
                                                               LosDev L, MixedPlan P, int shape) {
   constexpr int W = kPathThreads / 32;
@@ -918,7 +944,7 @@ __global__ void __launch_bounds__(kPathThreads, MINB) k_gas_m(CtlDev c, TblDev T
   const long long lp0 = P.toff[tile] - P.pt0;
   float* out = P.seg + ((lp0 * ndc + idl) * P.nseg + g) * 32 + rl;
   const long long ostep = (long long)ndc * P.nseg * 32;
-  const bool brg = (P.brmask >> g) & 1u;
+  const bool brg = FAST || ((P.brmask >> g) & 1u);
   GasState st;
   st.t = 1.f;
   st.e = 0.f;
@@ -932,12 +958,9 @@ __global__ void __launch_bounds__(kPathThreads, MINB) k_gas_m(CtlDev c, TblDev T
       const float pq = CGA ? fg[kFCgp * 32] : brg ? 0.f : f[F.p * 32];
       const float tq = CGA ? fg[kFCgt * 32] : brg ? 0.f : f[F.t * 32];
       const float ucg = CGA ? fg[kFCgu * 32] : 0.f;
-      const unsigned brw = brg ? __float_as_uint(fg[kb * 32]) : (kNoBracket | 1u);
-      const float wpre = brg ? fg[(kb + 1) * 32] : 0.f;
-      const float wta = brg ? fg[(kb + 2) * 32] : 0.f;
-      const float wtb = brg ? fg[(kb + 3) * 32] : 0.f;
+      const float4 cw = brg ? cell_words(fg + kb * 32, rl) : no_cell();
       bool sat = false;
-      const float eg = gas_eps_f<CGA>(T, dg, pq, tq, du, ucg, brw, wpre, wta, wtb, st, sat);
+      const float eg = gas_eps_f<CGA, FAST>(T, dg, pq, tq, du, ucg, cw, st, sat);
       if (sat) {
         stop = ip;
         break;
@@ -952,17 +975,14 @@ __global__ void __launch_bounds__(kPathThreads, MINB) k_gas_m(CtlDev c, TblDev T
   }
   const int nmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)n);
   // the next point's fields are loaded ahead of this point's chain
-  float nu = 0.f, npq = 0.f, ntq = 0.f, nw = 0.f, na = 0.f, nb = 0.f;
-  unsigned nbr = kNoBracket | 1u;
+  float nu = 0.f, npq = 0.f, ntq = 0.f;
+  float4 ncw = no_cell();
   auto fetch = [&](int ip) {
     if (ip >= n) return;
     const float* q = fg + (long long)ip * fstep;
     nu = CGA ? q[kFCgu * 32] : q[kFU * 32];
     if (brg) {
-      nbr = __float_as_uint(q[kb * 32]);
-      nw = q[(kb + 1) * 32];
-      na = q[(kb + 2) * 32];
-      nb = q[(kb + 3) * 32];
+      ncw = cell_words(q + kb * 32, rl);
     } else {
       npq = CGA ? q[kFCgp * 32] : f[(long long)ip * fstep + F.p * 32];
       ntq = CGA ? q[kFCgt * 32] : f[(long long)ip * fstep + F.t * 32];
@@ -978,7 +998,7 @@ __global__ void __launch_bounds__(kPathThreads, MINB) k_gas_m(CtlDev c, TblDev T
     if (!__any_sync(0xffffffffu, on)) break;
     const float u = nu, pq = npq, tq = ntq;
     CellFind cf{};
-    if (brg) cf.k = cell_packed(T, dg, nbr, nw, na, nb);
+    if (brg) cf.k = cell_packed(T, dg, ncw);
     else if (on) cf = cell_find<CGA>(T, dg, np, pq, tq, st.ipr);
     fetch(ip + 1);
     float mine = 0.f;
@@ -987,10 +1007,7 @@ __global__ void __launch_bounds__(kPathThreads, MINB) k_gas_m(CtlDev c, TblDev T
       const unsigned row = ((corner & 2) ? cf.k.rc : cf.k.ra) + (corner & 1);
       const float4 m = row_record<CGA>(T, row);
       cnt = row_count<CGA>(m);
-      if (cnt >= 2)
-        mine = (cnt & kOddRow)
-                   ? corner_odd<CGA>(T.ue + row * (unsigned)T.tu, cnt, st.e, u, u, &st.h[0])
-                   : corner_eps<CGA>(T, row, m, st.e, u, u, st.h[0]);
+      if (cnt >= 2) mine = corner_any<CGA, FAST>(T, row, m, cnt, st.e, u, u, st.h[0]);
     }
     const bool ok = ((__ballot_sync(0xffffffffu, cnt >= 2) >> (lane & ~3)) & 15u) == 15u;
     const float ox = __shfl_xor_sync(0xffffffffu, mine, 1);
@@ -1010,46 +1027,60 @@ __global__ void __launch_bounds__(kPathThreads, MINB) k_gas_m(CtlDev c, TblDev T
   if (r >= 0 && corner == 0) P.stop[((long long)(tl * ndc + idl) * ng + g) * 32 + rl] = stop;
 }
 
-// k_seg_m: one warp per (point, channel) joins the emitters' segments with the
-// continua, clouds and extinction and leaves src * eps and 1 - eps in the
-// first two of the point's entries.  Every point at once: nothing here
-// depends on the path.
+// k_seg_m: joins the emitters' segments with the continua, clouds and
+// extinction and leaves src * eps and 1 - eps in the first two of the point's
+// entries.  Nothing here depends on the path, so a warp takes a run of
+// kSegRun points of its (tile, channel): long enough that the channel's
+// constants and the rays' limits are read once per run, short enough to
+// spread a small batch (a warp per point took 398 instructions for what takes
+// 212 here; 3.3 -> 1.8 ms for 6.2e6 warp points, 5.5 GB of DRAM traffic).
+constexpr int kSegRun = 16;
+
 __global__ void __launch_bounds__(kPathThreads) k_seg_m(CtlDev c, TblDev T, BatchDev b, LosDev L,
                                                         MixedPlan P) {
   const int lane = threadIdx.x & 31;
   const int ng = c.ng, ndc = P.id1 - P.id0, nchb = (ndc + 3) / 4;
   const int idl = (int)(blockIdx.x % nchb) * 4 + (threadIdx.x >> 5);
-  const int ip = (int)(blockIdx.x / nchb);
+  const int ip0 = (int)(blockIdx.x / nchb) * kSegRun;
   const int tl = (int)blockIdx.y, tile = P.tile0 + tl;
   if (idl >= ndc) return;
   const int id = P.id0 + idl;
   const int r = P.perm[tile * 32 + lane];
-  if (r < 0 || ip >= L.count[r]) return;
-  if (b.obs_skip && b.obs_skip[b.ray_obs[r]]) return;
+  if (r < 0 || (b.obs_skip && b.obs_skip[b.ray_obs[r]])) return;
   if (b.skip_masked && b.mask[(long long)id * b.nray + r]) return;
+  // the run ends at the first saturated emitter, where k_scan_m stops
+  int n = min(L.count[r], ip0 + kSegRun);
+  const int* st = P.stop + (long long)(tl * ndc + idl) * ng * 32 + lane;
+  unsigned has = 0;  // emitters with a table
+  for (int g = 0; g < ng; g++)
+    if (__ldg(T.np + (long long)id * ng + g) >= 30) {
+      has |= 1u << g;
+      n = min(n, st[g * 32]);
+    }
   const Fields F = fields_of(c, P.brmask);
-  const long long pt = P.toff[tile] + ip;
+  const long long pt = P.toff[tile] + ip0;
   const float* f = P.data + pt * F.n * 32 + lane;
   float* seg = P.seg + ((pt - P.pt0) * ndc + idl) * (long long)P.nseg * 32 + lane;
-  const int* st = P.stop + (long long)(tl * ndc + idl) * ng * 32 + lane;
-  float E = 0.f;
-  for (int g = 0; g < ng; g++) {
-    if (__ldg(T.np + (long long)id * ng + g) < 30) continue;
-    if (ip >= st[g * 32]) return;  // saturated: k_scan_m stops before
-    E = join_f(E, seg[g * 32]);
-  }
-  const float* kc = T.chanf + id * kChanConsts;
-  const float p = f[F.p * 32], t = f[F.t * 32], ds = f[F.ds * 32];
-  float beta = c.nw > 0 ? f[(F.kw0 + __float_as_int(kc[kChanWindow])) * 32] : 0.f;
-  if (P.cloud) {
-    const float cl = P.cloud[(long long)id * b.nray + r];
+  const long long sstep = (long long)ndc * P.nseg * 32;
+  float kc[kChanWindow];
+  for (int k = 0; k < kChanWindow; k++) kc[k] = T.chanf[id * kChanConsts + k];
+  const int on = continua_on(c, kc[kChanSwitches]);
+  const int kw = c.nw > 0 ? (F.kw0 + __float_as_int(T.chanf[id * kChanConsts + kChanWindow])) * 32 : -1;
+  const float cl = P.cloud ? P.cloud[(long long)id * b.nray + r] : __int_as_float(0x7fc00000);
+  const float* srf = T.srf + (long long)id * kNS;
+  for (int ip = ip0; ip < n; ip++, f += F.n * 32, seg += sstep) {
+    float E = 0.f;
+    for (int g = 0; g < ng; g++)
+      if ((has >> g) & 1u) E = join_f(E, seg[g * 32]);
+    const float p = f[F.p * 32], t = f[F.t * 32], ds = f[F.ds * 32];
+    float beta = kw >= 0 ? f[kw] : 0.f;
     if (cl == cl) beta = __fmaf_rn(f[F.aux * 32], cl, beta);
+    beta = continua_f(c, F, kc, on, f, p, t, ds, beta);
+    const float src = source_f(srf, t);
+    const float eps = segment_f(E, beta, ds);
+    seg[0] = __fmul_rn(src, eps);
+    seg[32] = __fsub_rn(1.f, eps);
   }
-  beta = continua_f(c, F, kc, continua_on(c, kc[kChanSwitches]), f, p, t, ds, beta);
-  const float src = source_f(T.srf + (long long)id * kNS, t);
-  const float eps = segment_f(E, beta, ds);
-  seg[0] = __fmul_rn(src, eps);
-  seg[32] = __fsub_rn(1.f, eps);
 }
 
 // Cloud extinction of every (channel, ray), NaN without a cloud.
@@ -1127,7 +1158,7 @@ __global__ void k_rowmeta(long long nrow, int tu, const int* nu, const float* u,
 // The rows interleaved {u[i], eps[i]}: a probe of one brings the other; marks
 // odd rows (kOddRow, from the entry that shows it).
 __global__ void k_interleave(long long n, int tu, const int* nu, const float* u, const float* e,
-                             int cga, float2* ue, float4* meta) {
+                             int cga, float2* ue, float4* meta, int* any_odd) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float a = u[i], b = e[i];
@@ -1137,17 +1168,20 @@ __global__ void k_interleave(long long n, int tu, const int* nu, const float* u,
   if (cnt < 2 || k >= cnt) return;
   const bool fine = fabsf(a) < 4.2535296e37f && fabsf(b) < 4.2535296e37f &&  // 2^125
                     (k + 1 >= cnt || (a <= u[i + 1] && b <= e[i + 1]));
-  if (!fine)
+  if (!fine) {
     atomicOr(reinterpret_cast<int*>(cga ? &meta[r].x : &meta[2 * r].w), kOddRow);
+    *any_odd = 1;
+  }
 }
 
 void launch_rowmeta(long long nrow, int tu, const int* nu, const float* u, const float* e, int cga,
-                    float4* meta, float2* ue, cudaStream_t s) {
+                    float4* meta, float2* ue, int* any_odd, cudaStream_t s) {
   const int bs = 256;
   if (nrow > 0) {
     k_rowmeta<<<(unsigned)((nrow + bs - 1) / bs), bs, 0, s>>>(nrow, tu, nu, u, e, cga, meta);
     const long long n = nrow * tu;
-    k_interleave<<<(unsigned)((n + bs - 1) / bs), bs, 0, s>>>(n, tu, nu, u, e, cga, ue, meta);
+    k_interleave<<<(unsigned)((n + bs - 1) / bs), bs, 0, s>>>(n, tu, nu, u, e, cga, ue, meta,
+                                                               any_odd);
   }
 }
 
@@ -1187,16 +1221,19 @@ void launch_gas_v(const CtlDev& c, const TblDev& T, const BatchDev& b, const Los
   constexpr int W = kPathThreads / 32;
   if (lanes_per_ray == 4) {
     const unsigned nblk = (unsigned)((nt * ndc * c.ng * 4 + W - 1) / W);
-    k_gas_m<CGA, 4, 8><<<nblk, kPathThreads, 0, s>>>(c, T, b, L, P, 0);
+    if (P.fast) k_gas_m<CGA, 4, 8, true><<<nblk, kPathThreads, 0, s>>>(c, T, b, L, P, 0);
+    else k_gas_m<CGA, 4, 8, false><<<nblk, kPathThreads, 0, s>>>(c, T, b, L, P, 0);
     return;
   }
   const int shape = variant / 4;
   const unsigned nblk = (unsigned)(shape ? (nt + W - 1) / W * ndc * c.ng : (nt * ndc * c.ng + W - 1) / W);
+  auto go = [&](auto kern) { kern<<<nblk, kPathThreads, 0, s>>>(c, T, b, L, P, shape); };
+  if (!P.fast) return go(k_gas_m<CGA, 1, 8, false>);
   switch (variant % 4) {
-    case 0: k_gas_m<CGA, 1, 8><<<nblk, kPathThreads, 0, s>>>(c, T, b, L, P, shape); break;
-    case 1: k_gas_m<CGA, 1, 10><<<nblk, kPathThreads, 0, s>>>(c, T, b, L, P, shape); break;
-    case 2: k_gas_m<CGA, 1, 12><<<nblk, kPathThreads, 0, s>>>(c, T, b, L, P, shape); break;
-    default: k_gas_m<CGA, 1, 16><<<nblk, kPathThreads, 0, s>>>(c, T, b, L, P, shape); break;
+    case 0: go(k_gas_m<CGA, 1, 8, true>); break;
+    case 1: go(k_gas_m<CGA, 1, 10, true>); break;
+    case 2: go(k_gas_m<CGA, 1, 12, true>); break;
+    default: go(k_gas_m<CGA, 1, 16, true>); break;
   }
 }
 
@@ -1210,7 +1247,8 @@ void launch_gas_m(const CtlDev& c, const TblDev& T, const BatchDev& b, const Los
 void launch_seg_scan_m(const CtlDev& c, const TblDev& T, const ChanDev& ch, const BatchDev& b,
                        const LosDev& L, const MixedPlan& P, int longest, cudaStream_t s) {
   const long long nt = P.tile1 - P.tile0, ndc = P.id1 - P.id0, nchb = (ndc + 3) / 4;
-  k_seg_m<<<dim3((unsigned)(nchb * longest), (unsigned)nt), kPathThreads, 0, s>>>(c, T, b, L, P);
+  const long long runs = (longest + kSegRun - 1) / kSegRun;
+  k_seg_m<<<dim3((unsigned)(nchb * runs), (unsigned)nt), kPathThreads, 0, s>>>(c, T, b, L, P);
   k_scan_m<<<(unsigned)((nt * ndc + 3) / 4), kPathThreads, 0, s>>>(c, T, ch, b, L, P);
 }
 
@@ -1239,12 +1277,16 @@ void launch_path_resume(const CtlDev& c, const TblDev& T, const ChanDev& ch, con
     kern<<<nblk, kPathThreads, smem, s>>>(c, T, ch, b, L, P);
   };
   const bool share = P.seg_base != nullptr;
+  auto pick = [&](auto cga, auto fast) {
+    if (share) go(k_path_mixed<8, cga.value, true, fast.value>);
+    else go(k_path_mixed<8, cga.value, false, fast.value>);
+  };
   if (c.formod == 0) {
-    if (share) go(k_path_mixed<8, true, true>);
-    else go(k_path_mixed<8, true, false>);
+    if (P.fast) pick(std::true_type{}, std::true_type{});
+    else pick(std::true_type{}, std::false_type{});
   } else {
-    if (share) go(k_path_mixed<8, false, true>);
-    else go(k_path_mixed<8, false, false>);
+    if (P.fast) pick(std::false_type{}, std::true_type{});
+    else pick(std::false_type{}, std::false_type{});
   }
 }
 

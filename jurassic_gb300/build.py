@@ -28,6 +28,7 @@ UNITS = {
     "jgb_path64.cu": ["-fmad=false"],
     "jgb_mixed.cu": ["-prec-div=false", "-ftz=true"],
     "jgb_api.cu": [],
+    "jgb_cholinv.cu": [],
     "jgb_noalloc.cu": [],
     "jgb_normal.cu": ["-fmad=false"],
     "jgb_retrieval.cu": ["-fmad=false"],

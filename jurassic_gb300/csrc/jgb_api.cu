@@ -1657,7 +1657,7 @@ void jgb_destroy(jgb_ctx* x) {
                     &x->b_tp, &x->b_mask, &x->b_p, &x->los_off, &x->los_cnt, &x->los_cnt64,
                     &x->los_sft, &x->los_ends, &x->los_planes, &x->lev_slopes, &x->scan_tmp, &x->err_word,
                     &x->tiles_perm, &x->tiles_keys, &x->tiles_keys2, &x->tiles_vals,
-                    &x->tiles_off, &x->tiles_len, &x->tiles_data, &x->ne_desc, &x->ne_split, &x->seg,
+                    &x->tiles_off, &x->tiles_len, &x->tiles_data, &x->inv_work, &x->ne_desc, &x->ne_split, &x->seg,
                     &x->rs_start, &x->rs_lists, &x->rs_snap, &x->rs_base, &x->rs_seg, &x->rs_trace,
                     &x->d_fov, &x->fov_raw,
                     &x->kx_levoff, &x->kx_rayoff, &x->kx_rayobs, &x->kx_src, &x->kx_lev,

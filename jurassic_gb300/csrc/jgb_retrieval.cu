@@ -25,6 +25,7 @@
 #include <string>
 #include <vector>
 
+#include "jgb_cholinv.cuh"
 #include "jgb_ctx.h"
 #include "jgb_internal.h"
 
@@ -357,32 +358,27 @@ __global__ void k_diag_inverse(int nret, const RetDesc* d, const int* active, do
 }
 
 // The diagonal test of matrix_invert (retrieval.c:379-385: any element right
-// of the diagonal other than 0, NaN included, makes the matrix full):
-// diag[i] / full[i] select the two branches, status[i] starts at 0.
-__global__ void k_invert_flags(int nret, const RetDesc* d, const double* A, int* diag, int* full,
-                               int* status) {
+// of the diagonal other than 0, NaN included, makes the matrix full), the
+// reciprocal diagonal of the diagonal ones, and the others' flags.
+__global__ void k_invert_flags(const InvertDesc* d, double* A, int* full, int* status) {
   const int i = blockIdx.x;
-  if (i >= nret) return;
   const int n = d[i].n;
-  const double* M = A + d[i].so;
+  double* M = A + d[i].off;
   int nz = 0;
-  for (long long e = threadIdx.x; e < (long long)n * n; e += blockDim.x) {
-    const int r = (int)(e / n), c = (int)(e % n);
-    if (c > r && M[e] != 0) nz = 1;
+  for (int r = 0; r < n && !nz; r += 8) {  // rows at a time: a full matrix ends early
+    for (int q = r; q < min(r + 8, n); q++)
+      for (int c = q + 1 + threadIdx.x; c < n; c += blockDim.x) nz |= M[(long long)q * n + c] != 0;
+    nz = __syncthreads_or(nz);
   }
-  nz = __syncthreads_or(nz);
   if (threadIdx.x == 0) {
-    diag[i] = !nz;
     full[i] = nz;
     status[i] = 0;
   }
-}
-
-// Matrices whose factor failed (status 1) take no inverse: they keep their
-// input.
-__global__ void k_drop_failed(int nret, const int* status, int* full) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < nret && status[i]) full[i] = 0;
+  if (!nz)
+    for (int j = threadIdx.x; j < n; j += blockDim.x) {
+      double* v = M + (long long)j * n + j;
+      *v = 1 / *v;
+    }
 }
 
 // a-priori covariance (set_cov_apr, retrieval.c:808-920): per element
@@ -1863,41 +1859,33 @@ extern "C" int jgb_matrix_invert_dev(jgb_ctx* x, int nret, const int* n, double*
   rc = JGB_OK;  // tables are not needed: a context without them is fine
   cudaSetDevice(v.device);
   (void)cudaGetLastError();  // launch errors below are this call's
-  std::vector<RetDesc> desc(nret);
+  std::vector<InvertDesc> desc(nret);
   long long so = 0;
   int nmax = 1;
   for (int i = 0; i < nret; i++) {
     if (n[i] <= 0) return ctx_error(x, JGB_ERR_ARG, "empty matrix");
-    desc[i] = RetDesc{n[i], 0, 0, 0, so, 0};
+    desc[i] = InvertDesc{n[i], so};
     so += (long long)n[i] * n[i];
     nmax = std::max(nmax, n[i]);
   }
-  // scratch: descriptors, flags and status, the factors, the column solves
-  const size_t b_desc = (sizeof(RetDesc) * (size_t)nret + 255) & ~size_t(255);
-  const size_t b_flags = (sizeof(int) * 3 * (size_t)nret + 255) & ~size_t(255);
-  void* buf = nullptr;
-  if (cudaMalloc(&buf, b_desc + b_flags + sizeof(double) * 2 * (size_t)so) != cudaSuccess)
+  // scratch of the context (under its lock): descriptors, flags and status,
+  // the factors and their inverses
+  const size_t b_desc = (sizeof(InvertDesc) * (size_t)nret + 255) & ~size_t(255);
+  const size_t b_flags = (sizeof(int) * 2 * (size_t)nret + 255) & ~size_t(255);
+  if (x->inv_work.reserve(b_desc + b_flags + sizeof(double) * 2 * (size_t)so) != cudaSuccess)
     return ctx_error(x, JGB_ERR_CUDA, "cudaMalloc failed");
-  char* p = static_cast<char*>(buf);
-  RetDesc* d = reinterpret_cast<RetDesc*>(p);
-  int* diag = reinterpret_cast<int*>(p + b_desc);
-  int* full = diag + nret;
+  char* p = x->inv_work.as<char>();
+  InvertDesc* d = reinterpret_cast<InvertDesc*>(p);
+  int* full = reinterpret_cast<int*>(p + b_desc);
   int* st = full + nret;
   double* L = reinterpret_cast<double*>(p + b_desc + b_flags);
   double* W = L + so;
   cudaStream_t s = v.stream;
-  cudaEvent_t e0, e1;
-  cudaEventCreate(&e0);
-  cudaEventCreate(&e1);
-  cudaMemcpyAsync(d, desc.data(), sizeof(RetDesc) * nret, cudaMemcpyHostToDevice, s);
+  cudaEvent_t e0 = x->ev[0], e1 = x->ev[1];
+  cudaMemcpyAsync(d, desc.data(), sizeof(InvertDesc) * nret, cudaMemcpyHostToDevice, s);
   cudaEventRecord(e0, s);
-  k_invert_flags<<<nret, 256, 0, s>>>(nret, d, A, diag, full, st);
-  k_diag_inverse<<<nret, 128, 0, s>>>(nret, d, diag, A);
-  k_select_nn<<<dim3(16, nret), 256, 0, s>>>(nret, d, full, A, L);
-  k_chol_factor<<<nret, 1024, 0, s>>>(nret, d, full, L, st);
-  k_drop_failed<<<(nret + 255) / 256, 256, 0, s>>>(nret, st, full);
-  k_chol_inverse_cols<<<dim3((nmax + 63) / 64, nret), 64, 0, s>>>(nret, d, full, L, W);
-  k_sym_half<<<dim3(16, nret), 256, 0, s>>>(nret, d, full, W, A);
+  k_invert_flags<<<nret, 256, 0, s>>>(d, A, full, st);
+  matrix_invert_blocked(nret, nmax, d, full, st, A, L, W, s);
   cudaEventRecord(e1, s);
   cudaError_t err = cudaGetLastError();
   std::vector<int> hst(nret);
@@ -1906,9 +1894,6 @@ extern "C" int jgb_matrix_invert_dev(jgb_ctx* x, int nret, const int* n, double*
   if (err == cudaSuccess) err = cudaStreamSynchronize(s);
   if (err == cudaSuccess && kernel_ms) cudaEventElapsedTime(kernel_ms, e0, e1);
   if (err == cudaSuccess && status) std::memcpy(status, hst.data(), sizeof(int) * nret);
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  cudaFree(buf);
   if (err != cudaSuccess)
     return ctx_error(x, JGB_ERR_CUDA,
                      std::string("matrix inversion kernels: ") + cudaGetErrorString(err));

@@ -127,6 +127,48 @@ __device__ inline double solar_zenith(double sec, double lon, double lat) {
   return acos(sin(latr) * sin(dec) + cos(latr) * cos(dec) * cos(h)) * (180.0 / kPI);
 }
 
+#ifdef __CUDACC__
+// ---------------------------------------------------------------------------
+// FP64 values on the integer pipe.  A conversion or a compare of doubles holds
+// an SM for 16 to 19 cycles per warp instruction on GB300, like any other FP64
+// instruction.  The rare forms are calls: inline they become predicated
+// conversions that every value pays for.
+static __device__ __noinline__ double f2d_rare(float f) { return (double)f; }
+static __device__ __noinline__ float d2f_rare(double x) { return (float)x; }
+
+// (double)f: subnormal, infinite and NaN inputs by the conversion.
+__device__ __forceinline__ double f2d_bits(float f) {
+  const unsigned u = __float_as_uint(f);
+  if ((u & 0x7fffffffu) - 0x00800000u < 0x7f000000u)
+    return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + (896u << 20))),
+                            (int)(u << 29));
+  return u == 0u ? 0.0 : f2d_rare(f);
+}
+
+// (float)x, rounded to nearest even: results outside the normal range,
+// infinities and NaN by the conversion.
+__device__ __forceinline__ float d2f_bits(double x) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const unsigned mag = hi & 0x7fffffffu, rest = lo & 0x1fffffffu;
+  if (mag - (897u << 20) >= (253u << 20))
+    return (mag | lo) == 0u ? __uint_as_float(hi) : d2f_rare(x);
+  const unsigned f = ((mag - (896u << 20)) << 3) | (lo >> 29);
+  return __uint_as_float((hi & 0x80000000u) |
+                         (f + (rest > 0x10000000u || (rest == 0x10000000u && (f & 1u)) ? 1u : 0u)));
+}
+
+// a < b for doubles that are not NaN
+__device__ __forceinline__ long long order_key(double v) {
+  const long long k = __double_as_longlong(v);
+  return k < 0 ? (long long)(0x8000000000000000ULL - (unsigned long long)k) : k;  // -0 == 0
+}
+__device__ __forceinline__ bool lt(double a, double b) { return order_key(a) < order_key(b); }
+// false for NaN
+__device__ __forceinline__ bool is_number(double v) {
+  return (__double2hiint(v) & 0x7fffffff) <= 0x7ff00000;
+}
+#endif
+
 // ---------------------------------------------------------------------------
 // Device-resident views (plain pointers into context-owned buffers)
 

@@ -92,14 +92,6 @@ __global__ void k_level_slopes(CtlDev c, BatchDev b, double* out) {
   }
 }
 
-// Comparison of finite doubles on the integer pipe (an FP64 compare holds the
-// SM for 19 cycles).
-__device__ __forceinline__ long long order_key(double v) {
-  const long long k = __double_as_longlong(v);
-  return k ^ ((k >> 63) & 0x7fffffffffffffffLL);
-}
-__device__ __forceinline__ bool lt(double a, double b) { return order_key(a) < order_key(b); }
-
 // One level interval with its slopes.
 struct Lev64 {
   int i;
@@ -305,7 +297,7 @@ __device__ int walk(const CtlDev& c, const AtmView& a, const double* g, long lon
     }
     z = norm - kRE;
     // a position that is not a number is inside: the walk ends with an overflow
-    const bool num = (__double2hiint(z) & 0x7fffffff) <= 0x7ff00000;
+    const bool num = is_number(z);
     const bool low = num && lt(z, zmin), high = num && lt(zmax, z);
     if ((low || high) && n > 0) {
       if (!STORE) {  // the clipped last point ends the count
@@ -593,7 +585,7 @@ __global__ void __launch_bounds__(32)
     }
     double z = norm - kRE;
     // a position that is not a number is inside: the walk ends with an overflow
-    const bool num = (__double2hiint(z) & 0x7fffffff) <= 0x7ff00000;
+    const bool num = is_number(z);
     const bool low = num && lt(z, zmin), high = num && lt(zmax, z);
     if (alive && (low || high) && n > 0) {
       stop = low ? 2 : 1;

@@ -130,36 +130,6 @@ __global__ void k_wait_selftest(int arrive, unsigned long long* out) {
   out[1] = global_ns() - t0;
 }
 
-// Exact float -> double widening with integer operations on the two 32-bit
-// words (the FP64 pipe of GB300 is narrow): for a normal float the high word
-// is the sign, the exponent rebiased by 1023 - 127 and the top 20 mantissa
-// bits, the low word the last 3 mantissa bits; zero, subnormal, infinite
-// and NaN inputs take the conversion instruction, in a call: inline it
-// becomes a predicated conversion that every value pays for (16 cycles of the
-// SM per warp).
-__device__ __noinline__ double f2d_rare(float f) { return (double)f; }
-
-__device__ __forceinline__ double f2d_bits(float f) {
-  const unsigned u = __float_as_uint(f);
-  if ((u & 0x7fffffffu) - 0x00800000u >= 0x7f000000u)
-    return u == 0u ? 0.0 : f2d_rare(f);
-  const unsigned hi = (u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + (896u << 20));
-  return __hiloint2double((int)hi, (int)(u << 29));
-}
-
-// (float)x, rounded to nearest even on the integer pipe; results outside the
-// normal range, infinities and NaN by the conversion (as above, in a call).
-__device__ __noinline__ float d2f_rare(double x) { return (float)x; }
-
-__device__ __forceinline__ float d2f_bits(double x) {
-  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
-  const unsigned mag = hi & 0x7fffffffu, rest = lo & 0x1fffffffu;
-  if (mag - (897u << 20) >= (253u << 20)) return (mag | lo) == 0u ? __uint_as_float(hi) : d2f_rare(x);
-  const unsigned f = ((mag - (896u << 20)) << 3) | (lo >> 29);
-  return __uint_as_float((hi & 0x80000000u) |
-                         (f + (rest > 0x10000000u || (rest == 0x10000000u && (f & 1u)) ? 1u : 0u)));
-}
-
 // X = sqrt(W)[K | dy] of every problem, formed once in FP64 and split into
 // a TF32 high part and a TF32-rounded remainder, written in the operand
 // layout of the tensor-core product: per (column tile ti, chunk c of kChunk

@@ -223,7 +223,6 @@ __global__ void __launch_bounds__(128) k_prep64(CtlDev c, TblDev T, LosDev L, Pa
 // conversions and compares that every pass through the FP64 pipe pays for
 // (105 instead of 56 FP64 instructions per step of k_gas64).
 __device__ __noinline__ float round_down_slow(double x) { return __double2float_rd(x); }
-__device__ __noinline__ double widen_slow(float f) { return (double)f; }
 __device__ __noinline__ bool above_slow(double x, float g) { return x > (double)g; }
 
 // x rounded down to float (toward zero for x >= 0): for a float g, g <= x,
@@ -241,17 +240,6 @@ __device__ __forceinline__ float round_down_f(double x) {
 __device__ __forceinline__ bool above_f(double x, float d, float g) {
   if (d == g) return above_slow(x, g);
   return d > g;
-}
-
-// Exact widening on the integer pipe (subnormal, inf and NaN by the
-// conversion).
-__device__ __forceinline__ double widen(float f) {
-  const unsigned u = __float_as_uint(f);
-  if ((u & 0x7fffffffu) - 0x00800000u < 0x7f000000u)
-    return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + (896u << 20))),
-                            (int)(u << 29));
-  if (u == 0u) return 0.0;
-  return widen_slow(f);
 }
 
 // e < 1 ? e : 1, then e > 0 ? e : 0 (NaN gives 1), without FP64 compares
@@ -372,7 +360,7 @@ __device__ __forceinline__ double corner64(const TblDev& T, unsigned r, double e
       hi = k.b;
       inside = mono;
     }
-    u = widen(lo.x) + widen((hi.x - lo.x) / (hi.y - lo.y)) * (e - widen(lo.y)) + du;
+    u = f2d_bits(lo.x) + f2d_bits((hi.x - lo.x) / (hi.y - lo.y)) * (e - f2d_bits(lo.y)) + du;
     if (up) {
       u = u_above(un, en, e) + du;
       ib = n - 2;
@@ -406,7 +394,7 @@ __device__ __forceinline__ double corner64(const TblDev& T, unsigned r, double e
     }
   }
   if (up) return eps_above(un, en, u);
-  return widen(lo.y) + widen((hi.y - lo.y) / (hi.x - lo.x)) * (u - widen(lo.x));
+  return f2d_bits(lo.y) + f2d_bits((hi.y - lo.y) / (hi.x - lo.x)) * (u - f2d_bits(lo.x));
 }
 
 // ---------------------------------------------------------------------------

@@ -73,17 +73,26 @@ struct Lev {
   bool first, last; // lowest / highest interval (extrapolation below / above)
 };
 
+// x / y > 0, the division only where it might underflow or has special
+// operands: positive numbers between 1e-154 and 1e154 need none.
+static __device__ __noinline__ bool ratio_positive_rare(double x, double y) { return x / y > 0; }
+__device__ __forceinline__ bool ratio_positive(double x, double y) {
+  const unsigned hx = (unsigned)__double2hiint(x), hy = (unsigned)__double2hiint(y);
+  if (hx - (512u << 20) < (1023u << 20) && hy - (512u << 20) < (1023u << 20)) return true;
+  return ratio_positive_rare(x, y);
+}
+
 __device__ inline void lev_load(const AtmM& a, int i, Lev& L) {
   L.i = i;
   L.first = i == 0;
   L.last = i == a.np - 2;
   L.z0 = a.z[i];
-  L.dz = (float)(a.z[i + 1] - a.z[i]);
-  L.p0 = (float)a.p[i];
-  L.p1 = (float)a.p[i + 1];
-  L.t0 = (float)a.t[i];
-  L.t1 = (float)a.t[i + 1];
-  L.plog = (a.p[i + 1] / a.p[i]) > 0;
+  L.dz = d2f_bits(a.z[i + 1] - a.z[i]);
+  L.p0 = d2f_bits(a.p[i]);
+  L.p1 = d2f_bits(a.p[i + 1]);
+  L.t0 = d2f_bits(a.t[i]);
+  L.t1 = d2f_bits(a.t[i + 1]);
+  L.plog = ratio_positive(a.p[i + 1], a.p[i]);
   L.sp = L.plog ? logf(L.p1 / L.p0) / L.dz : (L.p1 - L.p0) / L.dz;
   L.st = (L.t1 - L.t0) / L.dz;
 }
@@ -102,13 +111,13 @@ __device__ inline bool lev_holds(const Lev& L, float dl) {
 // so the hints change no result.
 __device__ inline float lev_find(const AtmM& a, double z, Lev& L) {
   if (L.i >= 0) {
-    const float dl = (float)(z - L.z0);
+    const float dl = d2f_bits(z - L.z0);
     if (lev_holds(L, dl)) return dl;
     const int j = dl < 0.f ? L.i - 1 : L.i + 1;
     if (j >= 0 && j <= a.np - 2) {
       Lev M;
       lev_load(a, j, M);
-      const float dm = (float)(z - M.z0);
+      const float dm = d2f_bits(z - M.z0);
       if (lev_holds(M, dm)) {
         L = M;
         return dm;
@@ -116,7 +125,7 @@ __device__ inline float lev_find(const AtmM& a, double z, Lev& L) {
     }
   }
   lev_load(a, bracket_irr(a.z, a.np, z), L);
-  return (float)(z - L.z0);
+  return d2f_bits(z - L.z0);
 }
 
 __device__ inline void lev_pt(const Lev& L, float dl, float* p, float* t) {
@@ -196,7 +205,7 @@ __device__ __forceinline__ void level_values(const CtlDev& c, const AtmM& a, int
   const int nqk = c.ng + c.nw;
   for (int k = 0; k < nqk; k++) {
     const double* src = k < c.ng ? a.q + k * a.stride : a.k + (k - c.ng) * a.stride;
-    const float v0 = (float)src[i], v1 = (float)src[i + 1];
+    const float v0 = d2f_bits(src[i]), v1 = d2f_bits(src[i + 1]);
     qc[k * kTraceThreads] = v0;
     qc[(nqk + k) * kTraceThreads] = (v1 - v0) / dz;
   }
@@ -210,28 +219,20 @@ __host__ __device__ inline int trace_smem_floats(const CtlDev& c) {
   return 2 * (c.ng + c.nw) + c.ng + (c.formod == 0 ? 6 * c.ng : 0);
 }
 
-// STORE places every point with its final values: its trapezoid length
-// 0.5 (ds_(i-1) + ds_i), column densities 10 / k_B q p / T ds and CGA sums
-// are written when the next point is placed (the clip of the last segment
-// changes the previous point's raw length), so the walk keeps the raw
-// lengths of the last two points.
-// ROLE 1 keeps every point's position, direction, raw length and level
-// interval in sv; ROLE 2 with wf walks on from the state wf (a base ray's
-// walk).
-template <bool STORE, int ROLE = 0>
-__device__ int walk_m(const CtlDev& c, const AtmM& a, const double* g, long long nray, int r,
-                      const LosDev& L, long long base, int cap, double* sft_out, GeoKeep* gk,
-                      float* qc, unsigned* err, const WalkFrom* wf = nullptr,
-                      const TraceResume* sv = nullptr) {
-  const float h = 0.02f;
-  const double zrefrac = 60;
-  *sft_out = -999;
-  const double obsz = g[1 * nray + r], obslon = g[2 * nray + r], obslat = g[3 * nray + r];
-  const double vpz = g[4 * nray + r], vplon = g[5 * nray + r], vplat = g[6 * nray + r];
+// a < b on the integer pipe, false for NaN
+__device__ __forceinline__ bool less(double a, double b) {
+  return is_number(a) && is_number(b) && lt(a, b);
+}
+
+// The altitudes that end ray r: 1, or 0 for a ray above the atmosphere, -1 on
+// error.
+__device__ int ray_bounds_m(const CtlDev& c, const AtmM& a, const double* g, long long nray, int r,
+                            double* zlo, double* zhi, unsigned* err) {
+  const double obsz = g[1 * nray + r], vpz = g[4 * nray + r];
   double zmin = a.z[0], zmax = a.z[0];
   for (int i = 0; i < a.np; i++) {
-    zmin = a.z[i] < zmin ? a.z[i] : zmin;
-    zmax = a.z[i] > zmax ? a.z[i] : zmax;
+    zmin = less(a.z[i], zmin) ? a.z[i] : zmin;
+    zmax = less(zmax, a.z[i]) ? a.z[i] : zmax;
   }
   if (c.nsf > 0) {
     zmin = a.sfz > zmin ? a.sfz : zmin;
@@ -245,7 +246,57 @@ __device__ int walk_m(const CtlDev& c, const AtmM& a, const double* g, long long
     atomicOr(err, kErrObserverBelowSurface);
     return -1;
   }
-  if (vpz > zmax) return 0;
+  *zlo = zmin;
+  *zhi = zmax;
+  return vpz > zmax ? 0 : 1;
+}
+
+// Position, direction and altitude of ray r's first point.
+__device__ void ray_first_m(const double* g, long long nray, int r, double zmax, double* x,
+                            double* ex0, double* zout) {
+  const double obsz = g[1 * nray + r], obslon = g[2 * nray + r], obslat = g[3 * nray + r];
+  const double vpz = g[4 * nray + r], vplon = g[5 * nray + r], vplat = g[6 * nray + r];
+  double z;
+  double xobs[3], xvp[3];
+  to_cart(obsz, obslon, obslat, xobs);
+  to_cart(vpz, vplon, vplat, xvp);
+  for (int i = 0; i < 3; i++) ex0[i] = xvp[i] - xobs[i];
+  const double norm = sqrt(ex0[0] * ex0[0] + ex0[1] * ex0[1] + ex0[2] * ex0[2]);
+  for (int i = 0; i < 3; i++) {
+    ex0[i] /= norm;
+    x[i] = xobs[i];
+  }
+  z = obsz;
+  if (obsz > zmax) {  // entry into the atmosphere: bisection on the line of sight (FP64, once)
+    double dmax = norm, dmin = 0;
+    for (int guard = 0; fabs(dmin - dmax) > 0.001 && guard < 200; guard++) {
+      const double d = (dmax + dmin) / 2;
+      for (int i = 0; i < 3; i++) x[i] = xobs[i] + d * ex0[i];
+      z = sqrt(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]) - kRE;
+      if (z <= zmax && z > zmax - 0.001) break;
+      if (z < zmax - 0.0005) dmax = d; else dmin = d;
+    }
+  }
+  z = sqrt(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]) - kRE;
+  *zout = z;
+}
+
+// STORE places every point with its final values: its trapezoid length
+// 0.5 (ds_(i-1) + ds_i), column densities 10 / k_B q p / T ds and CGA sums
+// are written when the next point is placed (the clip of the last segment
+// changes the previous point's raw length), so the walk keeps the raw
+// lengths of the last two points.
+// With wf it walks on from the state wf (a base ray's walk).
+template <bool STORE>
+__device__ int walk_m(const CtlDev& c, const AtmM& a, const double* g, long long nray, int r,
+                      const LosDev& L, long long base, int cap, double* sft_out, GeoKeep* gk,
+                      float* qc, unsigned* err, const WalkFrom* wf = nullptr) {
+  const float h = 0.02f;
+  const double zrefrac = 60;
+  *sft_out = -999;
+  double zmin, zmax;
+  const int ok = ray_bounds_m(c, a, g, nray, r, &zmin, &zmax, err);
+  if (ok <= 0) return ok;
 
   // the direction stays FP64: renormalising an FP32 unit vector every step
   // would random-walk it by ~1e-7 rad per step (metres over a limb path)
@@ -254,7 +305,7 @@ __device__ int walk_m(const CtlDev& c, const AtmM& a, const double* g, long long
   Lev lv;
   lv.i = -1;
   int n = 0, stop = 0, qc_level = -1;
-  if (ROLE == 2 && wf) {  // on from a base's walk
+  if (STORE && wf) {  // on from a base's walk
     for (int i = 0; i < 3; i++) {
       x[i] = wf->x[i];
       ex0[i] = wf->e[i];
@@ -265,27 +316,7 @@ __device__ int walk_m(const CtlDev& c, const AtmM& a, const double* g, long long
     n = wf->n;
     lev_load(a, wf->lev_last, lv);
   } else {
-    double xobs[3], xvp[3];
-    to_cart(obsz, obslon, obslat, xobs);
-    to_cart(vpz, vplon, vplat, xvp);
-    for (int i = 0; i < 3; i++) ex0[i] = xvp[i] - xobs[i];
-    const double norm = sqrt(ex0[0] * ex0[0] + ex0[1] * ex0[1] + ex0[2] * ex0[2]);
-    for (int i = 0; i < 3; i++) {
-      ex0[i] /= norm;
-      x[i] = xobs[i];
-    }
-    z = obsz;
-    if (obsz > zmax) {  // entry into the atmosphere: bisection on the line of sight (FP64, once)
-      double dmax = norm, dmin = 0;
-      for (int guard = 0; fabs(dmin - dmax) > 0.001 && guard < 200; guard++) {
-        const double d = (dmax + dmin) / 2;
-        for (int i = 0; i < 3; i++) x[i] = xobs[i] + d * ex0[i];
-        z = sqrt(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]) - kRE;
-        if (z <= zmax && z > zmax - 0.001) break;
-        if (z < zmax - 0.0005) dmax = d; else dmin = d;
-      }
-    }
-    z = sqrt(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]) - kRE;
+    ray_first_m(g, nray, r, zmax, x, ex0, &z);
   }
   const int nqk = c.ng + c.nw;
   const float rayds = (float)c.rayds, raydz = (float)c.raydz;
@@ -297,7 +328,7 @@ __device__ int walk_m(const CtlDev& c, const AtmM& a, const double* g, long long
   float* cg = STORE ? pq + c.ng * kTraceThreads : nullptr;
   float raw_before = 0.f, raw_pend = 0.f, pend_p = 0.f, pend_t = 0.f;
   const int n0 = n;
-  if (ROLE == 2 && wf) raw_pend = wf->raw_last;
+  if (STORE && wf) raw_pend = wf->raw_last;
   if (STORE && L.cga)
     for (int k = 0; k < 6 * c.ng; k++) cg[k * kTraceThreads] = 0.f;
   auto finalize = [&](int k) {
@@ -337,8 +368,8 @@ __device__ int walk_m(const CtlDev& c, const AtmM& a, const double* g, long long
   for (;;) {
     // radial unit vector and radius at x
     const double rr = z + kRE;
-    const float rf = (float)rr, rinv = 1.f / rf;
-    float xh[3] = {(float)x[0] * rinv, (float)x[1] * rinv, (float)x[2] * rinv};
+    const float rf = d2f_bits(rr), rinv = 1.f / rf;
+    float xh[3] = {d2f_bits(x[0]) * rinv, d2f_bits(x[1]) * rinv, d2f_bits(x[2]) * rinv};
     // step length from this point (jurassic.c:4278-4287)
     float step = rayds;
     if (raydz > 0) {
@@ -347,7 +378,8 @@ __device__ int walk_m(const CtlDev& c, const AtmM& a, const double* g, long long
     }
     // ground or top of the atmosphere: clip the last segment (4292-4306;
     // the previous point's step becomes this point's step times frac)
-    if ((z < zmin || z > zmax) && n > 0) {
+    const bool low = less(z, zmin);
+    if ((low || less(zmax, z)) && n > 0) {
       if (!STORE) {
         if (n >= cap) {
           atomicOr(err, cap < c.nlos_max ? kErrSlabOverflow : kErrLosOverflow);
@@ -355,13 +387,12 @@ __device__ int walk_m(const CtlDev& c, const AtmM& a, const double* g, long long
         }
         return n + 1;
       }
-      stop = (z < zmin ? 2 : 1);
-      const double frac = ((z < zmin ? zmin : zmax) - last_z) / (z - last_z);
+      stop = low ? 2 : 1;
+      const double frac = ((low ? zmin : zmax) - last_z) / (z - last_z);
       for (int i = 0; i < 3; i++) x[i] = x_last[i] + frac * (x[i] - x_last[i]);
       z = last_z + frac * (z - last_z);
       const double dsc = (double)step * frac;
       raw_pend = (float)dsc;
-      if (ROLE == 1) sv->dsr[base + n - 1] = raw_pend;
       gk->ds_clip = dsc;
       step = 0.f;
     }
@@ -395,15 +426,6 @@ __device__ int walk_m(const CtlDev& c, const AtmM& a, const double* g, long long
       for (int iw = 0; iw < c.nw; iw++)
         L.f.kw[iw * L.cap + s] = qk_at(qc[(c.ng + iw) * kTraceThreads],
                                        qc[(nqk + c.ng + iw) * kTraceThreads], dl);
-      if (ROLE == 1) {
-        const long long bp = sv->bpts;
-        for (int i2 = 0; i2 < 3; i2++) {
-          sv->xs[i2 * bp + s] = x[i2];
-          sv->es[i2 * bp + s] = ex0[i2];
-        }
-        sv->lev[s] = i;
-        sv->dsr[s] = step;
-      }
       if (c.ncl > 0 && a.cldz > 0) {
         const float v = (float)((z - a.clz) / a.cldz);
         L.f.aux[s] = expf(-0.5f * v * v);
@@ -418,7 +440,7 @@ __device__ int walk_m(const CtlDev& c, const AtmM& a, const double* g, long long
         gk->ds_p1 = step;
         gk->want_p1 = false;
       }
-      if (n == 0 || z < gk->zmin_seen) {
+      if (n == 0 || less(z, gk->zmin_seen)) {
         gk->zmin_seen = z;
         gk->imin = n;
         gk->ds_m = step;
@@ -441,7 +463,7 @@ __device__ int walk_m(const CtlDev& c, const AtmM& a, const double* g, long long
     // refraction (jurassic.c:4388-4415): ex1 = (n ex0 + ds grad N) / |...|
     // = (ex0 + inc) / |ex0 + inc| with inc = ds grad N / n, the increment in
     // FP32 and the renormalisation as a series in delta = |ex0 + inc|^2 - 1
-    const bool bend = c.refrac && z <= zrefrac;
+    const bool bend = c.refrac && is_number(z) && !lt(zrefrac, z);
     double ex1[3] = {ex0[0], ex0[1], ex0[2]};
     if (bend) {
       const float nref = 1.f + kRefracC * p / t;
@@ -454,7 +476,7 @@ __device__ int walk_m(const CtlDev& c, const AtmM& a, const double* g, long long
       // midpoint offset in the point's interval (FP64 only when it leaves it)
       Lev lh = lv;
       float dlh = dl + dzh;
-      if (!lev_holds(lh, dlh)) dlh = lev_find(a, z + dzh, lh);
+      if (!lev_holds(lh, dlh)) dlh = lev_find(a, z + f2d_bits(dzh), lh);
       float ph, th;
       lev_pt(lh, dlh, &ph, &th);
       float inc[3];
@@ -467,7 +489,7 @@ __device__ int walk_m(const CtlDev& c, const AtmM& a, const double* g, long long
           dN = dN_in(lh, ph, th, dlk);
         } else {
           // split at the level boundary between the midpoint and zk
-          const double zh = lh.z0 + (double)dlh, zk = zh + dlk;
+          const double zh = lh.z0 + f2d_bits(dlh), zk = zh + f2d_bits(dlk);
           Lev lk = lh;
           const float dlk0 = lev_find(a, zk, lk);
           if (lk.i == lh.i) {
@@ -475,10 +497,10 @@ __device__ int walk_m(const CtlDev& c, const AtmM& a, const double* g, long long
           } else {
             const bool up = lk.i > lh.i;
             const double zb = up ? a.z[lh.i + 1] : a.z[lh.i];
-            const float d1 = (float)(zb - zh);
+            const float d1 = d2f_bits(zb - zh);
             const float dn1 = dN_in(lh, ph, th, d1);
             float pb, tb;
-            const float dlb = (float)(zb - lk.z0);
+            const float dlb = d2f_bits(zb - lk.z0);
             lev_pt(lk, dlb, &pb, &tb);
             dN = dn1 + dN_in(lk, pb, tb, dlk0 - dlb);
           }
@@ -487,10 +509,10 @@ __device__ int walk_m(const CtlDev& c, const AtmM& a, const double* g, long long
       }
       const float delta = 2.f * (ef[0] * inc[0] + ef[1] * inc[1] + ef[2] * inc[2]) +
                           (inc[0] * inc[0] + inc[1] * inc[1] + inc[2] * inc[2]);
-      for (int k = 0; k < 3; k++) ex1[k] = ex0[k] + (double)inc[k];
+      for (int k = 0; k < 3; k++) ex1[k] = ex0[k] + f2d_bits(inc[k]);
       if (fabsf(delta) < 1e-3f) {
         const float corr = delta * (-0.5f + delta * (0.375f - 0.3125f * delta));
-        for (int k = 0; k < 3; k++) ex1[k] += ex1[k] * (double)corr;
+        for (int k = 0; k < 3; k++) ex1[k] += ex1[k] * f2d_bits(corr);
       } else {
         const double nn = sqrt(ex1[0] * ex1[0] + ex1[1] * ex1[1] + ex1[2] * ex1[2]);
         for (int k = 0; k < 3; k++) ex1[k] /= nn;
@@ -498,16 +520,16 @@ __device__ int walk_m(const CtlDev& c, const AtmM& a, const double* g, long long
     }
     float D[3], efn[3];
     for (int k = 0; k < 3; k++) {
-      efn[k] = (float)ex1[k];
+      efn[k] = d2f_bits(ex1[k]);
       D[k] = 0.5f * step * (ef[k] + efn[k]);
     }
     const float dzs = dz_of(xh, rf, D);
     for (int k = 0; k < 3; k++) {
-      x[k] += (double)D[k];
+      x[k] += f2d_bits(D[k]);
       ex0[k] = ex1[k];
       ef[k] = efn[k];
     }
-    z += dzs;
+    z += f2d_bits(dzs);
   }
   return n;
 }
@@ -639,96 +661,11 @@ __device__ void copy_base_geometry(const CtlDev& c, const BatchDev& b, const Los
   }
 }
 
-// order (optional): thread t traces ray order[t], else ray r0 + t, so that a
-// warp's rays have similar LOS capacities and finish together; each ray's
-// outputs go to its own slots, so the order does not change any result.
-// ROLE 0: plain rays; 1: base rays of resumed perturbations (their walks are
-// kept in R); 2: the perturbations (R.plan; EGA only: the Curtis-Godson sums
-// run from the first point).
-template <int ROLE>
-__global__ void k_trace_fill_m(CtlDev c, BatchDev b, LosDev L, const int* order, int r0, int nr_l,
-                               TraceResume R, unsigned* err) {
-  const int th = blockIdx.x * blockDim.x + threadIdx.x;
-  if (th >= nr_l) return;
-  const int r = order ? order[th] : r0 + th;
-  if (b.obs_skip && b.obs_skip[b.ray_obs[r]]) {
-    L.count[r] = 0;
-    return;
-  }
-  const AtmM a = atm_m(b, c, b.ray_obs[r]);
+// What a ray leaves beside its points: count, surface temperature, tangent
+// point and ends.
+__device__ void ray_finish_m(const BatchDev& b, const LosDev& L, int r, int n, double sft,
+                             const GeoKeep& gk) {
   const long long base = L.off[r];
-  const int cap = L.count[r];
-  extern __shared__ float qcache[];  // trace_smem_floats(c) per thread
-  int4 pl = make_int4(-1, 0, 0, 0);
-  if (ROLE == 2) pl = R.plan[r];
-  if (ROLE == 2 && pl.z == 2) {
-    copy_base_geometry(c, b, L, a, r, pl.x, cap, R, qcache + threadIdx.x, err);
-    return;
-  }
-  double sft;
-  GeoKeep gk;
-  gk.want_p1 = false;
-  gk.imin = 0;
-  gk.zmin_seen = 0;
-  gk.ds_clip = 0;
-  gk.ds_m = gk.ds_p1 = 0.f;
-  for (int i = 0; i < 3; i++) gk.x_m1[i] = gk.x_p1[i] = gk.x_first[i] = gk.x_last[i] = 0;
-  // mode 1: points [0, m) are the base's (final values); the walk goes on
-  // from the base's state at m, its lon/lat bookkeeping restated from the
-  // base's points before m
-  int m = 0;
-  long long ob = 0;
-  WalkFrom wf;
-  if (ROLE == 2 && pl.z == 1) {
-    m = pl.y;
-    ob = L.off[pl.x];
-    if (m > cap) {
-      atomicOr(err, cap < c.nlos_max ? kErrSlabOverflow : kErrLosOverflow);
-      return;
-    }
-    const long long bp = R.bpts;
-    for (int ip = 0; ip < m; ip++) {
-      const long long q = ob + ip, s = base + ip;
-      L.z[s] = L.z[q];
-      L.f.p[s] = L.f.p[q];
-      L.f.t[s] = L.f.t[q];
-      L.f.ds[s] = L.f.ds[q];
-      L.f.aux[s] = L.f.aux[q];
-      if (c.ig_h2o >= 0) L.f.qh2o[s] = L.f.qh2o[q];
-      for (int ig = 0; ig < c.ng; ig++) L.f.u[ig * L.cap + s] = L.f.u[ig * L.cap + q];
-      for (int iw = 0; iw < c.nw; iw++) L.f.kw[iw * L.cap + s] = L.f.kw[iw * L.cap + q];
-    }
-    wf.n = m;
-    for (int i = 0; i < 3; i++) {
-      wf.x[i] = R.xs[i * bp + ob + m];
-      wf.e[i] = R.es[i * bp + ob + m];
-      wf.x_last[i] = R.xs[i * bp + ob + m - 1];
-      gk.x_first[i] = R.xs[i * bp + ob];
-    }
-    wf.z = L.z[ob + m];
-    wf.z_last = L.z[ob + m - 1];
-    wf.lev_last = R.lev[ob + m - 1];
-    wf.raw_last = R.dsr[ob + m - 1];
-    // the first lowest point so far and its neighbours
-    int imin = 0;
-    double zmin = L.z[ob];
-    for (int ip = 1; ip < m; ip++)
-      if (L.z[ob + ip] < zmin) {
-        zmin = L.z[ob + ip];
-        imin = ip;
-      }
-    gk.imin = imin;
-    gk.zmin_seen = zmin;
-    gk.want_p1 = imin == m - 1;
-    gk.ds_m = R.dsr[ob + imin];
-    if (imin + 1 < m) gk.ds_p1 = R.dsr[ob + imin + 1];
-    for (int i = 0; i < 3; i++) {
-      gk.x_m1[i] = imin > 0 ? R.xs[i * bp + ob + imin - 1] : 0.0;
-      gk.x_p1[i] = imin + 1 < m ? R.xs[i * bp + ob + imin + 1] : 0.0;
-    }
-  }
-  const int n = walk_m<true, ROLE>(c, a, b.geo, b.nray, r, L, base, cap, &sft, &gk,
-                                   qcache + threadIdx.x, err, m > 0 ? &wf : nullptr, &R);
   L.sft[r] = sft;
   if (n > 0) L.count[r] = n;
   const long long nr = b.nray;
@@ -778,6 +715,412 @@ __global__ void k_trace_fill_m(CtlDev c, BatchDev b, LosDev L, const int* order,
   e[5] = latl;
 }
 
+// order (optional): thread t traces ray order[t], else ray r0 + t, so that a
+// warp's rays have similar LOS capacities and finish together; each ray's
+// outputs go to its own slots, so the order does not change any result.
+// The perturbations of resumed tracing (R.plan; EGA only: the Curtis-Godson
+// sums run from the first point).
+__global__ void k_trace_fill_m(CtlDev c, BatchDev b, LosDev L, const int* order, int r0, int nr_l,
+                               TraceResume R, unsigned* err) {
+  const int th = blockIdx.x * blockDim.x + threadIdx.x;
+  if (th >= nr_l) return;
+  const int r = order ? order[th] : r0 + th;
+  if (b.obs_skip && b.obs_skip[b.ray_obs[r]]) {
+    L.count[r] = 0;
+    return;
+  }
+  const AtmM a = atm_m(b, c, b.ray_obs[r]);
+  const long long base = L.off[r];
+  const int cap = L.count[r];
+  extern __shared__ float qcache[];  // trace_smem_floats(c) per thread
+  const int4 pl = R.plan[r];
+  if (pl.z == 2) {
+    copy_base_geometry(c, b, L, a, r, pl.x, cap, R, qcache + threadIdx.x, err);
+    return;
+  }
+  double sft;
+  GeoKeep gk;
+  gk.want_p1 = false;
+  gk.imin = 0;
+  gk.zmin_seen = 0;
+  gk.ds_clip = 0;
+  gk.ds_m = gk.ds_p1 = 0.f;
+  for (int i = 0; i < 3; i++) gk.x_m1[i] = gk.x_p1[i] = gk.x_first[i] = gk.x_last[i] = 0;
+  // mode 1: points [0, m) are the base's (final values); the walk goes on
+  // from the base's state at m, its lon/lat bookkeeping restated from the
+  // base's points before m
+  int m = 0;
+  long long ob = 0;
+  WalkFrom wf;
+  if (pl.z == 1) {
+    m = pl.y;
+    ob = L.off[pl.x];
+    if (m > cap) {
+      atomicOr(err, cap < c.nlos_max ? kErrSlabOverflow : kErrLosOverflow);
+      return;
+    }
+    const long long bp = R.bpts;
+    for (int ip = 0; ip < m; ip++) {
+      const long long q = ob + ip, s = base + ip;
+      L.z[s] = L.z[q];
+      L.f.p[s] = L.f.p[q];
+      L.f.t[s] = L.f.t[q];
+      L.f.ds[s] = L.f.ds[q];
+      L.f.aux[s] = L.f.aux[q];
+      if (c.ig_h2o >= 0) L.f.qh2o[s] = L.f.qh2o[q];
+      for (int ig = 0; ig < c.ng; ig++) L.f.u[ig * L.cap + s] = L.f.u[ig * L.cap + q];
+      for (int iw = 0; iw < c.nw; iw++) L.f.kw[iw * L.cap + s] = L.f.kw[iw * L.cap + q];
+    }
+    wf.n = m;
+    for (int i = 0; i < 3; i++) {
+      wf.x[i] = R.xs[i * bp + ob + m];
+      wf.e[i] = R.es[i * bp + ob + m];
+      wf.x_last[i] = R.xs[i * bp + ob + m - 1];
+      gk.x_first[i] = R.xs[i * bp + ob];
+    }
+    wf.z = L.z[ob + m];
+    wf.z_last = L.z[ob + m - 1];
+    wf.lev_last = R.lev[ob + m - 1];
+    wf.raw_last = R.dsr[ob + m - 1];
+    // the first lowest point so far and its neighbours
+    int imin = 0;
+    double zmin = L.z[ob];
+    for (int ip = 1; ip < m; ip++)
+      if (L.z[ob + ip] < zmin) {
+        zmin = L.z[ob + ip];
+        imin = ip;
+      }
+    gk.imin = imin;
+    gk.zmin_seen = zmin;
+    gk.want_p1 = imin == m - 1;
+    gk.ds_m = R.dsr[ob + imin];
+    if (imin + 1 < m) gk.ds_p1 = R.dsr[ob + imin + 1];
+    for (int i = 0; i < 3; i++) {
+      gk.x_m1[i] = imin > 0 ? R.xs[i * bp + ob + imin - 1] : 0.0;
+      gk.x_p1[i] = imin + 1 < m ? R.xs[i * bp + ob + imin + 1] : 0.0;
+    }
+  }
+  const int n = walk_m<true>(c, a, b.geo, b.nray, r, L, base, cap, &sft, &gk,
+                                   qcache + threadIdx.x, err, m > 0 ? &wf : nullptr);
+  ray_finish_m(b, L, r, n, sft, gk);
+}
+
+// Four lanes walk one ray: lanes 0-2 the components of the FP64 position and
+// direction and the three refraction sub-points, the emitters and windows
+// dealt over all four.  A ray is a chain of dependent steps, bound by latency:
+// with one lane per ray a nadir step took 5000 cycles; the sub-points in turn,
+// the emitters in turn and 35 FP64 instructions (64 cycles of a warp each,
+// conversions and compares among them).  Here a step has 7 FP64 instructions,
+// conversions and compares run on the integer pipe and a step takes 3800.  One
+// nadir ray of 901 points: 2.4 to 1.87 ms; 1500 rays of 801: 2.7 to 2.12 ms.
+// 20000 limb rays stay at 2.25 ms: there the loads of the rays' level values
+// bind (cold lines of 20000 profiles; prefetches and a 96-register build with
+// more warps were slower, 3.1 ms).  Every value is formed as in walk_m, in the
+// same order, so both give the same LOS.  All lanes stay in the loop until the
+// warp's eight rays are done.
+constexpr int kWalk4 = 4;
+
+__device__ __forceinline__ float from4(float v, int k) {
+  return __shfl_sync(0xffffffffu, v, k, kWalk4);
+}
+__device__ __forceinline__ double from4(double v, int k) {
+  return __shfl_sync(0xffffffffu, v, k, kWalk4);
+}
+
+// float4 of shared memory per thread: per emitter or window of the lane's
+// share the current level's value and slope and (emitters) the mixing ratio of
+// the pending point, and the Curtis-Godson sums
+__host__ __device__ inline int trace4_smem_slots(const CtlDev& c) {
+  const int ng = (c.ng + kWalk4 - 1) / kWalk4, nw = (c.nw + kWalk4 - 1) / kWalk4;
+  return ng + nw + (c.formod == 0 ? 2 * ng : 0);
+}
+
+template <int ROLE>
+__global__ void __launch_bounds__(kTraceThreads)
+    k_trace_fill_m4(CtlDev c, BatchDev b, LosDev L, const int* order, int r0, int nr_l,
+                    TraceResume R, unsigned* err) {
+  extern __shared__ float4 sm4[];
+  __shared__ GeoKeep keep[kTraceThreads / kWalk4];
+  constexpr int S = kTraceThreads;
+  const int s = threadIdx.x & (kWalk4 - 1);
+  const int th = (int)(blockIdx.x * blockDim.x + threadIdx.x) / kWalk4;
+  GeoKeep& gk = keep[threadIdx.x / kWalk4];
+  int r = th < nr_l ? (order ? order[th] : r0 + th) : -1;
+  const bool skipped = r >= 0 && b.obs_skip && b.obs_skip[b.ray_obs[r]];
+  if (skipped) {
+    if (s == 0) L.count[r] = 0;
+    r = -1;
+  }
+  const AtmM a = atm_m(b, c, r >= 0 ? b.ray_obs[r] : 0);
+  const long long base = r >= 0 ? L.off[r] : 0;
+  const int cap = r >= 0 ? L.count[r] : 0;
+  const int k = s < 3 ? s : 0;  // component of this lane
+  const float h = 0.02f;
+  const double zrefrac = 60;
+  const float rayds = (float)c.rayds, raydz = (float)c.raydz;
+  double zmin = 0, zmax = 0, x = 0, e = 0, z = 0, sft = -999;
+  float xf[3] = {1.f, 0.f, 0.f}, ef[3] = {1.f, 0.f, 0.f};
+  int n = 0, stop = 0;
+  const int st = r >= 0 ? ray_bounds_m(c, a, b.geo, b.nray, r, &zmin, &zmax, err) : 0;
+  bool alive = st > 0;
+  if (st < 0) n = -1;
+  if (alive) {
+    double x0[3], e0[3];
+    ray_first_m(b.geo, b.nray, r, zmax, x0, e0, &z);
+    for (int i = 0; i < 3; i++) {
+      xf[i] = (float)x0[i];
+      ef[i] = (float)e0[i];
+      if (i == k) {
+        x = x0[i];
+        e = e0[i];
+      }
+    }
+  }
+  if (s == 0) {  // each field has one writer; read after the walk
+    gk.imin = 0;
+    gk.ds_clip = 0;
+    gk.ds_m = gk.ds_p1 = 0.f;
+  }
+  if (s < 3) gk.x_m1[s] = gk.x_p1[s] = gk.x_first[s] = gk.x_last[s] = 0;
+  bool want_p1 = false;
+  double zmin_seen = 0, last_z = 0, x_last = 0;
+  Lev lv;
+  lv.i = -1;
+  // this lane's emitters s, s + 4, ... and windows, in shared memory
+  const int nge = (c.ng - s + kWalk4 - 1) / kWalk4, nwe = (c.nw - s + kWalk4 - 1) / kWalk4;
+  const int jh2o = c.ig_h2o >= 0 && (c.ig_h2o & (kWalk4 - 1)) == s ? c.ig_h2o / kWalk4 : -1;
+  const int ng_max = (c.ng + kWalk4 - 1) / kWalk4, nw_max = (c.nw + kWalk4 - 1) / kWalk4;
+  float4* const qv = sm4 + threadIdx.x;
+  float4* const kv = qv + ng_max * S;
+  float4* const cg = kv + nw_max * S;
+  const long long stride4 = kWalk4 * L.cap;
+  float* const u0 = L.f.u + s * L.cap + base;
+  const bool cloud = c.ncl > 0 && a.cldz > 0;
+  if (L.cga)
+    for (int j = 0; j < 2 * nge; j++) cg[j * S] = make_float4(0.f, 0.f, 0.f, 0.f);
+  int qc_level = -1;
+  float raw_before = 0.f, raw_pend = 0.f, pend_p = 0.f, pend_t = 0.f;
+  auto finalize = [&](int ip) {
+    const float dsT = ip == 0 ? 0.5f * raw_pend : 0.5f * (raw_before + raw_pend);
+    if (s == 0) L.f.ds[base + ip] = dsT;
+    for (int j = 0; j < nge; j++) {
+      const float uu = col_density(qv[j * S].z, pend_p, pend_t, dsT);
+      u0[j * stride4 + ip] = uu;
+      if (L.cga) {  // compensated running sums {sum, compensation} of u, p, T
+        const float4 up = cg[2 * j * S];
+        float2 tt = *(const float2*)&cg[(2 * j + 1) * S];
+        float su = up.x, cu = up.y, sp = up.z, cp = up.w, st2 = tt.x, ct = tt.y;
+        float y = uu - cu, s2 = su + y;
+        cu = (s2 - su) - y;
+        su = s2;
+        y = uu * pend_p - cp;
+        s2 = sp + y;
+        cp = (s2 - sp) - y;
+        sp = s2;
+        y = uu * pend_t - ct;
+        s2 = st2 + y;
+        ct = (s2 - st2) - y;
+        st2 = s2;
+        cg[2 * j * S] = make_float4(su, cu, sp, cp);
+        *(float2*)&cg[(2 * j + 1) * S] = make_float2(st2, ct);
+        const long long sk = (s + kWalk4 * j) * L.cap + base + ip;
+        L.f.cgu[sk] = su;
+        L.f.cgp[sk] = sp / su;
+        L.f.cgt[sk] = st2 / su;
+      }
+    }
+  };
+  while (__any_sync(0xffffffffu, alive)) {
+    const float rf = d2f_bits(z + kRE), rinv = 1.f / rf;
+    float xh[3];
+    for (int i = 0; i < 3; i++) xh[i] = xf[i] * rinv;
+    float step = rayds;
+    if (raydz > 0) {
+      const float cosa = fabsf(ef[0] * xh[0] + ef[1] * xh[1] + ef[2] * xh[2]);
+      if (cosa != 0) step = rayds < raydz / cosa ? rayds : raydz / cosa;
+    }
+    const bool low = less(z, zmin), high = less(zmax, z);
+    if (alive && (low || high) && n > 0) {  // clip (see walk_m)
+      stop = low ? 2 : 1;
+      const double frac = ((low ? zmin : zmax) - last_z) / (z - last_z);
+      x = x_last + frac * (x - x_last);
+      z = last_z + frac * (z - last_z);
+      const double dsc = (double)step * frac;
+      raw_pend = (float)dsc;
+      if (s == 0) gk.ds_clip = dsc;
+      if (ROLE == 1 && s == 3) R.dsr[base + n - 1] = raw_pend;
+      step = 0.f;
+    }
+    if (alive && n >= cap) {
+      if (s == 0) atomicOr(err, cap < c.nlos_max ? kErrSlabOverflow : kErrLosOverflow);
+      alive = false;
+      n = -1;
+    }
+    float dl = 0.f, p = 0.f, t = 1.f;
+    if (alive) {
+      dl = lev_find(a, z, lv);
+      lev_pt(lv, dl, &p, &t);
+      if (n > 0) finalize(n - 1);
+      const long long q = base + n;
+      raw_before = raw_pend;
+      raw_pend = step;
+      pend_p = p;
+      pend_t = t;
+      if (s == 0) L.z[q] = z;
+      if (s == 1) L.f.p[q] = p;
+      if (s == 2) L.f.t[q] = t;
+      if (s == 3) {
+        float aux = 0.f;
+        if (cloud) {
+          const float v = (float)((z - a.clz) / a.cldz);
+          aux = expf(-0.5f * v * v);
+        }
+        L.f.aux[q] = aux;
+      }
+      if (lv.i != qc_level) {  // a new level: its values and slopes
+        qc_level = lv.i;
+        constexpr int kB = 3;  // loads in flight
+        for (int j0 = 0; j0 < nge + nwe; j0 += kB) {
+          double d0[kB], d1[kB];
+#pragma unroll
+          for (int m = 0; m < kB; m++) {
+            const int j = min(j0 + m, nge + nwe - 1);
+            const double* src = (j < nge ? a.q + (s + kWalk4 * j) * a.stride
+                                         : a.k + (s + kWalk4 * (j - nge)) * a.stride) + lv.i;
+            d0[m] = src[0];
+            d1[m] = src[1];
+          }
+#pragma unroll
+          for (int m = 0; m < kB; m++) {
+            const int j = min(j0 + m, nge + nwe - 1);
+            const float v0 = d2f_bits(d0[m]), v1 = d2f_bits(d1[m]);
+            *(float2*)(j < nge ? &qv[j * S] : &kv[(j - nge) * S]) =
+                make_float2(v0, (v1 - v0) / lv.dz);
+          }
+        }
+      }
+      for (int j = 0; j < nge; j++) {
+        const float2 vs = *(const float2*)&qv[j * S];
+        const float v = qk_at(vs.x, vs.y, dl);
+        qv[j * S].z = v;
+        if (j == jh2o) L.f.qh2o[q] = v;
+      }
+      for (int j = 0; j < nwe; j++) {
+        const float2 vs = *(const float2*)&kv[j * S];
+        L.f.kw[(s + kWalk4 * j) * L.cap + q] = qk_at(vs.x, vs.y, dl);
+      }
+      if (ROLE == 1) {
+        if (s < 3) {
+          R.xs[s * R.bpts + q] = x;
+          R.es[s * R.bpts + q] = e;
+        } else {
+          R.lev[q] = lv.i;
+          R.dsr[q] = step;
+        }
+      }
+      if (n == 0 && s < 3) gk.x_first[s] = x;
+      const bool newmin = n == 0 || less(z, zmin_seen);
+      if (want_p1) {
+        if (s < 3) gk.x_p1[s] = x;
+        if (s == 0) gk.ds_p1 = step;
+      }
+      if (newmin) {
+        zmin_seen = z;
+        if (s < 3) gk.x_m1[s] = x_last;  // the previous point
+        if (s == 0) {
+          gk.imin = n;
+          gk.ds_m = step;
+        }
+      }
+      want_p1 = newmin;
+      last_z = z;
+      x_last = x;
+      n++;
+      if (stop) {
+        sft = stop == 2 ? (c.nsf > 0 && a.sft > 0 ? a.sft : (double)t) : -999;
+        finalize(n - 1);
+        if (s < 3) gk.x_last[s] = x;
+        alive = false;
+      }
+    }
+    // refraction (see walk_m), a sub-point per lane
+    const bool bend = alive && c.refrac && is_number(z) && !lt(zrefrac, z);
+    const float nref = 1.f + kRefracC * p / t;
+    float inc_k = 0.f;
+    if (bend) {
+      const float d[3] = {0.5f * step * ef[0], 0.5f * step * ef[1], 0.5f * step * ef[2]};
+      const float dzh = dz_of(xh, rf, d);
+      const float rh = rf + dzh, rhinv = 1.f / rh;
+      const float xhh[3] = {(xh[0] * rf + d[0]) * rhinv, (xh[1] * rf + d[1]) * rhinv,
+                            (xh[2] * rf + d[2]) * rhinv};
+      Lev lh = lv;
+      float dlh = dl + dzh;
+      if (!lev_holds(lh, dlh)) dlh = lev_find(a, z + f2d_bits(dzh), lh);
+      float ph, thp;
+      lev_pt(lh, dlh, &ph, &thp);
+      const float dk[3] = {k == 0 ? h : 0.f, k == 1 ? h : 0.f, k == 2 ? h : 0.f};
+      const float dlk = dz_of(xhh, rh, dk);
+      float dN;
+      if (lev_holds(lh, dlh + dlk)) {
+        dN = dN_in(lh, ph, thp, dlk);
+      } else {
+        // split at the level boundary between the midpoint and zk
+        const double zh = lh.z0 + f2d_bits(dlh), zk = zh + f2d_bits(dlk);
+        Lev lk = lh;
+        const float dlk0 = lev_find(a, zk, lk);
+        if (lk.i == lh.i) {
+          dN = dN_in(lh, ph, thp, dlk);
+        } else {
+          const bool up = lk.i > lh.i;
+          const double zb = up ? a.z[lh.i + 1] : a.z[lh.i];
+          const float d1 = d2f_bits(zb - zh);
+          const float dn1 = dN_in(lh, ph, thp, d1);
+          float pb, tb;
+          const float dlb = d2f_bits(zb - lk.z0);
+          lev_pt(lk, dlb, &pb, &tb);
+          dN = dn1 + dN_in(lk, pb, tb, dlk0 - dlb);
+        }
+      }
+      inc_k = step * (dN / h) / nref;
+    }
+    float inc[3];
+    for (int i = 0; i < 3; i++) inc[i] = from4(inc_k, i);
+    double e1 = e;
+    if (bend) e1 = e + f2d_bits(inc_k);
+    const float delta = 2.f * (ef[0] * inc[0] + ef[1] * inc[1] + ef[2] * inc[2]) +
+                        (inc[0] * inc[0] + inc[1] * inc[1] + inc[2] * inc[2]);
+    const bool large = bend && !(fabsf(delta) < 1e-3f);
+    if (bend && !large) {
+      const float corr = delta * (-0.5f + delta * (0.375f - 0.3125f * delta));
+      e1 += e1 * f2d_bits(corr);
+    }
+    if (__any_sync(0xffffffffu, large)) {
+      const double e0 = from4(e1, 0), e1c = from4(e1, 1), e2 = from4(e1, 2);
+      if (large) e1 /= sqrt(e0 * e0 + e1c * e1c + e2 * e2);
+    }
+    const float en = d2f_bits(e1);
+    float D[3], efn[3];
+    for (int i = 0; i < 3; i++) {
+      efn[i] = from4(en, i);
+      D[i] = 0.5f * step * (ef[i] + efn[i]);
+    }
+    const float dzs = dz_of(xh, rf, D);
+    const float Dk = k == 0 ? D[0] : k == 1 ? D[1] : D[2];
+    if (alive) {
+      x += f2d_bits(Dk);
+      e = e1;
+      z += f2d_bits(dzs);
+    }
+    const float xn = d2f_bits(x);
+    for (int i = 0; i < 3; i++) {
+      xf[i] = from4(xn, i);
+      ef[i] = efn[i];
+    }
+  }
+  __syncwarp();
+  if (r >= 0 && s == 0) ray_finish_m(b, L, r, n, sft, gk);
+}
+
 }  // namespace
 
 void launch_trace_count_mixed(const CtlDev& c, const BatchDev& b, const LosDev& L, unsigned* err,
@@ -794,10 +1137,10 @@ void launch_los_bound_mixed(const CtlDev& c, const BatchDev& b, double scale, in
 
 void launch_trace_fill_mixed(const CtlDev& c, const BatchDev& b, const LosDev& L, const int* order,
                              unsigned* err, cudaStream_t s) {
-  const int bs = kTraceThreads;
-  const size_t smem = sizeof(float) * trace_smem_floats(c) * kTraceThreads;
-  k_trace_fill_m<0><<<(b.nray + bs - 1) / bs, bs, smem, s>>>(c, b, L, order, 0, b.nray,
-                                                              TraceResume{}, err);
+  const int rays = kTraceThreads / kWalk4;
+  const size_t smem = sizeof(float4) * trace4_smem_slots(c) * kTraceThreads;
+  k_trace_fill_m4<0><<<(b.nray + rays - 1) / rays, kTraceThreads, smem, s>>>(
+      c, b, L, order, 0, b.nray, TraceResume{}, err);
 }
 
 int trace_fill_resident(int sms) {
@@ -805,7 +1148,7 @@ int trace_fill_resident(int sms) {
   // emitters does not bind); computed once, thread-safely
   static const int per_sm = [] {
     int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trace_fill_m<2>, kTraceThreads, 0) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trace_fill_m, kTraceThreads, 0) !=
             cudaSuccess ||
         nb < 1)
       nb = 1;
@@ -817,13 +1160,15 @@ int trace_fill_resident(int sms) {
 void launch_trace_fill_resumed(const CtlDev& c, const BatchDev& b, const LosDev& L,
                                const int* order, int r0, int nr, const TraceResume& R, int role,
                                unsigned* err, cudaStream_t s) {
-  const int bs = kTraceThreads;
+  const int bs = kTraceThreads, rays = bs / kWalk4;
   if (nr <= 0) return;
-  const size_t smem = sizeof(float) * trace_smem_floats(c) * kTraceThreads;
   if (role == 1)
-    k_trace_fill_m<1><<<(nr + bs - 1) / bs, bs, smem, s>>>(c, b, L, order, r0, nr, R, err);
+    k_trace_fill_m4<1><<<(nr + rays - 1) / rays, bs,
+                         sizeof(float4) * trace4_smem_slots(c) * kTraceThreads, s>>>(
+        c, b, L, order, r0, nr, R, err);
   else
-    k_trace_fill_m<2><<<(nr + bs - 1) / bs, bs, smem, s>>>(c, b, L, order, r0, nr, R, err);
+    k_trace_fill_m<<<(nr + bs - 1) / bs, bs, sizeof(float) * trace_smem_floats(c) * kTraceThreads,
+                     s>>>(c, b, L, order, r0, nr, R, err);
 }
 
 }  // namespace jgb

@@ -214,6 +214,12 @@ __global__ void k_tiles(int nray, int ntile, int nfirst, int tfirst, int nsecond
   tpts[tile] = mx;
 }
 
+// Tile and lane (tile * 32 + lane) of every base ray.
+__global__ void k_base_slots(int n, const int* perm, int* slot) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n && perm[i] >= 0) slot[perm[i]] = i;
+}
+
 // Resume point of every ray of a batch of perturbations (ResumeSpec).  A
 // perturbed level value changes the atmosphere only on the two intervals
 // next to it, [z_lo, z_hi].  The position of LOS point p + 1 depends on the
@@ -297,12 +303,11 @@ __global__ void k_trace_plan(int nray, int nbase_rays, BatchDev b, LosDev L, con
 }
 
 // Sort key of a resumed batch: bases first (their tiles run first and save
-// the states), then by perturbation class (below: the perturbations that
-// cannot share emitters, class 15, before those that can, so that the two
-// form separate tile ranges), by measured channels, by the LOS points left
-// to do in 64-point buckets (longest first, so that no long warp is left for
-// the end) and by start point in 16-point buckets (so that the lanes of a
-// warp walk nearly the same range of points).
+// the states), then by perturbation class (below), by measured channels and by
+// the LOS points left to do in 64-point buckets (longest first, so that no long
+// warp is left for the end, and the lanes of a warp walk nearly the same range
+// of points).  Within a bucket the rays keep their order, one observation's
+// next to each other: they share table rows.
 // The perturbation class follows the channels: the perturbations of one
 // emitter's mixing ratio (class 1 + emitter) and of extinctions (class 0)
 // compute only that emitter (none) and take the others from their base, so
@@ -317,14 +322,13 @@ __global__ void k_resume_keys(int nray, int nbase_rays, int nd, const unsigned c
     m = 0;
     for (int id = 0; id < nd; id++) m += mask[(long long)id * nray + r] ? 0 : 1;
   }
-  const int left = count[r] - start[r];
   int cls = 0;
   if (pert) {  // emitters shared with the base
     const int4 pr = pert[ray_obs[r]];
     cls = pr.x == 2 ? 1 + min(pr.y, 13) : pr.x == 3 ? 0 : 15;
   }
   key[r] = ((r < nbase_rays ? 1 : 0) << 30) | (cls << 26) | (min(m, 511) << 17) |
-           (min(left >> 6, 127) << 10) | (min(start[r] >> 4, 255) << 2);
+           (min((count[r] - start[r]) >> 6, 127) << 10);
 }
 
 // Sort key of a batch whose masked pairs are skipped: rays with the same
@@ -445,11 +449,11 @@ struct PathChunk {
 // point_bytes, chan_bytes: workspace of a tile point, and of one per channel;
 // tile_bytes: of a (tile, channel).  The largest needs in *need_points (limited
 // to a quarter of kPathBytes) and *need_chan.
-void path_chunks(const std::vector<long long>& toff, int nd, size_t point_bytes, size_t chan_bytes,
-                 size_t tile_bytes, std::vector<PathChunk>& out, size_t* need_points,
-                 size_t* need_chan) {
+void path_chunks(const std::vector<long long>& toff, int tfirst, int nd, size_t point_bytes,
+                 size_t chan_bytes, size_t tile_bytes, std::vector<PathChunk>& out,
+                 size_t* need_points, size_t* need_chan) {
   const int ntile = (int)toff.size() - 1;
-  for (int t = 0; t < ntile;) {
+  for (int t = tfirst; t < ntile;) {
     PathChunk k{t, t, nd, 0};
     auto pts = [&](int t1) { return (size_t)(toff[t1] - toff[k.t0]); };
     do {
@@ -466,6 +470,10 @@ void path_chunks(const std::vector<long long>& toff, int nd, size_t point_bytes,
   }
 }
 
+// Up to here (warps of 32 rays per SM) a ray gets four lanes: a warp alone
+// walks its chain in a fifth of the time then, until the device is full.
+constexpr long long kFourLaneWarps = 8;
+
 // The autotuner of the mixed path: times every variant of the emitters'
 // kernel on a chunk (the results are the same) and keeps the fastest;
 // JGB_PATH_VARIANT takes one without timing.
@@ -480,7 +488,7 @@ int tune_gas(jgb_ctx* x, const TblDev& T, const BatchDev& b, const LosDev& L, co
   float best = 1e30f;
   for (int v = 0; v < nv; v++) {
     CK(cudaEventRecord(x->ev[4], s));
-    launch_gas_m(x->c, T, b, L, P, 1, v, s);
+    launch_gas_m(x->c, T, b, L, P, 1, v, 0, s);
     CK(cudaEventRecord(x->ev[5], s));
     CK(cudaEventSynchronize(x->ev[5]));
     float ms = 0;
@@ -519,7 +527,7 @@ int run_path64(jgb_ctx* x, const BatchDev& b, const LosDev& L, cudaStream_t s, i
   const size_t bch = 32 * sizeof(double) * (size_t)(c.ng + 2);  // per (point, channel)
   std::vector<PathChunk> chunks;
   size_t need_f = 0, need_w = 0;
-  path_chunks(toff, c.nd, bfd + bfu, bch, 32 * sizeof(int) * (size_t)std::max(c.ng, 1), chunks,
+  path_chunks(toff, 0, c.nd, bfd + bfu, bch, 32 * sizeof(int) * (size_t)std::max(c.ng, 1), chunks,
               &need_f, &need_w);
   CK(x->tiles_data.reserve(need_f));
   CK(x->seg.reserve(need_w));
@@ -809,33 +817,19 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
     }
     // resumed perturbations: start points and the base rays' snapshot lists
     const ResumeSpec* rs = x->resume;
-    const int nchb = (c.nd + 3) / 4;
     int nbase_rays = nray, tfirst = 0;
     int nplain_end = nray, tsecond = 0;  // resumed: end of the rays that share no emitter
     double resume_skip = 0.0;
     int* rstart = nullptr;
     int *snap_off = nullptr, *snap_ip = nullptr, *snap_ray = nullptr;
     // emitters shared between a perturbed ray and its base (see MixedPlan)
-    float* seg_base = nullptr;
-    unsigned *seg_satm = nullptr, *seg_final = nullptr;
-    int* seg_nvalid = nullptr;
-    const int2* seg_reuse = nullptr;
+    std::vector<int2> reuse;
+    bool any_reuse = false;
     bool share_emitters = false;
     if (rs) {
       nbase_rays = rs->h_ray_off[rs->nbase];
-      // sharing emitters with the base pays where most of the perturbed
-      // lookups can be taken from it (several emitters, mostly mixing-ratio
-      // perturbations); elsewhere its bookkeeping and the registers of the
-      // sharing kernel cost more than it saves
-      double shr = 0, tot = 0;
-      for (int e = rs->nbase; e < b.nobs; e++) {
-        const double wr = rs->h_ray_off[e + 1] - rs->h_ray_off[e];
-        const int4 pr = rs->h_pert[e];
-        tot += wr;
-        if (pr.x == 2 && c.ng > 1) shr += wr * (c.ng - 1.0) / c.ng;
-        else if (pr.x == 3) shr += wr;
-      }
-      share_emitters = x->fd_resume == 3 || (tot > 0 && shr / tot >= 0.3);
+      for (int e = rs->nbase; e < b.nobs; e++)
+        share_emitters |= (rs->h_pert[e].x == 2 && c.ng > 1) || rs->h_pert[e].x == 3;
       CK(x->rs_start.reserve(sizeof(int) * (size_t)nray));
       rstart = x->rs_start.as<int>();
       k_resume_points<<<(nray + 127) / 128, 128, 0, s>>>(nray, b, L, rs->nbase, rs->pert,
@@ -858,42 +852,49 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
         points += hc[r];
       }
       resume_skip = points > 0 ? (double)skipped / (double)points : 0.0;
-      // Does resuming pay?  Lanes of a warp walk the union of their point
-      // ranges, and the base tiles run before the others.  Estimate both
-      // schedules from their tile plans: a group of tiles takes the longer
-      // of its work over the tiles the device holds at once and its longest
-      // tile.
-      const double conc = std::max(1.0, (double)x->sms * 8.0 / nchb);
-      double waves = 0;  // of the plain plan: work over the longest tile
-      auto group_time = [&](const std::vector<int>& order, int k0, int k1, bool resumed) {
-        double sum = 0, mx = 0;
-        for (int t = k0; t < k1; t += 32) {
-          int hi = 0, lo = 1 << 30;
-          for (int l = t; l < std::min(t + 32, k1); l++) {
-            hi = std::max(hi, hc[order[l]]);
-            lo = std::min(lo, resumed ? hs[order[l]] : 0);
-          }
-          sum += hi - lo;
-          mx = std::max(mx, (double)(hi - lo));
-        }
-        waves = mx > 0 ? sum / conc / mx : 0;
-        return std::max(sum / conc, mx);
-      };
+      // Does resuming pay?  Both schedules from their tile plans, in points of
+      // a tile: the device holds conc tiles (of all channels and emitters) at
+      // once, and a group of tiles takes the longer of its work over that and
+      // its longest tile.  A resumed tile walks the union of its rays' points,
+      // for the share of its emitters that no base has (a quarter of the time
+      // goes to the segments in any case) and 1.4 times as slow per point as
+      // the plain batch, whose tiles hold one observation's nearly equal rays
+      // (0.47 against 0.29 ns per warp and point).  The bases come first and
+      // take 0.7 of a plain tile's time, 4 lanes per ray and nothing else to
+      // run beside them.
+      const double conc = std::max(1.0, (double)x->sms * 40.0 / ((double)c.nd * std::max(c.ng, 1)));
       std::vector<int> ord(nray);
       for (int r = 0; r < nray; r++) ord[r] = r;
       std::stable_sort(ord.begin(), ord.end(), [&](int a, int b2) { return hk[a] > hk[b2]; });
-      const double t_res = group_time(ord, 0, nbase_rays, false) + group_time(ord, nbase_rays, nray, true);
+      double sum_b = 0, sum_r = 0, mx = 1;
+      for (int t = 0; t < nray; t += 32) {
+        int hi = 0, lo = 1 << 30;
+        double share = 0;
+        const int t1 = std::min(t + 32, nray);
+        for (int l = t; l < t1; l++) {
+          const int r = ord[l], cls = (hk[r] >> 26) & 15;
+          hi = std::max(hi, hc[r]);
+          lo = std::min(lo, hs[r]);
+          share += cls == 15 || !share_emitters || t < nbase_rays ? 1.0 : cls > 0 ? 1.0 / c.ng : 0.0;
+        }
+        if (t < nbase_rays) sum_b += hi;
+        else sum_r += (hi - lo) * (0.25 + 0.75 * share / (t1 - t));
+        mx = std::max(mx, (double)hi);
+      }
+      const double t_res = std::max(sum_b / conc, 0.7 * mx) + std::max(1.4 * sum_r / conc, mx);
       // the plain plan: measured channels (key bits 17-25), then LOS length
       std::stable_sort(ord.begin(), ord.end(), [&](int a, int b2) {
         const int ma = (hk[a] >> 17) & 511, mb = (hk[b2] >> 17) & 511;
         return ma != mb ? ma > mb : hc[a] > hc[b2];
       });
-      const double t_plain = group_time(ord, 0, nray, false);
-      // measured: resumed chunks win from about ten waves on (48 serving
-      // requests: -6 %; 2048 nadir observations x 405 perturbations: +55 %
-      // throughput) and lose on a few waves, where the base tiles, which
-      // run first, cost more than the skipped points save
-      if (x->fd_resume == 1 && !(t_res < 0.9 * t_plain && waves >= 8.0)) {
+      double sum_p = 0;
+      for (int t = 0; t < nray; t += 32) {
+        int hi = 0;
+        for (int l = t; l < std::min(t + 32, nray); l++) hi = std::max(hi, hc[ord[l]]);
+        sum_p += hi;
+      }
+      const double t_plain = std::max(sum_p / conc, mx);
+      if (nbase_rays > 65535 * 32 || (x->fd_resume == 1 && !(t_res < 0.9 * t_plain))) {
         rs = nullptr;  // run the batch plainly (the base copies are computed too)
         nbase_rays = nray;
         resume_skip = 0.0;
@@ -940,13 +941,11 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
         CK(cudaMemcpyAsync(snap_ip, sip.data(), sizeof(int) * nsnap, cudaMemcpyHostToDevice, s));
         CK(cudaMemcpyAsync(snap_ray, sray.data(), sizeof(int) * nsnap, cudaMemcpyHostToDevice, s));
       }
-      CK(x->rs_snap.reserve(sizeof(float) * (size_t)nray * c.nd * path_state_words(c)));
       // a perturbation of one emitter's mixing ratio (array 2) or of an
       // extinction (array 3) leaves the LOS (refraction needs p and T only)
       // and the other emitters' inputs and states equal to the base's: those
       // emitters' segment emissivities are taken from the base's walk
-      std::vector<int2> reuse(nray, make_int2(-1, -1));
-      bool any_reuse = false;
+      reuse.assign(nray, make_int2(-1, -1));
       for (int r = nbase_rays; r < nray && share_emitters; r++) {
         const int e = ray_obs[r];
         const int4 pr = rs->h_pert[e];
@@ -955,27 +954,6 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
           reuse[r] = make_int2(rs->h_ray_off[eb] + (r - rs->h_ray_off[e]), pr.x == 2 ? pr.y : -1);
           any_reuse = true;
         }
-      }
-      if (any_reuse) {
-        long long bpts = 0;
-        CK(cudaMemcpyAsync(&bpts, L.off + nbase_rays, sizeof(long long), cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
-        const size_t nseg = (size_t)std::max(bpts, 1LL) * c.nd;
-        const size_t nst = (size_t)nbase_rays * c.nd;
-        const size_t sw = (size_t)path_state_words(c) - 3;
-        auto a16 = [](size_t b) { return (b + 15) & ~size_t(15); };
-        const size_t b_eps = a16(sizeof(float) * nseg * c.ng), b_satm = a16(sizeof(unsigned) * nseg);
-        const size_t b_nv = a16(sizeof(int) * nst), b_fin = a16(sizeof(unsigned) * nst * sw);
-        const size_t b_ru = a16(sizeof(int2) * (size_t)nray);
-        CK(x->rs_seg.reserve(b_eps + b_satm + b_nv + b_fin + b_ru));
-        char* sp = x->rs_seg.as<char>();
-        seg_base = reinterpret_cast<float*>(sp);
-        seg_satm = reinterpret_cast<unsigned*>(sp + b_eps);
-        seg_nvalid = reinterpret_cast<int*>(sp + b_eps + b_satm);
-        seg_final = reinterpret_cast<unsigned*>(sp + b_eps + b_satm + b_nv);
-        int2* d_reuse = reinterpret_cast<int2*>(sp + b_eps + b_satm + b_nv + b_fin);
-        CK(cudaMemcpyAsync(d_reuse, reuse.data(), sizeof(int2) * (size_t)nray, cudaMemcpyHostToDevice, s));
-        seg_reuse = d_reuse;
       }
       CK(cudaStreamSynchronize(s));  // the host lists go out of scope
       tfirst = (nbase_rays + 31) / 32;
@@ -1019,53 +997,105 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
     Pm.nfield = mixed_nfield(c, Pm.brmask);
     CK(x->tiles_data.reserve(sizeof(float) * 32 * (size_t)std::max(tile_points, 1LL) * Pm.nfield));
     Pm.data = x->tiles_data.as<float>();
+    Pm.start = rs ? rstart : nullptr;
     launch_pack_tiles_n(c, tbl_view(x), L, Pm, tile_points, s);
     CK(cudaGetLastError());
+    if (c.ncl > 0) {
+      CK(x->cloudf.reserve(sizeof(float) * (size_t)c.nd * nray));
+      launch_cloud_m(c, ch, bo, x->cloudf.as<float>(), s);
+      Pm.cloud = x->cloudf.as<float>();
+      launches += 1;
+    }
     if (rs) {
-      // bases (saving the states), then the perturbations (starting from them)
-      Pm.start = rstart;
+      // The bases (saving the states), then the perturbations (starting from
+      // them), for groups of channels whose base segments, states and the
+      // perturbations' segments each stay within kPathBytes.
+      const size_t np = (size_t)std::max(toff_h[tfirst], 1LL);
+      const int bseg = c.ng + 2;  // the emitters of a base's segments outlive its sums
+      const size_t b_seg = 32 * sizeof(float) * np * bseg;
+      const size_t b_stop = 32 * sizeof(int) * (size_t)tfirst * std::max(c.ng, 1);
+      const size_t b_state = gas_state_bytes() * (size_t)nray * c.ng, b_sums = 3 * sizeof(float) * (size_t)nray;
+      const size_t per = std::max(b_seg + b_stop, b_state + b_sums);
+      const int gnd = (int)std::min<size_t>(c.nd, std::max<size_t>(kPathBytes / per, 1));
+      auto a16 = [](size_t v) { return (v + 15) & ~size_t(15); };
+      const size_t o_stop = a16(b_seg * gnd), o_slot = o_stop + a16(b_stop * gnd);
+      const size_t o_reuse = o_slot + a16(sizeof(int) * (size_t)std::max(nbase_rays, 1));
+      CK(x->rs_seg.reserve(o_reuse + sizeof(int2) * (size_t)nray));
+      CK(x->rs_snap.reserve(a16(b_state * gnd) + b_sums * gnd));
+      char* sp = x->rs_seg.as<char>();
+      int* slot = reinterpret_cast<int*>(sp + o_slot);
+      k_base_slots<<<(tfirst * 32 + 127) / 128, 128, 0, s>>>(tfirst * 32, Pm.perm, slot);
       Pm.snap_off = snap_off;
       Pm.snap_ip = snap_ip;
       Pm.snap_ray = snap_ray;
-      Pm.snap = x->rs_snap.as<float>();
-      Pm.seg_base = seg_base;
-      Pm.seg_satm = seg_satm;
-      Pm.seg_nvalid = seg_nvalid;
-      Pm.seg_final = seg_final;
+      Pm.snap = x->rs_snap.as<unsigned>();
+      Pm.snap_sums = reinterpret_cast<float*>(x->rs_snap.as<char>() + a16(b_state * gnd));
+      Pm.base_seg = reinterpret_cast<float*>(sp);
+      Pm.base_stop = reinterpret_cast<int*>(sp + o_stop);
+      Pm.base_slot = slot;
+      Pm.base_nseg = bseg;
+      if (any_reuse) {
+        CK(cudaMemcpyAsync(sp + o_reuse, reuse.data(), sizeof(int2) * (size_t)nray,
+                           cudaMemcpyHostToDevice, s));
+        CK(cudaStreamSynchronize(s));
+        Pm.reuse = reinterpret_cast<int2*>(sp + o_reuse);
+      }
+      const size_t bch = 32 * sizeof(float) * (size_t)std::max(c.ng, 2);
+      std::vector<PathChunk> chunks;
+      size_t need = 0;
+      path_chunks(toff_h, tfirst, gnd, 0, bch, 32 * sizeof(int) * (size_t)std::max(c.ng, 1), chunks,
+                  nullptr, &need);
+      CK(x->seg.reserve(need));
       CK(cudaEventRecord(x->ev[4], s));
-      Pm.tile0 = 0;
-      Pm.tile1 = tfirst;
-      Pm.reuse = nullptr;       // the bases write their emitters' values
-      launch_path_resume(c, T, ch, bo, L, Pm, s);
-      MixedPlan Pp = Pm;        // perturbations that share no emitter
-      Pp.tile0 = tfirst;
-      Pp.tile1 = tsecond;
-      Pp.seg_base = nullptr;
-      launch_path_resume(c, T, ch, bo, L, Pp, s);
-      Pm.tile0 = tsecond;
-      Pm.tile1 = ntile;
-      Pm.reuse = seg_reuse;     // the perturbations that do read them
-      launch_path_resume(c, T, ch, bo, L, Pm, s);
-      launches += 10;
+      for (int g0 = 0; g0 < c.nd; g0 += gnd) {
+        MixedPlan P = Pm;
+        P.gid0 = g0;
+        P.gndc = std::min(c.nd - g0, gnd);
+        P.tile0 = 0;
+        P.tile1 = tfirst;
+        P.pt0 = 0;
+        P.id0 = g0;
+        P.id1 = g0 + P.gndc;
+        P.nseg = bseg;
+        P.seg = reinterpret_cast<float*>(sp);
+        P.stop = reinterpret_cast<int*>(sp + o_stop);
+        const long long warps = (long long)tfirst * P.gndc * c.ng;
+        long long longest = 1;
+        for (int t = 0; t < tfirst; t++) longest = std::max(longest, toff_h[t + 1] - toff_h[t]);
+        launch_gas_m(c, T, bo, L, P, warps <= kFourLaneWarps * x->sms ? 4 : 1, 0, 1, s);
+        launch_seg_scan_m(c, T, ch, bo, L, P, (int)longest, 1, s);
+        launches += 3;
+        P.nseg = std::max(c.ng, 2);
+        P.seg = x->seg.as<float>();
+        for (const PathChunk& k : chunks) {
+          P.tile0 = k.t0;
+          P.tile1 = k.t1;
+          P.pt0 = toff_h[k.t0];
+          const size_t pts = std::max<size_t>((size_t)(toff_h[k.t1] - toff_h[k.t0]), 1);
+          for (int id = g0; id < g0 + P.gndc; id += k.ndc) {
+            P.id0 = id;
+            P.id1 = std::min(g0 + P.gndc, id + k.ndc);
+            P.stop = reinterpret_cast<int*>(x->seg.as<char>() + pts * (P.id1 - P.id0) * bch);
+            launch_gas_m(c, T, bo, L, P, 1, 4, 2, s);
+            launch_seg_scan_m(c, T, ch, bo, L, P, std::max(k.longest, 1), 2, s);
+            launches += 3;
+          }
+        }
+        CK(cudaGetLastError());
+      }
+      launches += 8;
       x->stats.resume_skip = resume_skip;
     } else {
-      if (c.ncl > 0) {
-        CK(x->cloudf.reserve(sizeof(float) * (size_t)c.nd * nray));
-        launch_cloud_m(c, ch, bo, x->cloudf.as<float>(), s);
-        Pm.cloud = x->cloudf.as<float>();
-        launches += 1;
-      }
       Pm.nseg = std::max(c.ng, 2);
       // chunks of tiles whose segments stay within kPathBytes (and of channels
       // where one tile alone would not)
       const size_t bch = 32 * sizeof(float) * (size_t)Pm.nseg;
       std::vector<PathChunk> chunks;
       size_t need = 0;
-      path_chunks(toff_h, c.nd, 0, bch, 32 * sizeof(int) * (size_t)std::max(c.ng, 1), chunks, nullptr, &need);
+      path_chunks(toff_h, 0, c.nd, 0, bch, 32 * sizeof(int) * (size_t)std::max(c.ng, 1), chunks, nullptr, &need);
       CK(x->seg.reserve(need));
-      // a batch that leaves the schedulers idle gives each ray four lanes
       const long long warps = (long long)ntile * c.nd * c.ng;
-      const int lanes = x->path_split == 1 || (x->path_split < 0 && warps <= 8LL * x->sms) ? 4 : 1;
+      const int lanes = x->path_split == 1 || (x->path_split < 0 && warps <= kFourLaneWarps * x->sms) ? 4 : 1;
       bool timed = false;
       for (const PathChunk& k : chunks) {
         Pm.tile0 = k.t0;
@@ -1088,8 +1118,8 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
           if (k.t1 - k.t0 < 8) variant %= 4;
           if (!timed) CK(cudaEventRecord(x->ev[4], s));
           timed = true;
-          launch_gas_m(c, T, bo, L, Pm, lanes, variant, s);
-          launch_seg_scan_m(c, T, ch, bo, L, Pm, std::max(k.longest, 1), s);
+          launch_gas_m(c, T, bo, L, Pm, lanes, variant, 0, s);
+          launch_seg_scan_m(c, T, ch, bo, L, Pm, std::max(k.longest, 1), 0, s);
           CK(cudaGetLastError());
           launches += 3;
         }
@@ -1344,7 +1374,7 @@ int fd_core(jgb_ctx* x, const FdLayout& H, const FdInput& in, const std::vector<
     const int nob = (int)(i1 - i0);
     std::vector<int> eoff_l(1, 0), eoff_r(1, 0), esrc, e0(nob), ebase;
     std::vector<int4> pert;
-    // by default only chunks of many tile waves resume (see run_core)
+    // by default only chunks of more than a wave of warps may resume (see run_core)
     bool res_chunk = resume;
     if (resume && x->fd_resume == 1) {
       long long prays = 0;
@@ -1352,8 +1382,8 @@ int fd_core(jgb_ctx* x, const FdLayout& H, const FdInput& in, const std::vector<
         const int o = list[q];
         prays += (long long)H.ncnt[o] * (H.ray_off[o + 1] - H.ray_off[o]);
       }
-      const double waves = (double)((prays + 31) / 32) * ((c.nd + 3) / 4) / (8.0 * x->sms);
-      res_chunk = waves >= 8.0;
+      const double waves = (double)((prays + 31) / 32) * c.nd * c.ng / (40.0 * x->sms);
+      res_chunk = waves >= 1.5;
     }
     if (res_chunk)  // unperturbed base copies first
       for (size_t q = i0; q < i1; q++) {

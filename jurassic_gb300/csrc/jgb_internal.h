@@ -94,52 +94,49 @@ struct MixedPlan {
   float* seg;
   int* stop;
   const float* cloud;   // [nd][nray] cloud extinction (NaN: none), nullptr: no clouds
-  // resumed forward models (finite-difference perturbations): start[r] is
-  // the LOS point ray r starts at (its state read from snap, slot r); ray r
-  // saves the path state for the rays snap_ray[k] before its point
-  // snap_ip[k], k in [snap_off[r], snap_off[r+1]); nullptr: no resume
+  // Resumed forward models (finite-difference perturbations), for channels
+  // [gid0, gid0 + gndc): ray r starts at LOS point start[r], where its path
+  // equals its base ray's.  A base ray saves its state for the rays snap_ray[k]
+  // before its point snap_ip[k], k in [snap_off[r], snap_off[r+1]): every
+  // emitter's in snap[((ray * gndc + channel) * ng + emitter) * state words],
+  // the sums in snap_sums[(ray * gndc + channel) * 3].  A perturbation of one
+  // emitter's mixing ratio (or of an extinction) leaves the other emitters'
+  // inputs and path states equal to the base's: a ray with reuse[r] = {base
+  // ray, emitter} takes every emitter but that one (< 0: all) from its base's
+  // segments, base_seg (entries base_nseg) and base_stop, laid out as seg and
+  // stop over the base tiles, the base ray in tile and lane base_slot[ray].
+  // nullptr start: no resume; nullptr reuse: nothing shared.
+  int gid0, gndc;
   const int* start;
   const int* snap_off;
   const int* snap_ip;
   const int* snap_ray;
-  float* snap;          // [nray][nd][kStateWords * ng + 3]
-  // resumed launches, emitters shared with the base ray: a perturbation of
-  // one emitter's mixing ratio (or of an extinction) leaves the other
-  // emitters' inputs and path states equal to the base's.  The base launch
-  // (reuse == nullptr) writes every emitter's segment emissivity at
-  // seg_base[((L.off[rb] + ip) * nd + id) * ng + g] and the emitters'
-  // saturation flags as bits of seg_satm[(L.off[rb] + ip) * nd + id], the
-  // points it walked in seg_nvalid[rb * nd + id] and its final emitter states
-  // at seg_final[(rb * nd + id) * kStateWords * ng]; a perturbed ray r with
-  // reuse[r] = {rb, pg}, rb >= 0, takes every emitter but pg (pg < 0: all)
-  // from there while ip < nvalid and continues from the base's final states
-  // after that.  nullptr seg_base: nothing shared.
-  float* seg_base;
-  unsigned* seg_satm;
-  int* seg_nvalid;
-  unsigned* seg_final;
+  unsigned* snap;
+  float* snap_sums;
   const int2* reuse;
+  const int* base_slot;
+  const float* base_seg;
+  const int* base_stop;
+  int base_nseg;
 };
 int mixed_nfield(const CtlDev& c, unsigned brmask);
 void launch_pack_tiles_n(const CtlDev& c, const TblDev& T, const LosDev& L, const MixedPlan& P,
                          long long total_tile_points, cudaStream_t s);
 // the path of a chunk: the emitters' paths (lanes_per_ray 1 or 4; variant:
-// the autotuner's choice for 1), then segments and sums
+// the autotuner's choice for 1), then segments and sums; res 0, or 1 for the
+// base rays and 2 (one lane per ray) for the perturbations of a resumed batch
 int path_gas_variants();
 void launch_gas_m(const CtlDev& c, const TblDev& T, const BatchDev& b, const LosDev& L,
-                  const MixedPlan& P, int lanes_per_ray, int variant, cudaStream_t s);
+                  const MixedPlan& P, int lanes_per_ray, int variant, int res, cudaStream_t s);
 void launch_seg_scan_m(const CtlDev& c, const TblDev& T, const ChanDev& ch, const BatchDev& b,
-                       const LosDev& L, const MixedPlan& P, int longest, cudaStream_t s);
+                       const LosDev& L, const MixedPlan& P, int longest, int res, cudaStream_t s);
 void launch_cloud_m(const CtlDev& c, const ChanDev& ch, const BatchDev& b, float* out,
                     cudaStream_t s);
 // FP32 channel constants of the path
 size_t chan_const_bytes(const CtlDev& c);
 void launch_chan_consts(const CtlDev& c, const ChanDev& ch, float* out, cudaStream_t s);
-// the path of tiles [P.tile0, P.tile1) with resume points and state snapshots
-void launch_path_resume(const CtlDev& c, const TblDev& T, const ChanDev& ch, const BatchDev& b,
-                        const LosDev& L, const MixedPlan& P, cudaStream_t s);
-// words of one saved path state (per ray and channel)
-int path_state_words(const CtlDev& c);
+// bytes of an emitter's saved path state
+size_t gas_state_bytes();
 void launch_src_to_float(int nd, const double* sr, float* srf, cudaStream_t s);
 void launch_tables_to_float(long long n, const double* src, float* dst, cudaStream_t s);
 void launch_rowmeta(long long nrow, int tu, const int* nu, const float* u, const float* e, int cga,

@@ -300,7 +300,7 @@ __global__ void k_pack_tiles(CtlDev c, TblDev T, LosDev L, MixedPlan P, long lon
   const int r = P.perm[tile * 32 + lane];
   const Fields F = fields_of(c, P.brmask);
   float* out = P.data + tp * (long long)F.n * 32 + lane;
-  if (r < 0 || ip >= L.count[r]) return;  // never read
+  if (r < 0 || ip >= L.count[r] || (P.start && ip < P.start[r])) return;  // never read
   const long long q = L.off[r] + ip;
   const LosDev::F32& Lf = L.f;
   out[F.p * 32] = Lf.p[q];
@@ -690,199 +690,11 @@ __device__ __forceinline__ void write_radiance(const CtlDev& c, const TblDev& T,
   b.tau[oi] = (double)tau;
 }
 
-// The emitter loop runs over a runtime count with the per-emitter state in
-// shared memory: unrolling it over the emitters multiplies the code size
-// beyond the instruction cache and the register count beyond what keeps
-// enough warps resident to hide load latency, and thread-local arrays spill
-// through L1 into L2.
-// MINB is the minimum number of resident blocks per SM requested from the
-// register allocator.  This form (all emitters of a point in one warp, sums
-// along the way) serves the resumed batches of finite-difference
-// perturbations: rays start at P.start[r] from a saved state and save states
-// for other rays that share a path prefix.  Other batches take k_gas_m,
-// k_seg_m and k_scan_m, whose arithmetic per point is the same.
-template <int MINB, bool CGA, bool SHARE, bool FAST>
-__global__ void __launch_bounds__(kPathThreads, MINB) k_path_mixed(CtlDev c, TblDev T, ChanDev ch,
-                                                                   BatchDev b, LosDev L,
-                                                                   MixedPlan P) {
-  constexpr int nth = kPathThreads;
-  const int ng = c.ng;
-  const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
-  constexpr int W = nth / 32;  // warps of a block
-  // one channel of W consecutive tiles: the perturbations of one observation
-  // share table rows
-  const int tile = P.tile0 + (int)(blockIdx.x / c.nd) * W + warp;
-  const int id = (int)(blockIdx.x % c.nd);
-  if (tile >= P.tile1) return;
-  int r = P.perm[tile * 32 + lane];
-  if (r >= 0 && b.obs_skip && b.obs_skip[b.ray_obs[r]]) r = -1;  // lane idle, outputs untouched
-  const bool skip = r >= 0 && b.skip_masked && b.mask[(long long)id * b.nray + r];
-  const int n = r >= 0 && !skip ? L.count[r] : 0;
-  const Fields F = fields_of(c, P.brmask);
-  const float* base = P.data + P.toff[tile] * (long long)F.n * 32 + lane;
-
-  // per-emitter path state in shared memory, word-major per thread:
-  // sh[(g * kStateWords + w) * nth + threadIdx.x]
-  extern __shared__ unsigned sh_state[];
-  const int tid = threadIdx.x;
-  // behind the state: the channel's constants per warp and each thread's
-  // cloud extinction, read where used so that they hold no registers across
-  // the emitter loop
-  float* const sh_tail = reinterpret_cast<float*>(sh_state + kStateWords * nth * (ng > 0 ? ng : 1));
-  volatile float* kc = sh_tail + warp * kChanConsts;
-  volatile float* kthr = sh_tail + W * kChanConsts + tid;
-  if (lane < kChanConsts) kc[lane] = T.chanf[id * kChanConsts + lane];
-  bool has_cloud = false;
-  kthr[0] = r >= 0 ? cloud_of(c, ch, b, r, id, &has_cloud) : 0.f;
-  __syncwarp();
-  // the pressure-bracket word is only used where the bracket is searched
-  // here (pre = false); with a precomputed bracket it keeps its initial -1
-  auto sload = [&](int g, bool pre = false) {
-    const unsigned* q = sh_state + (g * kStateWords) * nth + tid;
-    GasState st;
-    st.t = __uint_as_float(q[0]);
-    st.e = __uint_as_float(q[nth]);
-    st.ipr = pre ? -1 : (int)q[2 * nth];
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-      const unsigned hw = q[(3 + k) * nth];
-      st.h[2 * k] = (int)(hw & 0xffffu);
-      st.h[2 * k + 1] = (int)(hw >> 16);
-    }
-    return st;
-  };
-  auto sstore = [&](int g, const GasState& st, bool pre = false) {
-    unsigned* q = sh_state + (g * kStateWords) * nth + tid;
-    q[0] = __float_as_uint(st.t);
-    q[nth] = __float_as_uint(st.e);
-    if (!pre) q[2 * nth] = (unsigned)st.ipr;
-#pragma unroll
-    for (int k = 0; k < 2; k++)
-      q[(3 + k) * nth] = (unsigned)st.h[2 * k] | ((unsigned)st.h[2 * k + 1] << 16);
-  };
-  for (int g = 0; g < ng; g++) {
-    GasState st;
-    st.t = 1.f;
-    st.e = 0.f;
-    st.ipr = -1;
-#pragma unroll
-    for (int k = 0; k < 4; k++) st.h[k] = 0;
-    sstore(g, st);
-  }
-  const long long dg0 = (long long)id * ng;
-  float rad = 0.f, comp = 0.f, tau = 1.f;
-
-  // resume: the state words of every emitter and rad, comp, tau
-  const int sw = kStateWords * ng;
-  auto snap_write = [&](int target) {
-    float* q = P.snap + ((long long)target * c.nd + id) * (sw + 3);
-    for (int k = 0; k < sw; k++) q[k] = __uint_as_float(sh_state[k * nth + tid]);
-    q[sw] = rad;
-    q[sw + 1] = comp;
-    q[sw + 2] = tau;
-  };
-  int start = 0, sn = 0, se = 0;
-  if (n > 0) {
-    start = P.start[r];
-    if (start > 0) {
-      const float* q = P.snap + ((long long)r * c.nd + id) * (sw + 3);
-      for (int k = 0; k < sw; k++) sh_state[k * nth + tid] = __float_as_uint(q[k]);
-      rad = q[sw];
-      comp = q[sw + 1];
-      tau = q[sw + 2];
-    }
-    sn = P.snap_off[r];
-    se = P.snap_off[r + 1];
-  }
-
-  // emitters shared with the base ray (see MixedPlan): rb >= 0 takes every
-  // emitter but pg from the base while ip < nvalid; a base lane writes them
-  const bool seg_write = SHARE && P.reuse == nullptr && r >= 0 && n > 0;
-  int rb = -1, pg = -1, nvalid = 0;
-  if (SHARE && P.reuse != nullptr && r >= 0 && n > 0) {
-    const int2 ru = P.reuse[r];
-    rb = ru.x;
-    pg = ru.y;
-    if (rb >= 0) nvalid = P.seg_nvalid[(long long)rb * c.nd + id];
-  }
-  int walked = n;  // points this lane walked (a base lane records it)
-  // LOS offset of the base ray whose entries this lane writes or reads
-  const long long soff = !SHARE ? 0 : rb >= 0 ? L.off[rb] : seg_write ? L.off[r] : 0;
-
-  // resumed lanes join the warp's walk at their own start point: every
-  // iteration reads one point of the tile for all lanes (coalesced)
-  const unsigned wmin = __reduce_min_sync(0xffffffffu, n > 0 ? (unsigned)start : 0xffffffffu);
-  for (int ip = wmin == 0xffffffffu ? 0 : (int)wmin; ip < n; ip++) {
-    if (ip < start) continue;
-    if (tau < kTauStop) {  // opaque from here on (see k_scan_m)
-      walked = ip;
-      break;
-    }
-    for (; sn < se && P.snap_ip[sn] == ip; sn++) snap_write(P.snap_ray[sn]);
-    // the base stopped here: the shared emitters continue from its final states
-    if (SHARE && rb >= 0 && ip == nvalid) {
-      const unsigned* q = P.seg_final + ((long long)rb * c.nd + id) * sw;
-      for (int g2 = 0; g2 < ng; g2++)
-        if (g2 != pg)
-          for (int k = 0; k < kStateWords; k++)
-            sh_state[(g2 * kStateWords + k) * nth + tid] = q[g2 * kStateWords + k];
-    }
-    const bool shared = SHARE && rb >= 0 && ip < nvalid;
-    const long long sbase = SHARE ? (soff + ip) * c.nd + id : 0;
-    const unsigned satm_in = shared ? P.seg_satm[sbase] : 0u;
-    unsigned satm_out = 0u;
-    const float* f = base + (long long)ip * F.n * 32;
-    const float p = f[F.p * 32], t = f[F.t * 32], ds = f[F.ds * 32];
-    float E = 0.f;
-    bool sat = false;
-#pragma unroll 1
-    for (int g = 0; g < ng; g++) {
-      float eg;
-      if (SHARE && shared && g != pg) {
-        eg = P.seg_base[sbase * ng + g];
-        if ((satm_in >> g) & 1u) sat = true;
-      } else {
-        constexpr int es = kEmitterFields(CGA), kb = kFBr(CGA);
-        const float* fg = f + (F.g0 + g * es) * 32;
-        const float du = CGA ? 0.f : fg[kFU * 32];
-        const float pq = CGA ? fg[kFCgp * 32] : p;
-        const float tq = CGA ? fg[kFCgt * 32] : t;
-        const float ucg = CGA ? fg[kFCgu * 32] : 0.f;
-        const bool brg = FAST || ((P.brmask >> g) & 1u);
-        const float4 cw = brg ? cell_words(fg + kb * 32, lane) : no_cell();
-        GasState st = sload(g, brg);
-        bool sg = false;
-        eg = gas_eps_f<CGA, FAST>(T, dg0 + g, pq, tq, du, ucg, cw, st, sg);
-        sstore(g, st, brg);
-        if (sg) sat = true;
-        if (SHARE && seg_write) {
-          P.seg_base[sbase * ng + g] = eg;
-          if (sg) satm_out |= 1u << g;
-        }
-      }
-      E = join_f(E, eg);
-    }
-    if (SHARE && seg_write) P.seg_satm[sbase] = satm_out;
-    if (!sat) {
-      float beta = c.nw > 0 ? f[(F.kw0 + __float_as_int(kc[kChanWindow])) * 32] : 0.f;
-      if (has_cloud) beta = __fmaf_rn(f[F.aux * 32], kthr[0], beta);
-      beta = continua_f(c, F, kc, continua_on(c, kc[kChanSwitches]), f, p, t, ds, beta);
-      const float src = source_f(T.srf + (long long)id * kNS, t);
-      const float eps = segment_f(E, beta, ds);
-      add_f(__fmul_rn(src, eps), __fsub_rn(1.f, eps), rad, comp, tau);
-    }
-  }
-  // states for resume points beyond the end of this walk (a path that became
-  // opaque earlier hands its final state on, so the resumed rays stop too)
-  for (; sn < se; sn++) snap_write(P.snap_ray[sn]);
-  if (SHARE && seg_write) {  // what a perturbed ray needs past this walk
-    P.seg_nvalid[(long long)r * c.nd + id] = walked;
-    unsigned* q = P.seg_final + ((long long)r * c.nd + id) * sw;
-    for (int k = 0; k < sw; k++) q[k] = sh_state[k * nth + tid];
-  }
-  if (r < 0) return;
-  write_radiance(c, T, ch, b, L, id, r, rad, tau, nullptr, 0, 0);
+// Does perturbed ray r take emitter g from its base ray?
+__device__ __forceinline__ bool shared_gas(const MixedPlan& P, int r, int g) {
+  if (!P.reuse) return false;
+  const int2 ru = P.reuse[r];
+  return ru.x >= 0 && ru.y != g;
 }
 
 // ---------------------------------------------------------------------------
@@ -901,7 +713,17 @@ __global__ void __launch_bounds__(kPathThreads, MINB) k_path_mixed(CtlDev c, Tbl
 // 17 ms in a kernel that held all emitters of a channel in a warp (527
 // instructions, state in shared memory).  What the register count costs
 // shows in the variants: spilling forms take 13.8 ms, 64 registers 12.9 ms.
-template <bool CGA, int LPR, int MINB, bool FAST>
+//
+// RES: 1 the base rays of resumed perturbations, which leave their state
+// before every start point of their perturbations; 2 the perturbations, which
+// walk on from there, and not at all for an emitter they share with the base.
+// 48 nadir observations x 405 perturbations, 150 channels, 4 emitters: 32 ms
+// here and 19 ms in k_seg_m (6.8e7 and 3.8e7 warp points; bound by issue as
+// above, with 1.6 times the plain batch's time per point since a warp's rays
+// come from several observations and share fewer rows), against 64 ms in a
+// kernel that held all emitters of a channel in a warp and joined the shared
+// ones there.
+template <bool CGA, int LPR, int MINB, bool FAST, int RES = 0>
 __global__ void __launch_bounds__(kPathThreads, MINB) k_gas_m(CtlDev c, TblDev T, BatchDev b,
                                                               LosDev L, MixedPlan P, int shape) {
   constexpr int W = kPathThreads / 32;
@@ -935,7 +757,8 @@ __global__ void __launch_bounds__(kPathThreads, MINB) k_gas_m(CtlDev c, TblDev T
   int r = P.perm[tile * 32 + rl];
   if (r >= 0 && b.obs_skip && b.obs_skip[b.ray_obs[r]]) r = -1;
   if (r >= 0 && b.skip_masked && b.mask[(long long)id * b.nray + r]) r = -1;
-  const int n = r >= 0 ? L.count[r] : 0;
+  int n = r >= 0 ? L.count[r] : 0;
+  if (RES == 2 && n > 0 && shared_gas(P, r, g)) n = 0;
   const Fields F = fields_of(c, P.brmask);
   constexpr int es = kEmitterFields(CGA), kb = kFBr(CGA);
   const float* f = P.data + P.toff[tile] * (long long)F.n * 32 + rl;
@@ -952,8 +775,65 @@ __global__ void __launch_bounds__(kPathThreads, MINB) k_gas_m(CtlDev c, TblDev T
 #pragma unroll
   for (int k = 0; k < 4; k++) st.h[k] = 0;
   int stop = n;  // the first point that is saturated: all later ones are too
+  // resumed perturbations: the state before a start point
+  int sn = 0, se = 0;
+  auto state_of = [&](int ray) {
+    return P.snap + (((long long)ray * P.gndc + (id - P.gid0)) * ng + g) * kStateWords;
+  };
+  auto save = [&](int target) {
+    if (shared_gas(P, target, g)) return;
+    unsigned* q = state_of(target);
+    if (LPR == 1 || corner == 0) {
+      q[0] = __float_as_uint(st.t);
+      q[1] = __float_as_uint(st.e);
+      q[2] = (unsigned)st.ipr;
+    }
+    unsigned short* h = reinterpret_cast<unsigned short*>(q + 3);
+    if (LPR == 4) h[corner] = (unsigned short)st.h[0];
+    else
+#pragma unroll
+      for (int k = 0; k < 4; k++) h[k] = (unsigned short)st.h[k];
+  };
+  if (RES == 1 && n > 0) {
+    sn = P.snap_off[r];
+    se = P.snap_off[r + 1];
+  }
+  int next = RES == 1 && sn < se ? P.snap_ip[sn] : 0x7fffffff;
+  auto save_at = [&](int ip) {
+    while (next == ip) {
+      save(P.snap_ray[sn]);
+      next = ++sn < se ? P.snap_ip[sn] : 0x7fffffff;
+    }
+  };
   if (LPR == 1) {
-    for (int ip = 0; ip < n; ip++) {
+    int start = 0, ip = 0;
+    if (RES == 2) {
+      start = n > 0 ? P.start[r] : 0x7fffffff;
+      ip = (int)__reduce_min_sync(0xffffffffu, (unsigned)start);
+      if (ip == 0x7fffffff) return;  // no lane walks
+      if (n > 0 && start > 0) {
+        const unsigned* q = state_of(r);
+        st.t = __uint_as_float(q[0]);
+        st.e = __uint_as_float(q[1]);
+        st.ipr = (int)q[2];
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+          st.h[2 * k] = (int)(q[3 + k] & 0xffffu);
+          st.h[2 * k + 1] = (int)(q[3 + k] >> 16);
+        }
+      }
+      out += ip * ostep;
+      f += (long long)ip * fstep;
+      fg += (long long)ip * fstep;
+    }
+    for (; ip < n; ip++) {
+      if (RES == 2 && ip < start) {  // one row of the tile for all lanes
+        out += ostep;
+        f += fstep;
+        fg += fstep;
+        continue;
+      }
+      if (RES == 1) save_at(ip);
       const float du = CGA ? 0.f : fg[kFU * 32];
       const float pq = CGA ? fg[kFCgp * 32] : brg ? 0.f : f[F.p * 32];
       const float tq = CGA ? fg[kFCgt * 32] : brg ? 0.f : f[F.t * 32];
@@ -970,6 +850,9 @@ __global__ void __launch_bounds__(kPathThreads, MINB) k_gas_m(CtlDev c, TblDev T
       f += fstep;
       fg += fstep;
     }
+    // beyond the walk's end a perturbation starts saturated, as its base ended
+    if (RES == 1)
+      for (; sn < se; sn++) save(P.snap_ray[sn]);
     if (r >= 0) P.stop[((long long)(tl * ndc + idl) * ng + g) * 32 + rl] = stop;
     return;
   }
@@ -990,6 +873,7 @@ __global__ void __launch_bounds__(kPathThreads, MINB) k_gas_m(CtlDev c, TblDev T
   };
   fetch(0);
   for (int ip = 0; ip < nmax; ip++) {
+    if (RES == 1) save_at(ip);
     bool on = ip < n && stop == n;
     if (on && st.t < 1e-9f) {
       stop = ip;
@@ -1024,6 +908,8 @@ __global__ void __launch_bounds__(kPathThreads, MINB) k_gas_m(CtlDev c, TblDev T
       else if (corner == 0) out[ip * ostep] = eg;
     }
   }
+  if (RES == 1)
+    for (; sn < se; sn++) save(P.snap_ray[sn]);
   if (r >= 0 && corner == 0) P.stop[((long long)(tl * ndc + idl) * ng + g) * 32 + rl] = stop;
 }
 
@@ -1036,6 +922,7 @@ __global__ void __launch_bounds__(kPathThreads, MINB) k_gas_m(CtlDev c, TblDev T
 // 212 here; 3.3 -> 1.8 ms for 6.2e6 warp points, 5.5 GB of DRAM traffic).
 constexpr int kSegRun = 16;
 
+template <int RES>
 __global__ void __launch_bounds__(kPathThreads) k_seg_m(CtlDev c, TblDev T, BatchDev b, LosDev L,
                                                         MixedPlan P) {
   const int lane = threadIdx.x & 31;
@@ -1051,12 +938,28 @@ __global__ void __launch_bounds__(kPathThreads) k_seg_m(CtlDev c, TblDev T, Batc
   // the run ends at the first saturated emitter, where k_scan_m stops
   int n = min(L.count[r], ip0 + kSegRun);
   const int* st = P.stop + (long long)(tl * ndc + idl) * ng * 32 + lane;
-  unsigned has = 0;  // emitters with a table
+  unsigned has = 0, own = ~0u;  // emitters with a table; of this ray, not of its base
+  const float* bseg = nullptr;
+  long long bstep = 0;
+  int start = 0;
+  const int* bst = nullptr;
+  if (RES == 2) {
+    start = P.start[r];
+    const int2 ru = P.reuse ? P.reuse[r] : make_int2(-1, -1);
+    if (ru.x >= 0) {
+      const int slot = P.base_slot[ru.x], bt = slot >> 5, gidl = id - P.gid0;
+      own = ru.y >= 0 ? 1u << ru.y : 0u;
+      bst = P.base_stop + (long long)(bt * P.gndc + gidl) * ng * 32 + (slot & 31);
+      bstep = (long long)P.gndc * P.base_nseg * 32;
+      bseg = P.base_seg + (P.toff[bt] + ip0) * bstep + (long long)gidl * P.base_nseg * 32 + (slot & 31);
+    }
+  }
   for (int g = 0; g < ng; g++)
     if (__ldg(T.np + (long long)id * ng + g) >= 30) {
       has |= 1u << g;
-      n = min(n, st[g * 32]);
+      n = min(n, RES == 2 && !((own >> g) & 1u) ? bst[g * 32] : st[g * 32]);
     }
+  if (RES == 2 && n <= start) return;
   const Fields F = fields_of(c, P.brmask);
   const long long pt = P.toff[tile] + ip0;
   const float* f = P.data + pt * F.n * 32 + lane;
@@ -1068,18 +971,25 @@ __global__ void __launch_bounds__(kPathThreads) k_seg_m(CtlDev c, TblDev T, Batc
   const int kw = c.nw > 0 ? (F.kw0 + __float_as_int(T.chanf[id * kChanConsts + kChanWindow])) * 32 : -1;
   const float cl = P.cloud ? P.cloud[(long long)id * b.nray + r] : __int_as_float(0x7fc00000);
   const float* srf = T.srf + (long long)id * kNS;
+  const int po = RES == 1 ? ng * 32 : 0;  // a base ray's emitters stay for its perturbations
   for (int ip = ip0; ip < n; ip++, f += F.n * 32, seg += sstep) {
     float E = 0.f;
+    if (RES == 2 && ip < start) {
+      bseg += bstep;
+      continue;
+    }
     for (int g = 0; g < ng; g++)
-      if ((has >> g) & 1u) E = join_f(E, seg[g * 32]);
+      if ((has >> g) & 1u)
+        E = join_f(E, RES == 2 && !((own >> g) & 1u) ? bseg[g * 32] : seg[g * 32]);
+    if (RES == 2) bseg += bstep;
     const float p = f[F.p * 32], t = f[F.t * 32], ds = f[F.ds * 32];
     float beta = kw >= 0 ? f[kw] : 0.f;
     if (cl == cl) beta = __fmaf_rn(f[F.aux * 32], cl, beta);
     beta = continua_f(c, F, kc, on, f, p, t, ds, beta);
     const float src = source_f(srf, t);
     const float eps = segment_f(E, beta, ds);
-    seg[0] = __fmul_rn(src, eps);
-    seg[32] = __fsub_rn(1.f, eps);
+    seg[po] = __fmul_rn(src, eps);
+    seg[po + 32] = __fsub_rn(1.f, eps);
   }
 }
 
@@ -1096,6 +1006,7 @@ __global__ void k_cloud_m(CtlDev c, ChanDev ch, BatchDev b, float* out) {
 // It stops at the first saturated emitter (nothing adds after it) and, without
 // surface reflection, once the path transmittance is below kTauStop: the rest
 // adds at most max(src) tau, below 1e-10 of the radiance.
+template <int RES>
 __global__ void __launch_bounds__(kPathThreads) k_scan_m(CtlDev c, TblDev T, ChanDev ch, BatchDev b,
                                                          LosDev L, MixedPlan P) {
   const int lane = threadIdx.x & 31;
@@ -1105,30 +1016,73 @@ __global__ void __launch_bounds__(kPathThreads) k_scan_m(CtlDev c, TblDev T, Cha
   if (tl >= P.tile1 - P.tile0) return;
   const int tile = P.tile0 + tl, id = P.id0 + idl;
   const int r = P.perm[tile * 32 + lane];
-  if (r < 0 || (b.obs_skip && b.obs_skip[b.ray_obs[r]])) return;
-  int n = b.skip_masked && b.mask[(long long)id * b.nray + r] ? 0 : L.count[r];
+  const bool idle = r < 0 || (b.obs_skip && b.obs_skip[b.ray_obs[r]]);
+  if (RES != 2 && idle) return;
+  int n = idle || (b.skip_masked && b.mask[(long long)id * b.nray + r]) ? 0 : L.count[r];
   const int* st = P.stop + (long long)(tl * ndc + idl) * ng * 32 + lane;
-  for (int g = 0; g < ng; g++)
-    if (n > 0 && __ldg(T.np + (long long)id * ng + g) >= 30) n = min(n, st[g * 32]);
-  const float* seg =
-      P.seg + ((P.toff[tile] - P.pt0) * ndc + idl) * (long long)P.nseg * 32 + lane;
-  const long long step = (long long)ndc * P.nseg * 32;
-  const bool refl = c.sftype >= 2 && c.nsf > 0 && L.sft[r] > 0 && sfeps_of(c, ch, b, r, id) < 1.f;
   float rad = 0.f, comp = 0.f, tau = 1.f;
+  int ip = 0, start = 0, sn = 0, se = 0;
+  const int* bst = nullptr;
+  unsigned own = ~0u;
+  auto sums_of = [&](int ray) { return P.snap_sums + ((long long)ray * P.gndc + (id - P.gid0)) * 3; };
+  if (RES == 2) {  // on from the base's sums, one row of the tile for all lanes
+    start = n > 0 ? P.start[r] : 0x7fffffff;
+    ip = (int)__reduce_min_sync(0xffffffffu, (unsigned)start);
+    if (idle) return;
+    if (n > 0) {
+      const int2 ru = P.reuse ? P.reuse[r] : make_int2(-1, -1);
+      if (ru.x >= 0) {
+        const int slot = P.base_slot[ru.x];
+        own = ru.y >= 0 ? 1u << ru.y : 0u;
+        bst = P.base_stop + (long long)((slot >> 5) * P.gndc + (id - P.gid0)) * ng * 32 + (slot & 31);
+      }
+      if (start > 0) {
+        const float* q = sums_of(r);
+        rad = q[0];
+        comp = q[1];
+        tau = q[2];
+      }
+    }
+  }
+  for (int g = 0; g < ng; g++)
+    if (n > 0 && __ldg(T.np + (long long)id * ng + g) >= 30)
+      n = min(n, RES == 2 && !((own >> g) & 1u) ? bst[g * 32] : st[g * 32]);
+  if (RES == 1 && !(b.skip_masked && b.mask[(long long)id * b.nray + r])) {
+    sn = P.snap_off[r];
+    se = P.snap_off[r + 1];
+  }
+  int next = sn < se ? P.snap_ip[sn] : 0x7fffffff;
+  auto save = [&]() {
+    float* q = sums_of(P.snap_ray[sn]);
+    q[0] = rad;
+    q[1] = comp;
+    q[2] = tau;
+    next = ++sn < se ? P.snap_ip[sn] : 0x7fffffff;
+  };
+  const float* seg = P.seg + ((P.toff[tile] - P.pt0) * ndc + idl) * (long long)P.nseg * 32 + lane +
+                     (RES == 1 ? ng * 32 : 0);
+  const long long step = (long long)ndc * P.nseg * 32;
+  const bool refl = RES == 0 && c.sftype >= 2 && c.nsf > 0 && L.sft[r] > 0 &&
+                    sfeps_of(c, ch, b, r, id) < 1.f;
   constexpr int U = 8;  // loads in flight ahead of the sums
-  for (int ip = 0; ip < n; ip += U) {
+  for (; ip < n; ip += U) {
     if (tau < kTauStop && !refl) break;
     float v[U], m[U];
 #pragma unroll
     for (int k = 0; k < U; k++) {
-      const bool in = ip + k < n;
+      const bool in = ip + k < n && (RES != 2 || ip + k >= start);
       v[k] = in ? seg[(ip + k) * step] : 0.f;
       m[k] = in ? seg[(ip + k) * step + 32] : 1.f;
     }
 #pragma unroll
-    for (int k = 0; k < U; k++)
-      if (ip + k < n && (refl || !(tau < kTauStop))) add_f(v[k], m[k], rad, comp, tau);
+    for (int k = 0; k < U; k++) {
+      if (RES == 1 && ip + k < n)
+        while (next == ip + k) save();
+      if (ip + k < n && (RES != 2 || ip + k >= start) && (refl || !(tau < kTauStop)))
+        add_f(v[k], m[k], rad, comp, tau);
+    }
   }
+  while (RES == 1 && sn < se) save();
   write_radiance(c, T, ch, b, L, id, r, rad, tau, refl ? seg : nullptr, step, n);
 }
 
@@ -1204,11 +1158,6 @@ void launch_pack_tiles_n(const CtlDev& c, const TblDev& T, const LosDev& L, cons
   k_pack_tiles<<<(unsigned)((nth + bs - 1) / bs), bs, 0, s>>>(c, T, L, P, total_tile_points);
 }
 
-size_t path_smem(const CtlDev& c) {
-  return sizeof(unsigned) * kStateWords * kPathThreads * (size_t)(c.ng > 0 ? c.ng : 1) +
-         sizeof(float) * ((kPathThreads / 32) * kChanConsts + kPathThreads);
-}
-
 // Variants of k_gas_m with one lane per ray, chosen by the autotuner: block
 // shape (v / 4) and minimum resident blocks per SM (v % 4: 8, 10, 12, 16, i.e.
 // at most 64, 48, 40 and 32 registers).
@@ -1216,18 +1165,20 @@ int path_gas_variants() { return 8; }
 
 template <bool CGA>
 void launch_gas_v(const CtlDev& c, const TblDev& T, const BatchDev& b, const LosDev& L,
-                  const MixedPlan& P, int lanes_per_ray, int variant, cudaStream_t s) {
+                  const MixedPlan& P, int lanes_per_ray, int variant, int res, cudaStream_t s) {
   const long long nt = P.tile1 - P.tile0, ndc = P.id1 - P.id0;
   constexpr int W = kPathThreads / 32;
-  if (lanes_per_ray == 4) {
-    const unsigned nblk = (unsigned)((nt * ndc * c.ng * 4 + W - 1) / W);
-    if (P.fast) k_gas_m<CGA, 4, 8, true><<<nblk, kPathThreads, 0, s>>>(c, T, b, L, P, 0);
-    else k_gas_m<CGA, 4, 8, false><<<nblk, kPathThreads, 0, s>>>(c, T, b, L, P, 0);
-    return;
-  }
-  const int shape = variant / 4;
-  const unsigned nblk = (unsigned)(shape ? (nt + W - 1) / W * ndc * c.ng : (nt * ndc * c.ng + W - 1) / W);
+  const int shape = lanes_per_ray == 4 ? 0 : variant / 4;
+  const unsigned nblk =
+      (unsigned)(lanes_per_ray == 4 ? (nt * ndc * c.ng * 4 + W - 1) / W
+                 : shape ? (nt + W - 1) / W * ndc * c.ng : (nt * ndc * c.ng + W - 1) / W);
   auto go = [&](auto kern) { kern<<<nblk, kPathThreads, 0, s>>>(c, T, b, L, P, shape); };
+  if (res == 1) {
+    if (lanes_per_ray == 4) return P.fast ? go(k_gas_m<CGA, 4, 8, true, 1>) : go(k_gas_m<CGA, 4, 8, false, 1>);
+    return P.fast ? go(k_gas_m<CGA, 1, 8, true, 1>) : go(k_gas_m<CGA, 1, 8, false, 1>);
+  }
+  if (res == 2) return P.fast ? go(k_gas_m<CGA, 1, 10, true, 2>) : go(k_gas_m<CGA, 1, 8, false, 2>);
+  if (lanes_per_ray == 4) return P.fast ? go(k_gas_m<CGA, 4, 8, true>) : go(k_gas_m<CGA, 4, 8, false>);
   if (!P.fast) return go(k_gas_m<CGA, 1, 8, false>);
   switch (variant % 4) {
     case 0: go(k_gas_m<CGA, 1, 8, true>); break;
@@ -1238,18 +1189,28 @@ void launch_gas_v(const CtlDev& c, const TblDev& T, const BatchDev& b, const Los
 }
 
 void launch_gas_m(const CtlDev& c, const TblDev& T, const BatchDev& b, const LosDev& L,
-                  const MixedPlan& P, int lanes_per_ray, int variant, cudaStream_t s) {
+                  const MixedPlan& P, int lanes_per_ray, int variant, int res, cudaStream_t s) {
   if (c.ng <= 0) return;
-  if (c.formod == 0) launch_gas_v<true>(c, T, b, L, P, lanes_per_ray, variant, s);
-  else launch_gas_v<false>(c, T, b, L, P, lanes_per_ray, variant, s);
+  if (c.formod == 0) launch_gas_v<true>(c, T, b, L, P, lanes_per_ray, variant, res, s);
+  else launch_gas_v<false>(c, T, b, L, P, lanes_per_ray, variant, res, s);
 }
 
 void launch_seg_scan_m(const CtlDev& c, const TblDev& T, const ChanDev& ch, const BatchDev& b,
-                       const LosDev& L, const MixedPlan& P, int longest, cudaStream_t s) {
+                       const LosDev& L, const MixedPlan& P, int longest, int res, cudaStream_t s) {
   const long long nt = P.tile1 - P.tile0, ndc = P.id1 - P.id0, nchb = (ndc + 3) / 4;
   const long long runs = (longest + kSegRun - 1) / kSegRun;
-  k_seg_m<<<dim3((unsigned)(nchb * runs), (unsigned)nt), kPathThreads, 0, s>>>(c, T, b, L, P);
-  k_scan_m<<<(unsigned)((nt * ndc + 3) / 4), kPathThreads, 0, s>>>(c, T, ch, b, L, P);
+  const dim3 gs((unsigned)(nchb * runs), (unsigned)nt);
+  const unsigned gn = (unsigned)((nt * ndc + 3) / 4);
+  if (res == 1) {
+    k_seg_m<1><<<gs, kPathThreads, 0, s>>>(c, T, b, L, P);
+    k_scan_m<1><<<gn, kPathThreads, 0, s>>>(c, T, ch, b, L, P);
+  } else if (res == 2) {
+    k_seg_m<2><<<gs, kPathThreads, 0, s>>>(c, T, b, L, P);
+    k_scan_m<2><<<gn, kPathThreads, 0, s>>>(c, T, ch, b, L, P);
+  } else {
+    k_seg_m<0><<<gs, kPathThreads, 0, s>>>(c, T, b, L, P);
+    k_scan_m<0><<<gn, kPathThreads, 0, s>>>(c, T, ch, b, L, P);
+  }
 }
 
 void launch_cloud_m(const CtlDev& c, const ChanDev& ch, const BatchDev& b, float* out,
@@ -1264,31 +1225,7 @@ void launch_chan_consts(const CtlDev& c, const ChanDev& ch, float* out, cudaStre
 
 size_t chan_const_bytes(const CtlDev& c) { return sizeof(float) * kChanConsts * (size_t)c.nd; }
 
-int path_state_words(const CtlDev& c) { return kStateWords * c.ng + 3; }
-
-void launch_path_resume(const CtlDev& c, const TblDev& T, const ChanDev& ch, const BatchDev& b,
-                        const LosDev& L, const MixedPlan& P, cudaStream_t s) {
-  const unsigned nblk = (unsigned)((long long)((P.tile1 - P.tile0 + 3) / 4) * c.nd);
-  if (nblk == 0) return;
-  const size_t smem = path_smem(c);
-  auto go = [&](auto kern) {
-    if (smem > 48 * 1024)  // many emitters: opt in to the larger shared memory
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    kern<<<nblk, kPathThreads, smem, s>>>(c, T, ch, b, L, P);
-  };
-  const bool share = P.seg_base != nullptr;
-  auto pick = [&](auto cga, auto fast) {
-    if (share) go(k_path_mixed<8, cga.value, true, fast.value>);
-    else go(k_path_mixed<8, cga.value, false, fast.value>);
-  };
-  if (c.formod == 0) {
-    if (P.fast) pick(std::true_type{}, std::true_type{});
-    else pick(std::true_type{}, std::false_type{});
-  } else {
-    if (P.fast) pick(std::false_type{}, std::true_type{});
-    else pick(std::false_type{}, std::false_type{});
-  }
-}
+size_t gas_state_bytes() { return sizeof(unsigned) * kStateWords; }
 
 void launch_src_to_float(int nd, const double* sr, float* srf, cudaStream_t s) {
   const int n = nd * kNS, bs = 256;

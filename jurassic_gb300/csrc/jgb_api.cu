@@ -471,8 +471,11 @@ void path_chunks(const std::vector<long long>& toff, int tfirst, int nd, size_t 
 }
 
 // Up to here (warps of 32 rays per SM) a ray gets four lanes: a warp alone
-// walks its chain in a fifth of the time then, until the device is full.
-constexpr long long kFourLaneWarps = 8;
+// walks its chain in a fifth of the time then, until the device is full.  One
+// lane and four, ms: 128 nadir rays x 500 channels and emitters (13 warps per
+// SM) 2.41 and 2.02, 224 (23) 2.68 and 3.06; 1184 limb rays (CGA, 23) 0.76 and
+// 0.64.
+constexpr long long kFourLaneWarps = 18;
 
 // The autotuner of the mixed path: times every variant of the emitters'
 // kernel on a chunk (the results are the same) and keeps the fastest;

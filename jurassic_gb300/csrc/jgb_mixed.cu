@@ -7,8 +7,8 @@
 // three kernels: k_gas_m walks the points for one (tile, channel, emitter)
 // per warp, k_seg_m joins the emitters' segments of every (point, channel)
 // with the continua, k_scan_m sums them along the rays.  Resumed
-// finite-difference perturbations take one kernel for all three
-// (k_path_mixed), which saves and restores path states.
+// finite-difference perturbations start in the middle of a path, from the
+// states that their base rays saved there.
 //
 // Numerics (same algorithm as intpol_tbl_ega/cga, jurassic.c:3710-3891, and
 // formod_pencil, 3196-3338):

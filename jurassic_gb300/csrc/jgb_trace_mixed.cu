@@ -805,19 +805,24 @@ __global__ void k_trace_fill_m(CtlDev c, BatchDev b, LosDev L, const int* order,
   ray_finish_m(b, L, r, n, sft, gk);
 }
 
-// Four lanes walk one ray: lanes 0-2 the components of the FP64 position and
-// direction and the three refraction sub-points, the emitters and windows
-// dealt over all four.  A ray is a chain of dependent steps, bound by latency:
-// with one lane per ray a nadir step took 5000 cycles; the sub-points in turn,
-// the emitters in turn and 35 FP64 instructions (64 cycles of a warp each,
-// conversions and compares among them).  Here a step has 7 FP64 instructions,
-// conversions and compares run on the integer pipe and a step takes 3800.  One
-// nadir ray of 901 points: 2.4 to 1.87 ms; 1500 rays of 801: 2.7 to 2.12 ms.
-// 20000 limb rays stay at 2.25 ms: there the loads of the rays' level values
-// bind (cold lines of 20000 profiles; prefetches and a 96-register build with
-// more warps were slower, 3.1 ms).  Every value is formed as in walk_m, in the
-// same order, so both give the same LOS.  All lanes stay in the loop until the
-// warp's eight rays are done.
+// The fill pass of a batch takes two kernels.  A ray's walk is a chain of
+// dependent steps, bound by latency, so k_walk_m does nothing but the chain and
+// leaves z, p, T, the trapezoid lengths and the level interval of every point;
+// k_points_m adds the mixing ratios, column densities and extinctions, which
+// no step needs, for all points at once.
+//
+// k_walk_m: four lanes per ray, lanes 0-2 the components of the FP64 position
+// and direction and the three refraction sub-points.  Conversions and compares
+// run on the integer pipe (an FP64 instruction, these among them, holds a warp
+// for 64 cycles; 7 are left per step).  Every value is formed as in walk_m, in
+// the same order, so both give the same LOS.  All lanes stay in the loop until
+// the warp's eight rays are done.
+// Walks of one nadir ray of 901 points, 1500 of 801 and 20000 limb rays (CGA),
+// both kernels: 1.49, 1.47 and 1.60 ms.  With the emitters in the same kernel,
+// dealt over the four lanes, 1.87, 2.12 and 2.27; with one lane per ray 2.40,
+// 2.70 and 2.28.  A step takes 3000 cycles of a warp at one ray; with many rays
+// the loads of their level values add to it (a build of 96 registers, for more
+// warps, was slower: 3.1 ms with the emitters inside against 2.3).
 constexpr int kWalk4 = 4;
 
 __device__ __forceinline__ float from4(float v, int k) {
@@ -827,21 +832,11 @@ __device__ __forceinline__ double from4(double v, int k) {
   return __shfl_sync(0xffffffffu, v, k, kWalk4);
 }
 
-// float4 of shared memory per thread: per emitter or window of the lane's
-// share the current level's value and slope and (emitters) the mixing ratio of
-// the pending point, and the Curtis-Godson sums
-__host__ __device__ inline int trace4_smem_slots(const CtlDev& c) {
-  const int ng = (c.ng + kWalk4 - 1) / kWalk4, nw = (c.nw + kWalk4 - 1) / kWalk4;
-  return ng + nw + (c.formod == 0 ? 2 * ng : 0);
-}
-
 template <int ROLE>
 __global__ void __launch_bounds__(kTraceThreads)
-    k_trace_fill_m4(CtlDev c, BatchDev b, LosDev L, const int* order, int r0, int nr_l,
+    k_walk_m(CtlDev c, BatchDev b, LosDev L, const int* order, int r0, int nr_l,
                     TraceResume R, unsigned* err) {
-  extern __shared__ float4 sm4[];
   __shared__ GeoKeep keep[kTraceThreads / kWalk4];
-  constexpr int S = kTraceThreads;
   const int s = threadIdx.x & (kWalk4 - 1);
   const int th = (int)(blockIdx.x * blockDim.x + threadIdx.x) / kWalk4;
   GeoKeep& gk = keep[threadIdx.x / kWalk4];
@@ -886,50 +881,9 @@ __global__ void __launch_bounds__(kTraceThreads)
   double zmin_seen = 0, last_z = 0, x_last = 0;
   Lev lv;
   lv.i = -1;
-  // this lane's emitters s, s + 4, ... and windows, in shared memory
-  const int nge = (c.ng - s + kWalk4 - 1) / kWalk4, nwe = (c.nw - s + kWalk4 - 1) / kWalk4;
-  const int jh2o = c.ig_h2o >= 0 && (c.ig_h2o & (kWalk4 - 1)) == s ? c.ig_h2o / kWalk4 : -1;
-  const int ng_max = (c.ng + kWalk4 - 1) / kWalk4, nw_max = (c.nw + kWalk4 - 1) / kWalk4;
-  float4* const qv = sm4 + threadIdx.x;
-  float4* const kv = qv + ng_max * S;
-  float4* const cg = kv + nw_max * S;
-  const long long stride4 = kWalk4 * L.cap;
-  float* const u0 = L.f.u + s * L.cap + base;
-  const bool cloud = c.ncl > 0 && a.cldz > 0;
-  if (L.cga)
-    for (int j = 0; j < 2 * nge; j++) cg[j * S] = make_float4(0.f, 0.f, 0.f, 0.f);
-  int qc_level = -1;
-  float raw_before = 0.f, raw_pend = 0.f, pend_p = 0.f, pend_t = 0.f;
-  auto finalize = [&](int ip) {
-    const float dsT = ip == 0 ? 0.5f * raw_pend : 0.5f * (raw_before + raw_pend);
-    if (s == 0) L.f.ds[base + ip] = dsT;
-    for (int j = 0; j < nge; j++) {
-      const float uu = col_density(qv[j * S].z, pend_p, pend_t, dsT);
-      u0[j * stride4 + ip] = uu;
-      if (L.cga) {  // compensated running sums {sum, compensation} of u, p, T
-        const float4 up = cg[2 * j * S];
-        float2 tt = *(const float2*)&cg[(2 * j + 1) * S];
-        float su = up.x, cu = up.y, sp = up.z, cp = up.w, st2 = tt.x, ct = tt.y;
-        float y = uu - cu, s2 = su + y;
-        cu = (s2 - su) - y;
-        su = s2;
-        y = uu * pend_p - cp;
-        s2 = sp + y;
-        cp = (s2 - sp) - y;
-        sp = s2;
-        y = uu * pend_t - ct;
-        s2 = st2 + y;
-        ct = (s2 - st2) - y;
-        st2 = s2;
-        cg[2 * j * S] = make_float4(su, cu, sp, cp);
-        *(float2*)&cg[(2 * j + 1) * S] = make_float2(st2, ct);
-        const long long sk = (s + kWalk4 * j) * L.cap + base + ip;
-        L.f.cgu[sk] = su;
-        L.f.cgp[sk] = sp / su;
-        L.f.cgt[sk] = st2 / su;
-      }
-    }
-  };
+  // lanes 1-3 write p, T and the offset in the level interval of a point
+  float* const dst = (s == 1 ? L.f.p : s == 2 ? L.f.t : L.f.aux) + base;
+  float raw_before = 0.f, raw_pend = 0.f;
   while (__any_sync(0xffffffffu, alive)) {
     const float rf = d2f_bits(z + kRE), rinv = 1.f / rf;
     float xh[3];
@@ -960,55 +914,14 @@ __global__ void __launch_bounds__(kTraceThreads)
     if (alive) {
       dl = lev_find(a, z, lv);
       lev_pt(lv, dl, &p, &t);
-      if (n > 0) finalize(n - 1);
+      if (n > 0 && s == 0)
+        L.f.ds[base + n - 1] = n == 1 ? 0.5f * raw_pend : 0.5f * (raw_before + raw_pend);
       const long long q = base + n;
       raw_before = raw_pend;
       raw_pend = step;
-      pend_p = p;
-      pend_t = t;
       if (s == 0) L.z[q] = z;
-      if (s == 1) L.f.p[q] = p;
-      if (s == 2) L.f.t[q] = t;
-      if (s == 3) {
-        float aux = 0.f;
-        if (cloud) {
-          const float v = (float)((z - a.clz) / a.cldz);
-          aux = expf(-0.5f * v * v);
-        }
-        L.f.aux[q] = aux;
-      }
-      if (lv.i != qc_level) {  // a new level: its values and slopes
-        qc_level = lv.i;
-        constexpr int kB = 3;  // loads in flight
-        for (int j0 = 0; j0 < nge + nwe; j0 += kB) {
-          double d0[kB], d1[kB];
-#pragma unroll
-          for (int m = 0; m < kB; m++) {
-            const int j = min(j0 + m, nge + nwe - 1);
-            const double* src = (j < nge ? a.q + (s + kWalk4 * j) * a.stride
-                                         : a.k + (s + kWalk4 * (j - nge)) * a.stride) + lv.i;
-            d0[m] = src[0];
-            d1[m] = src[1];
-          }
-#pragma unroll
-          for (int m = 0; m < kB; m++) {
-            const int j = min(j0 + m, nge + nwe - 1);
-            const float v0 = d2f_bits(d0[m]), v1 = d2f_bits(d1[m]);
-            *(float2*)(j < nge ? &qv[j * S] : &kv[(j - nge) * S]) =
-                make_float2(v0, (v1 - v0) / lv.dz);
-          }
-        }
-      }
-      for (int j = 0; j < nge; j++) {
-        const float2 vs = *(const float2*)&qv[j * S];
-        const float v = qk_at(vs.x, vs.y, dl);
-        qv[j * S].z = v;
-        if (j == jh2o) L.f.qh2o[q] = v;
-      }
-      for (int j = 0; j < nwe; j++) {
-        const float2 vs = *(const float2*)&kv[j * S];
-        L.f.kw[(s + kWalk4 * j) * L.cap + q] = qk_at(vs.x, vs.y, dl);
-      }
+      else dst[n] = s == 1 ? p : s == 2 ? t : dl;
+      if (s == 3) L.f.qh2o[q] = __int_as_float(lv.i);
       if (ROLE == 1) {
         if (s < 3) {
           R.xs[s * R.bpts + q] = x;
@@ -1038,7 +951,8 @@ __global__ void __launch_bounds__(kTraceThreads)
       n++;
       if (stop) {
         sft = stop == 2 ? (c.nsf > 0 && a.sft > 0 ? a.sft : (double)t) : -999;
-        finalize(n - 1);
+        if (s == 0)
+          L.f.ds[base + n - 1] = n == 1 ? 0.5f * raw_pend : 0.5f * (raw_before + raw_pend);
         if (s < 3) gk.x_last[s] = x;
         alive = false;
       }
@@ -1121,6 +1035,97 @@ __global__ void __launch_bounds__(kTraceThreads)
   if (r >= 0 && s == 0) ray_finish_m(b, L, r, n, sft, gk);
 }
 
+// k_points_m: a block per ray, a thread per point, over the points that
+// k_walk_m left (the level interval in qh2o, the offset in it in aux).  The
+// Curtis-Godson sums run along the ray: a thread per emitter walks the block's
+// points in shared memory, kSumGas emitters at a time.
+constexpr int kPointThreads = 128, kSumGas = 8;
+
+template <bool CGA>
+__global__ void __launch_bounds__(kPointThreads) k_points_m(CtlDev c, BatchDev b, LosDev L, int r0) {
+  __shared__ float su[CGA ? kSumGas : 1][kPointThreads], sp[CGA ? kSumGas : 1][kPointThreads],
+      st[CGA ? kSumGas : 1][kPointThreads], pt[2][CGA ? kPointThreads : 1];
+  const int r = r0 + (int)blockIdx.x, tid = threadIdx.x;
+  const int n = L.count[r];
+  if (n <= 0) return;
+  const long long base = L.off[r];
+  const AtmM a = atm_m(b, c, b.ray_obs[r]);
+  const bool cloud = c.ncl > 0 && a.cldz > 0;
+  float u_c, p_c, t_c, u_s, p_s, t_s;
+  const int groups = CGA ? (c.ng + kSumGas - 1) / kSumGas : 1;
+  // the groups after the first find the level interval already overwritten, so
+  // the last group writes the point's own values
+  for (int gr = 0; gr < max(groups, 1); gr++) {
+    const int g0 = gr * kSumGas, g1 = CGA ? min(g0 + kSumGas, c.ng) : c.ng;
+    const bool last = gr >= groups - 1;
+    u_c = p_c = t_c = u_s = p_s = t_s = 0.f;
+    for (int ip0 = 0; ip0 < n; ip0 += kPointThreads) {
+      const int ip = ip0 + tid;
+      const long long q = base + ip;
+      if (ip < n) {
+        const int i = __float_as_int(L.f.qh2o[q]);
+        const float dl = L.f.aux[q], p = L.f.p[q], t = L.f.t[q], ds = L.f.ds[q];
+        const float dz = d2f_bits(a.z[i + 1] - a.z[i]);
+        auto at = [&](const double* src) {
+          const float v0 = d2f_bits(src[i]), v1 = d2f_bits(src[i + 1]);
+          return qk_at(v0, (v1 - v0) / dz, dl);
+        };
+        if (CGA) {
+          pt[0][tid] = p;
+          pt[1][tid] = t;
+        }
+        for (int g = g0; g < g1; g++) {
+          const float u = col_density(at(a.q + g * a.stride), p, t, ds);
+          L.f.u[g * L.cap + q] = u;
+          if (CGA) su[g - g0][tid] = u;
+        }
+        if (last) {
+          for (int iw = 0; iw < c.nw; iw++) L.f.kw[iw * L.cap + q] = at(a.k + iw * a.stride);
+          if (c.ig_h2o >= 0) L.f.qh2o[q] = at(a.q + c.ig_h2o * a.stride);
+          float aux = 0.f;
+          if (cloud) {
+            const float v = (float)((L.z[q] - a.clz) / a.cldz);
+            aux = expf(-0.5f * v * v);
+          }
+          L.f.aux[q] = aux;
+        }
+      }
+      if (CGA) {
+        __syncthreads();
+        if (tid < g1 - g0) {  // compensated running sums
+          const int m = min(n - ip0, kPointThreads);
+          for (int k = 0; k < m; k++) {
+            const float uu = su[tid][k];
+            float y = uu - u_c, s2 = u_s + y;
+            u_c = (s2 - u_s) - y;
+            u_s = s2;
+            y = uu * pt[0][k] - p_c;
+            s2 = p_s + y;
+            p_c = (s2 - p_s) - y;
+            p_s = s2;
+            y = uu * pt[1][k] - t_c;
+            s2 = t_s + y;
+            t_c = (s2 - t_s) - y;
+            t_s = s2;
+            su[tid][k] = u_s;
+            sp[tid][k] = p_s;
+            st[tid][k] = t_s;
+          }
+        }
+        __syncthreads();
+        if (ip < n)
+          for (int g = g0; g < g1; g++) {
+            const float uu = su[g - g0][tid];
+            L.f.cgu[g * L.cap + q] = uu;
+            L.f.cgp[g * L.cap + q] = sp[g - g0][tid] / uu;
+            L.f.cgt[g * L.cap + q] = st[g - g0][tid] / uu;
+          }
+        __syncthreads();
+      }
+    }
+  }
+}
+
 }  // namespace
 
 void launch_trace_count_mixed(const CtlDev& c, const BatchDev& b, const LosDev& L, unsigned* err,
@@ -1135,12 +1140,22 @@ void launch_los_bound_mixed(const CtlDev& c, const BatchDev& b, double scale, in
   k_los_bound_m<<<(b.nray + bs - 1) / bs, bs, 0, s>>>(c, b, scale, cap);
 }
 
+namespace {
+template <int ROLE>
+void launch_walk(const CtlDev& c, const BatchDev& b, const LosDev& L, const int* order, int r0, int nr,
+                 const TraceResume& R, unsigned* err, cudaStream_t s) {
+  if (nr <= 0) return;
+  const int rays = kTraceThreads / kWalk4;
+  k_walk_m<ROLE><<<(nr + rays - 1) / rays, kTraceThreads, 0, s>>>(c, b, L, order, r0, nr, R, err);
+  if (L.cga) k_points_m<true><<<nr, kPointThreads, 0, s>>>(c, b, L, r0);
+  else k_points_m<false><<<nr, kPointThreads, 0, s>>>(c, b, L, r0);
+}
+}  // namespace
+
+// order: a permutation of the batch's rays
 void launch_trace_fill_mixed(const CtlDev& c, const BatchDev& b, const LosDev& L, const int* order,
                              unsigned* err, cudaStream_t s) {
-  const int rays = kTraceThreads / kWalk4;
-  const size_t smem = sizeof(float4) * trace4_smem_slots(c) * kTraceThreads;
-  k_trace_fill_m4<0><<<(b.nray + rays - 1) / rays, kTraceThreads, smem, s>>>(
-      c, b, L, order, 0, b.nray, TraceResume{}, err);
+  launch_walk<0>(c, b, L, order, 0, b.nray, TraceResume{}, err, s);
 }
 
 int trace_fill_resident(int sms) {
@@ -1160,12 +1175,10 @@ int trace_fill_resident(int sms) {
 void launch_trace_fill_resumed(const CtlDev& c, const BatchDev& b, const LosDev& L,
                                const int* order, int r0, int nr, const TraceResume& R, int role,
                                unsigned* err, cudaStream_t s) {
-  const int bs = kTraceThreads, rays = bs / kWalk4;
+  const int bs = kTraceThreads;
   if (nr <= 0) return;
   if (role == 1)
-    k_trace_fill_m4<1><<<(nr + rays - 1) / rays, bs,
-                         sizeof(float4) * trace4_smem_slots(c) * kTraceThreads, s>>>(
-        c, b, L, order, r0, nr, R, err);
+    launch_walk<1>(c, b, L, order, r0, nr, R, err, s);
   else
     k_trace_fill_m<<<(nr + bs - 1) / bs, bs, sizeof(float) * trace_smem_floats(c) * kTraceThreads,
                      s>>>(c, b, L, order, r0, nr, R, err);

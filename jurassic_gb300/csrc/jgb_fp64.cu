@@ -17,7 +17,8 @@
 //                 workspace (the allocation-free entry point; the others
 //                 take jgb_path64.cu).
 //   k_srcfunc     init_srcfunc (jurassic.c:3631-3681) on the device.
-//   k_hydrostatic hydrostatic (jurassic.c:3520-3582), one thread per profile.
+//   k_hydro_means, k_hydro_chain  hydrostatic (jurassic.c:3520-3582), a lane per
+//                 layer, then a thread per profile.
 #include "../../include/jurassic_gb300.h"
 #include "jgb_common.cuh"
 #include "jgb_internal.h"
@@ -957,43 +958,58 @@ __global__ void k_srcfunc(int nd, int id0, int nch, const int* fn_off, const dou
   sr[(long long)it * nd + id] = acc / fsum;
 }
 
-// hydrostatic (jurassic.c:3520-3582): one thread per profile
-__global__ void k_hydrostatic(CtlDev c, BatchDev b, double* p_out) {
-  const int o = blockIdx.x * blockDim.x + threadIdx.x;
+// hydrostatic (jurassic.c:3520-3582) in two kernels.  The mean of g M / (R T)
+// over a layer depends on nothing but the layer: a warp per profile, a lane per
+// layer, leaves mean * 1000 * dz in the place of the pressure that it leads to.
+// The pressures follow each other along the profile, a thread per profile.
+// Every value is formed as in a loop over the profile, one thread of which took
+// 2.04 ms for 1500 profiles of 77 levels: 20 means of 17 FP64 instructions per
+// layer, one after the other; 0.42 ms here.
+__device__ int hydro_ref(const double* z, int np, double hydz) {
+  double best = 1e99;
+  int iref = 0;
+  for (int ip = 0; ip < np; ip++)
+    if (fabs(z[ip] - hydz) < best) {
+      best = fabs(z[ip] - hydz);
+      iref = ip;
+    }
+  return iref;
+}
+
+__global__ void k_hydro_means(CtlDev c, BatchDev b, double* p_out) {
+  const int lane = threadIdx.x & 31;
+  const int o = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   if (o >= b.nobs || c.hydz < 0) return;
   if (b.obs_skip && b.obs_skip[o]) return;
   const int l0 = b.lev_off[o], np = b.lev_off[o + 1] - l0;
   const double* z = b.z + l0;
   const double* t = b.t + l0;
   const double* qw = c.ig_h2o >= 0 ? b.q + (long long)c.ig_h2o * b.nlev + l0 : nullptr;
-  double* p = p_out + l0;
   const double mmair = 28.96456e-3, mmh2o = 18.0153e-3;
   const int npts = 20;
-  double best = 1e99, e = 0;
-  int iref = 0;
-  for (int ip = 0; ip < np; ip++)
-    if (fabs(z[ip] - c.hydz) < best) {
-      best = fabs(z[ip] - c.hydz);
-      iref = ip;
-    }
-  for (int ip = iref + 1; ip < np; ip++) {
-    double mean = 0;
+  const int iref = hydro_ref(z, np, c.hydz);
+  for (int ip = lane; ip < np; ip += 32) {
+    if (ip == iref) continue;
+    const int i0 = ip > iref ? ip - 1 : ip + 1;
+    double mean = 0, e = 0;
     for (int i = 0; i < npts; i++) {
-      if (qw) e = lin(0.0, qw[ip - 1], npts - 1.0, qw[ip], (double)i);
+      if (qw) e = lin(0.0, qw[i0], npts - 1.0, qw[ip], (double)i);
       mean += (e * mmh2o + (1 - e) * mmair) * kG0 / kRI /
-              lin(0.0, t[ip - 1], npts - 1.0, t[ip], (double)i) / npts;
+              lin(0.0, t[i0], npts - 1.0, t[ip], (double)i) / npts;
     }
-    p[ip] = exp(log(p[ip - 1]) - mean * 1000 * (z[ip] - z[ip - 1]));
+    p_out[l0 + ip] = mean * 1000 * (z[ip] - z[i0]);
   }
-  for (int ip = iref - 1; ip >= 0; ip--) {
-    double mean = 0;
-    for (int i = 0; i < npts; i++) {
-      if (qw) e = lin(0.0, qw[ip + 1], npts - 1.0, qw[ip], (double)i);
-      mean += (e * mmh2o + (1 - e) * mmair) * kG0 / kRI /
-              lin(0.0, t[ip + 1], npts - 1.0, t[ip], (double)i) / npts;
-    }
-    p[ip] = exp(log(p[ip + 1]) - mean * 1000 * (z[ip] - z[ip + 1]));
-  }
+}
+
+__global__ void k_hydro_chain(CtlDev c, BatchDev b, double* p_out) {
+  const int o = blockIdx.x * blockDim.x + threadIdx.x;
+  if (o >= b.nobs || c.hydz < 0) return;
+  if (b.obs_skip && b.obs_skip[o]) return;
+  const int l0 = b.lev_off[o], np = b.lev_off[o + 1] - l0;
+  double* p = p_out + l0;
+  const int iref = hydro_ref(b.z + l0, np, c.hydz);
+  for (int ip = iref + 1; ip < np; ip++) p[ip] = exp(log(p[ip - 1]) - p[ip]);
+  for (int ip = iref - 1; ip >= 0; ip--) p[ip] = exp(log(p[ip + 1]) - p[ip]);
 }
 
 // ---------------------------------------------------------------------------
@@ -1101,8 +1117,8 @@ void launch_fov(const CtlDev& c, const BatchDev& b, const double* prad, const do
 }
 
 void launch_hydrostatic(const CtlDev& c, const BatchDev& b, double* p_out, cudaStream_t s) {
-  const int bs = 64;
-  k_hydrostatic<<<(b.nobs + bs - 1) / bs, bs, 0, s>>>(c, b, p_out);
+  k_hydro_means<<<(b.nobs + 3) / 4, 128, 0, s>>>(c, b, p_out);
+  k_hydro_chain<<<(b.nobs + 31) / 32, 32, 0, s>>>(c, b, p_out);
 }
 
 // Loads the FP64 forward-model kernels onto the current device (CUDA loads
@@ -1110,7 +1126,7 @@ void launch_hydrostatic(const CtlDev& c, const BatchDev& b, double* p_out, cudaS
 // later first launch allocates no device memory for their code.
 int preload_fp64_kernels() {
   cudaFuncAttributes a;
-  const void* fns[] = {(const void*)k_trace_count, (const void*)k_trace_fill, (const void*)k_path_fp64, (const void*)k_hydrostatic};
+  const void* fns[] = {(const void*)k_trace_count, (const void*)k_trace_fill, (const void*)k_path_fp64, (const void*)k_hydro_means, (const void*)k_hydro_chain};
   for (const void* f : fns)
     if (cudaFuncGetAttributes(&a, f) != cudaSuccess) return JGB_ERR_CUDA;
   return JGB_OK;

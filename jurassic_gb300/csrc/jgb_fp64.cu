@@ -4,7 +4,7 @@
 // expression is rounded like the reference's (no fused multiply-add), which
 // keeps the FP64 path within rounding of the reference results.
 //
-//   k_trace_fill, k_trace_fill8
+//   k_trace_fill; k_walk8, k_points64
 //                 raytrace (jurassic.c:4201-4438) + tangent_point
 //                 (jurassic.c:5223-5263), one or eight lanes per ray, in one
 //                 pass into per-ray capacities; k_trace_count counts the
@@ -505,26 +505,33 @@ __global__ void __launch_bounds__(kTrace64Threads)
 // A batch of few rays leaves the FP64 pipes idle while each ray waits for its
 // own chain (an instruction takes 64 cycles whether 1 or 32 lanes are active,
 // and three warps share an SM without slowing each other), so eight lanes walk
-// one ray: lanes 0-2 the refraction sub-points and the components of the
-// vectors, lane 3 the midpoint, the others the LOS point, whose five altitude
-// and atmosphere evaluations then run as one; the emitters are dealt over the
-// lanes.  Every value is formed as in walk(), so both give the same LOS.
-// Measured (trace stage, from the walk with one lane per ray in two passes,
-// slopes, compares and lon/lat at every point: 1247 FP64 instructions per
-// step): 10 limb rays 67.8 -> 9.7 ms, 273 limb rays 21.2 -> 2.9 ms, 1000 nadir
-// rays 49.1 -> 6.6 ms.
+// one ray (k_walk8): lanes 0-2 the components of the vectors and the refraction
+// sub-points, lane 3 the midpoint, the others the LOS point, whose five altitude
+// and atmosphere evaluations then run as one.  The lanes exchange squares and
+// products, formed once per component.  What no step needs (mixing ratios,
+// column densities, extinctions, Curtis-Godson sums) follows in k_points64.
+// Every value is formed as in walk(), in the same order, so both give the same
+// LOS.  Measured (trace stage, from the walk with one lane per ray in two
+// passes, slopes, compares and lon/lat at every point: 1247 FP64 instructions
+// per step; with the emitters dealt over the lanes and vectors in every lane:
+// 130; here about 100):
+// 10 limb rays 67.8, 9.7 and 7.3 ms; 273 limb rays 21.2, 2.9 and 2.2; 1000 nadir
+// rays 49.1, 6.6 and 5.1.
 // All lanes stay in the loop until the warp's four rays are done.
-constexpr int kWalk8Rays = 4;                   // rays of a warp
-constexpr int kWalk8Gases = (kMaxG + 7) / 8;    // emitters of a lane
-constexpr int kWalk8Windows = (kMaxW + 7) / 8;  // windows of a lane
+constexpr int kWalk8Rays = 4;  // rays of a warp
 
 __device__ __forceinline__ double from_lane(double v, int k) {
   return __shfl_sync(0xffffffffu, v, k, 8);
 }
+// the sum over the components of a value that lanes 0-2 hold, as x + y + z
+__device__ __forceinline__ double sum3(double v) {
+  const double x = from_lane(v, 0), y = from_lane(v, 1), z = from_lane(v, 2);
+  return x + y + z;
+}
 
 __global__ void __launch_bounds__(32)
-    k_trace_fill8(CtlDev c, BatchDev b, LosDev L, const int* order, const double* slopes,
-                  unsigned* err) {
+    k_walk8(CtlDev c, BatchDev b, LosDev L, const int* order, const double* slopes,
+            unsigned* err) {
   __shared__ Keep64 keep[kWalk8Rays];
   const int s = threadIdx.x & 7, th = (int)blockIdx.x * kWalk8Rays + (threadIdx.x >> 3);
   Keep64& kp = keep[threadIdx.x >> 3];
@@ -533,52 +540,33 @@ __global__ void __launch_bounds__(32)
   const AtmView a = atm_view(c, b, slopes, r >= 0 ? b.ray_obs[r] : 0);
   const long long base = r >= 0 ? L.off[r] : 0;
   const int cap = r >= 0 ? L.count[r] : 0;
-  double x[3] = {kRE, 0, 0}, ex0[3] = {1, 0, 0}, zmin = 0, zmax = 0;
-  int st = r >= 0 ? ray_start(c, a, b.geo, b.nray, r, x, ex0, &zmin, &zmax, err) : 0;
-  bool alive = st > 0;
-  const double h = 0.02, zrefrac = 60;
   const int k = s < 3 ? s : 0;  // component of this lane
+  double x = k == 0 ? kRE : 0, e = k == 0 ? 1 : 0, zmin = 0, zmax = 0;
+  int st = 0;
+  if (r >= 0) {
+    double x0[3] = {kRE, 0, 0}, e0[3] = {1, 0, 0};
+    st = ray_start(c, a, b.geo, b.nray, r, x0, e0, &zmin, &zmax, err);
+    for (int i = 0; i < 3; i++)
+      if (i == k) {
+        x = x0[i];
+        e = e0[i];
+      }
+  }
+  bool alive = st > 0;
+  const double h = 0.02, rh = 1 / h, zrefrac = 60;
   const bool sub = s < 3, main_pt = s >= 4;
-  double last_z = 0, last_x[3] = {0, 0, 0}, sft = -999;
-  double raw_before = 0, raw_pend = 0, pend_p = 0, pend_t = 0, pend_r = 0;
-  double pq[kWalk8Gases] = {}, cg[kWalk8Gases][3] = {};
+  double last_z = 0, last_x = 0, sft = -999, zmin_seen = 0;
+  double raw_before = 0, raw_pend = 0;
   int n = 0, stop = 0;
+  bool want_p1 = false;
   Lev64 lv;
   lv.i = -1;
-  if (s == 0) kp.want_p1 = false;
-  auto finalize = [&](int ip) {
-    const long long q = base + ip;
-    const double dsT = ip == 0 ? raw_pend * 0.5 : 0.5 * (raw_before + raw_pend);
-    if (s == 0) L.ds[q] = dsT;
-    const double kt = kKB * pend_t;
-#pragma unroll
-    for (int j = 0; j < kWalk8Gases; j++) {
-      const int ig = s + 8 * j;
-      if (ig >= a.ng) break;
-      const double u = div_by(10 * pq[j] * pend_p, kt, pend_r) * dsT;
-      L.u[ig * L.cap + q] = u;
-      if (L.cga) {
-        const double su = ip ? cg[j][0] + u : u;
-        const double sp = ip ? cg[j][1] + u * pend_p : u * pend_p;
-        const double st2 = ip ? cg[j][2] + u * pend_t : u * pend_t;
-        cg[j][0] = su;
-        cg[j][1] = sp;
-        cg[j][2] = st2;
-        const double ru = 1 / su;
-        L.cgu[ig * L.cap + q] = su;
-        L.cgp[ig * L.cap + q] = div_by(sp, su, ru);
-        L.cgt[ig * L.cap + q] = div_by(st2, su, ru);
-      }
-    }
-  };
+  __syncwarp();
   while (__any_sync(0xffffffffu, alive)) {
     double ds = c.rayds;
-    const double norm = sqrt(norm2(x));
+    const double norm = sqrt(sum3(x * x));
     if (c.raydz > 0) {
-      const double xc = x[k] / norm;
-      double xh[3];
-      for (int i = 0; i < 3; i++) xh[i] = from_lane(xc, i);
-      const double cosa = fabs(ex0[0] * xh[0] + ex0[1] * xh[1] + ex0[2] * xh[2]);
+      const double cosa = fabs(sum3(e * (x / norm)));
       if (__double_as_longlong(cosa) != 0) {
         const double v = c.raydz / cosa;
         ds = lt(c.rayds, v) ? c.rayds : v;
@@ -588,115 +576,178 @@ __global__ void __launch_bounds__(32)
     // a position that is not a number is inside: the walk ends with an overflow
     const bool num = is_number(z);
     const bool low = num && lt(z, zmin), high = num && lt(zmax, z);
-    if (alive && (low || high) && n > 0) {
-      stop = low ? 2 : 1;
-      const double frac = ((low ? zmin : zmax) - last_z) / (z - last_z);
-      double lz, llon, llat, xl[3];
-      to_geo(last_x, &lz, &llon, &llat);
-      to_cart(lz, llon, llat, xl);
-      for (int i = 0; i < 3; i++) x[i] = xl[i] + frac * (x[i] - xl[i]);
-      z = sqrt(norm2(x)) - kRE;
-      raw_pend = ds * frac;
-      if (s == 0) kp.ds_clip = raw_pend;
-      ds = 0;
+    const bool clip = alive && (low || high) && n > 0;
+    if (__any_sync(0xffffffffu, clip)) {
+      double xs[3], xl[3];
+      for (int i = 0; i < 3; i++) {
+        xs[i] = from_lane(x, i);
+        xl[i] = from_lane(last_x, i);
+      }
+      if (clip) {
+        stop = low ? 2 : 1;
+        const double frac = ((low ? zmin : zmax) - last_z) / (z - last_z);
+        double lz, llon, llat, xc[3];
+        to_geo(xl, &lz, &llon, &llat);
+        to_cart(lz, llon, llat, xc);
+        for (int i = 0; i < 3; i++) {
+          xs[i] = xc[i] + frac * (xs[i] - xc[i]);
+          if (i == k) x = xs[i];
+        }
+        z = sqrt(norm2(xs)) - kRE;
+        raw_pend = ds * frac;
+        if (s == 0) kp.ds_clip = raw_pend;
+        ds = 0;
+      }
     }
     if (alive && n >= cap) {
       if (s == 0) atomicOr(err, cap < c.nlos_max ? kErrSlabOverflow : kErrLosOverflow);
       alive = false;
       n = -1;
     }
-    // this lane's evaluation point: midpoint, sub-point (the reference adds h
+    // this lane's evaluation point: midpoint m, sub-point (the reference adds h
     // to a component and takes it off again before the next) or LOS point
-    const double hds = 0.5 * ds, hl = main_pt ? 0.0 : hds;
-    double y[3];
-    for (int i = 0; i < 3; i++) {
-      const double m = x[i] + hl * ex0[i];
-      y[i] = (m + (sub && i <= s ? h : 0.0)) - (sub && i < s ? h : 0.0);
+    const double hds = 0.5 * ds;
+    double zl;
+    {
+      const double m = x + hds * e, mh = m + h, mr = mh - h;
+      const double qm = m * m, qh = mh * mh, qr = mr * mr;
+      const double m0 = from_lane(qm, 0), m1 = from_lane(qm, 1), m2 = from_lane(qm, 2);
+      const double h0 = from_lane(qh, 0), h1 = from_lane(qh, 1), h2 = from_lane(qh, 2);
+      const double r0 = from_lane(qr, 0), r1 = from_lane(qr, 1);
+      const double y0 = !sub ? m0 : s == 0 ? h0 : r0;
+      const double y1 = !sub || s < 1 ? m1 : s == 1 ? h1 : r1;
+      const double y2 = !sub || s < 2 ? m2 : h2;
+      zl = main_pt ? z : sqrt(y0 + y1 + y2) - kRE;
     }
-    const double zl = main_pt ? z : sqrt(norm2(y)) - kRE;
     double pl, tl;
     if (alive) lev64_find(a, zl, lv);
     else if (lv.i < 0) lev64_load(a, 0, lv);
     lev64_pt(a, lv, zl, &pl, &tl);
     const double nl = kRefrac * pl / tl;
-    const double p = from_lane(pl, 4), t = from_lane(tl, 4), nmain = from_lane(nl, 4),
-                 nmid = from_lane(nl, 3);
-    const int i0 = __shfl_sync(0xffffffffu, lv.i, 4, 8);
-    const double dz = from_lane(zl - lv.z0, 4);
+    const double nmain = from_lane(nl, 4), nmid = from_lane(nl, 3), t = from_lane(tl, 4);
     if (alive) {
-      if (n > 0) finalize(n - 1);
       const long long q = base + n;
+      if (n > 0 && s == 0)
+        L.ds[q - 1] = n == 1 ? raw_pend * 0.5 : 0.5 * (raw_before + raw_pend);
       raw_before = raw_pend;
       raw_pend = ds;
-      pend_p = p;
-      pend_t = t;
-      pend_r = 1 / (kKB * t);
-      if (s == 4) L.p[q] = p;
-      if (s == 5) L.t[q] = t;
-      if (s == 6)
-        L.aux[q] = (c.ncl > 0 && a.cldz > 0) ? exp(-0.5 * ((z - a.clz) / a.cldz) * ((z - a.clz) / a.cldz)) : 0.0;
-#pragma unroll
-      for (int j = 0; j < kWalk8Gases; j++) {
-        const int ig = s + 8 * j;
-        if (ig >= a.ng) break;
-        pq[j] = a.q[ig * a.stride + i0] + a.sq[ig * a.stride + i0] * dz;
-        if (ig == c.ig_h2o) L.qh2o[q] = pq[j];
-      }
-#pragma unroll
-      for (int j = 0; j < kWalk8Windows; j++) {
-        const int iw = s + 8 * j;
-        if (iw >= a.nw) break;
-        L.kw[iw * L.cap + q] = a.k[iw * a.stride + i0] + a.sk[iw * a.stride + i0] * dz;
+      // for k_points64: the altitude and its level interval in aux and qh2o
+      if (s == 4) L.p[q] = pl;
+      if (s == 5) L.t[q] = tl;
+      if (s == 6) L.aux[q] = zl;
+      if (s == 7) L.qh2o[q] = __longlong_as_double(lv.i);
+      const bool newmin = n == 0 || lt(z, zmin_seen);
+      if (s < 3) {
+        if (n == 0) kp.x0[s] = x;
+        if (want_p1) kp.xp[s] = x;
+        if (newmin) kp.xm[s] = last_x;
       }
       if (s == 0) {
-        if (n == 0) {
-          kp.z0 = z;
-          for (int i = 0; i < 3; i++) kp.x0[i] = x[i];
-        }
-        if (kp.want_p1) {
-          kp.want_p1 = false;
+        if (n == 0) kp.z0 = z;
+        if (want_p1) {
           kp.zp1 = z;
           kp.ds_p1 = ds;
-          for (int i = 0; i < 3; i++) kp.xp[i] = x[i];
         }
-        if (n == 0 || lt(z, kp.zmin)) {
+        if (newmin) {
           kp.zmin = z;
           kp.imin = n;
           kp.ds_m = ds;
           kp.zm1 = last_z;
-          for (int i = 0; i < 3; i++) kp.xm[i] = last_x[i];
-          kp.want_p1 = true;
         }
       }
+      if (newmin) zmin_seen = z;
+      want_p1 = newmin;
       last_z = z;
-      for (int i = 0; i < 3; i++) last_x[i] = x[i];
+      last_x = x;
       n++;
       if (stop) {
         sft = stop == 2 ? (c.nsf > 0 && a.sft > 0 ? a.sft : t) : -999;
-        finalize(n - 1);
         if (s == 0) {
+          L.ds[q] = n == 1 ? raw_pend * 0.5 : 0.5 * (raw_before + raw_pend);
           kp.zl = z;
-          for (int i = 0; i < 3; i++) kp.xl[i] = x[i];
         }
+        if (s < 3) kp.xl[s] = x;
         alive = false;
       }
     }
     const bool bend = c.refrac && !lt(zrefrac, z);
-    const double ec = bend ? ex0[k] * (1 + nmain) + ds * ((nl - nmid) / h) : ex0[k];
-    double ex1[3];
-    for (int i = 0; i < 3; i++) ex1[i] = from_lane(ec, i);
-    const double en = ec / sqrt(norm2(ex1));
-    const double xn = x[k] + hds * (ex0[k] + en);
-    for (int i = 0; i < 3; i++) {
-      const double e = from_lane(en, i), xi = from_lane(xn, i);
-      if (alive) {
-        ex0[i] = e;
-        x[i] = xi;
-      }
+    const double ec = bend ? e * (1 + nmain) + ds * div_by(nl - nmid, h, rh) : e;
+    const double en = ec / sqrt(sum3(ec * ec));
+    if (alive) {
+      x += hds * (e + en);
+      e = en;
     }
   }
   __syncwarp();
   if (r >= 0 && s == 0) ray_finish(b, L, r, st < 0 ? -1 : n, sft, kp);
+}
+
+// A block per ray, a thread per point: what k_walk8 left out.  The sums of a
+// ray's column densities run along it, a thread per emitter over the block's
+// points in shared memory, kSumGas emitters at a time.
+constexpr int kPointThreads = 128, kSumGas = 8;
+
+template <bool CGA>
+__global__ void __launch_bounds__(kPointThreads)
+    k_points64(CtlDev c, BatchDev b, LosDev L, const double* slopes) {
+  __shared__ double su[CGA ? kSumGas : 1][kPointThreads], sp[CGA ? kSumGas : 1][kPointThreads],
+      st[CGA ? kSumGas : 1][kPointThreads];
+  const int r = blockIdx.x, tid = threadIdx.x;
+  const int n = L.count[r];
+  if (n <= 0) return;
+  const long long base = L.off[r];
+  const AtmView a = atm_view(c, b, slopes, b.ray_obs[r]);
+  const bool cloud = c.ncl > 0 && a.cldz > 0;
+  const int groups = CGA ? max((c.ng + kSumGas - 1) / kSumGas, 1) : 1;
+  for (int gr = 0; gr < groups; gr++) {
+    const int g0 = gr * kSumGas, g1 = CGA ? min(g0 + kSumGas, c.ng) : c.ng;
+    double u_s = 0, p_s = 0, t_s = 0;
+    for (int ip0 = 0; ip0 < n; ip0 += kPointThreads) {
+      const int ip = ip0 + tid;
+      const long long q = base + ip;
+      if (ip < n) {
+        const int i = (int)__double_as_longlong(L.qh2o[q]);
+        const double z = L.aux[q], dz = z - a.z[i], p = L.p[q], t = L.t[q], ds = L.ds[q];
+        const double kt = kKB * t, rt = 1 / kt;
+        for (int g = g0; g < g1; g++) {
+          const double v = a.q[g * a.stride + i] + a.sq[g * a.stride + i] * dz;
+          const double u = div_by(10 * v * p, kt, rt) * ds;
+          L.u[g * L.cap + q] = u;
+          if (CGA) {
+            su[g - g0][tid] = u;
+            sp[g - g0][tid] = u * p;
+            st[g - g0][tid] = u * t;
+          }
+        }
+        if (gr == groups - 1) {  // the point's altitude and interval end here
+          for (int iw = 0; iw < a.nw; iw++)
+            L.kw[iw * L.cap + q] = a.k[iw * a.stride + i] + a.sk[iw * a.stride + i] * dz;
+          if (c.ig_h2o >= 0)
+            L.qh2o[q] = a.q[c.ig_h2o * a.stride + i] + a.sq[c.ig_h2o * a.stride + i] * dz;
+          L.aux[q] = cloud ? exp(-0.5 * ((z - a.clz) / a.cldz) * ((z - a.clz) / a.cldz)) : 0.0;
+        }
+      }
+      if (CGA) {
+        __syncthreads();
+        if (tid < g1 - g0)
+          for (int j = 0; j < min(n - ip0, kPointThreads); j++) {
+            const bool first = ip0 + j == 0;
+            su[tid][j] = u_s = first ? su[tid][j] : u_s + su[tid][j];
+            sp[tid][j] = p_s = first ? sp[tid][j] : p_s + sp[tid][j];
+            st[tid][j] = t_s = first ? st[tid][j] : t_s + st[tid][j];
+          }
+        __syncthreads();
+        if (ip < n)
+          for (int g = g0; g < g1; g++) {
+            const double uu = su[g - g0][tid], ru = 1 / uu;
+            L.cgu[g * L.cap + q] = uu;
+            L.cgp[g * L.cap + q] = div_by(sp[g - g0][tid], uu, ru);
+            L.cgt[g * L.cap + q] = div_by(st[g - g0][tid], uu, ru);
+          }
+        __syncthreads();
+      }
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1015,10 +1066,10 @@ __global__ void k_hydro_chain(CtlDev c, BatchDev b, double* p_out) {
 // ---------------------------------------------------------------------------
 // launch wrappers
 
-// Eight lanes per ray up to here: a step is about 130 FP64 instructions of a
+// Eight lanes per ray up to here: a step is about 100 FP64 instructions of a
 // warp (4 rays) against 330 (32 rays), 64 cycles each until about three warps
-// share an SM, 19 of the SM's then, so the two forms meet near 6000 rays on
-// 152 SMs.
+// share an SM, 19 of the SM's then, so the two forms meet between 6000 and
+// 7000 rays on 152 SMs.
 constexpr int kWalk8MaxRays = 6144;
 
 size_t level_slope_bytes(const CtlDev& c, long long nlev) {
@@ -1039,7 +1090,9 @@ void launch_trace_count(const CtlDev& c, const BatchDev& b, const LosDev& L, con
 void launch_trace_fill(const CtlDev& c, const BatchDev& b, const LosDev& L, const int* order,
                        const double* slopes, unsigned* err, cudaStream_t s) {
   if (slopes && b.nray <= kWalk8MaxRays) {
-    k_trace_fill8<<<(b.nray + kWalk8Rays - 1) / kWalk8Rays, 32, 0, s>>>(c, b, L, order, slopes, err);
+    k_walk8<<<(b.nray + kWalk8Rays - 1) / kWalk8Rays, 32, 0, s>>>(c, b, L, order, slopes, err);
+    if (L.cga) k_points64<true><<<b.nray, kPointThreads, 0, s>>>(c, b, L, slopes);
+    else k_points64<false><<<b.nray, kPointThreads, 0, s>>>(c, b, L, slopes);
     return;
   }
   const int bs = kTrace64Threads;

@@ -137,37 +137,44 @@ __global__ void k_wait_selftest(int arrive, unsigned long long* out) {
 // each 128 columns x kChunk rows in the core-matrix order of tc_off, zero
 // outside m x (n + 1).  Block bi = ti * nch + c of a problem starts at
 // xoff + bi * kBlockFloats (16 KB apart: whole blocks go to shared memory
-// with one bulk copy).  A block is assembled in shared memory and written
-// with 16-byte stores.
+// with one bulk copy).  A thread takes a column of a block: its kChunk loads,
+// lanes along a row, are in flight together, and four rows of a column are 16
+// bytes of a plane, eight columns' 128 bytes, so the stores go straight to
+// memory.  512 problems of 150 x 405: 63 us (0.5 GB, 47 us at the
+// measured bandwidth); assembled in shared memory by 4-byte stores, with two
+// barriers per block, 97 us.
 __global__ void __launch_bounds__(128) k_split_x(const NeDesc* desc, const double* Kall,
                                                  const double* wall, const double* dyall,
                                                  float* xbuf) {
-  __shared__ __align__(16) float blk[kBlockFloats];
   const NeDesc d = desc[blockIdx.y];
   const int na = d.n + 1;
   const int nt = (na + kTile - 1) / kTile, nch = (d.m + kChunk - 1) / kChunk;
   const int tid = threadIdx.x;
   for (int bi = blockIdx.x; bi < nt * nch; bi += gridDim.x) {
     const int ti = bi / nch, c = bi - ti * nch;
-    const int col = ti * kTile + tid;
-#pragma unroll 4
-    for (int k = 0; k < kChunk; k++) {
-      const int row = c * kChunk + k;
-      float x = 0.f;
-      if (row < d.m && col < na) {
-        const double v = col < d.n ? Kall[d.koff + (long long)row * d.n + col] : dyall[d.moff + row];
-        x = d2f_bits(v * wall[d.moff + row]);
+    const int col = ti * kTile + tid, row0 = c * kChunk;
+    // column n of the augmented matrix is dy, contiguous
+    const double* src = col < d.n ? Kall + d.koff + (long long)row0 * d.n + col : dyall + d.moff + row0;
+    const int step = col < d.n ? d.n : 1;
+    const double* w = wall + d.moff + row0;
+    const int nrow = col < na ? min(d.m - row0, kChunk) : 0;
+    double v[kChunk];
+#pragma unroll
+    for (int k = 0; k < kChunk; k++) v[k] = k < nrow ? src[(long long)k * step] : 0.0;
+    float* dst = xbuf + d.xoff + (long long)bi * kBlockFloats;
+#pragma unroll
+    for (int k = 0; k < kChunk; k += 4) {
+      float hi[4], lo[4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const float x = k + j < nrow ? d2f_bits(v[k + j] * w[k + j]) : 0.f;
+        hi[j] = __uint_as_float(tf32_of(x));
+        lo[j] = __uint_as_float(tf32_of(x - hi[j]));
       }
-      const float hi = __uint_as_float(tf32_of(x));
       const int o = tc_off(tid, k) >> 2;
-      blk[o] = hi;
-      blk[kTile * kChunk + o] = __uint_as_float(tf32_of(x - hi));
+      *reinterpret_cast<float4*>(dst + o) = make_float4(hi[0], hi[1], hi[2], hi[3]);
+      *reinterpret_cast<float4*>(dst + kTile * kChunk + o) = make_float4(lo[0], lo[1], lo[2], lo[3]);
     }
-    __syncthreads();
-    float4* dst = reinterpret_cast<float4*>(xbuf + d.xoff + (long long)bi * kBlockFloats);
-    const float4* src = reinterpret_cast<const float4*>(blk);
-    for (int i = tid; i < kBlockFloats / 4; i += blockDim.x) dst[i] = src[i];
-    __syncthreads();
   }
 }
 
@@ -228,7 +235,9 @@ __device__ __forceinline__ void epi_sync() {
 //    back ("empty").
 // So the copies, the MMAs of one tile and the epilogue of the previous one
 // overlap.  The epilogue sets the pace (without its stores the kernel runs
-// in about half the time, and four stages instead of two change nothing), so
+// in about half the time, and four stages instead of two change nothing; with
+// two columns per lane in the direct entries, half a sector per store, 512
+// problems of 150 x 405 took 185 us, 152 now), so
 // the CTA keeps two stages and a 64-column staging tile, 97 KB of shared
 // memory, and two CTAs share an SM (32 epilogue warps, all 512 columns of
 // tensor memory).  Every wait is bounded; one that gives up flags the error, the
@@ -406,22 +415,16 @@ __global__ void __launch_bounds__(kNeThreads, 2) k_normal_tc(const NeDesc* desc,
             A[(long long)col * d.n + row] = f2d_bits(__uint_as_float(v[j]));
         }
         epi_sync();
-        // direct entries, rows >= columns (and b, the augmented row n): two
-        // columns per lane, lanes along the row
-        const int colp = tj * kTile + h * kEpiCols + 2 * lane;
+        // direct entries, rows >= columns (and b, the augmented row n): lanes
+        // along the row, so that a store covers whole sectors
         for (int rr = ew; rr < kTile; rr += kEpiThreads / 32) {
           const int row2 = ti * kTile + rr;
-          if (row2 > d.n || colp >= d.n) break;
-          const float2 x2 = *reinterpret_cast<const float2*>(stile + rr * kEpiPad + 2 * lane);
+          if (row2 > d.n) break;
+          double* dst = row2 == d.n ? bv : A + (long long)row2 * d.n;
 #pragma unroll
-          for (int k = 0; k < 2; k++) {
-            const int col = colp + k;
-            if (col >= d.n) break;
-            const double x = f2d_bits(k ? x2.y : x2.x);
-            if (row2 == d.n)
-              bv[col] = x;
-            else if (row2 >= col)
-              A[(long long)row2 * d.n + col] = x;
+          for (int k = 0; k < kEpiCols; k += 32) {
+            const int col = tj * kTile + h * kEpiCols + k + lane;
+            if (col < d.n && col <= row2) dst[col] = f2d_bits(stile[rr * kEpiPad + k + lane]);
           }
         }
         epi_sync();  // the staging tile is free for the next pass

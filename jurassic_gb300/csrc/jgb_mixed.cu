@@ -1177,7 +1177,7 @@ void launch_gas_v(const CtlDev& c, const TblDev& T, const BatchDev& b, const Los
     if (lanes_per_ray == 4) return P.fast ? go(k_gas_m<CGA, 4, 8, true, 1>) : go(k_gas_m<CGA, 4, 8, false, 1>);
     return P.fast ? go(k_gas_m<CGA, 1, 8, true, 1>) : go(k_gas_m<CGA, 1, 8, false, 1>);
   }
-  if (res == 2) return P.fast ? go(k_gas_m<CGA, 1, 10, true, 2>) : go(k_gas_m<CGA, 1, 8, false, 2>);
+  if (res == 2) return P.fast ? go(k_gas_m<CGA, 1, 8, true, 2>) : go(k_gas_m<CGA, 1, 8, false, 2>);
   if (lanes_per_ray == 4) return P.fast ? go(k_gas_m<CGA, 4, 8, true>) : go(k_gas_m<CGA, 4, 8, false>);
   if (!P.fast) return go(k_gas_m<CGA, 1, 8, false>);
   switch (variant % 4) {

@@ -707,12 +707,12 @@ __device__ __forceinline__ bool shared_gas(const MixedPlan& P, int r, int g) {
 // cell, for batches that leave the device idle.  shape 1: the warps of a
 // block take consecutive tiles of one (channel, emitter), whose rows they
 // share in L1; shape 0: consecutive channels of one tile.
-// Bound by instruction issue and the L1 data pipe together (73 % and 62 %
-// busy on 62 nadir tiles x 100 channels x 5 emitters, 345 instructions per
-// point and emitter, DRAM 5 %): 12.3 ms for those 3.1e7 warp steps, against
+// Bound by instruction issue and the L1 data pipe together (77 % and 70 %
+// busy on 62 nadir tiles x 100 channels x 5 emitters, 354 instructions per
+// point and emitter, DRAM 5 %): 12.1 ms for those 3.1e7 warp steps, against
 // 17 ms in a kernel that held all emitters of a channel in a warp (527
 // instructions, state in shared memory).  What the register count costs
-// shows in the variants: spilling forms take 13.8 ms, 64 registers 12.9 ms.
+// shows in the variants: 12.8 to 14.7 ms.
 //
 // RES: 1 the base rays of resumed perturbations, which leave their state
 // before every start point of their perturbations; 2 the perturbations, which

@@ -244,15 +244,15 @@ class Context:
         self._check(load().jgb_set_los_bound_scale(self.h, float(scale)))
 
     def set_path_split(self, mode: int):
-        """Mixed path loop split over the emitters: -1 for batches too small
-        to fill the device (default), 0 never, 1 always."""
+        """Four lanes per ray in the mixed path: -1 for batches too small to
+        fill the device (default), 0 never, 1 always."""
         self._check(load().jgb_set_path_split(self.h, int(mode)))
 
     def set_fd_resume(self, mode: int):
         """Resume perturbed paths of mixed Jacobians from their base's saved
-        state: 1 when the estimated schedule is shorter (default), 2 always,
-        0 never; 3 always, with the emitters a perturbation leaves unchanged
-        always taken from the base (the results do not depend on it)."""
+        state (and the emitters a perturbation leaves unchanged from the
+        base): 1 when the estimated schedule is shorter (default), 2 and 3
+        always, 0 never (the results do not depend on it)."""
         self._check(load().jgb_set_fd_resume(self.h, int(mode)))
 
     def _check(self, rc):

@@ -118,6 +118,7 @@ struct MixedPlan {
   const float* base_seg;
   const int* base_stop;
   int base_nseg;
+  int gstep;  // perturbations: emitter g in entry g * gstep (0: a tile's one emitter)
 };
 int mixed_nfield(const CtlDev& c, unsigned brmask);
 void launch_pack_tiles_n(const CtlDev& c, const TblDev& T, const LosDev& L, const MixedPlan& P,

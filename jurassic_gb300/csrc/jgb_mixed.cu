@@ -717,9 +717,9 @@ __device__ __forceinline__ bool shared_gas(const MixedPlan& P, int r, int g) {
 // RES: 1 the base rays of resumed perturbations, which leave their state
 // before every start point of their perturbations; 2 the perturbations, which
 // walk on from there, and not at all for an emitter they share with the base.
-// 48 nadir observations x 405 perturbations, 150 channels, 4 emitters: 32 ms
-// here and 19 ms in k_seg_m (6.8e7 and 3.8e7 warp points; bound by issue as
-// above, with 1.6 times the plain batch's time per point since a warp's rays
+// 48 nadir observations x 405 perturbations, 150 channels, 4 emitters: 29 ms
+// here and 17 ms in k_seg_m (6.8e7 and 3.8e7 warp points; bound by issue as
+// above, with 1.5 times the plain batch's time per point since a warp's rays
 // come from several observations and share fewer rows), against 64 ms in a
 // kernel that held all emitters of a channel in a warp and joined the shared
 // ones there.
@@ -765,7 +765,7 @@ __global__ void __launch_bounds__(kPathThreads, MINB) k_gas_m(CtlDev c, TblDev T
   const float* fg = f + (F.g0 + g * es) * 32;
   const int fstep = F.n * 32;
   const long long lp0 = P.toff[tile] - P.pt0;
-  float* out = P.seg + ((lp0 * ndc + idl) * P.nseg + g) * 32 + rl;
+  float* out = P.seg + ((lp0 * ndc + idl) * P.nseg + (RES == 2 ? g * P.gstep : g)) * 32 + rl;
   const long long ostep = (long long)ndc * P.nseg * 32;
   const bool brg = FAST || ((P.brmask >> g) & 1u);
   GasState st;
@@ -980,7 +980,7 @@ __global__ void __launch_bounds__(kPathThreads) k_seg_m(CtlDev c, TblDev T, Batc
     }
     for (int g = 0; g < ng; g++)
       if ((has >> g) & 1u)
-        E = join_f(E, RES == 2 && !((own >> g) & 1u) ? bseg[g * 32] : seg[g * 32]);
+        E = join_f(E, RES != 2 ? seg[g * 32] : (own >> g) & 1u ? seg[g * P.gstep * 32] : bseg[g * 32]);
     if (RES == 2) bseg += bstep;
     const float p = f[F.p * 32], t = f[F.t * 32], ds = f[F.ds * 32];
     float beta = kw >= 0 ? f[kw] : 0.f;

@@ -140,18 +140,17 @@ def peaks():
         return 6800.0, "fallback"
 
 
-# ncu counters of k_path_mixed per LOS point of the nadir workload (all 100
-# channels, 5 emitters), from one capture of the 4000-observation launch
-# with the same channels, emitters and tables (the nadir observations are
-# alike, so the counters scale with the LOS points):
-#   JGB_PATH_VARIANT=14 ncu --set full --clock-control none -k regex:k_path_mixed \
-#       -s 1 -c 1 -o path python bench.py --nobs 4000 --steps 2 --warmup 1 \
-#       --fp64-steps 0 --no-cpu --serve-requests 0 --no-extra
-#   (variant 14: the one the autotuner picks on the 1e5-observation launch)
-#   smsp__inst_executed.sum 3.2978e10, dram__bytes_read.sum + write.sum 862.5 MB,
-#   4,004,179 LOS points in the launch.
-PATH_NCU_NADIR = {"warp_inst_per_los_point": 32978257734 / 4004179,
-                  "dram_bytes_per_los_point": 862.547456e6 / 4004179}
+# ncu counters of the mixed path's kernels (k_gas_m, k_seg_m, k_scan_m) per LOS
+# point of the nadir workload (all 100 channels, 5 emitters), from one capture
+# of one chunk of 1984 observations with the same channels, emitters and tables
+# (the nadir observations are alike, so the counters scale with the LOS points):
+#   JGB_PATH_VARIANT=6 ncu --clock-control none -k "regex:k_gas_m|k_seg_m|k_scan_m" \
+#       --metrics smsp__inst_executed.sum,dram__bytes_read.sum,dram__bytes_write.sum -c 3
+#   (variant 6: the one the autotuner picks on the 1e5-observation launch)
+#   smsp__inst_executed.sum 1.0998e10 + 1.3128e9 + 1.274e8, dram__bytes_read.sum +
+#   write.sum 4.872 + 5.509 + 1.571 GB, 1,986,084 LOS points.
+PATH_NCU_NADIR = {"warp_inst_per_los_point": 12438274756 / 1986084,
+                  "dram_bytes_per_los_point": 11951.956e6 / 1986084}
 
 
 def sm_count(device=0):
@@ -185,7 +184,7 @@ def compulsory_bytes(ctl, tables, los_points, nray):
 
 
 def issue_roofline(los_points, path_ms, sm_mhz, sms, ctl, tables, nray, hbm, hbm_kind):
-    """Binding roofline of k_path_mixed: warp instructions issued per second
+    """Binding roofline of the path's kernels: warp instructions issued per second
     (ncu instructions per LOS point x the launch's LOS points / CUDA-event
     time) against the issue peak of the SMs (4 schedulers x SMs x the SM
     clock sampled during the timed region); the compulsory-byte HBM
@@ -195,11 +194,11 @@ def issue_roofline(los_points, path_ms, sm_mhz, sms, ctl, tables, nray, hbm, hbm
     achieved = inst / t / 1e9
     peak = 4.0 * sms * sm_mhz * 1e6 / 1e9 if sm_mhz and sms else None
     comp = compulsory_bytes(ctl, tables, los_points, nray)
-    return {"bound": "issue", "kernel": "k_path_mixed", "achieved": achieved,
+    return {"bound": "issue", "kernel": "k_gas_m + k_seg_m + k_scan_m", "achieved": achieved,
             "peak": peak, "unit": "G warp-instructions/s",
             "frac": achieved / peak if peak else None,
             "traffic": PATH_NCU_NADIR["dram_bytes_per_los_point"] * los_points,
-            "traffic_note": "ncu dram__bytes_read+write per LOS point (4000-observation capture) "
+            "traffic_note": "ncu dram__bytes_read+write per LOS point (1984-observation capture) "
                             "x LOS points of this launch",
             "warp_instructions_per_launch": inst,
             "peak_note": "4 warp schedulers x %d SMs x %.0f MHz (median SM clock sampled in "
@@ -840,14 +839,9 @@ def main():
                 "stage_ms": {k: stats[k] for k in ("hydro_ms", "trace_ms", "pack_ms", "path_ms")},
                 "trace_passes": stats["trace_passes"],
                 "autotune": {"path_variant": stats["path_variant"], "variant_ms": stats["tune_ms"][:16],
-                             "caps": ["no register cap", "5 blocks/SM (<=102 regs)",
-                                      "6 blocks/SM (<=85 regs)", "4 blocks/SM (<=128 regs)",
-                                      "8 blocks/SM (<=64 regs)", "10 blocks/SM (<=51 regs)",
-                                      "12 blocks/SM (<=42 regs)"],
-                             "note": "variant v < 14: register cap v % 7; block = 4 channels x 1 "
-                                     "tile (v < 7) or 1 channel x 4 tiles (7 <= v < 14); v = 14, "
-                                     "15: block = 1 channel x 8 tiles (256 threads), <= 64 or "
-                                     "<= 51 registers"},
+                             "note": "variant v: at most 64, 48, 40 or 32 registers (v % 4); "
+                                     "block = 4 channels x 1 tile (v < 4) or 1 channel and "
+                                     "emitter x 4 tiles (v >= 4)"},
                 "wall_s_timed": wall,
                 "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(h2d),
                         "d2h_bytes_per_step": int(d2h), "ms_per_step": statistics.mean(e2e_ms),

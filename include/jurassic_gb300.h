@@ -96,12 +96,11 @@ typedef struct {
   long long los_points;          /* LOS points of the batch */
   int path_launches;             /* kernels launched by the last call */
   int path_variant;              /* mixed path kernel variant chosen by the autotuner:
-                                    0-13: register cap (path_variant % 7) and block
-                                    shape (path_variant / 7: 0 = 4 channels of one
-                                    tile, 1 = one channel of 4 tiles); 14, 15: one
-                                    channel of 8 tiles (256 threads), at most 64 or
-                                    51 registers */
-  float tune_ms[16];             /* autotuner timings of the variants [ms] */
+                                    register cap (path_variant % 4: 64, 48, 40 or
+                                    32) and block shape (path_variant / 4: 0 = 4
+                                    channels of one tile, 1 = 4 tiles of one channel
+                                    and emitter); -1 = none timed yet */
+  float tune_ms[16];             /* autotuner timings of the 8 variants [ms], then 0 */
   int trace_passes;              /* ray-tracing passes over the batch: 1 = one
                                     pass, 2 = count + fill, 3 = a capacity
                                     bound was exceeded and the rays were
@@ -156,20 +155,19 @@ int jgb_write_table_file(const char *path, int tblfmt, int np, const double *p, 
    off.  Not available in jgb_formod_batch_dev_noalloc. */
 int jgb_set_fov(jgb_ctx *ctx, int n, const double *dz, const double *w);
 
-/* Mixed-precision ray tracing of a batch larger than 2^23 / NLOS rays runs
-   in one pass into per-ray capacities from a geometric bound of the LOS
-   points (a ray that outgrows its capacity makes the batch count its rays
-   first, as FP64 always does).  scale multiplies the bound (memory against
+/* Ray tracing of a batch (mixed precision: one larger than 2^23 / NLOS rays)
+   runs in one pass into per-ray capacities from a geometric bound of the LOS
+   points (a ray that outgrows its capacity, or in FP64 capacities that do not
+   fit the device, make the batch count its rays first).  scale multiplies the bound (memory against
    the chance of a second pass); 0 always counts first.  Default 1.  The
    results do not depend on it. */
 int jgb_set_los_bound_scale(jgb_ctx *ctx, double scale);
 
-/* Mixed-precision path loop of a batch too small to fill the device (at most
-   32 x SMs warps of tile x channel x emitter): split over the emitters, one
-   warp per (tile, channel, emitter) for the emitters' path states, then one
-   per (tile, channel) for their combination and the radiance.  mode -1 (the
-   default) decides by that size, 0 never splits, 1 always does.  The results
-   do not depend on it. */
+/* Mixed-precision path of a batch too small to fill the device (at most 18 x
+   SMs warps of tile x channel x emitter): four lanes per ray, one per corner of
+   the p-T cell, walk an emitter's path instead of one.  mode -1 (the default)
+   decides by that size, 0 never, 1 always takes four.  The results do not
+   depend on it. */
 int jgb_set_path_split(jgb_ctx *ctx, int mode);
 
 /* Mixed-precision finite-difference Jacobians: a perturbation of a level
@@ -178,13 +176,13 @@ int jgb_set_path_split(jgb_ctx *ctx, int mode);
    path restarts from its unperturbed base's saved state there (exact; not
    with hydrostatic pressures, a field of view or surface reflection).  The
    bases run first and the lanes of a warp walk the union of their ranges,
-   so it pays on large batches: mode 1 (default) resumes a Jacobian chunk
-   when the estimated schedule of its tiles is shorter, 2 always, 0 never.
+   so it pays on all but the smallest batches: mode 1 (default) resumes a
+   Jacobian chunk when the estimated schedule of its tiles is shorter, 2 and 3
+   always, 0 never.
    A perturbation of one emitter's mixing ratio (or of an extinction) also
    leaves the other emitters' path states equal to the base's: resumed
    chunks then take those emitters' segment emissivities from the base's
-   walk and compute only the perturbed one, where at least 30 % of the
-   perturbed lookups can be shared (mode 3: always resume and always share).
+   walk and compute only the perturbed one.
    In EGA, modes 2 and 3 also trace the perturbed rays from their bases'
    walks (a perturbed mixing ratio or extinction takes the base's geometry,
    a perturbed temperature walks on from the base's state); mode 1 does so

@@ -166,7 +166,7 @@ __global__ void k_widen(int n, const int* a, long long* b) {
 // Batches of mixed precision with at most this many rays x NLOS points are
 // traced in one pass into fixed per-ray slabs (small batches, e.g. the
 // retrieval's damped trials, are latency-bound and the counting pass would
-// double the ray-tracing time); larger ones count first.
+// double the ray-tracing time); larger ones take capacities from a bound.
 constexpr long long kSinglePassPoints = 1LL << 23;
 
 // Fixed slabs of LOS points per ray (single-pass tracing): ray r owns

@@ -440,6 +440,14 @@ int plan_tiles(jgb_ctx* x, int nray, const int* keys, const int* count, int ntil
 // emitters' kernel tens of warps per scheduler.
 constexpr size_t kPathBytes = size_t(4) << 30;
 
+// A workspace of that limit did not fit the device: try a quarter of it, down
+// to 64 MiB (results do not depend on the chunks).
+bool smaller_chunks(cudaError_t e, size_t limit) {
+  if (e != cudaErrorMemoryAllocation || limit <= (size_t(64) << 20)) return false;
+  (void)cudaGetLastError();
+  return true;
+}
+
 struct PathChunk {
   int t0, t1;   // tiles
   int ndc;      // channels at a time
@@ -448,9 +456,9 @@ struct PathChunk {
 
 // point_bytes, chan_bytes: workspace of a tile point, and of one per channel;
 // tile_bytes: of a (tile, channel).  The largest needs in *need_points (limited
-// to a quarter of kPathBytes) and *need_chan.
-void path_chunks(const std::vector<long long>& toff, int tfirst, int nd, size_t point_bytes,
-                 size_t chan_bytes, size_t tile_bytes, std::vector<PathChunk>& out,
+// to a quarter of limit) and *need_chan (limited to limit).
+void path_chunks(const std::vector<long long>& toff, int tfirst, int nd, size_t limit,
+                 size_t point_bytes, size_t chan_bytes, size_t tile_bytes, std::vector<PathChunk>& out,
                  size_t* need_points, size_t* need_chan) {
   const int ntile = (int)toff.size() - 1;
   for (int t = tfirst; t < ntile;) {
@@ -459,10 +467,10 @@ void path_chunks(const std::vector<long long>& toff, int tfirst, int nd, size_t 
     do {
       k.longest = std::max(k.longest, (int)(toff[k.t1 + 1] - toff[k.t1]));
       k.t1++;
-    } while (k.t1 < ntile && k.t1 - k.t0 < 65535 && pts(k.t1 + 1) * point_bytes <= kPathBytes / 4 &&
-             pts(k.t1 + 1) * nd * chan_bytes <= kPathBytes);
+    } while (k.t1 < ntile && k.t1 - k.t0 < 65535 && pts(k.t1 + 1) * point_bytes <= limit / 4 &&
+             pts(k.t1 + 1) * nd * chan_bytes <= limit);
     const size_t np = std::max<size_t>(pts(k.t1), 1);
-    if (np * nd * chan_bytes > kPathBytes) k.ndc = (int)std::max<size_t>(kPathBytes / (np * chan_bytes), 1);
+    if (np * nd * chan_bytes > limit) k.ndc = (int)std::max<size_t>(limit / (np * chan_bytes), 1);
     if (need_points) *need_points = std::max(*need_points, np * point_bytes);
     *need_chan = std::max(*need_chan, np * k.ndc * chan_bytes + (size_t)(k.t1 - k.t0) * k.ndc * tile_bytes);
     out.push_back(k);
@@ -529,11 +537,18 @@ int run_path64(jgb_ctx* x, const BatchDev& b, const LosDev& L, cudaStream_t s, i
   path64_point_bytes(c, &bfd, &bfu);
   const size_t bch = 32 * sizeof(double) * (size_t)(c.ng + 2);  // per (point, channel)
   std::vector<PathChunk> chunks;
-  size_t need_f = 0, need_w = 0;
-  path_chunks(toff, 0, c.nd, bfd + bfu, bch, 32 * sizeof(int) * (size_t)std::max(c.ng, 1), chunks,
-              &need_f, &need_w);
-  CK(x->tiles_data.reserve(need_f));
-  CK(x->seg.reserve(need_w));
+  for (size_t limit = kPathBytes;; limit /= 4) {
+    chunks.clear();
+    size_t need_f = 0, need_w = 0;
+    path_chunks(toff, 0, c.nd, limit, bfd + bfu, bch, 32 * sizeof(int) * (size_t)std::max(c.ng, 1),
+                chunks, &need_f, &need_w);
+    cudaError_t e = x->tiles_data.reserve(need_f);
+    if (e == cudaSuccess) e = x->seg.reserve(need_w);
+    if (!smaller_chunks(e, limit)) {
+      CK(e);
+      break;
+    }
+  }
   CK(cudaEventRecord(x->ev[4], s));
   Path64 P{};
   P.perm = Pm.perm;
@@ -1019,12 +1034,39 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
       const size_t b_stop = 32 * sizeof(int) * (size_t)tfirst * std::max(c.ng, 1);
       const size_t b_state = gas_state_bytes() * (size_t)nray * c.ng, b_sums = 3 * sizeof(float) * (size_t)nray;
       const size_t per = std::max(b_seg + b_stop, b_state + b_sums);
-      const int gnd = (int)std::min<size_t>(c.nd, std::max<size_t>(kPathBytes / per, 1));
       auto a16 = [](size_t v) { return (v + 15) & ~size_t(15); };
-      const size_t o_stop = a16(b_seg * gnd), o_slot = o_stop + a16(b_stop * gnd);
-      const size_t o_reuse = o_slot + a16(sizeof(int) * (size_t)std::max(nbase_rays, 1));
-      CK(x->rs_seg.reserve(o_reuse + sizeof(int2) * (size_t)nray));
-      CK(x->rs_snap.reserve(a16(b_state * gnd) + b_sums * gnd));
+      // rays that share emitters keep one emitter's segments (two entries, for
+      // the products), so that more of their tiles run side by side: most of
+      // a chunk's warps have nothing to walk (48 nadir observations x 405
+      // perturbations: 64.1 ms with ng entries, 59.8 with two)
+      struct Part {
+        std::vector<PathChunk> chunks;
+        int nseg, gstep;
+      };
+      Part parts[2] = {{{}, std::max(c.ng, 2), 1}, {{}, 2, 0}};
+      const size_t tile_bytes = 32 * sizeof(int) * (size_t)std::max(c.ng, 1);
+      const std::vector<long long> toff_own(toff_h.begin(), toff_h.begin() + tsecond + 1);
+      int gnd = 1;
+      size_t o_stop = 0, o_slot = 0, o_reuse = 0;
+      for (size_t limit = kPathBytes;; limit /= 4) {
+        gnd = (int)std::min<size_t>(c.nd, std::max<size_t>(limit / per, 1));
+        o_stop = a16(b_seg * gnd);
+        o_slot = o_stop + a16(b_stop * gnd);
+        o_reuse = o_slot + a16(sizeof(int) * (size_t)std::max(nbase_rays, 1));
+        size_t need = 0;
+        for (Part& part : parts) {
+          part.chunks.clear();
+          path_chunks(part.gstep ? toff_own : toff_h, part.gstep ? tfirst : tsecond, gnd, limit, 0,
+                      32 * sizeof(float) * part.nseg, tile_bytes, part.chunks, nullptr, &need);
+        }
+        cudaError_t e = x->rs_seg.reserve(o_reuse + sizeof(int2) * (size_t)nray);
+        if (e == cudaSuccess) e = x->rs_snap.reserve(a16(b_state * gnd) + b_sums * gnd);
+        if (e == cudaSuccess) e = x->seg.reserve(need);
+        if (!smaller_chunks(e, limit)) {
+          CK(e);
+          break;
+        }
+      }
       char* sp = x->rs_seg.as<char>();
       int* slot = reinterpret_cast<int*>(sp + o_slot);
       k_base_slots<<<(tfirst * 32 + 127) / 128, 128, 0, s>>>(tfirst * 32, Pm.perm, slot);
@@ -1043,22 +1085,6 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
         CK(cudaStreamSynchronize(s));
         Pm.reuse = reinterpret_cast<int2*>(sp + o_reuse);
       }
-      // rays that share emitters keep one emitter's segments (two entries, for
-      // the products), so that more of their tiles run side by side: most of
-      // a chunk's warps have nothing to walk (48 nadir observations x 405
-      // perturbations: 64.1 ms with ng entries, 59.8 with two)
-      struct Part {
-        std::vector<PathChunk> chunks;
-        int nseg, gstep;
-      };
-      Part parts[2] = {{{}, std::max(c.ng, 2), 1}, {{}, 2, 0}};
-      size_t need = 0;
-      const size_t tile_bytes = 32 * sizeof(int) * (size_t)std::max(c.ng, 1);
-      path_chunks(std::vector<long long>(toff_h.begin(), toff_h.begin() + tsecond + 1), tfirst, gnd, 0,
-                  32 * sizeof(float) * parts[0].nseg, tile_bytes, parts[0].chunks, nullptr, &need);
-      path_chunks(toff_h, tsecond, gnd, 0, 32 * sizeof(float) * parts[1].nseg, tile_bytes,
-                  parts[1].chunks, nullptr, &need);
-      CK(x->seg.reserve(need));
       CK(cudaEventRecord(x->ev[4], s));
       for (int g0 = 0; g0 < c.nd; g0 += gnd) {
         MixedPlan P = Pm;
@@ -1108,9 +1134,17 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
       // where one tile alone would not)
       const size_t bch = 32 * sizeof(float) * (size_t)Pm.nseg;
       std::vector<PathChunk> chunks;
-      size_t need = 0;
-      path_chunks(toff_h, 0, c.nd, 0, bch, 32 * sizeof(int) * (size_t)std::max(c.ng, 1), chunks, nullptr, &need);
-      CK(x->seg.reserve(need));
+      for (size_t limit = kPathBytes;; limit /= 4) {
+        chunks.clear();
+        size_t need = 0;
+        path_chunks(toff_h, 0, c.nd, limit, 0, bch, 32 * sizeof(int) * (size_t)std::max(c.ng, 1),
+                    chunks, nullptr, &need);
+        const cudaError_t e = x->seg.reserve(need);
+        if (!smaller_chunks(e, limit)) {
+          CK(e);
+          break;
+        }
+      }
       const long long warps = (long long)ntile * c.nd * c.ng;
       const int lanes = x->path_split == 1 || (x->path_split < 0 && warps <= kFourLaneWarps * x->sms) ? 4 : 1;
       bool timed = false;

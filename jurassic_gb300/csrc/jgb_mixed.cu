@@ -969,7 +969,7 @@ __global__ void __launch_bounds__(kPathThreads) k_seg_m(CtlDev c, TblDev T, Batc
   for (int k = 0; k < kChanWindow; k++) kc[k] = T.chanf[id * kChanConsts + k];
   const int on = continua_on(c, kc[kChanSwitches]);
   const int kw = c.nw > 0 ? (F.kw0 + __float_as_int(T.chanf[id * kChanConsts + kChanWindow])) * 32 : -1;
-  const float cl = P.cloud ? P.cloud[(long long)id * b.nray + r] : __int_as_float(0x7fc00000);
+  const float cl = P.cloud ? P.cloud[(long long)id * b.nray + r] : 0.f;
   const float* srf = T.srf + (long long)id * kNS;
   const int po = RES == 1 ? ng * 32 : 0;  // a base ray's emitters stay for its perturbations
   for (int ip = ip0; ip < n; ip++, f += F.n * 32, seg += sstep) {
@@ -984,7 +984,7 @@ __global__ void __launch_bounds__(kPathThreads) k_seg_m(CtlDev c, TblDev T, Batc
     if (RES == 2) bseg += bstep;
     const float p = f[F.p * 32], t = f[F.t * 32], ds = f[F.ds * 32];
     float beta = kw >= 0 ? f[kw] : 0.f;
-    if (cl == cl) beta = __fmaf_rn(f[F.aux * 32], cl, beta);
+    if (P.cloud) beta = __fmaf_rn(f[F.aux * 32], cl, beta);
     beta = continua_f(c, F, kc, on, f, p, t, ds, beta);
     const float src = source_f(srf, t);
     const float eps = segment_f(E, beta, ds);
@@ -993,13 +993,14 @@ __global__ void __launch_bounds__(kPathThreads) k_seg_m(CtlDev c, TblDev T, Batc
   }
 }
 
-// Cloud extinction of every (channel, ray), NaN without a cloud.
+// Cloud extinction of every (channel, ray), 0 without a cloud (whose factor aux
+// is 0 at every point then): an extinction that is not a number stays one.
 __global__ void k_cloud_m(CtlDev c, ChanDev ch, BatchDev b, float* out) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (long long)c.nd * b.nray) return;
   bool has = false;
   const float v = cloud_of(c, ch, b, (int)(i % b.nray), (int)(i / b.nray), &has);
-  out[i] = has ? v : __int_as_float(0x7fc00000);
+  out[i] = has ? v : 0.f;
 }
 
 // k_scan_m: one thread per (ray, channel) sums the segments along the path.

@@ -3,8 +3,8 @@
 // matrix_invert, retrieval.c:373-399), blocked in tiles of 32 x 32:
 //
 //   for every panel k: k_chol_diag   L_kk and its inverse, one warp
-//                      k_chol_panel  L_ik = A_ik L_kk^-T, a tile per block
-//                      k_chol_update A_ij -= L_ik L_jk^T, a tile per block
+//                      k_chol_panel  L_ik = (A - S)_ik L_kk^-T, a tile per block
+//                      k_chol_update S_ij += L_ik L_jk^T, a tile per block
 //   k_tri_inverse      W = L^-1, one block per block column
 //   k_gram             A^-1 = W^T W, a tile pair per block, both triangles
 //
@@ -14,10 +14,16 @@
 // instructions per multiply-add, 1.7 n^3 in all, with a block-wide barrier
 // twice per column; tiles spread every matrix over the device, a thread keeps
 // 4 x 4 sums in registers, and 32 x 32 tiles waste little on the diagonals.
-// 96 matrices of up to 405 x 405 (48 of them smaller): 44.6 -> 7.7 ms, of
+// 96 matrices of up to 405 x 405 (48 of them smaller): 44.6 -> 7.8 ms, of
 // which k_tri_inverse 2.8 (its longest column is 1.5), k_gram 1.8,
-// k_chol_update 1.5, k_chol_diag 0.9 (13 panels, a warp's chain of roots),
-// k_chol_panel 0.6; the multiply-adds alone are 4.1 ms.
+// k_chol_update 1.5, k_chol_diag 1.1 (13 panels, a warp's chain of roots),
+// k_chol_panel 0.7; the multiply-adds alone are 4.1 ms.
+//
+// Rounding: sums are formed apart and subtracted once, a tile's products apart
+// from the sum over the tiles, quotients are correctly rounded.  Error against
+// inverses refined in long double, over the error of a block per matrix that
+// subtracted whole sums (geometric means, n from 12 to 405): covariances 1.06,
+// Gauss-Newton matrices 0.76.
 #include <algorithm>
 
 #include "../../include/jurassic_gb300.h"
@@ -78,50 +84,66 @@ __device__ __forceinline__ void tile_fma(const double (*a)[kPad], const double (
   }
 }
 
-// Copy of the matrices' lower triangles into the factors.
-__global__ void k_chol_copy(int nret, const InvertDesc* d, const int* full, const double* A,
-                            double* L) {
-  const int i = blockIdx.y;
-  if (!full[i]) return;
-  const long long nn = (long long)d[i].n * d[i].n;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < nn;
-       e += (long long)gridDim.x * blockDim.x)
-    L[d[i].off + e] = A[d[i].off + e];
+__device__ __forceinline__ void tile_add(double (&acc)[4][4], const double (&part)[4][4]) {
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++) acc[i][j] += part[i][j];
 }
 
-// Diagonal tile of panel k: lane r holds row r.  Columns beyond the matrix are
+// a / w from the reciprocal r of w > 0: quotient, exact remainder, one correction
+// (Markstein, IBM J. Res. Dev. 34, 1990); 0 for an infinite w.
+__device__ __forceinline__ double quotient(double a, double w, double r) {
+  const double q = a * r;
+  return __double2hiint(w) == 0x7ff00000 ? q : fma(fma(-q, w, a), r, q);
+}
+
+// Diagonal tile of panel k: lane r holds row r.  Every entry of the factor is (A -
+// sum) / L_jj with its sum formed apart and subtracted once, the sums over the
+// panels before it (S, where the factor will be) and over this tile's columns:
+// taking the products off A one by one rounds at the size of A every time and
+// made covariances' inverses 2.3 times as wrong.  Columns beyond the matrix are
 // those of the identity.
 __global__ void __launch_bounds__(32) k_chol_diag(const InvertDesc* d, const int* full, int* status,
-                                                  double* Lall, double* Wall, int k) {
+                                                  const double* Aall, double* Lall, double* Wall,
+                                                  int k) {
   const int i = blockIdx.x, lane = threadIdx.x;
   Mat m;
   if (!mat_at(d, full, status, Lall, Wall, i, m)) return;
   const int base = k * kB;
   if (base >= m.n) return;
   const int nb = min(kB, m.n - base);
-  double row[kB];
+  __shared__ double a[kB][kB + 1], s[kB][kB + 1];
+  const double* A = Aall + d[i].off;
+#pragma unroll 16
+  for (int r = 0; r < kB; r++) {  // lanes along a row
+    const bool in = r < nb && lane <= r;
+    const long long e = (long long)(base + r) * m.n + base + lane;
+    a[r][lane] = in ? A[e] : (r == lane ? 1.0 : 0.0);
+    s[r][lane] = in && k > 0 ? m.L[e] : 0.0;
+  }
+  __syncwarp();
+  double row[kB], sum[kB];
 #pragma unroll
-  for (int c = 0; c < kB; c++)
-    row[c] = lane < nb && c <= lane ? m.L[(long long)(base + lane) * m.n + base + c]
-                                    : (c == lane ? 1.0 : 0.0);
+  for (int c = 0; c < kB; c++) sum[c] = 0.0;
   bool bad = false;
-  double inv = 0.0;  // reciprocal of this lane's diagonal entry
+  double diag = 1.0, recip = 1.0;  // this lane's diagonal entry and its reciprocal
 #pragma unroll
   for (int j = 0; j < kB; j++) {
-    const double dj = __shfl_sync(0xffffffffu, row[j], j);
+    const double v = a[lane][j] - (s[lane][j] + sum[j]);
+    const double dj = __shfl_sync(0xffffffffu, v, j);
     bad |= !(dj > 0);
     const double lj = sqrt(dj), rj = 1 / lj;
     if (lane == j) {
-      row[j] = lj;
-      inv = rj;
-    } else if (lane > j) {
-      row[j] *= rj;
+      diag = lj;
+      recip = rj;
     }
-    const double mine = lane > j ? row[j] : 0.0;
+    const double mine = lane > j ? quotient(v, lj, rj) : 0.0;
+    row[j] = lane == j ? lj : mine;
 #pragma unroll
     for (int c = j + 1; c < kB; c++) {
       const double lc = __shfl_sync(0xffffffffu, mine, c);
-      row[c] = fma(-mine, lc, row[c]);
+      sum[c] = fma(mine, lc, sum[c]);
     }
   }
   if (bad) {
@@ -136,10 +158,11 @@ __global__ void __launch_bounds__(32) k_chol_diag(const InvertDesc* d, const int
   double x[kB];
 #pragma unroll
   for (int r = 0; r < kB; r++) {
-    double s = r == lane ? 1.0 : 0.0;
+    double t = 0.0;
 #pragma unroll
-    for (int q = 0; q < r; q++) s = fma(-__shfl_sync(0xffffffffu, row[q], r), x[q], s);
-    x[r] = s * __shfl_sync(0xffffffffu, inv, r);
+    for (int q = 0; q < r; q++) t = fma(__shfl_sync(0xffffffffu, row[q], r), x[q], t);
+    x[r] = quotient((r == lane ? 1.0 : 0.0) - t, __shfl_sync(0xffffffffu, diag, r),
+                    __shfl_sync(0xffffffffu, recip, r));
   }
   if (lane < nb)
 #pragma unroll
@@ -147,16 +170,22 @@ __global__ void __launch_bounds__(32) k_chol_diag(const InvertDesc* d, const int
       if (r < nb && r >= lane) m.W[(long long)(base + r) * m.n + base + lane] = x[r];
 }
 
-// L_ik = A_ik L_kk^-T below the diagonal tile (L_kk^-1 in W).
+// L_ik = (A - S)_ik L_kk^-T below the diagonal tile (L_kk^-1 in W; S, the sum over
+// the panels before, where L_ik goes).
 __global__ void __launch_bounds__(kT) k_chol_panel(const InvertDesc* d, const int* full,
-                                                   const int* status, double* Lall, double* Wall,
-                                                   int k) {
+                                                   const int* status, const double* Aall,
+                                                   double* Lall, double* Wall, int k) {
   Mat m;
   if (!mat_at(d, full, status, Lall, Wall, blockIdx.y, m)) return;
   const int bi = k + 1 + (int)blockIdx.x;
   if (bi * kB >= m.n) return;
   __shared__ __align__(16) double a[kB][kPad], b[kB][kPad];
-  load_tile<true, false>(m.L, m.n, bi, k, a);  // a[q][i] = A_iq
+  const double* A = Aall + d[blockIdx.y].off;
+  for (int e = threadIdx.x; e < kB * kB; e += kT) {  // a[q][i] = (A - S)_iq
+    const int r = e / kB, c = e % kB, row = bi * kB + r;
+    const long long g = (long long)row * m.n + k * kB + c;  // panel k lies whole in the matrix
+    a[c][r] = row < m.n ? (k > 0 ? A[g] - m.L[g] : A[g]) : 0.0;
+  }
   load_tile<true, true>(m.W, m.n, k, k, b);    // b[q][j] = (L_kk^-1)_jq
   __syncthreads();
   double acc[4][4] = {};
@@ -175,7 +204,7 @@ __device__ __forceinline__ void tri_pair(int g, int& ti, int& tj) {
   tj = g - ti * (ti + 1) / 2;
 }
 
-// A_ij -= L_ik L_jk^T for the tiles behind panel k.
+// S_ij += L_ik L_jk^T for the tiles behind panel k (the first panel writes S).
 __global__ void __launch_bounds__(kT) k_chol_update(const InvertDesc* d, const int* full,
                                                     const int* status, double* Lall, double* Wall,
                                                     int k) {
@@ -197,7 +226,7 @@ __global__ void __launch_bounds__(kT) k_chol_update(const InvertDesc* d, const i
     for (int j = 0; j < 4; j++)
       if (i0 + i < m.n && j0 + j <= i0 + i) {
         double* p = m.L + (long long)(i0 + i) * m.n + j0 + j;
-        *p -= acc[i][j];
+        *p = k > 0 ? *p + acc[i][j] : acc[i][j];
       }
 }
 
@@ -213,14 +242,16 @@ __global__ void __launch_bounds__(kT) k_tri_inverse(const InvertDesc* d, const i
   __shared__ __align__(16) double a[kB][kPad], b[kB][kPad];
   const int i0 = 4 * (threadIdx.x >> 3), j0 = 4 * (threadIdx.x & 7);
   for (int bi = bj + 1; bi < nt; bi++) {
-    double acc[4][4] = {};
+    double acc[4][4] = {};  // a tile's products apart, then the tiles: fewer roundings
     for (int k = bj; k < bi; k++) {
+      double part[4][4] = {};
       __syncthreads();
       load_tile<true, false>(m.L, m.n, bi, k, a);  // a[q][i] = L_iq
       if (k == bj) load_tile<false, true>(m.W, m.n, k, bj, b);
       else load_tile<false, false>(m.W, m.n, k, bj, b);  // b[q][j] = W_qj
       __syncthreads();
-      tile_fma(a, b, acc);
+      tile_fma(a, b, part);
+      tile_add(acc, part);
     }
     __syncthreads();
     load_tile<true, true>(m.W, m.n, bi, bi, a);  // a[q][i] = (L_ii^-1)_iq
@@ -250,12 +281,14 @@ __global__ void __launch_bounds__(kT) k_gram(const InvertDesc* d, const int* ful
   __shared__ __align__(16) double a[kB][kPad], b[kB][kPad];
   double acc[4][4] = {};
   for (int k = bi; k < nt; k++) {
+    double part[4][4] = {};
     __syncthreads();
     if (k == bi) load_tile<false, true>(m.W, m.n, k, bi, a);
     else load_tile<false, false>(m.W, m.n, k, bi, a);
     if (bi != bj) load_tile<false, false>(m.W, m.n, k, bj, b);
     __syncthreads();
-    tile_fma(a, bi != bj ? b : a, acc);
+    tile_fma(a, bi != bj ? b : a, part);
+    tile_add(acc, part);
   }
   double* out = A + d[blockIdx.y].off;
   const int i0 = bi * kB + 4 * (threadIdx.x >> 3), j0 = bj * kB + 4 * (threadIdx.x & 7);
@@ -272,12 +305,11 @@ __global__ void __launch_bounds__(kT) k_gram(const InvertDesc* d, const int* ful
 void matrix_invert_blocked(int nret, int nmax, const InvertDesc* d, const int* full, int* status,
                            double* A, double* L, double* W, cudaStream_t s) {
   const int nt = (nmax + kB - 1) / kB;
-  k_chol_copy<<<dim3(16, nret), 256, 0, s>>>(nret, d, full, A, L);
   for (int k = 0; k < nt; k++) {
     const int below = nt - 1 - k;
-    k_chol_diag<<<nret, 32, 0, s>>>(d, full, status, L, W, k);
+    k_chol_diag<<<nret, 32, 0, s>>>(d, full, status, A, L, W, k);
     if (below > 0) {
-      k_chol_panel<<<dim3(below, nret), kT, 0, s>>>(d, full, status, L, W, k);
+      k_chol_panel<<<dim3(below, nret), kT, 0, s>>>(d, full, status, A, L, W, k);
       k_chol_update<<<dim3(below * (below + 1) / 2, nret), kT, 0, s>>>(d, full, status, L, W, k);
     }
   }

@@ -73,7 +73,8 @@ void ctm_coefficients(double nu, double* out) {
       out[5] = sfac * c296;
       out[6] = c260 / c296;
       out[7] = cfrn * fscal;
-      out[14] = c260 > 0 && c296 > 0 ? std::log(out[6]) : std::nan("");
+      if (c260 > 0 && c296 > 0) log_parts(out[6], &out[14], &out[15]);
+      else out[14] = std::nan("");
     }
   }
   auto cia = [&](int ob, int obeta, int onu, int n, double* o) {

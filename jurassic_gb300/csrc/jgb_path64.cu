@@ -569,8 +569,8 @@ __global__ void __launch_bounds__(128) k_seg64(CtlDev c, TblDev T, ChanDev ch, B
   }
   if (c.ctm_h2o && c.ig_h2o >= 0 && cc[4] != 0) {
     const double* f = fd + F.h2o * 32;
-    const double nu = ch.nu[id], x = f[32], lc = cc[14];  // lc = log(cc[6]), NaN: no logarithm
-    const double self = cc[5] * (lc == lc ? exp(lc * x) : pow(cc[6], x));
+    const double nu = ch.nu[id], x = f[32], lc = cc[14];  // log(cc[6]), NaN: no logarithm
+    const double self = cc[5] * (lc == lc ? pow_of_log(lc, cc[15], x) : pow(cc[6], x));
     beta = fma(nu * tanh(f[0] * nu), fma(f[64], self, f[96] * cc[7]), beta);
   }
   if ((c.ctm_n2 && cc[8] != 0) || (c.ctm_o2 && cc[11] != 0)) {

@@ -93,7 +93,7 @@ struct MixedPlan {
   int nseg;
   float* seg;
   int* stop;
-  const float* cloud;   // [nd][nray] cloud extinction (0: no cloud), nullptr: no clouds
+  const float* cloud;   // [nd][nray] cloud extinction (-0: no cloud), nullptr: no clouds
   // Resumed forward models (finite-difference perturbations), for channels
   // [gid0, gid0 + gndc): ray r starts at LOS point start[r], where its path
   // equals its base ray's.  A base ray saves its state for the rays snap_ray[k]

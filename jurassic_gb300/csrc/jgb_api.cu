@@ -1025,6 +1025,16 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
       Pm.cloud = x->cloudf.as<float>();
       launches += 1;
     }
+    // four lanes per ray where the batch leaves the device idle; with one, and for
+    // perturbations, opaque rays end early (small batches wait for their longest)
+    const long long path_warps = (long long)ntile * c.nd * c.ng;
+    const int lanes = x->path_split == 1 || (x->path_split < 0 && path_warps <= kFourLaneWarps * x->sms) ? 4 : 1;
+    if ((c.nw > 0 || c.ncl > 0) && (rs || lanes == 1)) {
+      CK(x->ext_sum.reserve(sizeof(float) * (size_t)(c.nw + 1) * nray));
+      launch_ext_sums(c, L, nray, x->ext_sum.as<float>(), s);
+      Pm.ext_sum = x->ext_sum.as<float>();
+      launches += 1;
+    }
     if (rs) {
       // The bases (saving the states), then the perturbations (starting from
       // them), for groups of channels whose base segments, states and the
@@ -1045,7 +1055,7 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
         int nseg, gstep;
       };
       Part parts[2] = {{{}, std::max(c.ng, 2), 1}, {{}, 2, 0}};
-      const size_t tile_bytes = 32 * sizeof(int) * (size_t)std::max(c.ng, 1);
+      const size_t tile_bytes = 32 * sizeof(int) * (size_t)(c.ng + 1);  // stop and ends
       const std::vector<long long> toff_own(toff_h.begin(), toff_h.begin() + tsecond + 1);
       int gnd = 1;
       size_t o_stop = 0, o_slot = 0, o_reuse = 0;
@@ -1119,9 +1129,11 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
               P.id1 = std::min(g0 + P.gndc, id + k.ndc);
               P.stop = reinterpret_cast<int*>(x->seg.as<char>() + pts * (P.id1 - P.id0) * 32 *
                                                                       sizeof(float) * part.nseg);
+              P.ends = P.stop + (size_t)(k.t1 - k.t0) * (P.id1 - P.id0) * c.ng * 32;
+              launch_path_ends(c, T, ch, bo, L, P, 2, s);
               launch_gas_m(c, T, bo, L, P, 1, 4, 2, s);
               launch_seg_scan_m(c, T, ch, bo, L, P, std::max(k.longest, 1), 2, s);
-              launches += 3;
+              launches += 4;
             }
           }
         }
@@ -1138,16 +1150,14 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
       for (size_t limit = kPathBytes;; limit /= 4) {
         chunks.clear();
         size_t need = 0;
-        path_chunks(toff_h, 0, c.nd, limit, 0, bch, 32 * sizeof(int) * (size_t)std::max(c.ng, 1),
-                    chunks, nullptr, &need);
+        path_chunks(toff_h, 0, c.nd, limit, 0, bch, 32 * sizeof(int) * (size_t)(c.ng + 1), chunks,
+                    nullptr, &need);
         const cudaError_t e = x->seg.reserve(need);
         if (!smaller_chunks(e, limit)) {
           CK(e);
           break;
         }
       }
-      const long long warps = (long long)ntile * c.nd * c.ng;
-      const int lanes = x->path_split == 1 || (x->path_split < 0 && warps <= kFourLaneWarps * x->sms) ? 4 : 1;
       bool timed = false;
       for (const PathChunk& k : chunks) {
         Pm.tile0 = k.t0;
@@ -1159,8 +1169,13 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
           Pm.id1 = std::min(c.nd, id + k.ndc);
           Pm.seg = x->seg.as<float>();
           Pm.stop = reinterpret_cast<int*>(x->seg.as<char>() + np * (Pm.id1 - Pm.id0) * bch);
+          if (lanes == 1) {
+            Pm.ends = Pm.stop + (size_t)(k.t1 - k.t0) * (Pm.id1 - Pm.id0) * c.ng * 32;
+            launch_path_ends(c, T, ch, bo, L, Pm, 0, s);
+            launches += 1;
+          }
           int variant = x->path_variant;
-          if (lanes == 1 && variant < 0 && warps > 32LL * x->sms) {
+          if (lanes == 1 && variant < 0 && path_warps > 32LL * x->sms) {
             const int rc = tune_gas(x, T, bo, L, Pm, s);
             if (rc) return rc;
             variant = x->path_variant;
@@ -1732,7 +1747,7 @@ void jgb_destroy(jgb_ctx* x) {
     for (jgb_engine* E : x->engines) engine_detach(E);
     x->engines.clear();
   }
-  DevBuf* bufs[] = {&x->d_nu, &x->d_window, &x->d_clnu, &x->d_sfnu, &x->d_ctm, &x->d_chanf, &x->cloudf, &x->t_np,
+  DevBuf* bufs[] = {&x->d_nu, &x->d_window, &x->d_clnu, &x->d_sfnu, &x->d_ctm, &x->d_chanf, &x->cloudf, &x->ext_sum, &x->t_np,
                     &x->t_p, &x->t_nt, &x->t_t, &x->t_nu, &x->t_u, &x->t_eps, &x->t_pf,
                     &x->t_tf, &x->t_meta, &x->t_ue, &x->t_odd, &x->s_st, &x->s_sr, &x->s_srf, &x->s_srd, &x->b_levoff, &x->b_rayoff,
                     &x->b_rayobs, &x->b_lev, &x->b_scal, &x->b_geo, &x->b_rad, &x->b_tau,

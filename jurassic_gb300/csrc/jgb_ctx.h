@@ -95,6 +95,7 @@ struct jgb_ctx {
   jgb::DevBuf los_off, los_cnt, los_cnt64, los_sft, los_ends, los_planes, lev_slopes, scan_tmp, err_word;
   jgb::DevBuf tiles_perm, tiles_keys, tiles_keys2, tiles_vals, tiles_off, tiles_len, tiles_data;
   jgb::DevBuf cloudf;   // mixed path: cloud extinction per (channel, ray)
+  jgb::DevBuf ext_sum;  // extinction sums per (window and cloud, ray)
   jgb::DevBuf inv_work;  // matrix_invert: descriptors, factors, their inverses
   jgb::DevBuf ne_desc, ne_split;  // normal equations: descriptors, operand blocks
   // finite-difference Jacobian: expanded batch and bookkeeping

@@ -94,6 +94,12 @@ struct MixedPlan {
   float* seg;
   int* stop;
   const float* cloud;   // [nd][nray] cloud extinction (-0: no cloud), nullptr: no clouds
+  // opaque rays (k_path_ends): sums along the rays of extinction x length per
+  // window and of cloud factor x length ([nw + 1][nray], nullptr: neither), and
+  // the points that a (tile, channel, lane) of the chunk walks (one lane per ray
+  // only; nullptr otherwise)
+  const float* ext_sum;
+  int* ends;
   // Resumed forward models (finite-difference perturbations), for channels
   // [gid0, gid0 + gndc): ray r starts at LOS point start[r], where its path
   // equals its base ray's.  A base ray saves its state for the rays snap_ray[k]
@@ -133,6 +139,10 @@ void launch_seg_scan_m(const CtlDev& c, const TblDev& T, const ChanDev& ch, cons
                        const LosDev& L, const MixedPlan& P, int longest, int res, cudaStream_t s);
 void launch_cloud_m(const CtlDev& c, const ChanDev& ch, const BatchDev& b, float* out,
                     cudaStream_t s);
+// opaque rays of the mixed path: sums per ray, then P.ends of a chunk
+void launch_ext_sums(const CtlDev& c, const LosDev& L, int nray, float* out, cudaStream_t s);
+void launch_path_ends(const CtlDev& c, const TblDev& T, const ChanDev& ch, const BatchDev& b,
+                      const LosDev& L, const MixedPlan& P, int res, cudaStream_t s);
 // FP32 channel constants of the path
 size_t chan_const_bytes(const CtlDev& c);
 void launch_chan_consts(const CtlDev& c, const ChanDev& ch, float* out, cudaStream_t s);

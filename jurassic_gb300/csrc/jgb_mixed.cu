@@ -698,6 +698,115 @@ __device__ __forceinline__ bool shared_gas(const MixedPlan& P, int r, int g) {
 }
 
 // ---------------------------------------------------------------------------
+// opaque rays
+//
+// Behind a thick cloud or window extinction a ray's path adds nothing (kTauStop),
+// but the emitters' kernel does not know the other factors of the ray's
+// transmittance.  The extinctions' optical depth depends on no emitter, and the
+// emitters' transmittances are at most 1: from the point where it reaches
+// kOpaqueDepth the transmittance is below 1e-13 (the CO2 continuum's
+// extrapolation to 100 K could take 0.1 off the depth, two segments that are
+// opaque by themselves and round to 1 a factor of 4), so that k_scan_m would have
+// stopped there or before.  8000 nadir observations x 50 channels x 5 emitters, 5
+// per km below 80, 40 and 20 km: 31.6, 31.3 and 31.5 ms without these ends, 8.6,
+// 20.3 and 27.0 with them; the kernel that held all emitters of a channel in a
+// warp and left at kTauStop took 11.1, 26.9 and 37.1, and 43.8 on clear scenes
+// (31.5 here).
+constexpr float kOpaqueDepth = 30.f;
+
+// Sums along every ray, a warp per ray: extinction x length of every window, then
+// cloud factor x length; -infinity where a value is negative (such a ray keeps
+// all its points).
+__global__ void __launch_bounds__(128) k_ext_sums(CtlDev c, LosDev L, int nray, float* out) {
+  const int lane = threadIdx.x & 31;
+  const long long r = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (r >= nray) return;
+  const int n = L.count[r];
+  const long long base = L.off[r];
+  for (int w = 0; w <= c.nw; w++) {
+    const float* k = (w < c.nw ? L.f.kw + w * L.cap : L.f.aux) + base;
+    float sum = 0.f;
+    bool negative = false;
+    if (w < c.nw || c.ncl > 0)
+      for (int ip = lane; ip < n; ip += 32) {
+        const float v = k[ip];
+        sum += v * L.f.ds[base + ip];
+        negative |= v < 0.f;
+      }
+    for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    negative = __any_sync(0xffffffffu, negative);
+    if (lane == 0) out[(long long)w * nray + r] = negative ? __int_as_float(0xff800000) : sum;
+  }
+}
+
+// Does the surface of ray r reflect in channel id?  Its sum needs every point.
+__device__ __forceinline__ bool reflects(const CtlDev& c, const ChanDev& ch, const BatchDev& b,
+                                         const LosDev& L, int r, int id) {
+  return c.sftype >= 2 && c.nsf > 0 && L.sft[r] > 0 && sfeps_of(c, ch, b, r, id) < 1.f;
+}
+
+// P.ends of a chunk, a warp per (tile, channel): the points that a lane walks, 0
+// where it is empty, skipped or masked.  A perturbed ray (RES 2) sums from its
+// start point on, and needs no point beyond it where its base was opaque there.
+template <int RES>
+__global__ void __launch_bounds__(128) k_path_ends(CtlDev c, TblDev T, ChanDev ch, BatchDev b,
+                                                   LosDev L, MixedPlan P) {
+  const int lane = threadIdx.x & 31, ndc = P.id1 - P.id0;
+  const long long w = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+  const int idl = (int)(w % ndc), tl = (int)(w / ndc);
+  if (tl >= P.tile1 - P.tile0) return;
+  const int tile = P.tile0 + tl, id = P.id0 + idl;
+  const int r = P.perm[tile * 32 + lane];
+  const int n = r >= 0 && !(b.obs_skip && b.obs_skip[b.ray_obs[r]]) &&
+                        !(b.skip_masked && b.mask[(long long)id * b.nray + r])
+                    ? L.count[r] : 0;
+  int start = 0, end = n;
+  if (RES == 2 && n > 0) {
+    start = P.start[r];
+    if (start > 0 && P.snap_sums[((long long)r * P.gndc + (id - P.gid0)) * 3 + 2] < kTauStop) end = start;
+  }
+  bool walk = false;
+  float cl = 0.f;
+  const Fields F = fields_of(c, P.brmask);
+  const int win = c.nw > 0 ? __float_as_int(T.chanf[id * kChanConsts + kChanWindow]) : -1;
+  if (P.ext_sum && n > 0 && end == n) {
+    if (P.cloud) cl = P.cloud[(long long)id * b.nray + r];
+    const float depth = (win >= 0 ? P.ext_sum[(long long)win * b.nray + r] : 0.f) +
+                        cl * P.ext_sum[(long long)c.nw * b.nray + r];
+    walk = depth >= kOpaqueDepth && !(cl < 0.f) && (RES != 0 || !reflects(c, ch, b, L, r, id));
+  }
+  if (__any_sync(0xffffffffu, walk)) {
+    const float* f = P.data + P.toff[tile] * (long long)F.n * 32 + lane;
+    const int kw = win >= 0 ? (F.kw0 + win) * 32 : -1;
+    float depth = 0.f;
+    int ip = (int)__reduce_min_sync(0xffffffffu, walk ? (unsigned)start : 0x7fffffffu);
+    const int last = (int)(P.toff[tile + 1] - P.toff[tile]) - 1;
+    const bool cloudy = P.cloud != nullptr;
+    constexpr int U = 8;  // points in flight: every lane loads, the walking ones use them
+    for (; __any_sync(0xffffffffu, walk); ip += U) {
+      float v[U], a[U], ds[U];
+#pragma unroll
+      for (int k = 0; k < U; k++) {
+        const float* q = f + (long long)min(ip + k, last) * F.n * 32;
+        v[k] = kw >= 0 ? q[kw] : 0.f;
+        a[k] = cloudy ? q[F.aux * 32] : 0.f;
+        ds[k] = q[F.ds * 32];
+      }
+#pragma unroll
+      for (int k = 0; k < U; k++) {
+        if (ip + k >= start && ip + k < n) depth += (v[k] + a[k] * cl) * ds[k];
+        if (walk && depth >= kOpaqueDepth) {
+          end = min(ip + k + 1, n);
+          walk = false;
+        }
+      }
+      walk = walk && ip + U < n;
+    }
+  }
+  P.ends[(long long)w * 32 + lane] = end;
+}
+
+// ---------------------------------------------------------------------------
 // the path of a batch, in three kernels
 //
 // k_gas_m: the emitters' paths are independent (one tau_path per emitter in
@@ -754,10 +863,16 @@ __global__ void __launch_bounds__(kPathThreads, MINB) k_gas_m(CtlDev c, TblDev T
   const int np = __ldg(T.np + dg);
   if (np < 30) return;  // no table: k_seg_m leaves this emitter out
   const int rl = LPR == 4 ? part8 * 8 + (lane >> 2) : lane, corner = lane & 3;
-  int r = P.perm[tile * 32 + rl];
-  if (r >= 0 && b.obs_skip && b.obs_skip[b.ray_obs[r]]) r = -1;
-  if (r >= 0 && b.skip_masked && b.mask[(long long)id * b.nray + r]) r = -1;
-  int n = r >= 0 ? L.count[r] : 0;
+  int r = 0, n = 0;
+  if (LPR == 1 && RES != 1) {
+    n = P.ends[(long long)(tl * ndc + idl) * 32 + rl];
+    if (RES == 2) r = P.perm[tile * 32 + rl];
+  } else {
+    r = P.perm[tile * 32 + rl];
+    if (r >= 0 && b.obs_skip && b.obs_skip[b.ray_obs[r]]) r = -1;
+    if (r >= 0 && b.skip_masked && b.mask[(long long)id * b.nray + r]) r = -1;
+    n = r >= 0 ? L.count[r] : 0;
+  }
   if (RES == 2 && n > 0 && shared_gas(P, r, g)) n = 0;
   const Fields F = fields_of(c, P.brmask);
   constexpr int es = kEmitterFields(CGA), kb = kFBr(CGA);
@@ -964,6 +1079,7 @@ __global__ void __launch_bounds__(kPathThreads) k_seg_m(CtlDev c, TblDev T, Batc
       has |= 1u << g;
       n = min(n, RES == 2 && !((own >> g) & 1u) ? bst[g * 32] : st[g * 32]);
     }
+  if (RES != 1 && P.ends) n = min(n, P.ends[(long long)(tl * ndc + idl) * 32 + lane]);
   if (RES == 2 && n <= start) return;
   const Fields F = fields_of(c, P.brmask);
   const long long pt = P.toff[tile] + ip0;
@@ -1049,6 +1165,7 @@ __global__ void __launch_bounds__(kPathThreads) k_scan_m(CtlDev c, TblDev T, Cha
       }
     }
   }
+  if (RES != 1 && P.ends && n > 0) n = min(n, P.ends[(long long)(tl * ndc + idl) * 32 + lane]);
   for (int g = 0; g < ng; g++)
     if (n > 0 && __ldg(T.np + (long long)id * ng + g) >= 30)
       n = min(n, RES == 2 && !((own >> g) & 1u) ? bst[g * 32] : st[g * 32]);
@@ -1067,8 +1184,7 @@ __global__ void __launch_bounds__(kPathThreads) k_scan_m(CtlDev c, TblDev T, Cha
   const float* seg = P.seg + ((P.toff[tile] - P.pt0) * ndc + idl) * (long long)P.nseg * 32 + lane +
                      (RES == 1 ? ng * 32 : 0);
   const long long step = (long long)ndc * P.nseg * 32;
-  const bool refl = RES == 0 && c.sftype >= 2 && c.nsf > 0 && L.sft[r] > 0 &&
-                    sfeps_of(c, ch, b, r, id) < 1.f;
+  const bool refl = RES == 0 && reflects(c, ch, b, L, r, id);
   constexpr int U = 8;  // loads in flight ahead of the sums
   for (; ip < n; ip += U) {
     if (tau < kTauStop && !refl) break;
@@ -1222,6 +1338,18 @@ void launch_cloud_m(const CtlDev& c, const ChanDev& ch, const BatchDev& b, float
                     cudaStream_t s) {
   const long long n = (long long)c.nd * b.nray;
   k_cloud_m<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(c, ch, b, out);
+}
+
+void launch_ext_sums(const CtlDev& c, const LosDev& L, int nray, float* out, cudaStream_t s) {
+  k_ext_sums<<<(unsigned)((nray + 3) / 4), 128, 0, s>>>(c, L, nray, out);
+}
+
+void launch_path_ends(const CtlDev& c, const TblDev& T, const ChanDev& ch, const BatchDev& b,
+                      const LosDev& L, const MixedPlan& P, int res, cudaStream_t s) {
+  const long long warps = (long long)(P.tile1 - P.tile0) * (P.id1 - P.id0);
+  const unsigned nblk = (unsigned)((warps + 3) / 4);
+  if (res == 2) k_path_ends<2><<<nblk, 128, 0, s>>>(c, T, ch, b, L, P);
+  else k_path_ends<0><<<nblk, 128, 0, s>>>(c, T, ch, b, L, P);
 }
 
 void launch_chan_consts(const CtlDev& c, const ChanDev& ch, float* out, cudaStream_t s) {

@@ -8,6 +8,8 @@
 //   k_tri_inverse      W = L^-1, one block per block column
 //   k_gram             A^-1 = W^T W, a tile pair per block, both triangles
 //
+// and invert_small for matrices of a tile or less, a warp each.
+//
 // What bounds it: n^3 / 2 FP64 multiply-adds per matrix at 19 cycles of an SM
 // per warp instruction (the tensor form of FP64 runs at the same rate).  A
 // block per matrix left 56 of 152 SMs idle for 96 matrices and spent two
@@ -23,7 +25,7 @@
 // from the sum over the tiles, quotients are correctly rounded.  Error against
 // inverses refined in long double, over the error of a block per matrix that
 // subtracted whole sums (geometric means, n from 12 to 405): covariances 1.06,
-// Gauss-Newton matrices 0.76.
+// Gauss-Newton matrices 0.76 (with the small matrices' solves 1.02 and 0.74).
 #include <algorithm>
 
 #include "../../include/jurassic_gb300.h"
@@ -44,7 +46,7 @@ struct Mat {
 
 __device__ __forceinline__ bool mat_at(const InvertDesc* d, const int* full, const int* status,
                                        double* Lall, double* Wall, int i, Mat& m) {
-  if (!full[i] || status[i]) return false;
+  if (!full[i] || status[i] || d[i].n <= kB) return false;
   m.n = d[i].n;
   m.L = Lall + d[i].off;
   m.W = Wall + d[i].off;
@@ -98,76 +100,136 @@ __device__ __forceinline__ double quotient(double a, double w, double r) {
   return __double2hiint(w) == 0x7ff00000 ? q : fma(fma(-q, w, a), r, q);
 }
 
-// Diagonal tile of panel k: lane r holds row r.  Every entry of the factor is (A -
-// sum) / L_jj with its sum formed apart and subtracted once, the sums over the
-// panels before it (S, where the factor will be) and over this tile's columns:
-// taking the products off A one by one rounds at the size of A every time and
-// made covariances' inverses 2.3 times as wrong.  Columns beyond the matrix are
-// those of the identity.
+// Cholesky factor of an n x n tile (n <= kB) by a warp: l holds the lower triangle of
+// A and receives the factor, rec its reciprocal diagonal; lane r holds row r.  An entry
+// is (A - sum) / L_jj with its sum formed apart and subtracted once: the sum over the
+// columns before the tile (s, if SUMS) and over the tile's own.  Taking the products
+// off A one by one rounds at the size of A every time and made covariances' inverses
+// 2.4 times as wrong.  The loops end at n: the FP64 instructions of a column (root,
+// reciprocal, products) are what a tile costs.  False: not positive definite.
+template <bool SUMS>
+__device__ __forceinline__ bool factor_tile(double (*l)[kB + 1], const double (*s)[kB + 1], int n,
+                                            double* rec) {
+  const int lane = threadIdx.x & 31;
+  double sum[kB];
+#pragma unroll
+  for (int c = 0; c < kB; c++) sum[c] = 0.0;
+#pragma unroll
+  for (int j = 0; j < kB; j++) {
+    if (j >= n) break;
+    double v = 0.0;
+    if (lane >= j && lane < n) v = l[lane][j] - (SUMS ? s[lane][j] + sum[j] : sum[j]);
+    const double dj = __shfl_sync(0xffffffffu, v, j);
+    if (!(dj > 0)) return false;
+    const double lj = sqrt(dj), rj = 1 / lj;
+    const double mine = lane > j ? quotient(v, lj, rj) : 0.0;
+    if (lane >= j) l[lane][j] = lane == j ? lj : mine;
+    if (lane == j) rec[j] = rj;
+#pragma unroll
+    for (int c = j + 1; c < kB; c++) {
+      if (c >= n) break;
+      sum[c] = fma(mine, __shfl_sync(0xffffffffu, mine, c), sum[c]);
+    }
+  }
+  __syncwarp();
+  return true;
+}
+
+// L x = e_c for lane c.
+__device__ __forceinline__ void forward_tile(const double (*l)[kB + 1], const double* rec, int n,
+                                             double (&x)[kB]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int r = 0; r < kB; r++) {
+    if (r >= n) break;
+    double t = 0.0;
+#pragma unroll
+    for (int q = 0; q < r; q++) t = fma(l[r][q], x[q], t);
+    x[r] = quotient((r == lane ? 1.0 : 0.0) - t, l[r][r], rec[r]);
+  }
+}
+
+// Inverse of a matrix of one tile or less by a warp: lane c solves for column c, and
+// the two triangles are averaged.  20000 matrices of 2 x 2, 8 x 8 and 32 x 32: 0.18,
+// 0.45 and 2.41 ms; by the kernels for several tiles, whose columns beyond the matrix
+// cost as much as its own then, 1.80, 3.02 and 3.24, with a block per matrix 0.82,
+// 2.57 and 14.3.
+__device__ __forceinline__ void invert_small(double* A, int n, double (*l)[kB + 1], double* rec,
+                                             int* status) {
+  const int lane = threadIdx.x;
+  for (int r = 0; r < n; r++) l[r][lane] = lane <= r ? A[r * n + lane] : 0.0;
+  __syncwarp();
+  if (!factor_tile<false>(l, nullptr, n, rec)) {
+    if (lane == 0) *status = 1;
+    return;
+  }
+  double x[kB];
+  forward_tile(l, rec, n, x);
+#pragma unroll
+  for (int r = kB - 1; r >= 0; r--) {  // L^T x = y
+    if (r >= n) continue;
+    double t = 0.0;
+#pragma unroll
+    for (int q = r + 1; q < kB; q++) {
+      if (q >= n) break;
+      t = fma(l[q][r], x[q], t);
+    }
+    x[r] = quotient(x[r] - t, l[r][r], rec[r]);
+  }
+  __syncwarp();
+#pragma unroll
+  for (int r = 0; r < kB; r++) {
+    if (r >= n) break;
+    l[r][lane] = x[r];
+  }
+  __syncwarp();
+  if (lane < n)
+    for (int r = 0; r < n; r++) A[r * n + lane] = 0.5 * (l[r][lane] + l[lane][r]);
+}
+
+__global__ void __launch_bounds__(32) k_invert_small(const InvertDesc* d, const int* full,
+                                                     int* status, double* Aall) {
+  __shared__ double l[kB][kB + 1], rec[kB];
+  const int i = blockIdx.x;
+  if (full[i]) invert_small(Aall + d[i].off, d[i].n, l, rec, status + i);
+}
+
+// Diagonal tile of panel k, a warp per matrix; S, the sums over the panels before,
+// lies where the factor goes.  The first panel's launch inverts the small matrices.
 __global__ void __launch_bounds__(32) k_chol_diag(const InvertDesc* d, const int* full, int* status,
-                                                  const double* Aall, double* Lall, double* Wall,
-                                                  int k) {
+                                                  double* Aall, double* Lall, double* Wall, int k) {
+  __shared__ double l[kB][kB + 1], s[kB][kB + 1], rec[kB];
   const int i = blockIdx.x, lane = threadIdx.x;
+  if (k == 0 && full[i] && d[i].n <= kB) {
+    invert_small(Aall + d[i].off, d[i].n, l, rec, status + i);
+    return;
+  }
   Mat m;
   if (!mat_at(d, full, status, Lall, Wall, i, m)) return;
   const int base = k * kB;
   if (base >= m.n) return;
   const int nb = min(kB, m.n - base);
-  __shared__ double a[kB][kB + 1], s[kB][kB + 1];
-  const double* A = Aall + d[i].off;
+  const double* A = Aall + d[i].off + (long long)base * (m.n + 1);
+  double* L = m.L + (long long)base * (m.n + 1);
+  double* W = m.W + (long long)base * (m.n + 1);
 #pragma unroll 16
-  for (int r = 0; r < kB; r++) {  // lanes along a row
-    const bool in = r < nb && lane <= r;
-    const long long e = (long long)(base + r) * m.n + base + lane;
-    a[r][lane] = in ? A[e] : (r == lane ? 1.0 : 0.0);
-    s[r][lane] = in && k > 0 ? m.L[e] : 0.0;
+  for (int r = 0; r < nb; r++) {
+    l[r][lane] = lane <= r ? A[(long long)r * m.n + lane] : 0.0;
+    s[r][lane] = lane <= r && k > 0 ? L[(long long)r * m.n + lane] : 0.0;
   }
   __syncwarp();
-  double row[kB], sum[kB];
-#pragma unroll
-  for (int c = 0; c < kB; c++) sum[c] = 0.0;
-  bool bad = false;
-  double diag = 1.0, recip = 1.0;  // this lane's diagonal entry and its reciprocal
-#pragma unroll
-  for (int j = 0; j < kB; j++) {
-    const double v = a[lane][j] - (s[lane][j] + sum[j]);
-    const double dj = __shfl_sync(0xffffffffu, v, j);
-    bad |= !(dj > 0);
-    const double lj = sqrt(dj), rj = 1 / lj;
-    if (lane == j) {
-      diag = lj;
-      recip = rj;
-    }
-    const double mine = lane > j ? quotient(v, lj, rj) : 0.0;
-    row[j] = lane == j ? lj : mine;
-#pragma unroll
-    for (int c = j + 1; c < kB; c++) {
-      const double lc = __shfl_sync(0xffffffffu, mine, c);
-      sum[c] = fma(mine, lc, sum[c]);
-    }
-  }
-  if (bad) {
+  if (!factor_tile<true>(l, s, nb, rec)) {
     if (lane == 0) status[i] = 1;
     return;
   }
-  if (lane < nb)
-#pragma unroll
-    for (int c = 0; c < kB; c++)
-      if (c <= lane) m.L[(long long)(base + lane) * m.n + base + c] = row[c];
-  // inverse of the tile: lane c solves for column c, L x = e_c
   double x[kB];
-#pragma unroll
-  for (int r = 0; r < kB; r++) {
-    double t = 0.0;
-#pragma unroll
-    for (int q = 0; q < r; q++) t = fma(__shfl_sync(0xffffffffu, row[q], r), x[q], t);
-    x[r] = quotient((r == lane ? 1.0 : 0.0) - t, __shfl_sync(0xffffffffu, diag, r),
-                    __shfl_sync(0xffffffffu, recip, r));
-  }
+  forward_tile(l, rec, nb, x);
+  for (int r = 0; r < nb; r++)
+    if (lane <= r) L[(long long)r * m.n + lane] = l[r][lane];
   if (lane < nb)
 #pragma unroll
     for (int r = 0; r < kB; r++)
-      if (r < nb && r >= lane) m.W[(long long)(base + r) * m.n + base + lane] = x[r];
+      if (r < nb && r >= lane) W[(long long)r * m.n + lane] = x[r];
 }
 
 // L_ik = (A - S)_ik L_kk^-T below the diagonal tile (L_kk^-1 in W; S, the sum over
@@ -304,6 +366,10 @@ __global__ void __launch_bounds__(kT) k_gram(const InvertDesc* d, const int* ful
 
 void matrix_invert_blocked(int nret, int nmax, const InvertDesc* d, const int* full, int* status,
                            double* A, double* L, double* W, cudaStream_t s) {
+  if (nmax <= kB) {
+    k_invert_small<<<nret, 32, 0, s>>>(d, full, status, A);
+    return;
+  }
   const int nt = (nmax + kB - 1) / kB;
   for (int k = 0; k < nt; k++) {
     const int below = nt - 1 - k;
@@ -313,7 +379,7 @@ void matrix_invert_blocked(int nret, int nmax, const InvertDesc* d, const int* f
       k_chol_update<<<dim3(below * (below + 1) / 2, nret), kT, 0, s>>>(d, full, status, L, W, k);
     }
   }
-  if (nt > 1) k_tri_inverse<<<dim3(nret, nt - 1), kT, 0, s>>>(d, full, status, L, W);
+  k_tri_inverse<<<dim3(nret, nt - 1), kT, 0, s>>>(d, full, status, L, W);
   k_gram<<<dim3(nt * (nt + 1) / 2, nret), kT, 0, s>>>(d, full, status, L, W, A);
 }
 

@@ -447,6 +447,7 @@ __global__ void __launch_bounds__(kNeThreads, 2) k_normal_tc(const NeDesc* desc,
 // still spreads over the SMs (91 blocks).  The blocks behind the tiles take b, a
 // thread per element.  512 problems of up to 150 x 405 take 7.5
 // ms instead of 28.0, one 0.074 instead of 0.175 (bound by the FP64 pipe).
+// Problems of up to kNe64 columns take k_normal_fp64_small.
 constexpr int kNe64 = 32, kNe64Threads = 256;
 
 __global__ void __launch_bounds__(kNe64Threads) k_normal_fp64(const NeDesc* desc, const double* Kall,
@@ -454,6 +455,7 @@ __global__ void __launch_bounds__(kNe64Threads) k_normal_fp64(const NeDesc* desc
                                                               double* Aall, double* ball) {
   __shared__ double xi[kNe64][kNe64 + 1], xj[kNe64][kNe64 + 1];
   const NeDesc d = desc[blockIdx.y];
+  if (d.n <= kNe64) return;
   const int nt = (d.n + kNe64 - 1) / kNe64, ntri = nt * (nt + 1) / 2;
   const int nb = (d.n + kNe64Threads - 1) / kNe64Threads, tid = threadIdx.x;
   const double* K = Kall + d.koff;
@@ -503,6 +505,55 @@ __global__ void __launch_bounds__(kNe64Threads) k_normal_fp64(const NeDesc* desc
   }
 }
 
+// The same for problems of one tile or less: a block per problem, a thread per entry
+// of the lower triangle and of b, so that few columns cost few multiply-adds (the
+// tile above forms all 1024).  Rows of [w K | K | w^2 dy] come kNe64 at a time
+// through shared memory.  1000 problems of 300 x 8 and 3000 x 3: 0.11 and 0.64 ms; in
+// tiles 0.69 and 6.57, with a thread per entry that read both factors from L2 0.27
+// and 1.63.  At the line: 200 x 32 here 0.23, 200 x 33 in tiles 0.70.
+__host__ __device__ inline int small_entries(int n) { return n * (n + 1) / 2 + n; }
+
+__global__ void k_normal_fp64_small(const NeDesc* desc, const double* Kall, const double* wall,
+                                    const double* dyall, double* Aall, double* ball) {
+  __shared__ double rows[kNe64 * (2 * kNe64 + 1)];
+  const NeDesc d = desc[blockIdx.x];
+  const int n = d.n, tid = threadIdx.x, stride = 2 * n + 1;
+  if (n > kNe64) return;
+  const double* K = Kall + d.koff;
+  const double* w = wall + d.moff;
+  const double* dy = dyall + d.moff;
+  const int ntri = n * (n + 1) / 2;
+  int i = (int)((sqrtf(8.f * tid + 1.f) - 1.f) * 0.5f);
+  if ((i + 1) * (i + 2) / 2 <= tid) i++;
+  if (i * (i + 1) / 2 > tid) i--;
+  const int j = tid < ntri ? tid - i * (i + 1) / 2 : tid - ntri;
+  double s = 0;
+  for (int k0 = 0; k0 < d.m; k0 += kNe64) {
+    const int kn = min(kNe64, d.m - k0);
+    __syncthreads();
+    for (int e = tid; e < kn * n; e += blockDim.x) {
+      const int k = e / n, c = e - k * n;
+      const double v = K[(long long)k0 * n + e];
+      rows[k * stride + c] = w[k0 + k] * v;
+      rows[k * stride + n + c] = v;
+    }
+    for (int k = tid; k < kn; k += blockDim.x)
+      rows[k * stride + 2 * n] = dy[k0 + k] * (w[k0 + k] * w[k0 + k]);
+    __syncthreads();
+    if (tid < ntri)
+      for (int k = 0; k < kn; k++) s = fma(rows[k * stride + i], rows[k * stride + j], s);
+    else if (tid < ntri + n)
+      for (int k = 0; k < kn; k++) s += rows[k * stride + n + j] * rows[k * stride + 2 * n];
+  }
+  if (tid < ntri) {
+    double* A = Aall + d.aoff;
+    A[i * n + j] = s;
+    A[j * n + i] = s;
+  } else if (tid < ntri + n) {
+    ball[d.boff + j] = s;
+  }
+}
+
 }  // namespace
 
 int normal_equations_dev(int nret, const int* m, const int* n, const double* K, const double* w,
@@ -513,7 +564,7 @@ int normal_equations_dev(int nret, const int* m, const int* n, const double* K, 
   // (one more entry holds the tensor-core kernel's error word)
   std::vector<NeDesc> hd(nret + 1);
   long long ko = 0, mo = 0, ao = 0, bo = 0, xo = 0, ntiles = 0;
-  int maxn = 0, maxblk = 0, nsel = 0;
+  int maxn = 0, maxsmall = 0, maxblk = 0, nsel = 0;  // maxsmall: largest n up to kNe64
   for (int i = 0; i < nret; i++) {
     if (!sel || sel[i]) {
       hd[nsel++] = NeDesc{m[i], n[i], ko, mo, ao, bo, xo, ntiles};
@@ -523,6 +574,7 @@ int normal_equations_dev(int nret, const int* m, const int* n, const double* K, 
       ntiles += (long long)nt * (nt + 1) / 2;
       maxblk = nblk > maxblk ? nblk : maxblk;
       maxn = n[i] > maxn ? n[i] : maxn;
+      if (n[i] <= kNe64) maxsmall = n[i] > maxsmall ? n[i] : maxsmall;
     }
     ko += (long long)m[i] * n[i];
     mo += m[i];
@@ -556,10 +608,15 @@ int normal_equations_dev(int nret, const int* m, const int* n, const double* K, 
     cudaMemcpyAsync(&herr, err, sizeof(herr), cudaMemcpyDeviceToHost, s);
     if (cudaStreamSynchronize(s) != cudaSuccess || herr) return JGB_ERR_CUDA;
   } else {
-    const long long nt = (maxn + kNe64 - 1) / kNe64;
-    const long long nblk = nt * (nt + 1) / 2 + (maxn + kNe64Threads - 1) / kNe64Threads;
-    dim3 grid((unsigned)(nblk < 4096 ? nblk : 4096), nsel);
-    k_normal_fp64<<<grid, kNe64Threads, 0, s>>>(static_cast<const NeDesc*>(desc_dev), K, w, dy, A, b);
+    const NeDesc* dd = static_cast<const NeDesc*>(desc_dev);
+    if (maxsmall > 0)
+      k_normal_fp64_small<<<nsel, (small_entries(maxsmall) + 31) / 32 * 32, 0, s>>>(dd, K, w, dy, A, b);
+    if (maxn > kNe64) {
+      const long long nt = (maxn + kNe64 - 1) / kNe64;
+      const long long nblk = nt * (nt + 1) / 2 + (maxn + kNe64Threads - 1) / kNe64Threads;
+      dim3 grid((unsigned)(nblk < 4096 ? nblk : 4096), nsel);
+      k_normal_fp64<<<grid, kNe64Threads, 0, s>>>(dd, K, w, dy, A, b);
+    }
   }
   return cudaGetLastError() == cudaSuccess ? JGB_OK : JGB_ERR_CUDA;
 }

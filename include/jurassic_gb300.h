@@ -163,6 +163,18 @@ int jgb_set_fov(jgb_ctx *ctx, int n, const double *dz, const double *w);
    results do not depend on it. */
 int jgb_set_los_bound_scale(jgb_ctx *ctx, double scale);
 
+/* Device memory of the path between its kernels.  A context keeps its workspaces
+   until it is destroyed: segments of a chunk of the batch, up to bytes (default
+   4 GiB, 0 restores it, at least 1 MiB) and an eighth, in FP64 also a quarter of
+   it for fields, in resumed Jacobians three times it.  Larger batches run in
+   more chunks.  Where the device has no room, a call gives the workspaces back and
+   goes on with a quarter of the limit, down to 64 MiB, which then stays the
+   context's limit.  Setting the limit gives the workspaces back.  The results do
+   not depend on it.  get: the limit in force, and the bytes held by the workspaces
+   and the tiles of line-of-sight points. */
+int jgb_set_path_workspace(jgb_ctx *ctx, unsigned long long bytes);
+int jgb_get_path_workspace(jgb_ctx *ctx, unsigned long long *limit, unsigned long long *held);
+
 /* Mixed-precision path of a batch too small to fill the device (at most 18 x
    SMs warps of tile x channel x emitter): four lanes per ray, one per corner of
    the p-T cell, walk an emitter's path instead of one.  mode -1 (the default)

@@ -435,18 +435,43 @@ int plan_tiles(jgb_ctx* x, int nray, const int* keys, const int* count, int ntil
   return JGB_OK;
 }
 
-// Workspace of the path between its kernels (segments of every point, channel
-// and emitter): a batch runs in chunks of tiles within it, of channels where
-// one tile alone would exceed it.  4 GiB is 1.4 % of the device and gives the
-// emitters' kernel tens of warps per scheduler.
-constexpr size_t kPathBytes = size_t(4) << 30;
+// Workspaces of the path between its kernels (segments of every point, channel and
+// emitter): a batch runs in chunks of tiles within the context's path_limit, of
+// channels where one tile alone would exceed it.  The results do not depend on
+// the chunks.
 
-// A workspace of that limit did not fit the device: try a quarter of it, down
-// to 64 MiB (results do not depend on the chunks).
-bool smaller_chunks(cudaError_t e, size_t limit) {
-  if (e != cudaErrorMemoryAllocation || limit <= (size_t(64) << 20)) return false;
-  (void)cudaGetLastError();
-  return true;
+// Gives the path's workspaces back (nothing in them outlives a call; fields:
+// also tiles_data, while it holds nothing).
+void release_path(jgb_ctx* x, bool fields) {
+  x->seg.release();
+  x->rs_seg.release();
+  x->rs_snap.release();
+  if (fields) x->tiles_data.release();
+}
+
+// Reserves a chunk plan's workspaces, reserve(limit): where the device has no room
+// for them, from empty workspaces, then with a quarter of the limit, down to 64 MiB
+// (or the caller's own limit).  What fitted stays the context's limit.
+constexpr size_t kMinPathBytes = size_t(64) << 20;
+
+template <typename F>
+int reserve_path(jgb_ctx* x, bool fields, F reserve) {
+  for (bool empty = false;; empty = true) {
+    const cudaError_t e = reserve(x->path_limit);
+    if (e == cudaSuccess) return JGB_OK;
+    if (e != cudaErrorMemoryAllocation || (empty && x->path_limit <= kMinPathBytes))
+      return fail(x, JGB_ERR_CUDA, std::string("path workspaces: ") + cudaGetErrorString(e));
+    release_path(x, fields);
+    if (empty) x->path_limit = std::max(x->path_limit / 4, kMinPathBytes);
+  }
+}
+
+// Any other buffer of the call: the path's workspaces make room for it.
+cudaError_t reserve_first(jgb_ctx* x, DevBuf& buf, size_t bytes, bool fields) {
+  cudaError_t e = buf.reserve(bytes);
+  if (e != cudaErrorMemoryAllocation) return e;
+  release_path(x, fields);
+  return buf.reserve(bytes);
 }
 
 struct PathChunk {
@@ -456,8 +481,9 @@ struct PathChunk {
 };
 
 // point_bytes, chan_bytes: workspace of a tile point, and of one per channel;
-// tile_bytes: of a (tile, channel).  The largest needs in *need_points (limited
-// to a quarter of limit) and *need_chan (limited to limit).
+// tile_bytes: of a (tile, channel), which bounds the tiles of rays without points.
+// The largest needs in *need_points (limited to a quarter of limit) and *need_chan
+// (limited to limit).
 void path_chunks(const std::vector<long long>& toff, int tfirst, int nd, size_t limit,
                  size_t point_bytes, size_t chan_bytes, size_t tile_bytes, std::vector<PathChunk>& out,
                  size_t* need_points, size_t* need_chan) {
@@ -465,15 +491,17 @@ void path_chunks(const std::vector<long long>& toff, int tfirst, int nd, size_t 
   for (int t = tfirst; t < ntile;) {
     PathChunk k{t, t, nd, 0};
     auto pts = [&](int t1) { return (size_t)(toff[t1] - toff[k.t0]); };
+    auto per_chan = [&](int t1) {
+      return std::max<size_t>(pts(t1), 1) * chan_bytes + (size_t)(t1 - k.t0) * tile_bytes;
+    };
     do {
       k.longest = std::max(k.longest, (int)(toff[k.t1 + 1] - toff[k.t1]));
       k.t1++;
     } while (k.t1 < ntile && k.t1 - k.t0 < 65535 && pts(k.t1 + 1) * point_bytes <= limit / 4 &&
-             pts(k.t1 + 1) * nd * chan_bytes <= limit);
-    const size_t np = std::max<size_t>(pts(k.t1), 1);
-    if (np * nd * chan_bytes > limit) k.ndc = (int)std::max<size_t>(limit / (np * chan_bytes), 1);
-    if (need_points) *need_points = std::max(*need_points, np * point_bytes);
-    *need_chan = std::max(*need_chan, np * k.ndc * chan_bytes + (size_t)(k.t1 - k.t0) * k.ndc * tile_bytes);
+             per_chan(k.t1 + 1) * nd <= limit);
+    k.ndc = (int)std::min<size_t>(nd, std::max<size_t>(limit / per_chan(k.t1), 1));
+    if (need_points) *need_points = std::max(*need_points, std::max<size_t>(pts(k.t1), 1) * point_bytes);
+    *need_chan = std::max(*need_chan, per_chan(k.t1) * k.ndc);
     out.push_back(k);
     t = k.t1;
   }
@@ -538,18 +566,15 @@ int run_path64(jgb_ctx* x, const BatchDev& b, const LosDev& L, cudaStream_t s, i
   path64_point_bytes(c, &bfd, &bfu);
   const size_t bch = 32 * sizeof(double) * (size_t)(c.ng + 2);  // per (point, channel)
   std::vector<PathChunk> chunks;
-  for (size_t limit = kPathBytes;; limit /= 4) {
+  rc = reserve_path(x, true, [&](size_t limit) {
     chunks.clear();
     size_t need_f = 0, need_w = 0;
     path_chunks(toff, 0, c.nd, limit, bfd + bfu, bch, 32 * sizeof(int) * (size_t)std::max(c.ng, 1),
                 chunks, &need_f, &need_w);
-    cudaError_t e = x->tiles_data.reserve(need_f);
-    if (e == cudaSuccess) e = x->seg.reserve(need_w);
-    if (!smaller_chunks(e, limit)) {
-      CK(e);
-      break;
-    }
-  }
+    const cudaError_t e = x->tiles_data.reserve(need_f);
+    return e == cudaSuccess ? x->seg.reserve(need_w) : e;
+  });
+  if (rc) return rc;
   CK(cudaEventRecord(x->ev[4], s));
   Path64 P{};
   P.perm = Pm.perm;
@@ -683,12 +708,12 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
     const size_t plane_bytes = precision == JGB_MIXED
                                    ? (sizeof(double) + sizeof(float) * nplanes) * (size_t)cap
                                    : sizeof(double) * (size_t)cap * nplanes;
-    if (mode == kBound && x->los_planes.reserve(plane_bytes) == cudaErrorMemoryAllocation) {
-      (void)cudaGetLastError();  // the exact counts may still fit
-      mode = kCount;
+    const cudaError_t fits = reserve_first(x, x->los_planes, plane_bytes, true);
+    if (mode == kBound && fits == cudaErrorMemoryAllocation) {
+      mode = kCount;  // the exact counts may still fit
       continue;
     }
-    CK(x->los_planes.reserve(plane_bytes));
+    CK(fits);
     double* P = x->los_planes.as<double>();
     if (precision == JGB_MIXED) {  // z in FP64, the point data in FP32 planes
       float* F = reinterpret_cast<float*>(P + cap);
@@ -734,7 +759,7 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
       const size_t o_plan = o_lev + a16(sizeof(int) * (size_t)bpts);
       const size_t o_key = o_plan + a16(sizeof(int4) * (size_t)nray);
       const size_t nk = (size_t)std::max(npr, 1);
-      CK(x->rs_trace.reserve(o_key + 4 * a16(sizeof(int) * nk)));
+      CK(reserve_first(x, x->rs_trace, o_key + 4 * a16(sizeof(int) * nk), true));
       char* tb = x->rs_trace.as<char>();
       TraceResume R{};
       R.bpts = bpts;
@@ -816,7 +841,7 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
   // with a field of view the path kernels write pencil beams to scratch
   BatchDev bo = b;
   if (c.fov) {
-    CK(x->fov_raw.reserve(sizeof(double) * 2 * (size_t)c.nd * nray));
+    CK(reserve_first(x, x->fov_raw, sizeof(double) * 2 * (size_t)c.nd * nray, true));
     bo.rad = x->fov_raw.as<double>();
     bo.tau = bo.rad + (size_t)c.nd * nray;
   }
@@ -1014,13 +1039,14 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
     Pm.brmask = x->grid_mask;
     Pm.fast = !x->odd_rows && x->grid_mask == (1u << c.ng) - 1u;
     Pm.nfield = mixed_nfield(c, Pm.brmask);
-    CK(x->tiles_data.reserve(sizeof(float) * 32 * (size_t)std::max(tile_points, 1LL) * Pm.nfield));
+    CK(reserve_first(x, x->tiles_data, sizeof(float) * 32 * (size_t)std::max(tile_points, 1LL) * Pm.nfield,
+                     false));
     Pm.data = x->tiles_data.as<float>();
     Pm.start = rs ? rstart : nullptr;
     launch_pack_tiles_n(c, tbl_view(x), L, Pm, tile_points, s);
     CK(cudaGetLastError());
     if (c.ncl > 0) {
-      CK(x->cloudf.reserve(sizeof(float) * (size_t)c.nd * nray));
+      CK(reserve_first(x, x->cloudf, sizeof(float) * (size_t)c.nd * nray, false));
       launch_cloud_m(c, ch, bo, x->cloudf.as<float>(), s);
       Pm.cloud = x->cloudf.as<float>();
       launches += 1;
@@ -1038,7 +1064,7 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
     if (rs) {
       // The bases (saving the states), then the perturbations (starting from
       // them), for groups of channels whose base segments, states and the
-      // perturbations' segments each stay within kPathBytes.
+      // perturbations' segments each stay within the limit.
       const size_t np = (size_t)std::max(toff_h[tfirst], 1LL);
       const int bseg = c.ng + 2;  // the emitters of a base's segments outlive its sums
       const size_t b_seg = 32 * sizeof(float) * np * bseg;
@@ -1059,7 +1085,7 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
       const std::vector<long long> toff_own(toff_h.begin(), toff_h.begin() + tsecond + 1);
       int gnd = 1;
       size_t o_stop = 0, o_slot = 0, o_reuse = 0;
-      for (size_t limit = kPathBytes;; limit /= 4) {
+      const int fits = reserve_path(x, false, [&](size_t limit) {
         gnd = (int)std::min<size_t>(c.nd, std::max<size_t>(limit / per, 1));
         o_stop = a16(b_seg * gnd);
         o_slot = o_stop + a16(b_stop * gnd);
@@ -1072,12 +1098,9 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
         }
         cudaError_t e = x->rs_seg.reserve(o_reuse + sizeof(int2) * (size_t)nray);
         if (e == cudaSuccess) e = x->rs_snap.reserve(a16(b_state * gnd) + b_sums * gnd);
-        if (e == cudaSuccess) e = x->seg.reserve(need);
-        if (!smaller_chunks(e, limit)) {
-          CK(e);
-          break;
-        }
-      }
+        return e == cudaSuccess ? x->seg.reserve(need) : e;
+      });
+      if (fits) return fits;
       char* sp = x->rs_seg.as<char>();
       int* slot = reinterpret_cast<int*>(sp + o_slot);
       k_base_slots<<<(tfirst * 32 + 127) / 128, 128, 0, s>>>(tfirst * 32, Pm.perm, slot);
@@ -1143,21 +1166,18 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
       x->stats.resume_skip = resume_skip;
     } else {
       Pm.nseg = std::max(c.ng, 2);
-      // chunks of tiles whose segments stay within kPathBytes (and of channels
+      // chunks of tiles whose segments stay within the limit (and of channels
       // where one tile alone would not)
       const size_t bch = 32 * sizeof(float) * (size_t)Pm.nseg;
       std::vector<PathChunk> chunks;
-      for (size_t limit = kPathBytes;; limit /= 4) {
+      const int fits = reserve_path(x, false, [&](size_t limit) {
         chunks.clear();
         size_t need = 0;
         path_chunks(toff_h, 0, c.nd, limit, 0, bch, 32 * sizeof(int) * (size_t)(c.ng + 1), chunks,
                     nullptr, &need);
-        const cudaError_t e = x->seg.reserve(need);
-        if (!smaller_chunks(e, limit)) {
-          CK(e);
-          break;
-        }
-      }
+        return x->seg.reserve(need);
+      });
+      if (fits) return fits;
       bool timed = false;
       for (const PathChunk& k : chunks) {
         Pm.tile0 = k.t0;
@@ -1876,6 +1896,23 @@ int jgb_set_fd_resume(jgb_ctx* x, int mode) {
   jgb::CtxLock lock(x);
   if (!x || mode < 0 || mode > 3) return fail(x, JGB_ERR_ARG, "bad resume setting");
   x->fd_resume = mode;
+  return JGB_OK;
+}
+
+int jgb_set_path_workspace(jgb_ctx* x, unsigned long long bytes) {
+  jgb::CtxLock lock(x);
+  if (!x || (bytes && bytes < (1ULL << 20))) return fail(x, JGB_ERR_ARG, "workspace below 1 MiB");
+  x->path_limit = bytes ? (size_t)bytes : kPathBytes;
+  cudaSetDevice(x->device);
+  release_path(x, true);
+  return JGB_OK;
+}
+
+int jgb_get_path_workspace(jgb_ctx* x, unsigned long long* limit, unsigned long long* held) {
+  jgb::CtxLock lock(x);
+  if (!x) return JGB_ERR_ARG;
+  if (limit) *limit = x->path_limit;
+  if (held) *held = x->seg.n + x->rs_seg.n + x->rs_snap.n + x->tiles_data.n;
   return JGB_OK;
 }
 

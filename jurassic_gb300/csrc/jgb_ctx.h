@@ -13,6 +13,10 @@
 
 namespace jgb {
 
+// Default of a context's path_limit: 1.4 % of the device, and tens of warps per
+// scheduler for the emitters' kernel of the mixed path.
+constexpr size_t kPathBytes = size_t(4) << 30;
+
 // Grow-only device buffer.
 struct DevBuf {
   void* p = nullptr;
@@ -26,9 +30,17 @@ struct DevBuf {
     if (p) cudaFree(p);
     p = nullptr;
     n = 0;
-    const size_t want = bytes + bytes / 8;  // headroom for slightly larger batches
+    size_t want = bytes + bytes / 8;  // headroom for slightly larger batches
     cudaError_t e = cudaMalloc(&p, want);
-    if (e == cudaSuccess) n = want;
+    if (e == cudaErrorMemoryAllocation) {  // without it
+      e = cudaMalloc(&p, want = bytes);
+    }
+    if (e == cudaSuccess) {
+      n = want;
+    } else {
+      p = nullptr;
+      (void)cudaGetLastError();  // reported here, not by the next call's check
+    }
     return e;
   }
   template <typename T>
@@ -118,7 +130,12 @@ struct jgb_ctx {
   // retrieval engines made from this context (detached by jgb_destroy)
   std::vector<jgb_engine*> engines;
   int sms = 152;          // multiprocessors of the device
-  jgb::DevBuf seg;        // workspace of the path between its kernels
+  // workspaces of the path between its kernels: seg, for resumed perturbations
+  // also rs_seg and rs_snap, each up to path_limit; FP64 fields in tiles_data up
+  // to a quarter of it.  An allocation that fails lowers the limit for the calls
+  // that follow.
+  jgb::DevBuf seg;
+  size_t path_limit = jgb::kPathBytes;
   std::vector<float> tune_ms;
   jgb_stats stats{};
   std::string err;

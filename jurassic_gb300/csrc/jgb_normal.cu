@@ -712,17 +712,16 @@ extern "C" int jgb_normal_equations_dev(jgb_ctx* x, int nret, const int* m, cons
   void* ddesc = x->ne_desc.p;
   cudaEvent_t e0 = x->ev[0], e1 = x->ev[1];
   cudaStream_t s = v.stream;
-  // descriptors are uploaded (and the stream synchronised) inside; the
-  // events bracket the kernel launch that follows
   rc = normal_equations_dev(nret, m, n, K, w, dy, A, b, precision, nullptr, ddesc, x->ne_split, s);
-  // time a second identical launch only when asked: the first one above
-  // included the descriptor upload
+  // time a second identical call only when asked: the first one may have grown
+  // the buffers
   if (rc == JGB_OK && kernel_ms) {
     cudaEventRecord(e0, s);
     rc = normal_equations_dev(nret, m, n, K, w, dy, A, b, precision, nullptr, ddesc, x->ne_split, s);
     cudaEventRecord(e1, s);
   }
   if (cudaStreamSynchronize(s) != cudaSuccess) rc = JGB_ERR_CUDA;
+  if (x->ne_split.n > x->path_limit) x->ne_split.release();  // large scratch is not kept
   if (rc == JGB_OK && kernel_ms) cudaEventElapsedTime(kernel_ms, e0, e1);
   return rc ? ctx_fail(x, rc, "normal-equation kernel failed") : JGB_OK;
 }

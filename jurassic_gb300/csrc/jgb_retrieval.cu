@@ -1894,6 +1894,7 @@ extern "C" int jgb_matrix_invert_dev(jgb_ctx* x, int nret, const int* n, double*
   if (err == cudaSuccess) err = cudaStreamSynchronize(s);
   if (err == cudaSuccess && kernel_ms) cudaEventElapsedTime(kernel_ms, e0, e1);
   if (err == cudaSuccess && status) std::memcpy(status, hst.data(), sizeof(int) * nret);
+  if (x->inv_work.n > x->path_limit) x->inv_work.release();  // large scratch is not kept
   if (err != cudaSuccess)
     return ctx_error(x, JGB_ERR_CUDA,
                      std::string("matrix inversion kernels: ") + cudaGetErrorString(err));

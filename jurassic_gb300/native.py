@@ -122,6 +122,8 @@ SIGNATURES = {
     "jgb_set_fov": (C.c_int, [C.c_void_p, C.c_int, _dp, _dp]),
     "jgb_set_los_bound_scale": (C.c_int, [C.c_void_p, C.c_double]),
     "jgb_set_path_split": (C.c_int, [C.c_void_p, C.c_int]),
+    "jgb_set_path_workspace": (C.c_int, [C.c_void_p, C.c_ulonglong]),
+    "jgb_get_path_workspace": (C.c_int, [C.c_void_p, C.POINTER(C.c_ulonglong), C.POINTER(C.c_ulonglong)]),
     "jgb_set_fd_resume": (C.c_int, [C.c_void_p, C.c_int]),
     "jgb_set_srcfunc": (C.c_int, [C.c_void_p, _dp]),
     "jgb_get_srcfunc": (C.c_int, [C.c_void_p, _dp, _dp]),
@@ -247,6 +249,17 @@ class Context:
         """Four lanes per ray in the mixed path: -1 for batches too small to
         fill the device (default), 0 never, 1 always."""
         self._check(load().jgb_set_path_split(self.h, int(mode)))
+
+    def set_path_workspace(self, nbytes: int):
+        """Limit of the path's workspaces on the device (0: the default, 4 GiB);
+        gives the present ones back.  The results do not depend on it."""
+        self._check(load().jgb_set_path_workspace(self.h, int(nbytes)))
+
+    def path_workspace(self):
+        """(limit in force, bytes held) of the path's workspaces."""
+        a, b = C.c_ulonglong(), C.c_ulonglong()
+        self._check(load().jgb_get_path_workspace(self.h, C.byref(a), C.byref(b)))
+        return a.value, b.value
 
     def set_fd_resume(self, mode: int):
         """Resume perturbed paths of mixed Jacobians from their base's saved

@@ -190,7 +190,7 @@ __global__ void k_iota(int n, int* v, int from = 0) {
 // a tile; nsecond = nfirst, tsecond = tfirst: two; nfirst = nray, tfirst =
 // ntile: one)
 __global__ void k_tiles(int nray, int ntile, int nfirst, int tfirst, int nsecond, int tsecond,
-                        const int* count, const int* sorted_ray, int* perm, int* tlen,
+                        const int* count, const int* sorted_ray, int* perm,
                         long long* tpts) {
   const int tile = blockIdx.x * blockDim.x + threadIdx.x;
   if (tile >= ntile) return;
@@ -211,7 +211,6 @@ __global__ void k_tiles(int nray, int ntile, int nfirst, int tfirst, int nsecond
     perm[tile * 32 + l] = k < k1 ? sorted_ray[k] : -1;
     if (k < k1) mx = max(mx, count[sorted_ray[k]]);
   }
-  tlen[tile] = mx;
   tpts[tile] = mx;
 }
 
@@ -401,7 +400,6 @@ int plan_tiles(jgb_ctx* x, int nray, const int* keys, const int* count, int ntil
   CK(x->tiles_keys2.reserve(sizeof(int) * (size_t)nray));
   CK(x->tiles_vals.reserve(sizeof(int) * 2 * (size_t)nray));
   CK(x->tiles_perm.reserve(sizeof(int) * 32 * (size_t)ntile));
-  CK(x->tiles_len.reserve(sizeof(int) * (size_t)ntile));
   CK(x->tiles_off.reserve(sizeof(long long) * (size_t)(2 * ntile + 2)));
   int* vals_in = x->tiles_vals.as<int>();
   int* vals_out = vals_in + nray;
@@ -419,12 +417,11 @@ int plan_tiles(jgb_ctx* x, int nray, const int* keys, const int* count, int ntil
   }
   P.ntile = ntile;
   P.perm = x->tiles_perm.as<int>();
-  P.tlen = x->tiles_len.as<int>();
   P.toff = toff;
   P.tile0 = 0;
   P.tile1 = ntile;
   k_tiles<<<(ntile + 127) / 128, 128, 0, s>>>(nray, ntile, nfirst, tfirst, nsecond, tsecond, count,
-                                               sorted ? vals_out : vals_in, P.perm, P.tlen, tpts);
+                                               sorted ? vals_out : vals_in, P.perm, tpts);
   CK(cudaMemsetAsync(toff, 0, sizeof(long long), s));
   cub::DeviceScan::InclusiveSum(nullptr, sb2, tpts, toff + 1, ntile, s);
   CK(x->scan_tmp.reserve(std::max(sb, sb2) + 16));
@@ -1038,7 +1035,7 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
     const long long tile_points = toff_h[ntile];
     Pm.brmask = x->grid_mask;
     Pm.fast = !x->odd_rows && x->grid_mask == (1u << c.ng) - 1u;
-    Pm.nfield = mixed_nfield(c, Pm.brmask);
+    Pm.nfield = mixed_nfield(c);
     CK(reserve_first(x, x->tiles_data, sizeof(float) * 32 * (size_t)std::max(tile_points, 1LL) * Pm.nfield,
                      false));
     Pm.data = x->tiles_data.as<float>();
@@ -1774,7 +1771,7 @@ void jgb_destroy(jgb_ctx* x) {
                     &x->b_tp, &x->b_mask, &x->b_p, &x->los_off, &x->los_cnt, &x->los_cnt64,
                     &x->los_sft, &x->los_ends, &x->los_planes, &x->lev_slopes, &x->scan_tmp, &x->err_word,
                     &x->tiles_perm, &x->tiles_keys, &x->tiles_keys2, &x->tiles_vals,
-                    &x->tiles_off, &x->tiles_len, &x->tiles_data, &x->inv_work, &x->ne_desc, &x->ne_split, &x->seg,
+                    &x->tiles_off, &x->tiles_data, &x->inv_work, &x->ne_desc, &x->ne_split, &x->seg,
                     &x->rs_start, &x->rs_lists, &x->rs_snap, &x->rs_base, &x->rs_seg, &x->rs_trace,
                     &x->d_fov, &x->fov_raw,
                     &x->kx_levoff, &x->kx_rayoff, &x->kx_rayobs, &x->kx_src, &x->kx_lev,

@@ -105,7 +105,7 @@ struct jgb_ctx {
   // per-call scratch
   jgb::DevBuf b_levoff, b_rayoff, b_rayobs, b_lev, b_scal, b_geo, b_rad, b_tau, b_tp, b_mask, b_p;
   jgb::DevBuf los_off, los_cnt, los_cnt64, los_sft, los_ends, los_planes, lev_slopes, scan_tmp, err_word;
-  jgb::DevBuf tiles_perm, tiles_keys, tiles_keys2, tiles_vals, tiles_off, tiles_len, tiles_data;
+  jgb::DevBuf tiles_perm, tiles_keys, tiles_keys2, tiles_vals, tiles_off, tiles_data;
   jgb::DevBuf cloudf;   // mixed path: cloud extinction per (channel, ray)
   jgb::DevBuf ext_sum;  // extinction sums per (window and cloud, ray)
   jgb::DevBuf inv_work;  // matrix_invert: descriptors, factors, their inverses
@@ -121,8 +121,8 @@ struct jgb_ctx {
   double los_bound_scale = 1.0;  // factor on the per-ray LOS bound (0: count first)
   int path_split = -1;    // four lanes per ray in the mixed path: -1 small batches, 0 never, 1 always
   int fd_resume = 1;      // resume perturbed paths from their base's state: 0 never,
-                          // 1 when the estimated schedule is shorter, 2 always,
-                          // 3 always and with the emitters shared with the base
+                          // 1 when the estimated schedule is shorter, 2 and 3
+                          // (its alias) always
   const ResumeSpec* resume = nullptr;  // set by fd_core for the run_core call it makes
   jgb::DevBuf rs_start, rs_lists, rs_snap, rs_base, rs_seg;
   // resumed tracing: the base rays' walks and the perturbed rays' plan

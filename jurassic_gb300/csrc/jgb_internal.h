@@ -78,7 +78,6 @@ struct MixedPlan {
   int ntile;
   int* perm;            // [ntile*32]
   long long* toff;      // [ntile+1]
-  int* tlen;            // [ntile]
   float* data;          // tile planes
   int nfield;
   unsigned brmask;      // emitters with p-T brackets precomputed per LOS point
@@ -126,7 +125,7 @@ struct MixedPlan {
   int base_nseg;
   int gstep;  // perturbations: emitter g in entry g * gstep (0: a tile's one emitter)
 };
-int mixed_nfield(const CtlDev& c, unsigned brmask);
+int mixed_nfield(const CtlDev& c);
 void launch_pack_tiles_n(const CtlDev& c, const TblDev& T, const LosDev& L, const MixedPlan& P,
                          long long total_tile_points, cudaStream_t s);
 // the path of a chunk: the emitters' paths (lanes_per_ray 1 or 4; variant:
@@ -149,7 +148,6 @@ void launch_chan_consts(const CtlDev& c, const ChanDev& ch, float* out, cudaStre
 // bytes of an emitter's saved path state
 size_t gas_state_bytes();
 void launch_src_to_float(int nd, const double* sr, float* srf, cudaStream_t s);
-void launch_tables_to_float(long long n, const double* src, float* dst, cudaStream_t s);
 void launch_rowmeta(long long nrow, int tu, const int* nu, const float* u, const float* e, int cga,
                     float4* meta, float2* ue, int* any_odd, cudaStream_t s);
 

@@ -47,8 +47,7 @@ constexpr int kFCgp = 1, kFCgt = 2, kFCgu = 3;  // CGA means
 __host__ __device__ constexpr int kEmitterFields(bool cga) { return cga ? 8 : 5; }
 __host__ __device__ constexpr int kFBr(bool cga) { return cga ? 4 : 1; }  // then pw, wa, wb
 
-__host__ __device__ inline Fields fields_of(const CtlDev& c, unsigned brmask) {
-  (void)brmask;
+__host__ __device__ inline Fields fields_of(const CtlDev& c) {
   Fields f;
   f.p = 0;
   f.t = 1;
@@ -62,7 +61,7 @@ __host__ __device__ inline Fields fields_of(const CtlDev& c, unsigned brmask) {
   return f;
 }
 
-int mixed_nfield(const CtlDev& c, unsigned brmask) { return fields_of(c, brmask).n; }
+int mixed_nfield(const CtlDev& c) { return fields_of(c).n; }
 
 constexpr unsigned kNoBracket = 0x80000000u;
 
@@ -298,7 +297,7 @@ __global__ void k_pack_tiles(CtlDev c, TblDev T, LosDev L, MixedPlan P, long lon
   const int tile = lo;
   const int ip = (int)(tp - P.toff[tile]);
   const int r = P.perm[tile * 32 + lane];
-  const Fields F = fields_of(c, P.brmask);
+  const Fields F = fields_of(c);
   float* out = P.data + tp * (long long)F.n * 32 + lane;
   if (r < 0 || ip >= L.count[r] || (P.start && ip < P.start[r])) return;  // never read
   const long long q = L.off[r] + ip;
@@ -767,7 +766,7 @@ __global__ void __launch_bounds__(128) k_path_ends(CtlDev c, TblDev T, ChanDev c
   }
   bool walk = false;
   float cl = 0.f;
-  const Fields F = fields_of(c, P.brmask);
+  const Fields F = fields_of(c);
   const int win = c.nw > 0 ? __float_as_int(T.chanf[id * kChanConsts + kChanWindow]) : -1;
   if (P.ext_sum && n > 0 && end == n) {
     if (P.cloud) cl = P.cloud[(long long)id * b.nray + r];
@@ -874,7 +873,7 @@ __global__ void __launch_bounds__(kPathThreads, MINB) k_gas_m(CtlDev c, TblDev T
     n = r >= 0 ? L.count[r] : 0;
   }
   if (RES == 2 && n > 0 && shared_gas(P, r, g)) n = 0;
-  const Fields F = fields_of(c, P.brmask);
+  const Fields F = fields_of(c);
   constexpr int es = kEmitterFields(CGA), kb = kFBr(CGA);
   const float* f = P.data + P.toff[tile] * (long long)F.n * 32 + rl;
   const float* fg = f + (F.g0 + g * es) * 32;
@@ -1081,7 +1080,7 @@ __global__ void __launch_bounds__(kPathThreads) k_seg_m(CtlDev c, TblDev T, Batc
     }
   if (RES != 1 && P.ends) n = min(n, P.ends[(long long)(tl * ndc + idl) * 32 + lane]);
   if (RES == 2 && n <= start) return;
-  const Fields F = fields_of(c, P.brmask);
+  const Fields F = fields_of(c);
   const long long pt = P.toff[tile] + ip0;
   const float* f = P.data + pt * F.n * 32 + lane;
   float* seg = P.seg + ((pt - P.pt0) * ndc + idl) * (long long)P.nseg * 32 + lane;
@@ -1267,11 +1266,6 @@ __global__ void k_src_to_float(int nd, const double* sr, float* srf) {
   srf[gid] = (float)sr[(long long)it * nd + id];
 }
 
-__global__ void k_to_float(long long n, const double* src, float* dst) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) dst[i] = (float)src[i];
-}
-
 void launch_pack_tiles_n(const CtlDev& c, const TblDev& T, const LosDev& L, const MixedPlan& P,
                          long long total_tile_points, cudaStream_t s) {
   const long long nth = total_tile_points * 32;
@@ -1363,11 +1357,6 @@ size_t gas_state_bytes() { return sizeof(unsigned) * kStateWords; }
 void launch_src_to_float(int nd, const double* sr, float* srf, cudaStream_t s) {
   const int n = nd * kNS, bs = 256;
   k_src_to_float<<<(n + bs - 1) / bs, bs, 0, s>>>(nd, sr, srf);
-}
-
-void launch_tables_to_float(long long n, const double* src, float* dst, cudaStream_t s) {
-  const int bs = 256;
-  if (n > 0) k_to_float<<<(unsigned)((n + bs - 1) / bs), bs, 0, s>>>(n, src, dst);
 }
 
 }  // namespace jgb

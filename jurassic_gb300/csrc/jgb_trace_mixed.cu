@@ -213,10 +213,10 @@ __device__ __forceinline__ void level_values(const CtlDev& c, const AtmM& a, int
 
 // Per-thread shared memory of the fill pass, stride kTraceThreads: the
 // current level's emitter and window values and slopes (qc[k], qc[nqk + k],
-// nqk = ng + nw), the mixing ratios of the point waiting for its trapezoid
-// length (pq[ig]) and, in CGA, the running compensated sums (cg[6 ig + j]).
+// nqk = ng + nw) and the mixing ratios of the point waiting for its trapezoid
+// length (pq[ig]).
 __host__ __device__ inline int trace_smem_floats(const CtlDev& c) {
-  return 2 * (c.ng + c.nw) + c.ng + (c.formod == 0 ? 6 * c.ng : 0);
+  return 2 * (c.ng + c.nw) + c.ng;
 }
 
 // a < b on the integer pipe, false for NaN
@@ -282,11 +282,11 @@ __device__ void ray_first_m(const double* g, long long nray, int r, double zmax,
 }
 
 // STORE places every point with its final values: its trapezoid length
-// 0.5 (ds_(i-1) + ds_i), column densities 10 / k_B q p / T ds and CGA sums
-// are written when the next point is placed (the clip of the last segment
-// changes the previous point's raw length), so the walk keeps the raw
-// lengths of the last two points.
-// With wf it walks on from the state wf (a base ray's walk).
+// 0.5 (ds_(i-1) + ds_i) and column densities 10 / k_B q p / T ds are written
+// when the next point is placed (the clip of the last segment changes the
+// previous point's raw length), so the walk keeps the raw lengths of the last
+// two points.  It serves resumed perturbations, which are EGA only (no
+// Curtis-Godson sums).  With wf it walks on from the state wf (a base's walk).
 template <bool STORE>
 __device__ int walk_m(const CtlDev& c, const AtmM& a, const double* g, long long nray, int r,
                       const LosDev& L, long long base, int cap, double* sft_out, GeoKeep* gk,
@@ -325,12 +325,9 @@ __device__ int walk_m(const CtlDev& c, const AtmM& a, const double* g, long long
   // the point waiting for its final values (STORE): raw lengths of it and
   // of the point before, its p and T; its mixing ratios in pq
   float* pq = STORE ? qc + 2 * nqk * kTraceThreads : nullptr;
-  float* cg = STORE ? pq + c.ng * kTraceThreads : nullptr;
   float raw_before = 0.f, raw_pend = 0.f, pend_p = 0.f, pend_t = 0.f;
   const int n0 = n;
   if (STORE && wf) raw_pend = wf->raw_last;
-  if (STORE && L.cga)
-    for (int k = 0; k < 6 * c.ng; k++) cg[k * kTraceThreads] = 0.f;
   auto finalize = [&](int k) {
     const long long sk = base + k;
     const float dsT = k == 0 ? 0.5f * raw_pend : 0.5f * (raw_before + raw_pend);
@@ -338,31 +335,6 @@ __device__ int walk_m(const CtlDev& c, const AtmM& a, const double* g, long long
     for (int ig = 0; ig < c.ng; ig++) {
       const float uu = col_density(pq[ig * kTraceThreads], pend_p, pend_t, dsT);
       L.f.u[ig * L.cap + sk] = uu;
-      if (L.cga) {  // compensated running sums
-        float* q = cg + 6 * ig * kTraceThreads;
-        float su = q[0], sp = q[kTraceThreads], st = q[2 * kTraceThreads];
-        float cu = q[3 * kTraceThreads], cp = q[4 * kTraceThreads], ct = q[5 * kTraceThreads];
-        float y = uu - cu, s2 = su + y;
-        cu = (s2 - su) - y;
-        su = s2;
-        y = uu * pend_p - cp;
-        s2 = sp + y;
-        cp = (s2 - sp) - y;
-        sp = s2;
-        y = uu * pend_t - ct;
-        s2 = st + y;
-        ct = (s2 - st) - y;
-        st = s2;
-        q[0] = su;
-        q[kTraceThreads] = sp;
-        q[2 * kTraceThreads] = st;
-        q[3 * kTraceThreads] = cu;
-        q[4 * kTraceThreads] = cp;
-        q[5 * kTraceThreads] = ct;
-        L.f.cgu[ig * L.cap + sk] = su;
-        L.f.cgp[ig * L.cap + sk] = sp / su;
-        L.f.cgt[ig * L.cap + sk] = st / su;
-      }
     }
   };
   for (;;) {

@@ -93,6 +93,24 @@ void ctm_coefficients(double nu, double* out) {
 }  // namespace
 
 
+namespace jgb {
+// Gives the path's workspaces back (nothing in them outlives a call; fields:
+// also tiles_data, while it holds nothing).
+static void release_path(jgb_ctx* x, bool fields) {
+  x->seg.release();
+  x->rs_seg.release();
+  x->rs_snap.release();
+  if (fields) x->tiles_data.release();
+}
+
+cudaError_t reserve_first(jgb_ctx* x, DevBuf& buf, size_t bytes, bool fields) {
+  cudaError_t e = buf.reserve(bytes);
+  if (e != cudaErrorMemoryAllocation) return e;
+  release_path(x, fields);
+  return buf.reserve(bytes);
+}
+}  // namespace jgb
+
 namespace {
 
 int fail(jgb_ctx* x, int code, const std::string& msg) {
@@ -437,15 +455,6 @@ int plan_tiles(jgb_ctx* x, int nray, const int* keys, const int* count, int ntil
 // channels where one tile alone would exceed it.  The results do not depend on
 // the chunks.
 
-// Gives the path's workspaces back (nothing in them outlives a call; fields:
-// also tiles_data, while it holds nothing).
-void release_path(jgb_ctx* x, bool fields) {
-  x->seg.release();
-  x->rs_seg.release();
-  x->rs_snap.release();
-  if (fields) x->tiles_data.release();
-}
-
 // Reserves a chunk plan's workspaces, reserve(limit): where the device has no room
 // for them, from empty workspaces, then with a quarter of the limit, down to 64 MiB
 // (or the caller's own limit).  What fitted stays the context's limit.
@@ -461,14 +470,6 @@ int reserve_path(jgb_ctx* x, bool fields, F reserve) {
     release_path(x, fields);
     if (empty) x->path_limit = std::max(x->path_limit / 4, kMinPathBytes);
   }
-}
-
-// Any other buffer of the call: the path's workspaces make room for it.
-cudaError_t reserve_first(jgb_ctx* x, DevBuf& buf, size_t bytes, bool fields) {
-  cudaError_t e = buf.reserve(bytes);
-  if (e != cudaErrorMemoryAllocation) return e;
-  release_path(x, fields);
-  return buf.reserve(bytes);
 }
 
 struct PathChunk {
@@ -1493,17 +1494,17 @@ int fd_core(jgb_ctx* x, const FdLayout& H, const FdInput& in, const std::vector<
     }
     const int ne = (int)esrc.size();
     const long long nlev_e = eoff_l.back(), nray_e = eoff_r.back();
-    CK(x->kx_levoff.reserve(sizeof(int) * (ne + 1)));
-    CK(x->kx_rayoff.reserve(sizeof(int) * (ne + 1)));
-    CK(x->kx_src.reserve(sizeof(int) * ne));
-    CK(x->kx_pert.reserve(sizeof(int4) * ne));
-    CK(x->kx_h.reserve(sizeof(double) * ne));
-    CK(x->kx_lev.reserve(sizeof(double) * (size_t)nlev_e * nplanes));
-    CK(x->kx_scal.reserve(sizeof(double) * (size_t)ne * nscal));
-    CK(x->kx_geo.reserve(sizeof(double) * 7 * (size_t)nray_e));
-    CK(x->kx_tp.reserve(sizeof(double) * ((size_t)c.nd * 2 + 3) * (size_t)nray_e));
-    CK(x->kx_mask.reserve((size_t)c.nd * nray_e));
-    CK(x->kx_rayobs.reserve(sizeof(int) * nray_e));
+    CK(reserve_first(x, x->kx_levoff, sizeof(int) * (ne + 1), true));
+    CK(reserve_first(x, x->kx_rayoff, sizeof(int) * (ne + 1), true));
+    CK(reserve_first(x, x->kx_src, sizeof(int) * ne, true));
+    CK(reserve_first(x, x->kx_pert, sizeof(int4) * ne, true));
+    CK(reserve_first(x, x->kx_h, sizeof(double) * ne, true));
+    CK(reserve_first(x, x->kx_lev, sizeof(double) * (size_t)nlev_e * nplanes, true));
+    CK(reserve_first(x, x->kx_scal, sizeof(double) * (size_t)ne * nscal, true));
+    CK(reserve_first(x, x->kx_geo, sizeof(double) * 7 * (size_t)nray_e, true));
+    CK(reserve_first(x, x->kx_tp, sizeof(double) * ((size_t)c.nd * 2 + 3) * (size_t)nray_e, true));
+    CK(reserve_first(x, x->kx_mask, (size_t)c.nd * nray_e, true));
+    CK(reserve_first(x, x->kx_rayobs, sizeof(int) * nray_e, true));
     CK(cudaMemcpyAsync(x->kx_levoff.p, eoff_l.data(), sizeof(int) * (ne + 1), cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(x->kx_rayoff.p, eoff_r.data(), sizeof(int) * (ne + 1), cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(x->kx_src.p, esrc.data(), sizeof(int) * ne, cudaMemcpyHostToDevice, s));
@@ -1591,7 +1592,7 @@ int fd_core(jgb_ctx* x, const FdLayout& H, const FdInput& in, const std::vector<
     const size_t o_mc = carve(sizeof(int) * nob), o_nc = carve(sizeof(int) * nob);
     const size_t o_yo = carve(sizeof(int) * nob), o_e0 = carve(sizeof(int) * nob);
     const size_t o_br = carve(sizeof(int) * nob), o_ym = carve(sizeof(int2) * H.ymap.size());
-    CK(x->kx_ymap.reserve(off + 16));
+    CK(reserve_first(x, x->kx_ymap, off + 16, true));
     char* qp = x->kx_ymap.as<char>();
     long long* d_kb = reinterpret_cast<long long*>(qp + o_kb);
     long long* d_kd = reinterpret_cast<long long*>(qp + o_kd);
@@ -2019,16 +2020,16 @@ int jgb_formod_batch(jgb_ctx* x, const jgb_batch* hb, int precision) {
       ob[1] = o1;
     }
   }
-  CK(x->b_levoff.reserve(sizeof(int) * (nobs + 2)));
-  CK(x->b_rayoff.reserve(sizeof(int) * (nobs + 2)));
-  CK(x->b_rayobs.reserve(sizeof(int) * nray));
-  CK(x->b_lev.reserve(sizeof(double) * (size_t)nlev * nlevf));
-  CK(x->b_scal.reserve(sizeof(double) * (size_t)nobs * nscal));
-  CK(x->b_geo.reserve(sizeof(double) * 7 * (size_t)nray));
-  CK(x->b_rad.reserve(sizeof(double) * (size_t)c.nd * nray));
-  CK(x->b_tau.reserve(sizeof(double) * (size_t)c.nd * nray));
-  CK(x->b_tp.reserve(sizeof(double) * 3 * (size_t)nray));
-  CK(x->b_mask.reserve((size_t)c.nd * nray));
+  CK(reserve_first(x, x->b_levoff, sizeof(int) * (nobs + 2), true));
+  CK(reserve_first(x, x->b_rayoff, sizeof(int) * (nobs + 2), true));
+  CK(reserve_first(x, x->b_rayobs, sizeof(int) * nray, true));
+  CK(reserve_first(x, x->b_lev, sizeof(double) * (size_t)nlev * nlevf, true));
+  CK(reserve_first(x, x->b_scal, sizeof(double) * (size_t)nobs * nscal, true));
+  CK(reserve_first(x, x->b_geo, sizeof(double) * 7 * (size_t)nray, true));
+  CK(reserve_first(x, x->b_rad, sizeof(double) * (size_t)c.nd * nray, true));
+  CK(reserve_first(x, x->b_tau, sizeof(double) * (size_t)c.nd * nray, true));
+  CK(reserve_first(x, x->b_tp, sizeof(double) * 3 * (size_t)nray, true));
+  CK(reserve_first(x, x->b_mask, (size_t)c.nd * nray, true));
   struct Chunk {
     int o0, o1, l0, l1, r0, r1;
     BatchDev b;
@@ -2196,8 +2197,8 @@ int jgb_formod_batch_dev(jgb_ctx* x, const jgb_batch* db, int precision) {
   CK(cudaMemcpy(&nlev, db->lev_off + nobs, sizeof(int), cudaMemcpyDeviceToHost));
   CK(cudaMemcpy(&nray, db->ray_off + nobs, sizeof(int), cudaMemcpyDeviceToHost));
   if (nlev <= 0 || nray <= 0) return fail(x, JGB_ERR_ARG, "no levels or rays");
-  CK(x->b_rayobs.reserve(sizeof(int) * nray));
-  CK(x->b_mask.reserve((size_t)c.nd * nray));
+  CK(reserve_first(x, x->b_rayobs, sizeof(int) * nray, true));
+  CK(reserve_first(x, x->b_mask, (size_t)c.nd * nray, true));
   BatchDev b{};
   b.nobs = nobs;
   b.nlev = nlev;

@@ -179,6 +179,10 @@ int normal_equations_dev(int nret, const int* m, const int* n, const double* K, 
 size_t normal_desc_bytes(int nret);
 int ctx_fail(jgb_ctx* x, int code, const char* msg);
 
+// jgb_api.cu: reserves a buffer for which the path's workspaces of the context make
+// room (fields: also tiles_data, while it holds nothing).
+cudaError_t reserve_first(jgb_ctx* x, DevBuf& buf, size_t bytes, bool fields);
+
 // The context's (recursive) lock for the duration of a public call: host
 // threads may share a context, and their calls run one after another.
 void ctx_lock(jgb_ctx* x);

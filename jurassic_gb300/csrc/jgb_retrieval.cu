@@ -897,7 +897,7 @@ int build_workset(jgb_engine* E, WorkSet& w, WorkSet* old, const std::vector<Req
     std::copy(q->sael.begin(), q->sael.end(), sael.begin() + w.desc[i].xo);
   }
   const size_t bytes = workset_bytes(c, nret, w.nlev, w.nray, nx, w.ny, nss, w.nk, err_ana);
-  ECK(w.mem.reserve(bytes));
+  ECK(reserve_first(E->x, w.mem, bytes, true));
   char* mp = w.mem.as<char>();
   auto take = [&](size_t nbytes) {
     char* p = mp;
@@ -1872,7 +1872,7 @@ extern "C" int jgb_matrix_invert_dev(jgb_ctx* x, int nret, const int* n, double*
   // the factors and their inverses
   const size_t b_desc = (sizeof(InvertDesc) * (size_t)nret + 255) & ~size_t(255);
   const size_t b_flags = (sizeof(int) * 2 * (size_t)nret + 255) & ~size_t(255);
-  if (x->inv_work.reserve(b_desc + b_flags + sizeof(double) * 2 * (size_t)so) != cudaSuccess)
+  if (reserve_first(x, x->inv_work, b_desc + b_flags + sizeof(double) * 2 * (size_t)so, true) != cudaSuccess)
     return ctx_error(x, JGB_ERR_CUDA, "cudaMalloc failed");
   char* p = x->inv_work.as<char>();
   InvertDesc* d = reinterpret_cast<InvertDesc*>(p);
@@ -1914,7 +1914,7 @@ extern "C" int jgb_matrix_invert(jgb_ctx* x, int nret, const int* n, double* A, 
   if (rc != JGB_OK && rc != JGB_ERR_STATE) return rc;
   cudaSetDevice(v.device);
   jgb::DevBuf dA;
-  if (dA.reserve(sizeof(double) * (size_t)so) != cudaSuccess)
+  if (reserve_first(x, dA, sizeof(double) * (size_t)so, true) != cudaSuccess)
     return ctx_error(x, JGB_ERR_CUDA, "cudaMalloc failed");
   if (cudaMemcpyAsync(dA.p, A, sizeof(double) * so, cudaMemcpyHostToDevice, v.stream) != cudaSuccess)
     return ctx_error(x, JGB_ERR_CUDA, "copy to the device failed");

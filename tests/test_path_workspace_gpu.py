@@ -101,14 +101,22 @@ def test_no_room_on_the_device(built_lib):
     held = ctx.path_workspace()[1]
     ctx.set_path_workspace(0)
     assert held > 2500 * MIB and ctx.path_workspace()[1] == 0
+    z = np.linspace(0, 60, 1000)
+    spd = np.exp(-np.abs(z[:, None] - z[None, :]) / 3.0)
     block = L.jgb_dev_alloc(_free_bytes() - 700 * MIB)
     assert block
     try:
         out = [ctx.formod_batch(w.batch.fresh_outputs(), p) for p in (native.FP64, native.MIXED, native.FP64)]
-        limit = ctx.path_workspace()[0]
+        limit, held = ctx.path_workspace()
+        # inverses of 20 matrices of 1000 x 1000: 160 MB and 320 MB of scratch, for
+        # which the workspaces make room
+        inv, st = ctx.matrix_invert([spd] * 20)
+        after = ctx.path_workspace()[1]
     finally:
         L.jgb_dev_free(ctypes.c_void_p(block))
     ctx.close()
     for a, b in zip(out, ref + ref[:1]):
         assert np.array_equal(a.rad, b.rad) and np.array_equal(a.tau, b.tau)
     assert 64 * MIB <= limit <= 512 * MIB
+    assert held > 200 * MIB and after < held and not np.any(st)
+    assert np.max(np.abs(inv[-1] @ spd - np.eye(1000))) < 1e-9

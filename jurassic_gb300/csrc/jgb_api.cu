@@ -596,7 +596,11 @@ int run_path64(jgb_ctx* x, const BatchDev& b, const LosDev& L, cudaStream_t s, i
       P.om = x->seg.as<double>();
       P.se = P.om + np * ndc * c.ng * 32;
       P.stop = reinterpret_cast<int*>(P.se + np * ndc * 2 * 32);
-      // four lanes per ray while the warps of one per ray leave schedulers idle
+      // four lanes per ray while the warps of one per ray leave schedulers idle; the
+      // line is on the safe side.  One lane and four, ms (20 channels, 3 emitters):
+      // nadir 0.4 warps per SM 5.42 and 2.26, 1.6 5.83 and 2.94, 5.1 7.33 and 6.61,
+      // 6.3 7.67 and 10.42; limb (CGA) 0.4 2.77 and 1.08, 5.1 3.19 and 2.30, 9.9 3.69
+      // and 3.66
       const long long warps = (long long)(k.t1 - k.t0) * ndc * c.ng;
       launch_path64(c, T, ch, b, L, P, std::max(k.longest, 1), warps <= 2LL * x->sms ? 4 : 1, s);
       CK(cudaGetLastError());
@@ -903,7 +907,10 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
       // the plain batch, whose tiles hold one observation's nearly equal rays
       // (0.47 against 0.29 ns per warp and point).  The bases come first and
       // take 0.7 of a plain tile's time, 4 lanes per ray and nothing else to
-      // run beside them.
+      // run beside them.  Fitted on nadir batches of 405 elements (1, 2, 4, 8 and 16
+      // observations of 20 to 150 channels) and a limb batch: estimated ratios 1.33,
+      // 0.72, 0.59, 1.27, 0.46, 0.71, measured 1.02, 0.90, 0.78, 1.05, 0.60, 0.88; so
+      // the line at 0.9 errs towards the plain plan.
       const double conc = std::max(1.0, (double)x->sms * 40.0 / ((double)c.nd * std::max(c.ng, 1)));
       std::vector<int> ord(nray);
       for (int r = 0; r < nray; r++) ord[r] = r;
@@ -1198,7 +1205,11 @@ int jgb::run_core(jgb_ctx* x, BatchDev& b, int precision, bool timed_h2d) {
             if (rc) return rc;
             variant = x->path_variant;
           }
-          // few tiles: no consecutive ones to share rows between
+          // few tiles: hardly any consecutive ones to share rows between.  Channels
+          // of a tile side by side and tiles of a channel, ms: 2 nadir tiles 6.63 and
+          // 7.05, 4 7.02 and 6.83, 7 7.60 and 7.39; limb (CGA) 2.49 and 2.64, 2.11 and
+          // 2.22, 1.98 and 1.96: within 6 % either way up to the line, 3 to 4 % for
+          // tiles of a channel beyond it (24 tiles 10.10 and 9.68)
           if (variant < 0) variant = 6;
           if (k.t1 - k.t0 < 8) variant %= 4;
           if (!timed) CK(cudaEventRecord(x->ev[4], s));

@@ -16,7 +16,7 @@
 // instructions per multiply-add, 1.7 n^3 in all, with a block-wide barrier
 // twice per column; tiles spread every matrix over the device, a thread keeps
 // 4 x 4 sums in registers, and 32 x 32 tiles waste little on the diagonals.
-// 96 matrices of up to 405 x 405 (48 of them smaller): 44.6 -> 7.8 ms, of
+// 96 matrices of up to 405 x 405 (48 of them smaller): 44.6 -> 7.9 ms, of
 // which k_tri_inverse 2.8 (its longest column is 1.5), k_gram 1.8,
 // k_chol_update 1.5, k_chol_diag 1.1 (13 panels, a warp's chain of roots),
 // k_chol_panel 0.7; the multiply-adds alone are 4.1 ms.
@@ -24,8 +24,8 @@
 // Rounding: sums are formed apart and subtracted once, a tile's products apart
 // from the sum over the tiles, quotients are correctly rounded.  Error against
 // inverses refined in long double, over the error of a block per matrix that
-// subtracted whole sums (geometric means, n from 12 to 405): covariances 1.06,
-// Gauss-Newton matrices 0.76 (with the small matrices' solves 1.02 and 0.74).
+// subtracted whole sums (geometric means, n from 12 to 405): covariances 1.02,
+// Gauss-Newton matrices 0.74.
 #include <algorithm>
 
 #include "../../include/jurassic_gb300.h"

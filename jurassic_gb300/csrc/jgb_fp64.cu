@@ -1069,7 +1069,9 @@ __global__ void k_hydro_chain(CtlDev c, BatchDev b, double* p_out) {
 // Eight lanes per ray up to here: a step is about 100 FP64 instructions of a
 // warp (4 rays) against 330 (32 rays), 64 cycles each until about three warps
 // share an SM, 19 of the SM's then, so the two forms meet between 6000 and
-// 7000 rays on 152 SMs.
+// 7000 rays on 152 SMs.  Eight lanes and one, ms: nadir 500 rays 4.06 and 9.57, 5000
+// 8.25 and 9.91, 6144 9.65 and 9.99, 7000 10.53 and 10.01, 12000 20.7 and 10.2; limb
+// 6144 3.90 and 5.13, 8192 4.87 and 5.22, 12000 6.18 and 5.40.
 constexpr int kWalk8MaxRays = 6144;
 
 size_t level_slope_bytes(const CtlDev& c, long long nlev) {

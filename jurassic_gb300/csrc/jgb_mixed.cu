@@ -1273,6 +1273,8 @@ void launch_pack_tiles_n(const CtlDev& c, const TblDev& T, const LosDev& L, cons
   k_pack_tiles<<<(unsigned)((nth + bs - 1) / bs), bs, 0, s>>>(c, T, L, P, total_tile_points);
 }
 
+// The resumed kernels take at most 64 registers (16 observations x 405 elements, emitters'
+// kernel: 24.6 ms; 48, 40 and 32 registers 24.8, 25.1 and 26.6).
 // Variants of k_gas_m with one lane per ray, chosen by the autotuner: block
 // shape (v / 4) and minimum resident blocks per SM (v % 4: 8, 10, 12, 16, i.e.
 // at most 64, 48, 40 and 32 registers).

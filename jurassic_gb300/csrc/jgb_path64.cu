@@ -242,11 +242,14 @@ __device__ __forceinline__ bool above_f(double x, float d, float g) {
   return d > g;
 }
 
-// e < 1 ? e : 1, then e > 0 ? e : 0 (NaN gives 1), without FP64 compares
+// e clamped to [0, 1] without FP64 compares.  What is not a number gives 0, as in
+// k_path_fp64 and the mixed path: an emitter without a column has no Curtis-Godson
+// pressure (0 / 0), and adds nothing.
 __device__ __forceinline__ double clamp01(double e) {
   const unsigned hi = (unsigned)__double2hiint(e);
   if (hi < 0x3ff00000u) return e;
-  return (long long)__double_as_longlong(e) < 0 && hi <= 0xfff00000u ? 0.0 : 1.0;
+  const bool number = hi < 0x7ff00000u || (hi == 0x7ff00000u && __double2loint(e) == 0);
+  return number ? 1.0 : 0.0;  // negative numbers are above 0x7ff00000 as well
 }
 
 // a < b for doubles that are not negative (and not NaN), on the integer pipe

@@ -417,13 +417,14 @@ __global__ void __launch_bounds__(kNeThreads, 2) k_normal_tc(const NeDesc* desc,
         epi_sync();
         // direct entries, rows >= columns (and b, the augmented row n): lanes
         // along the row, so that a store covers whole sectors
-        for (int rr = ew; rr < kTile; rr += kEpiThreads / 32) {
+        const int col0 = tj * kTile + h * kEpiCols;
+        const int rows = col0 < d.n ? min(kTile, d.n + 1 - ti * kTile) : 0;
+        for (int rr = ew; rr < rows; rr += kEpiThreads / 32) {
           const int row2 = ti * kTile + rr;
-          if (row2 > d.n) break;
           double* dst = row2 == d.n ? bv : A + (long long)row2 * d.n;
 #pragma unroll
           for (int k = 0; k < kEpiCols; k += 32) {
-            const int col = tj * kTile + h * kEpiCols + k + lane;
+            const int col = col0 + k + lane;
             if (col < d.n && col <= row2) dst[col] = f2d_bits(stile[rr * kEpiPad + k + lane]);
           }
         }
